@@ -1,4 +1,5 @@
-"""Builds libfa_sm100.so in-tree with nvcc for sm_100a.
+"""Builds libfa_sm100.so (kernels and C ABI, nvcc for sm_100a) and _fa_torch.so (the PyTorch
+launch path on top of it, host compiler) in-tree.
 
 Run as ``python -m triton_flashattn_b200.build`` (add ``--force`` to rebuild
 everything, ``--verbose`` for ptxas register/shared-memory statistics).  Objects
@@ -11,12 +12,15 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 BUILD_DIR = os.path.join(PKG_DIR, "build")
 LIB_PATH = os.path.join(PKG_DIR, "libfa_sm100.so")
+BINDING_SRC = os.path.join(CSRC, "torch_binding.cpp")
+BINDING_PATH = os.path.join(PKG_DIR, "_fa_torch.so")
 INCLUDE_DIR = os.path.join(os.path.dirname(PKG_DIR), "include")
 
 SOURCES = [
@@ -52,7 +56,7 @@ def _stale(target: str, deps: list[str]) -> bool:
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile every translation unit and link the shared library; returns its path."""
+    """Compile every translation unit and link the two shared libraries; returns the kernels' path."""
     os.makedirs(BUILD_DIR, exist_ok=True)
     nvcc = _nvcc()
     headers = _headers()
@@ -91,7 +95,33 @@ def build(force: bool = False, verbose: bool = False) -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    build_binding(force)
     return LIB_PATH
+
+
+def build_binding(force: bool = False) -> str:
+    """Compile the PyTorch launch path against the installed torch and link it to libfa_sm100.so
+    (found beside it at run time); returns its path."""
+    import torch
+
+    deps = [BINDING_SRC] + [h for h in _headers() if h.endswith(".h")]
+    if not force and not _stale(BINDING_PATH, deps):
+        return BINDING_PATH
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    cmd = [
+        shutil.which("g++") or "c++", "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden",
+        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+        "-I", os.path.join(root, "include"), "-I", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+        "-I", sysconfig.get_path("include"), "-I", os.path.join(cuda, "include"), "-I", INCLUDE_DIR,
+        BINDING_SRC, "-o", BINDING_PATH,
+        "-L", PKG_DIR, "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN",
+        "-L", os.path.join(root, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
+    ]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for {BINDING_SRC}:\n{r.stdout}\n{r.stderr}")
+    return BINDING_PATH
 
 
 def main() -> None:
