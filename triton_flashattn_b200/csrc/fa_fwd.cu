@@ -506,8 +506,6 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
                     s[i + 3] = f2_hi(x1);
                   }
                   b_phase ^= 1u << bs;
-                  __syncwarp();
-                  if (lane == 0) mbar_arrive(&bias_empty[bs]);
                 }
                 if (!ok) break;
               } else if (BIAS == 1) {
@@ -542,11 +540,6 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
                   }
                 }
               }
-              if (BIAS == 1 || (BIAS == 2 && h == 1)) {
-                b_phase ^= 1u << bs;
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bias_empty[bs]);
-              }
             }
             // ---- bounds and causal masks (only on halves that need them)
             if ((n0 + 64 > p.N) || (p.causal && n0 + 63 > m0)) {
@@ -570,7 +563,18 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
             mx1 = max3(mx1, s[62], s[63]);
             const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * mul;  // log2 domain
             const bool need = mx > m_used + 8.0f;
-            if (__any_sync(0xffffffffu, need)) {
+            const bool any_need = __any_sync(0xffffffffu, need);
+            // The bias units go back to their producer only after the vote, which needs the maximum of
+            // every lane and so every value read from them.  (Right after the reads is too early: the
+            // arrival may then take effect while reads of the warp are still under way, and the next
+            // bulk load overwrote rows before they were read about once in ten full-size passes.)
+            if (BIAS == 1 || (BIAS == 2 && h == 1)) {
+              b_phase ^= 1u << bs;
+              if (lane == 0) mbar_arrive(&bias_empty[bs]);
+            } else if (BIAS == 3 && lane < 2) {
+              mbar_arrive(&bias_empty[(unit + lane) % NB]);
+            }
+            if (any_need) {
               const float m_new = need ? mx : m_used;
               const float alpha = need ? ex2(m_used - m_new) : 1.0f;
               l *= alpha;
