@@ -138,6 +138,20 @@ int fa_fwd(const fa_params* p, void* stream);
 int fa_bwd(const fa_params* p, void* stream);
 
 /*
+ * Backward with scratch: the same results as fa_bwd, faster wherever dS has no tensor of its own
+ * (no bias, a mask, a bias without gradient, an fp32 bias, D = 256).  The dK/dV stage leaves
+ * dS in `workspace` as 16-bit values and the dQ stage is one streamed product over it, where
+ * fa_bwd computes the scores a second time; `ds16` is not needed then.  The (batch, head)
+ * problems are worked through in parts that fit the workspace.
+ *   workspace: 16-byte aligned device memory, contents unspecified before and after;
+ *   bytes: any size; fa_bwd_workspace_bytes(p) is what the call works best with (0: it has no
+ *     use for one).  Less than the dS of one problem (M rows of N 16-bit values, rows padded
+ *     to 16 bytes), or a null workspace: the call is fa_bwd.
+ */
+uint64_t fa_bwd_workspace_bytes(const fa_params* p);
+int fa_bwd_workspace(const fa_params* p, void* workspace, uint64_t bytes, void* stream);
+
+/*
  * Backward for callers that cannot allocate device memory (a plugin living inside a
  * host runtime with a frozen memory plan, a real-time loop, a foreign-language
  * binding without an allocator).  Same as fa_bwd, except that `p->delta` is ignored:

@@ -68,6 +68,8 @@ EXPORTED_SYMBOLS = (
     "fa_status_string",
     "fa_fwd",
     "fa_bwd",
+    "fa_bwd_workspace",
+    "fa_bwd_workspace_bytes",
     "fa_bwd_static_scratch",
     "fa_bwd_pre",
     "fa_bwd_dkdv",
@@ -107,6 +109,10 @@ def load() -> ctypes.CDLL:
         fn = getattr(lib, name)
         fn.restype = ctypes.c_int
         fn.argtypes = [P, ctypes.c_void_p]
+    lib.fa_bwd_workspace_bytes.restype = ctypes.c_uint64
+    lib.fa_bwd_workspace_bytes.argtypes = [P]
+    lib.fa_bwd_workspace.restype = ctypes.c_int
+    lib.fa_bwd_workspace.argtypes = [P, ctypes.c_void_p, ctypes.c_uint64, ctypes.c_void_p]
     lib.fa_last_device_status.restype = ctypes.c_int
     lib.fa_last_device_status.argtypes = [ctypes.c_int, ctypes.POINTER(ctypes.c_int32)]
     lib.fa_reset_device_status.restype = ctypes.c_int

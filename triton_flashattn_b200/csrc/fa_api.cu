@@ -149,7 +149,8 @@ int validate_common(const fa_params* p) {
   return FA_OK;
 }
 
-int validate_bwd(const fa_params* p) {
+// `workspace`: dS may go to scratch slabs, so the call needs no ds16 tensor
+int validate_bwd(const fa_params* p, bool workspace = false) {
   int r = validate_common(p);
   if (r) return r;
   if (!p->d_o || !p->dq || !p->dk || !p->dv || !p->delta) return FA_ERR_NULL;
@@ -157,9 +158,68 @@ int validate_bwd(const fa_params* p) {
     if (p->bias_kind != FA_BIAS_SAME && p->bias_kind != FA_BIAS_F32) return FA_ERR_DTYPE;
     if (!p->dbias) return FA_ERR_NULL;
   }
+  if (workspace) return FA_OK;
   if (p->bias_kind == FA_BIAS_F32 && !p->ds16) return FA_ERR_NULL;
   // head dim 256: dQ is always the streamed product over the 16-bit dS
   if (p->D == 256 && !(p->write_dbias && p->bias_kind == FA_BIAS_SAME) && !p->ds16) return FA_ERR_NULL;
+  return FA_OK;
+}
+
+// ---- backward through dS slabs ------------------------------------------------------------
+// Whether dS already has a place of its own: the gradient of a 16-bit bias is dS.
+bool ds_is_dbias(const fa_params& p) { return p.write_dbias && p.bias_kind == FA_BIAS_SAME; }
+
+int64_t slab_pitch(const fa_params& p) { return ((int64_t)p.N + 7) / 8 * 8; }
+uint64_t slab_bytes(const fa_params& p) { return (uint64_t)slab_pitch(p) * p.M * 2; }
+
+// Problems per part of the backward, at most `most`: the number that makes the persistent dK/dV
+// grids of all parts together need the fewest turns of one work unit per SM, where every part
+// costs about a third of a turn more for its two launches and its drained tail.
+int problems_per_part(const fa_params& p, int most) {
+  const int total = p.B * p.H;
+  if (most >= total) return total;
+  const int keys = p.D == 256 ? 64 : 128;
+  const int tiles = (p.N + keys - 1) / keys;
+  const bool pairs = p.causal && p.D != 256;  // a causal unit is a heavy and a light tile
+  const int sms = persistent_grid(1 << 30);
+  auto turns = [&](int n) {
+    const int64_t units = pairs ? ((int64_t)n * tiles + 1) / 2 : (int64_t)n * tiles;
+    return (units + sms - 1) / sms;
+  };
+  int best = most;
+  int64_t best_cost = -1;
+  for (int n = most; n >= 1 && n > most / 2; --n) {
+    const int parts = total / n, rest = total % n;
+    const int64_t cost = 3 * (parts * turns(n) + (rest ? turns(rest) : 0)) + parts + (rest ? 1 : 0);
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best = n;
+    }
+  }
+  return best;
+}
+
+// The scratch a backward works best with: room for the dS of all problems, or of as many as
+// kSlabCap holds.  Slabs of 1.5 GiB hold tens of long-sequence heads, enough work units to fill
+// the SMs several times, so more would not shorten the turns by more than a few per cent.
+constexpr uint64_t kSlabCap = 3ull << 29;
+
+uint64_t bwd_workspace_bytes(const fa_params& p) {
+  if (ds_is_dbias(p)) return 0;
+  const uint64_t one = slab_bytes(p);
+  const uint64_t fit = kSlabCap / one;
+  return one * (uint64_t)problems_per_part(p, fit < 1 ? 1 : (fit > 65535 ? 65535 : (int)fit));
+}
+
+int bwd_in_parts(const fa_params& p, void* ws, uint64_t bytes, cudaStream_t s, int* st) {
+  const uint64_t fit = bytes / slab_bytes(p);
+  const int total = p.B * p.H;
+  const int n = problems_per_part(p, fit > (uint64_t)total ? total : (int)fit);
+  for (int bh0 = 0; bh0 < total; bh0 += n) {
+    const DsSlab slab = {ws, slab_pitch(p), bh0, n < total - bh0 ? n : total - bh0};
+    if (int e = launch_bwd_dkdv(p, s, st, &slab)) return e;
+    if (int e = launch_bwd_dq(p, s, st, &slab)) return e;
+  }
   return FA_OK;
 }
 
@@ -240,6 +300,29 @@ int fa_bwd(const fa_params* p, void* stream) {
     e = launch_bwd_dkdv(*p, s, st);
     if (e) return e;
     return launch_bwd_dq(*p, s, st);
+  });
+}
+
+uint64_t fa_bwd_workspace_bytes(const fa_params* p) {
+  if (validate_common(p)) return 0;
+  uint64_t bytes = 0;
+  with_device(p->device, [&](int*) {
+    bytes = bwd_workspace_bytes(*p);
+    return (int)FA_OK;
+  });
+  return bytes;
+}
+
+int fa_bwd_workspace(const fa_params* p, void* workspace, uint64_t bytes, void* stream) {
+  const bool slabs = p && workspace && !validate_common(p) && !ds_is_dbias(*p) && bytes >= slab_bytes(*p);
+  int r = validate_bwd(p, slabs);
+  if (r) return r;
+  if (!slabs) return fa_bwd(p, stream);
+  if (reinterpret_cast<uintptr_t>(workspace) % 16 != 0) return FA_ERR_ALIGN;
+  return with_device(p->device, [&](int* st) {
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (int e = launch_bwd_pre(*p, s, st)) return e;
+    return bwd_in_parts(*p, workspace, bytes, s, st);
   });
 }
 

@@ -60,7 +60,9 @@ struct DkdvParams {
   int64_t bias_sB, bias_sH, bias_sM;
   int64_t dk_sB, dk_sN, dk_sH, dv_sB, dv_sN, dv_sH;
   int H, M, N, D;
-  int n_nblk, n_tiles;  // key blocks per (batch, head); tiles = n_nblk * B * H
+  int n_nblk, n_tiles;  // key blocks per (batch, head); tiles of this launch
+  int bh0;              // first (batch, head) of this launch
+  int ds_flat;          // dS goes to slabs numbered from bh0 instead of a (B, H, M, N) tensor
   int causal, bias_vec32, bias_b_mul, bias_h_mul;
   int dkv_vec32;  // dk / dv bases and strides are multiples of 32 bytes
   int store_ds;    // the 16-bit dS tiles go out through map_dbias (as dbias, or as scratch for dQ)
@@ -130,6 +132,7 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
     if (k >= p.n_tiles) return false;
     bh = k / p.n_nblk;
     const int pos = k - bh * p.n_nblk;
+    bh += p.bh0;
     nb = p.causal ? ((pos & 1) ? p.n_nblk - 1 - (pos >> 1) : (pos >> 1)) : pos;
     i_start = p.causal ? min(nb, n_mblk) : 0;
     T_steps = n_mblk - i_start;
@@ -343,6 +346,7 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
       int bh, nb, i_start, T_steps;
       for (int it = 0; ok && tile_at(it, bh, nb, i_start, T_steps); ++it) {
         const int b = bh / p.H, h = bh - b * p.H, n0 = nb * 128;
+        const int ds_h = p.ds_flat ? bh - p.bh0 : h, ds_b = p.ds_flat ? 0 : b;
         if (p.zero_tiles) {
           ok = wait_warp(&zero_ready, it & 1, ctx, kSiteZeroReady, it);
           if (!ok) break;
@@ -398,8 +402,8 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
             mma_commit(&dk_done);
             if (stores_here) {
               const int m0 = (i_start + t) * 128;
-              tma_store_4d(&p.map_dbias, smem + L::kDs, n0, m0, h, b);
-              if (n0 + 64 < p.N) tma_store_4d(&p.map_dbias, smem + L::kDs + kBlk, n0 + 64, m0, h, b);
+              tma_store_4d(&p.map_dbias, smem + L::kDs, n0, m0, ds_h, ds_b);
+              if (n0 + 64 < p.N) tma_store_4d(&p.map_dbias, smem + L::kDs + kBlk, n0 + 64, m0, ds_h, ds_b);
               tma_store_commit();
               tma_store_wait_read<0>();
               mbar_arrive(&st_done);
@@ -774,8 +778,8 @@ int launch_bias(const DkdvParams& kp, int bias_kind, dim3 grid, cudaStream_t str
 }  // namespace
 
 
-int launch_bwd_dkdv(const fa_params& p, cudaStream_t stream, int* status) {
-  if (p.D == 256) return launch_bwd_dkdv_d256(p, stream, status);
+int launch_bwd_dkdv(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab) {
+  if (p.D == 256) return launch_bwd_dkdv_d256(p, stream, status, slab);
   DkdvParams kp;
   int r = make_tmap_bshd(&kp.map_q, p.q, p.B, p.M, p.H, p.D, p.q_stride, 128);
   if (r) return r;
@@ -786,11 +790,16 @@ int launch_bwd_dkdv(const fa_params& p, cudaStream_t stream, int* status) {
   r = make_tmap_bshd(&kp.map_do, p.d_o, p.B, p.M, p.H, p.D, p.do_stride, 128);
   if (r) return r;
   const bool f32 = p.bias_kind == FA_BIAS_F32;
-  kp.store_ds = f32 ? 1 : (p.write_dbias ? 1 : 0);
+  kp.ds_flat = slab != nullptr;
+  kp.bh0 = slab ? slab->bh0 : 0;
+  kp.store_ds = slab || f32 || p.write_dbias;
   kp.zero_tiles = !f32 && p.write_dbias && p.causal;
   kp.dbias_f32 = nullptr;
   kp.dbf_sB = kp.dbf_sH = kp.dbf_sM = 0;
-  if (kp.store_ds) {
+  if (slab) {
+    r = make_tmap_slab(&kp.map_dbias, *slab, p.M, p.N);
+    if (r) return r;
+  } else if (kp.store_ds) {
     // the 16-bit dS tiles: the bias gradient itself, or (fp32 bias) the scratch the dQ stage reads
     const void* dst = f32 ? p.ds16 : p.dbias;
     const int64_t* dst_stride = f32 ? p.ds16_stride : p.dbias_stride;
@@ -869,7 +878,7 @@ int launch_bwd_dkdv(const fa_params& p, cudaStream_t stream, int* status) {
   kp.scale_log2 = p.sm_scale * kLog2e;
   kp.sm_scale = p.sm_scale;
   kp.n_nblk = (p.N + 127) / 128;
-  kp.n_tiles = kp.n_nblk * p.B * p.H;
+  kp.n_tiles = kp.n_nblk * (slab ? slab->n_bh : p.B * p.H);
   const int units = p.causal ? (kp.n_tiles + 1) / 2 : kp.n_tiles;
   const dim3 grid(persistent_grid(units));
   const int dp = padded_head_dim(p.D);

@@ -50,6 +50,8 @@ struct Dkdv256Params {
   int64_t dbf_sB, dbf_sH, dbf_sM;
   int64_t dk_sB, dk_sN, dk_sH, dv_sB, dv_sN, dv_sH;
   int H, M, N;
+  int bh0;      // first (batch, head) of this launch
+  int ds_flat;  // ds16 holds slabs numbered from bh0 (ds_sH apart) instead of a (B, H, M, N) tensor
   int causal, bias_vec32;
   float scale_log2;  // sm_scale * log2(e)
   float sm_scale;
@@ -83,7 +85,7 @@ __global__ void __launch_bounds__(192, 1) dkdv256_kernel(const __grid_constant__
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lane = tid & 31;
   const int n0 = static_cast<int>(blockIdx.x) * 64;
-  const int bh = blockIdx.y;
+  const int bh = p.bh0 + blockIdx.y;
   const int b = bh / p.H, h = bh - b * p.H;
   const int n_mblk = (p.M + 127) >> 7;
   // causal (top-left aligned): query block i sees key n0 when 128 i + 127 >= n0
@@ -196,6 +198,7 @@ __global__ void __launch_bounds__(192, 1) dkdv256_kernel(const __grid_constant__
     const uint32_t sp_row = smem_u32(smem + kOffP) + static_cast<uint32_t>(r) * 128u;
     const uint32_t sds_row = smem_u32(smem + kOffDs) + static_cast<uint32_t>(r) * 128u;
     const int64_t bias_bh = b * p.bias_sB + h * p.bias_sH;
+    const int64_t ds_bh = p.ds_flat ? (bh - p.bh0) * p.ds_sH : b * p.ds_sB + h * p.ds_sH;
     bool ok = live;
 #pragma unroll 1
     for (int s = 0; s < steps && ok; ++s) {
@@ -270,7 +273,7 @@ __global__ void __launch_bounds__(192, 1) dkdv256_kernel(const __grid_constant__
                  dsu[c * 4 + 2], dsu[c * 4 + 3]);
         if (row_ok && col0 < p.N) {
           // the 16-bit dS row segment: 64 contiguous bytes
-          T* drow = reinterpret_cast<T*>(p.ds16) + b * p.ds_sB + h * p.ds_sH + static_cast<int64_t>(m) * p.ds_sM + col0;
+          T* drow = reinterpret_cast<T*>(p.ds16) + ds_bh + static_cast<int64_t>(m) * p.ds_sM + col0;
           if (col0 + 32 <= p.N) {
 #pragma unroll
             for (int c = 0; c < 4; ++c)
@@ -381,7 +384,7 @@ const void* d256_ds_tensor(const fa_params& p, const int64_t** stride) {
   return p.ds16;
 }
 
-int launch_bwd_dkdv_d256(const fa_params& p, cudaStream_t stream, int* status) {
+int launch_bwd_dkdv_d256(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab) {
   Dkdv256Params kp;
   int r = make_tmap_bshd(&kp.map_q, p.q, p.B, p.M, p.H, p.D, p.q_stride, 128);
   if (r) return r;
@@ -391,8 +394,11 @@ int launch_bwd_dkdv_d256(const fa_params& p, cudaStream_t stream, int* status) {
   if (r) return r;
   r = make_tmap_bshd(&kp.map_do, p.d_o, p.B, p.M, p.H, p.D, p.do_stride, 128);
   if (r) return r;
-  const int64_t* ds_stride = nullptr;
-  const void* ds = d256_ds_tensor(p, &ds_stride);
+  const int64_t slab_stride[3] = {0, slab ? slab->pitch * p.M : 0, slab ? slab->pitch : 0};
+  const int64_t* ds_stride = slab_stride;
+  const void* ds = slab ? slab->base : d256_ds_tensor(p, &ds_stride);
+  kp.bh0 = slab ? slab->bh0 : 0;
+  kp.ds_flat = slab != nullptr;
   if (!ds) return FA_ERR_NULL;
   if (reinterpret_cast<uintptr_t>(ds) % 16 != 0 || ds_stride[0] % 8 || ds_stride[1] % 8 || ds_stride[2] % 8)
     return FA_ERR_ALIGN;
@@ -446,7 +452,7 @@ int launch_bwd_dkdv_d256(const fa_params& p, cudaStream_t stream, int* status) {
   kp.causal = p.causal ? 1 : 0;
   kp.scale_log2 = p.sm_scale * kLog2e;
   kp.sm_scale = p.sm_scale;
-  const dim3 grid((p.N + 63) / 64, p.B * p.H);
+  const dim3 grid((p.N + 63) / 64, slab ? slab->n_bh : p.B * p.H);
   return p.dtype == FA_BF16 ? launch_bias<__nv_bfloat16>(kp, p.bias_kind, grid, stream)
                             : launch_bias<__half>(kp, p.bias_kind, grid, stream);
 }

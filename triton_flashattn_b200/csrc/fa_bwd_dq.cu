@@ -14,9 +14,9 @@
 // The S and dP columns are handed back to the MMA issuer as soon as they sit in
 // registers, so the next block's products run while the row threads compute.
 //
-// (2) dq_from_ds_kernel -- used when the dK/dV kernel has just written dS as
-// dbias in the same 16-bit dtype as q: dQ = sm_scale * dS . K is then a plain
-// streamed GEMM whose A operand is loaded by TMA from the dbias tensor
+// (2) dq_from_ds_kernel -- used when the dK/dV kernel has just written dS as 16-bit
+// values, either as dbias or into scratch slabs: dQ = sm_scale * dS . K is then a plain
+// streamed GEMM whose A operand is loaded by TMA from that tensor
 // (64-key stages, two CTAs per SM).  The reference itself rounds dS to the
 // 16-bit dtype before this product (flash_attention.py line 517), so the
 // result is the same.
@@ -42,6 +42,7 @@ struct DqParams {
   int64_t bias_sB, bias_sH, bias_sM;
   int64_t dq_sB, dq_sM, dq_sH;
   int H, M, N, D;
+  int bh0, ds_flat;     // variant (2): first (batch, head) of this launch; dS slabs numbered from it
   int n_mblk, n_tiles;  // query blocks per (batch, head); tiles = n_mblk * B * H
   int causal, bias_vec32;
   float scale_log2;
@@ -440,7 +441,7 @@ __global__ void __launch_bounds__(192, 2) dq_from_ds_kernel(const __grid_constan
   const int m_block = gridDim.x - 1 - blockIdx.x;
   // the (batch, head) problems in reverse: the dS tiles written last by the dK/dV kernel are
   // still in L2 when this kernel starts
-  const int bh = gridDim.y - 1 - blockIdx.y;
+  const int bh = p.bh0 + gridDim.y - 1 - blockIdx.y;
   const int b = bh / p.H;
   const int h = bh - b * p.H;
   const int m0 = m_block * 128;
@@ -476,6 +477,7 @@ __global__ void __launch_bounds__(192, 2) dq_from_ds_kernel(const __grid_constan
       tma_prefetch_desc(&p.map_ds);
       tma_prefetch_desc(&p.map_k);
       const uint64_t pol_stream = policy_evict_first();
+      const int ds_h = p.ds_flat ? bh - p.bh0 : h, ds_b = p.ds_flat ? 0 : b;
       bool ok = true;
       for (int s = 0; s < nsteps && ok; ++s) {
         const int st = s % L::kStages;
@@ -484,7 +486,7 @@ __global__ void __launch_bounds__(192, 2) dq_from_ds_kernel(const __grid_constan
         if (!ok) break;
         uint8_t* base = smem + st * L::kStage;
         mbar_expect_tx(&full[st], L::kStage);
-        tma_load_4d_hint(base, &p.map_ds, &full[st], s * 64, m0, h, b, pol_stream);
+        tma_load_4d_hint(base, &p.map_ds, &full[st], s * 64, m0, ds_h, ds_b, pol_stream);
         for (int kb = 0; kb < KB; ++kb)
           tma_load_4d(base + L::kDsBytes + kb * (64 * 128), &p.map_k, &full[st], kb * 64, h, s * 64,
                       b);
@@ -586,19 +588,21 @@ int launch_bias(const DqParams& kp, int bias_kind, bool from_ds, dim3 grid, cuda
 
 }  // namespace
 
-int launch_bwd_dq(const fa_params& p, cudaStream_t stream, int* status) {
+int launch_bwd_dq(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab) {
   DqParams kp;
-  // When the dK/dV stage has just left dS in a 16-bit tensor (the bias gradient itself, or the
-  // scratch an fp32 bias comes with) the streamed GEMM variant is used, otherwise the general
-  // kernel.
+  // When the dK/dV stage has just left dS in a 16-bit tensor (the bias gradient itself, or
+  // scratch) the streamed GEMM variant is used, otherwise the general kernel.
   // At head dimension 256 only the streamed variant exists: its dK/dV kernel always leaves dS.
   const bool f32 = p.bias_kind == FA_BIAS_F32;
   const bool d256 = p.D == 256;
-  if (f32 && !p.ds16) return FA_ERR_NULL;
-  const bool from_ds = d256 || f32 || (p.write_dbias && p.bias_kind == FA_BIAS_SAME);
+  if (f32 && !p.ds16 && !slab) return FA_ERR_NULL;
+  const bool from_ds = slab || d256 || f32 || (p.write_dbias && p.bias_kind == FA_BIAS_SAME);
+  kp.bh0 = slab ? slab->bh0 : 0;
+  kp.ds_flat = slab != nullptr;
   const int64_t* ds_stride = f32 ? p.ds16_stride : p.dbias_stride;
   const void* ds = f32 ? p.ds16 : p.dbias;
-  if (d256) ds = d256_ds_tensor(p, &ds_stride);
+  if (slab) ds = slab->base;
+  else if (d256) ds = d256_ds_tensor(p, &ds_stride);
   if (from_ds && !ds) return FA_ERR_NULL;
   int r = make_tmap_bshd(&kp.map_q, p.q, p.B, p.M, p.H, p.D, p.q_stride, 128);
   if (r) return r;
@@ -608,7 +612,10 @@ int launch_bwd_dq(const fa_params& p, cudaStream_t stream, int* status) {
   if (r) return r;
   r = make_tmap_bshd(&kp.map_do, p.d_o, p.B, p.M, p.H, p.D, p.do_stride, 128);
   if (r) return r;
-  if (from_ds) {
+  if (slab) {
+    r = make_tmap_slab(&kp.map_ds, *slab, p.M, p.N);
+    if (r) return r;
+  } else if (from_ds) {
     int bm, hm;
     r = make_tmap_bhmn(&kp.map_ds, ds, 2, p.B, p.H, p.M, p.N, ds_stride, 64, 128, &bm, &hm);
     if (r) return r;
@@ -651,7 +658,7 @@ int launch_bwd_dq(const fa_params& p, cudaStream_t stream, int* status) {
   kp.sm_scale = p.sm_scale;
   kp.n_mblk = (p.M + 127) / 128;
   kp.n_tiles = kp.n_mblk * p.B * p.H;
-  const dim3 grid((p.M + 127) / 128, p.B * p.H);  // streamed-dS variant: one CTA per tile
+  const dim3 grid((p.M + 127) / 128, slab ? slab->n_bh : p.B * p.H);  // streamed-dS variant: one CTA per tile
   const int dp = padded_head_dim(p.D);
   if (dp == 256)
     return p.dtype == FA_BF16 ? launch_from_ds<256, __nv_bfloat16>(kp, grid, stream)

@@ -294,15 +294,25 @@ void backward(const Shape& s, const Tensor& grad, const View& q, const View& k, 
     p.dbias = dbias.mutable_data_ptr();
     set_stride(p.dbias_stride, dbias.strides().data());
   }
-  Tensor ds16;
-  if (bias.kind == FA_BIAS_F32 || (s.D == 256 && !(dbias.defined() && bias.kind == FA_BIAS_SAME))) {
-    // the dK/dV stage hands dS to the dQ stage through a 16-bit scratch tensor (fp32 bias; at head
-    // dim 256 always, unless the 16-bit bias gradient itself is that tensor)
-    ds16 = pitched_empty(o, {s.B, s.H, s.M, s.N}, s.dtype, false);
-    p.ds16 = ds16.mutable_data_ptr();
-    set_stride(p.ds16_stride, ds16.strides().data());
+  // Scratch for dS where it has no tensor of its own.  Without the memory for all the library asks
+  // for, one problem's share; without that, the scores are recomputed where the kernels can.
+  uint64_t bytes = fa_bwd_workspace_bytes(&p);
+  Tensor ws;
+  if (bytes > 0) {
+    const uint64_t one = static_cast<uint64_t>((s.N + 7) / 8 * 8 * s.M * 2);
+    try {
+      ws = empty_on(o, {static_cast<int64_t>(bytes)}, at::kByte);
+    } catch (const c10::OutOfMemoryError&) {
+      bytes = one;
+      try {
+        ws = empty_on(o, {static_cast<int64_t>(bytes)}, at::kByte);
+      } catch (const c10::OutOfMemoryError&) {
+        if (s.D == 256 || bias.kind == FA_BIAS_F32) throw;
+        bytes = 0;
+      }
+    }
   }
-  check_code(fa_bwd(&p, stream_of(s.device)), "fa_bwd");
+  check_code(fa_bwd_workspace(&p, bytes ? ws.mutable_data_ptr() : nullptr, bytes, stream_of(s.device)), "fa_bwd");
 }
 
 // empty_like (strides preserved, as the reference's flash_attention.py 796-798) when the kernels
