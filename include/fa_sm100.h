@@ -131,6 +131,13 @@ const char* fa_status_string(int code);
 int fa_fwd(const fa_params* p, void* stream);
 
 /*
+ * Whether fa_fwd reads the bias of a problem with M query rows of head dim D element by element
+ * (few rows: a decode step).  Such a bias needs a unit innermost stride and nothing else: any
+ * address, any other strides, 0 for M included.
+ */
+int fa_fwd_takes_any_bias(int M, int D);
+
+/*
  * Backward, all three stages in order on `stream`.  Replaces _flash_attn_bwd
  * (FA:688-763): the eager pre-scaled copies of k and bias (FA:699-704) and the
  * zero fill of dbias (FA:799) are folded into the kernels.

@@ -108,6 +108,22 @@ def test_head_dim_256_fp32_bias_and_packed_qkv(causal, device_ok):
     assert torch.equal(kk.grad, qkv_g.grad[:, :, 1]) and torch.equal(vv.grad, qkv_g.grad[:, :, 2])
 
 
+@pytest.mark.parametrize("M,N", [(1, 1), (1, 17), (8, 63), (9, 16), (16, 1000), (3, 4099)])
+@pytest.mark.parametrize("D,dtype", [(16, HF), (32, BF), (64, HF), (128, BF), (128, HF)])
+@pytest.mark.parametrize("bias_kind,causal", [(None, False), (None, True), ("float", False), ("f32", False), ("bool", True)])
+def test_few_query_rows(M, N, D, dtype, bias_kind, causal, device_ok):
+    """M <= 16 runs a kernel of its own: one or two groups of 8 rows, 16-key tiles spread over the
+    warps of 1 to 16 CTAs, warps and whole CTAs without a key among them.  B * H = 3 leaves room
+    for the largest cluster."""
+    q, k, v, bias, do = make_inputs(1, M, N, 3, D, dtype, "float" if bias_kind == "f32" else bias_kind, 15)
+    if bias_kind == "f32":
+        bias = bias.float()
+    ours = run_ours(q, k, v, bias, causal, None, do)
+    ours.pop("dbias", None)
+    compare(ours, q, k, v, bias, causal, None, do, dtype, label=f"M{M} N{N} D{D} {bias_kind} causal={causal}: ",
+            verbose=False)
+
+
 @pytest.mark.parametrize("D", [16, 32])
 @pytest.mark.parametrize("bias_kind", [None, "float"])
 def test_small_head_dims(D, bias_kind, device_ok):

@@ -67,6 +67,7 @@ EXPORTED_SYMBOLS = (
     "fa_launch_count",
     "fa_status_string",
     "fa_fwd",
+    "fa_fwd_takes_any_bias",
     "fa_bwd",
     "fa_bwd_workspace",
     "fa_bwd_workspace_bytes",

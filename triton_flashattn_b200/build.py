@@ -27,6 +27,7 @@ SOURCES = [
     "fa_api.cu",
     "fa_selftest.cu",
     "fa_fwd.cu",
+    "fa_decode.cu",
     "fa_bwd_pre.cu",
     "fa_bwd_dkdv.cu",
     "fa_bwd_dq.cu",

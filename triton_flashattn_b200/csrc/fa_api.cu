@@ -266,6 +266,8 @@ int fa_fwd(const fa_params* p, void* stream) {
                      [&](int* st) { return launch_fwd(*p, static_cast<cudaStream_t>(stream), st); });
 }
 
+int fa_fwd_takes_any_bias(int M, int D) { return decode_takes(M, D) ? 1 : 0; }
+
 int fa_bwd_pre(const fa_params* p, void* stream) {
   int r = validate_bwd(p);
   if (r) return r;

@@ -1,0 +1,436 @@
+// Forward attention for a handful of query rows (decoding: one or a few new tokens against a long
+// key / value cache) on sm_100a.
+//
+// With M <= 16 the path is a stream over K and V: 2 N D elements are read once and each takes part in
+// at most 16 multiply-adds, a few per cent of what the 128-row tile kernel would spend on its
+// padding.  What matters is bytes in flight, so K and V go straight from global memory into
+// registers in the layout the warp-level matrix instruction wants (no shared memory, no barriers),
+// one 16-key tile ahead, and the keys of a (batch, head) are spread over all warps of a cluster
+// of CTAs, so that even a few heads fill the chip.  (The tile kernel gives each head to one CTA.)
+// The warp-level matrix instruction is enough: at the HBM rate an SM has 350 cycles for the 32 products
+// of a tile, and tcgen05 would want the operands in shared memory and 128 rows of queries.
+//   B8 H32 N4096 D128, M=1, bf16:  119 -> 89 us (6.0 TB/s);  B1 H32 N20011:  277 -> 61 us;
+//   B64 H32 N2048: 316 us (6.8 TB/s).  A ring of asynchronous copies in shared memory in place of the
+//   register tiles, two or three tiles deep, was slower (109 and 71 us for the first two).
+//
+// Per warp and tile of 16 keys (r = lane / 4, t = lane % 4):
+//   S^T [16 keys x 8 queries] = K Q^T    the four lanes of a row load 16 bytes each: 64 contiguous
+//        bytes of a key.  Which of the loaded elements meet in one k16 step is free as long as Q is
+//        read the same way, so the words of a 16-byte load feed two steps.
+//   P^T = exp2(S^T - m), transposed in registers (movmatrix) into the B operand
+//   O^T [D x 8 queries] += V^T P^T       lane r loads elements 8r .. 8r+7 of keys 2t, 2t+1, 2t+8, 2t+9
+//        (eight lanes: 128 contiguous bytes) and pairs the keys with byte permutes.
+// The running maximum is raised only when some score passes it by more than 8 (log2 units), so the
+// common tile needs one vote and no shuffles; row sums stay per lane until the end.
+// Partial results are merged in shared memory, then over the cluster through distributed shared
+// memory; every merge runs in a fixed order, so results do not vary from run to run.
+//
+// Replaces _attn_fwd of the reference (flash_attention.py 12-194) for short queries: same masks,
+// bias, base-2 softmax and log-sum-exp as the tile kernel.
+#include <cooperative_groups.h>
+
+#include <mutex>
+
+#include "fa_common.cuh"
+#include "fa_host.cuh"
+
+namespace fa {
+namespace {
+
+namespace cg = cooperative_groups;
+
+struct DecodeParams {
+  const void* q;
+  const void* k;
+  const void* v;
+  const void* bias;
+  void* o;
+  float* lse;
+  int* status;
+  int64_t q_sB, q_sM, q_sH, k_sB, k_sN, k_sH, v_sB, v_sN, v_sH, o_sB, o_sM, o_sH;
+  int64_t bias_sB, bias_sH, bias_sM;
+  int H, M, N, D;
+  int n_keys;  // keys some row sees: N, or min(N, M) when causal
+  int causal;
+  float sm_scale;
+};
+
+__device__ __forceinline__ uint4 ldg_stream(const void* ptr, bool ok) {
+  uint4 v = make_uint4(0, 0, 0, 0);
+  if (ok)
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(ptr));
+  return v;
+}
+
+template <typename T>
+__device__ __forceinline__ void mma16816(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                         uint32_t b1) {
+  if constexpr (Pack2<T>::kIsBf16)
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  else
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+__device__ __forceinline__ uint32_t transpose8x8(uint32_t x) {
+  uint32_t y;
+  asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+  return y;
+}
+
+template <int BIAS, typename T>
+__device__ __forceinline__ float load_bias(const DecodeParams& p, int64_t off) {
+  if constexpr (BIAS == 1) return static_cast<float>(static_cast<const T*>(p.bias)[off]);
+  if constexpr (BIAS == 2) return static_cast<const uint8_t*>(p.bias)[off] ? 0.f : -INFINITY;
+  if constexpr (BIAS == 3) return static_cast<const float*>(p.bias)[off];
+  return 0.f;
+}
+
+// DP: head dim rounded up to 64 or 128; NQ: groups of 8 query rows; W: warps per CTA.
+// Grid: (cluster size, B * H).  The CTAs of a cluster share one (batch, head).
+template <int DP, int NQ, int W, typename T, int BIAS>
+__global__ void __launch_bounds__(W * 32) decode_kernel(const DecodeParams p) {
+  using P2 = Pack2<T>;
+  constexpr int KG = DP / 32;  // 16-byte loads per lane and key row of K
+  constexpr int VG = DP / 64;  // ... of V
+  constexpr int QR = NQ * 8;
+
+  __shared__ float s_o[W][QR][DP + 4];  // +4: rows a few banks apart
+  __shared__ float s_m[W][QR], s_l[W][QR];
+  __shared__ float c_o[QR][DP];  // this CTA's partial result, read by the whole cluster
+  __shared__ float c_m[QR], c_l[QR];
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int r = lane >> 2, t = lane & 3;
+  const int bh = blockIdx.y, b = bh / p.H, h = bh - b * p.H;
+  grid_dep_launch_next();
+  grid_dep_wait();  // the previous kernel's results (and the status word) are visible from here
+  const bool live = *reinterpret_cast<volatile int*>(p.status) == 0;
+
+  const int n_tiles = live ? (p.n_keys + 15) >> 4 : 0;
+  const int stride = static_cast<int>(gridDim.x) * W;
+  const int first = static_cast<int>(blockIdx.x) * W + warp;
+
+  // Q as the B operand: row = query, the same 16-byte pieces of the head dim as a key's
+  uint4 q[NQ][KG];
+  const T* qb = static_cast<const T*>(p.q) + b * p.q_sB + h * p.q_sH;
+#pragma unroll
+  for (int n = 0; n < NQ; ++n)
+#pragma unroll
+    for (int g = 0; g < KG; ++g) {
+      const int m = n * 8 + r, d = g * 32 + t * 8;
+      q[n][g] = m < p.M && d < p.D ? __ldcg(reinterpret_cast<const uint4*>(qb + m * p.q_sM + d)) : make_uint4(0, 0, 0, 0);
+    }
+
+  const T* kb = static_cast<const T*>(p.k) + b * p.k_sB + h * p.k_sH + t * 8;
+  const T* vb = static_cast<const T*>(p.v) + b * p.v_sB + h * p.v_sH + r * 8;
+  const int64_t bias_bh = b * p.bias_sB + h * p.bias_sH;
+
+  uint4 kf[2][KG], vf[4][VG];
+  auto load_k = [&](int tile) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int n = tile * 16 + r + 8 * i;
+      const T* row = kb + n * p.k_sN;
+#pragma unroll
+      for (int g = 0; g < KG; ++g) kf[i][g] = ldg_stream(row + g * 32, n < p.n_keys && (DP == 128 || g * 32 + t * 8 < p.D));
+    }
+  };
+  auto load_v = [&](int tile) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int n = tile * 16 + 2 * t + (i & 1) + 8 * (i >> 1);
+      const T* row = vb + n * p.v_sN;
+#pragma unroll
+      for (int g = 0; g < VG; ++g) vf[i][g] = ldg_stream(row + g * 64, n < p.n_keys && (DP == 128 || r * 8 < p.D));
+    }
+  };
+  float bf[NQ][4];
+  auto load_b = [&](int tile) {
+    if constexpr (BIAS != 0) {
+#pragma unroll
+      for (int n = 0; n < NQ; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int m = n * 8 + 2 * t + (i & 1), key = tile * 16 + r + 8 * (i >> 1);
+          bf[n][i] = m < p.M && key < p.n_keys ? load_bias<BIAS, T>(p, bias_bh + m * p.bias_sM + key) : 0.f;
+        }
+    }
+  };
+
+  float o[NQ][VG * 4][4];  // O^T: [query group][16 head-dim rows][fragment]
+#pragma unroll
+  for (int n = 0; n < NQ; ++n)
+#pragma unroll
+    for (int i = 0; i < VG * 4; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[n][i][e] = 0.f;
+  float mx[NQ][2], l[NQ][2];  // of queries 2t, 2t+1: running maximum (log2 units), this lane's part of the sum
+#pragma unroll
+  for (int n = 0; n < NQ; ++n) mx[n][0] = mx[n][1] = -INFINITY, l[n][0] = l[n][1] = 0.f;
+
+  if (first < n_tiles) {
+    load_k(first);
+    load_b(first);
+    load_v(first);
+  }
+#pragma unroll 1
+  for (int tile = first; tile < n_tiles; tile += stride) {
+    float s[NQ][4];
+#pragma unroll
+    for (int n = 0; n < NQ; ++n) {
+      s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
+#pragma unroll
+      for (int g = 0; g < KG; ++g) {
+        mma16816<T>(s[n], kf[0][g].x, kf[1][g].x, kf[0][g].y, kf[1][g].y, q[n][g].x, q[n][g].y);
+        mma16816<T>(s[n], kf[0][g].z, kf[1][g].z, kf[0][g].w, kf[1][g].w, q[n][g].z, q[n][g].w);
+      }
+    }
+    const bool more = tile + stride < n_tiles;
+    if (more) load_k(tile + stride);
+    // scores in log2 units, -inf where masked
+    bool need = false;
+#pragma unroll
+    for (int n = 0; n < NQ; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float x = s[n][i] * p.sm_scale;
+        if (BIAS != 0) x += bf[n][i];
+        const int key = tile * 16 + r + 8 * (i >> 1);
+        if (key >= p.n_keys || (p.causal && key > n * 8 + 2 * t + (i & 1))) x = -INFINITY;
+        s[n][i] = x * kLog2e;
+        need = need || s[n][i] > mx[n][i & 1] + 8.f;
+      }
+    if (more) load_b(tile + stride);
+    if (__any_sync(0xffffffffu, need)) {
+#pragma unroll
+      for (int n = 0; n < NQ; ++n)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float m_new = fmaxf(mx[n][j], fmaxf(s[n][j], s[n][j + 2]));
+          for (int off = 4; off < 32; off <<= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, off));
+          const float alpha = m_new == -INFINITY ? 1.f : ex2(mx[n][j] - m_new);
+          mx[n][j] = m_new;
+          l[n][j] *= alpha;
+#pragma unroll
+          for (int i = 0; i < VG * 4; ++i) o[n][i][j] *= alpha, o[n][i][j + 2] *= alpha;
+        }
+    }
+    uint32_t pb[NQ][2];
+#pragma unroll
+    for (int n = 0; n < NQ; ++n) {
+      const float m0 = mx[n][0] == -INFINITY ? 0.f : mx[n][0], m1 = mx[n][1] == -INFINITY ? 0.f : mx[n][1];
+      const float p0 = ex2(s[n][0] - m0), p1 = ex2(s[n][1] - m1), p2 = ex2(s[n][2] - m0), p3 = ex2(s[n][3] - m1);
+      l[n][0] += p0 + p2;
+      l[n][1] += p1 + p3;
+      pb[n][0] = transpose8x8(P2::pack(p0, p1));
+      pb[n][1] = transpose8x8(P2::pack(p2, p3));
+    }
+#pragma unroll
+    for (int g = 0; g < VG; ++g) {
+      const uint32_t w[4][4] = {{vf[0][g].x, vf[0][g].y, vf[0][g].z, vf[0][g].w},
+                                {vf[1][g].x, vf[1][g].y, vf[1][g].z, vf[1][g].w},
+                                {vf[2][g].x, vf[2][g].y, vf[2][g].z, vf[2][g].w},
+                                {vf[3][g].x, vf[3][g].y, vf[3][g].z, vf[3][g].w}};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t a0 = __byte_perm(w[0][i], w[1][i], 0x5410), a1 = __byte_perm(w[0][i], w[1][i], 0x7632);
+        const uint32_t a2 = __byte_perm(w[2][i], w[3][i], 0x5410), a3 = __byte_perm(w[2][i], w[3][i], 0x7632);
+#pragma unroll
+        for (int n = 0; n < NQ; ++n) mma16816<T>(o[n][g * 4 + i], a0, a1, a2, a3, pb[n][0], pb[n][1]);
+      }
+    }
+    if (more) load_v(tile + stride);
+  }
+
+  // ---- this warp's part: maximum and sum per query, O^T with lane (r, t) holding head-dim rows
+  // 64 g + 8 r + 2 i (+1) of queries 2t, 2t+1
+#pragma unroll
+  for (int n = 0; n < NQ; ++n)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      for (int off = 4; off < 32; off <<= 1) l[n][j] += __shfl_xor_sync(0xffffffffu, l[n][j], off);
+      const int m = n * 8 + 2 * t + j;
+      if (r == 0) s_m[warp][m] = mx[n][j], s_l[warp][m] = l[n][j];
+#pragma unroll
+      for (int g = 0; g < VG; ++g)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          s_o[warp][m][g * 64 + r * 8 + 2 * i] = o[n][g * 4 + i][j];
+          s_o[warp][m][g * 64 + r * 8 + 2 * i + 1] = o[n][g * 4 + i][j + 2];
+        }
+    }
+  __syncthreads();
+  // ---- this CTA's part
+  for (int e = tid; e < QR * DP; e += W * 32) {
+    const int m = e / DP, d = e - m * DP;
+    float m_all = s_m[0][m];
+#pragma unroll
+    for (int w = 1; w < W; ++w) m_all = fmaxf(m_all, s_m[w][m]);
+    float acc = 0.f, sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      const float f = m_all == -INFINITY ? 0.f : ex2(s_m[w][m] - m_all);
+      acc += f * s_o[w][m][d];
+      sum += f * s_l[w][m];
+    }
+    c_o[m][d] = acc;
+    if (d == 0) c_m[m] = m_all, c_l[m] = sum;
+  }
+  // ---- the cluster's result: each CTA finishes a share of the elements
+  const int parts = static_cast<int>(gridDim.x);
+  cg::cluster_group cluster = cg::this_cluster();
+  if (parts > 1)
+    cluster.sync();
+  else
+    __syncthreads();
+  for (int e = static_cast<int>(blockIdx.x) * W * 32 + tid; live && e < p.M * DP; e += parts * W * 32) {
+    const int m = e / DP, d = e - m * DP;
+    float m_all = -INFINITY;
+    for (int c = 0; c < parts; ++c) m_all = fmaxf(m_all, parts > 1 ? *cluster.map_shared_rank(&c_m[m], c) : c_m[m]);
+    float acc = 0.f, sum = 0.f;
+    for (int c = 0; c < parts; ++c) {
+      const float mc = parts > 1 ? *cluster.map_shared_rank(&c_m[m], c) : c_m[m];
+      const float f = m_all == -INFINITY ? 0.f : ex2(mc - m_all);
+      acc += f * (parts > 1 ? *cluster.map_shared_rank(&c_o[m][d], c) : c_o[m][d]);
+      sum += f * (parts > 1 ? *cluster.map_shared_rank(&c_l[m], c) : c_l[m]);
+    }
+    // a row whose keys are all masked out: output 0, log-sum-exp +inf
+    const bool any_key = m_all != -INFINITY && sum > 0.f;
+    if (d < p.D)
+      (static_cast<T*>(p.o) + b * p.o_sB + m * p.o_sM + h * p.o_sH)[d] = static_cast<T>(any_key ? acc / sum : 0.f);
+    if (d == 0) p.lse[static_cast<int64_t>(bh) * p.M + m] = any_key ? m_all + log2f(sum) : INFINITY;
+  }
+  if (parts > 1) cluster.sync();  // no CTA leaves while another still reads its shared memory
+}
+
+// How many clusters of 1 .. 16 CTAs of a kernel the current device holds at once (asked once).
+constexpr int kMaxParts = 16;
+template <auto kern>  // one table per kernel
+const int* resident_clusters(int warps) {
+  static int table[64][kMaxParts + 1] = {};
+  static std::mutex mu;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> lock(mu);
+  int* t = table[dev];
+  if (t[0] == 0) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return nullptr;
+    for (int parts = 1; parts <= kMaxParts; ++parts) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(parts, 1);
+      cfg.blockDim = dim3(warps * 32);
+      cudaLaunchAttribute attr;
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = parts;
+      attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+      cfg.attrs = &attr;
+      cfg.numAttrs = 1;
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;  // this size is not launched
+      }
+      t[parts] = n;
+    }
+    t[0] = 1;
+  }
+  return t;
+}
+
+// The split of a (batch, head)'s key tiles over `parts` CTAs of `warps` warps: the one with the least
+// (turns of the resident clusters) x (tiles per warp + the start and the merge of a CTA, which take
+// about as long as six tiles).  A single turn that fills the SMs wins where there are few heads,
+// several turns of longer CTAs where there are many.  B1 H32 N20011 D128: 10 CTAs a head 61 us,
+// 8: 70, 11 (no longer one turn): 95; B8 H32 N4096: 3 a head 90 us, 1: 108, 2: 117, 4: 99.
+struct Split {
+  int parts = 0, warps = 0;
+  int64_t cost = -1;
+};
+void consider(Split& best, const int* resident, int warps, int bh, int tiles) {
+  if (!resident) return;
+  for (int parts = 1; parts <= kMaxParts; ++parts) {
+    if (resident[parts] < 1 || (parts > 1 && (parts - 1) * warps >= tiles)) continue;
+    const int64_t turns = (bh + resident[parts] - 1) / resident[parts];
+    const int64_t cost = turns * ((tiles + parts * warps - 1) / (parts * warps) + 6);
+    if (best.cost < 0 || cost < best.cost) best = {parts, warps, cost};
+  }
+}
+
+template <int DP, int NQ, typename T, int BIAS>
+int launch_inst(const DecodeParams& dp, int bh, cudaStream_t stream) {
+  const int tiles = (dp.n_keys + 15) / 16;
+  Split s;
+  consider(s, resident_clusters<decode_kernel<DP, NQ, 4, T, BIAS>>(4), 4, bh, tiles);
+  // twice the warps per head where even 16 CTAs leave SMs idle (one group of rows only: two groups
+  // of partial results would not fit the static shared memory)
+  if constexpr (NQ == 1) consider(s, resident_clusters<decode_kernel<DP, NQ, 8, T, BIAS>>(8), 8, bh, tiles);
+  if (s.cost < 0) return FA_ERR_CUDA;
+  if constexpr (NQ == 1)
+    if (s.warps == 8)
+      return launch_overlapped(decode_kernel<DP, NQ, 8, T, BIAS>, dim3(s.parts, bh), 256, 0, stream, dp, s.parts);
+  return launch_overlapped(decode_kernel<DP, NQ, 4, T, BIAS>, dim3(s.parts, bh), 128, 0, stream, dp, s.parts);
+}
+
+template <int DP, typename T, int BIAS>
+int launch_rows(const DecodeParams& dp, int bh, cudaStream_t stream) {
+  return dp.M <= 8 ? launch_inst<DP, 1, T, BIAS>(dp, bh, stream) : launch_inst<DP, 2, T, BIAS>(dp, bh, stream);
+}
+
+template <int DP, typename T>
+int launch_bias(const DecodeParams& dp, int bias_kind, int bh, cudaStream_t stream) {
+  switch (bias_kind) {
+    case FA_BIAS_NONE: return launch_rows<DP, T, 0>(dp, bh, stream);
+    case FA_BIAS_SAME: return launch_rows<DP, T, 1>(dp, bh, stream);
+    case FA_BIAS_BOOL: return launch_rows<DP, T, 2>(dp, bh, stream);
+    case FA_BIAS_F32: return launch_rows<DP, T, 3>(dp, bh, stream);
+    default: return FA_ERR_UNSUPPORTED;
+  }
+}
+
+template <typename T>
+int launch_dtype(const DecodeParams& dp, int bias_kind, int bh, cudaStream_t stream) {
+  return dp.D <= 64 ? launch_bias<64, T>(dp, bias_kind, bh, stream)
+                    : launch_bias<128, T>(dp, bias_kind, bh, stream);
+}
+
+}  // namespace
+
+// 16 rows are what two groups of 8 queries cover; at head dim 256 the operands no longer fit a
+// thread's registers.
+bool decode_takes(int M, int D) { return M <= 16 && D <= 128; }
+
+int launch_decode(const fa_params& p, cudaStream_t stream, int* status) {
+  auto bad = [](const void* ptr, const int64_t s[3]) {
+    return reinterpret_cast<uintptr_t>(ptr) % 16 != 0 || s[0] % 8 || s[1] % 8 || s[2] % 8;
+  };
+  if (bad(p.q, p.q_stride) || bad(p.k, p.k_stride) || bad(p.v, p.v_stride) || bad(p.o, p.o_stride)) return FA_ERR_ALIGN;
+  DecodeParams d;
+  d.q = p.q;
+  d.k = p.k;
+  d.v = p.v;
+  d.bias = p.bias;
+  d.o = p.o;
+  d.lse = p.lse;
+  d.status = status;
+  d.q_sB = p.q_stride[0], d.q_sM = p.q_stride[1], d.q_sH = p.q_stride[2];
+  d.k_sB = p.k_stride[0], d.k_sN = p.k_stride[1], d.k_sH = p.k_stride[2];
+  d.v_sB = p.v_stride[0], d.v_sN = p.v_stride[1], d.v_sH = p.v_stride[2];
+  d.o_sB = p.o_stride[0], d.o_sM = p.o_stride[1], d.o_sH = p.o_stride[2];
+  d.bias_sB = p.bias_stride[0], d.bias_sH = p.bias_stride[1], d.bias_sM = p.bias_stride[2];
+  d.H = p.H, d.M = p.M, d.N = p.N, d.D = p.D;
+  d.n_keys = p.causal && p.M < p.N ? p.M : p.N;
+  d.causal = p.causal ? 1 : 0;
+  d.sm_scale = p.sm_scale;
+  const int bh = p.B * p.H;
+  return p.dtype == FA_BF16 ? launch_dtype<__nv_bfloat16>(d, p.bias_kind, bh, stream)
+                            : launch_dtype<__half>(d, p.bias_kind, bh, stream);
+}
+
+}  // namespace fa

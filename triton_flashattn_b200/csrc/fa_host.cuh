@@ -36,6 +36,10 @@ struct DsSlab {
 };
 
 int launch_fwd(const fa_params& p, cudaStream_t stream, int* status);
+// Forward for a few query rows: whether it takes the problem, and its launch.  It reads the bias
+// element by element, so that needs no alignment there.
+bool decode_takes(int M, int D);
+int launch_decode(const fa_params& p, cudaStream_t stream, int* status);
 int launch_bwd_pre(const fa_params& p, cudaStream_t stream, int* status);
 // Without a slab: all problems, dS going where the parameters say (dbias, ds16 or nowhere).
 int launch_bwd_dkdv(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab = nullptr);
@@ -61,17 +65,20 @@ extern std::atomic<uint64_t> g_kernel_launches;
 // Launch with the programmatic-stream-serialization attribute (see grid_dep_wait()).
 template <typename Kern, typename Params>
 inline int launch_overlapped(Kern kern, dim3 grid, int threads, size_t smem, cudaStream_t stream,
-                             const Params& params) {
+                             const Params& params, int cluster_x = 1) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster_x;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster_x > 1 ? 2 : 1;
   if (cudaLaunchKernelEx(&cfg, kern, params) != cudaSuccess) return FA_ERR_CUDA;
   g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
   return FA_OK;

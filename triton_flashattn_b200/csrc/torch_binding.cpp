@@ -139,30 +139,35 @@ Tensor bias_ready(const Tensor& bias) {
   return out.expand(sz);
 }
 
-struct Bias {
-  Tensor t;  // what the kernels read; undefined without a bias
-  int kind = FA_BIAS_NONE;
-};
-
-Bias classify_bias(const Tensor& bias, at::ScalarType q_dtype) {
-  if (!bias.defined()) return {};
-  const auto dt = bias.scalar_type();
-  if (dt == at::kBool) return {bias_ready(bias), FA_BIAS_BOOL};
-  if (!at::isFloatingType(dt))
-    fail(PyExc_TypeError, std::string("bias must be a bool or floating tensor, got ") + toString(dt));
-  if (dt == q_dtype) return {bias_ready(bias), FA_BIAS_SAME};
-  // Any other float dtype is streamed as fp32 (the reference also adds the bias in fp32,
-  // flash_attention.py 52, 292): nothing is rounded to 16 bits, the gradient comes back in fp32.
-  return {bias_ready(dt == at::kFloat ? bias : bias.to(at::kFloat)), FA_BIAS_F32};
-}
-
-// ---------------------------------------------------------------------------- argument checks
 struct Shape {
   int64_t B, M, N, H, D;
   at::ScalarType dtype;
   int device;
 };
 
+struct Bias {
+  Tensor t;  // what the kernels read; undefined without a bias
+  int kind = FA_BIAS_NONE;
+};
+
+// `any_layout`: the reader takes it with any strides but the innermost
+Bias classify_bias(const Tensor& bias, at::ScalarType q_dtype, bool any_layout = false) {
+  if (!bias.defined()) return {};
+  const auto dt = bias.scalar_type();
+  const auto ready = [&](const Tensor& t) { return any_layout && t.stride(3) == 1 ? t : bias_ready(t); };
+  if (dt == at::kBool) return {ready(bias), FA_BIAS_BOOL};
+  if (!at::isFloatingType(dt))
+    fail(PyExc_TypeError, std::string("bias must be a bool or floating tensor, got ") + toString(dt));
+  if (dt == q_dtype) return {ready(bias), FA_BIAS_SAME};
+  // Any other float dtype is streamed as fp32 (the reference also adds the bias in fp32,
+  // flash_attention.py 52, 292): nothing is rounded to 16 bits, the gradient comes back in fp32.
+  return {ready(dt == at::kFloat ? bias : bias.to(at::kFloat)), FA_BIAS_F32};
+}
+Bias forward_bias(const Shape& s, const Tensor& bias) {
+  return classify_bias(bias, s.dtype, fa_fwd_takes_any_bias(static_cast<int>(s.M), static_cast<int>(s.D)) != 0);
+}
+
+// ---------------------------------------------------------------------------- argument checks
 std::string shape_text(at::IntArrayRef s) {
   std::string t = "(";
   for (size_t i = 0; i < s.size(); ++i) t += (i ? ", " : "") + std::to_string(s[i]);
@@ -426,7 +431,7 @@ Tensor attention(const Tensor& a, const Tensor& k, const Tensor& v, const Tensor
   Bias b;
   {
     at::AutoDispatchBelowADInplaceOrView guard;
-    b = classify_bias(bias, s.dtype);
+    b = forward_bias(s, bias);
     if (packed) {
       const Tensor t = packed_ready(a);
       std::tie(out, lse) = forward(s, t, slice_of(t, 0), slice_of(t, 1), slice_of(t, 2), b, causal, scale);
@@ -532,7 +537,7 @@ PyObject* py_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor q = tile_ready(q0), k = tile_ready(k0), v = tile_ready(v0);
     Tensor out, lse;
     std::tie(out, lse) =
-        forward(s, q, view_of(q), view_of(k), view_of(v), classify_bias(bias, s.dtype), causal, scale);
+        forward(s, q, view_of(q), view_of(k), view_of(v), forward_bias(s, bias), causal, scale);
     return PyTuple_Pack(2, THPObjectPtr(THPVariable_Wrap(out)).get(), THPObjectPtr(THPVariable_Wrap(lse)).get());
   });
 }
