@@ -146,6 +146,21 @@ def test_many_tiles_per_persistent_cta(max_ctas, D, bias_kind, causal, device_ok
     check_case(2, 3 * 128 + 40, 5 * 128 - 9, 3, D, BF, bias_kind, causal, seed=21, bias_scale=0.5)
 
 
+@pytest.mark.parametrize("max_ctas", ["1", "2"])
+@pytest.mark.parametrize("M,N,causal,bias_kind,trainable", [
+    (1, 129, False, None, False), (129, 128, True, "bool", False), (384, 192, False, "float", True),
+    (130, 400, True, "float", True), (257, 65, False, "float", False), (300, 300, True, None, False)])
+def test_head_dim_256_tile_edges(max_ctas, M, N, causal, bias_kind, trainable, device_ok, monkeypatch):
+    """Head dimension 256 with several key tiles per CTA: one query block and several, a last key tile of one
+    key, of 64 and of 65, key tiles that no query row sees (M < N, causal).  Bounds as in test_head_dim_256."""
+    monkeypatch.setenv("FA_MAX_CTAS", max_ctas)
+    q, k, v, bias, do = make_inputs(2, M, N, 2, 256, BF, bias_kind, 22)
+    ours = run_ours(q, k, v, bias, causal, None, do, trainable)
+    ref = oracle.attention_backward(q, k, v, bias, causal, None, do, o_saved=ours["out"])
+    for n, t in ours.items():
+        accept(n, account(t, ref[n], BF), BF, label=f"D256 M{M} N{N} bias={bias_kind} causal={causal} {n}: ")
+
+
 def test_non_trainable_float_bias(device_ok):
     check_case(1, 256, 256, 2, 128, BF, "float", True, seed=6, trainable_bias=False)
 

@@ -178,9 +178,8 @@ uint64_t slab_bytes(const fa_params& p) { return (uint64_t)slab_pitch(p) * p.M *
 int problems_per_part(const fa_params& p, int most) {
   const int total = p.B * p.H;
   if (most >= total) return total;
-  const int keys = p.D == 256 ? 64 : 128;
-  const int tiles = (p.N + keys - 1) / keys;
-  const bool pairs = p.causal && p.D != 256;  // a causal unit is a heavy and a light tile
+  const int tiles = (p.N + 127) / 128;
+  const bool pairs = p.causal != 0;  // a causal unit is a heavy and a light tile
   const int sms = persistent_grid(1 << 30);
   auto turns = [&](int n) {
     const int64_t units = pairs ? ((int64_t)n * tiles + 1) / 2 : (int64_t)n * tiles;

@@ -20,20 +20,34 @@
 // (64-key stages, two CTAs per SM).  The reference itself rounds dS to the
 // 16-bit dtype before this product (flash_attention.py line 517), so the
 // result is the same.
+// At head dimension 256 the same kernel, reading the dS tiles the other way round, gives
+// dK = sm_scale * dS^T . Q as well (that dK/dV kernel has no tensor memory for dK).
 //
-// Both replace _attn_bwd_dq / _attn_bwd_dq_inner (flash_attention.py 458-646).
+// All replace _attn_bwd_dq / _attn_bwd_dq_inner (flash_attention.py 458-646).
 #include "fa_common.cuh"
 #include "fa_host.cuh"
 
 namespace fa {
 namespace {
 
+struct FromDsParams {
+  CUtensorMap map_ds;  // box of 64 keys x 128 (dQ) or 64 (dK) query rows
+  CUtensorMap map_b;   // K or Q, box of 64 rows
+  void* out;           // dQ or dK
+  int* status;
+  int64_t out_sB, out_sR, out_sH;
+  int H, M, N, D;
+  int bh0, ds_flat;  // first (batch, head) of this launch; dS slabs numbered from it
+  int ascending;     // (batch, head) problems in ascending order
+  int causal;
+  float sm_scale;
+};
+
 struct DqParams {
   CUtensorMap map_q;
   CUtensorMap map_k;
   CUtensorMap map_v;
   CUtensorMap map_do;
-  CUtensorMap map_ds;  // dbias viewed as the A operand of variant (2)
   const void* bias;
   void* dq;
   const float* lse;
@@ -42,7 +56,6 @@ struct DqParams {
   int64_t bias_sB, bias_sH, bias_sM;
   int64_t dq_sB, dq_sM, dq_sH;
   int H, M, N, D;
-  int bh0, ds_flat;     // variant (2): first (batch, head) of this launch; dS slabs numbered from it
   int n_mblk, n_tiles;  // query blocks per (batch, head); tiles = n_mblk * B * H
   int causal, bias_vec32;
   float scale_log2;
@@ -407,24 +420,28 @@ __global__ void __launch_bounds__(608, 1) dq_recompute_kernel(const __grid_const
 }
 
 // ----------------------------------------------------------------------------
-// variant (2): dQ = sm_scale * dS . K with dS streamed from the dbias tensor
+// variant (2): dQ = sm_scale * dS . K (KEYS: dK = sm_scale * dS^T . Q), dS streamed from global memory
 // ----------------------------------------------------------------------------
+// Two CTAs per SM.  At head dim 256 a stage is 48 KB: two stages each, so that two producer threads
+// and four stages are under way per SM (one CTA with three stages: one thread's stream of bulk loads
+// was the bound).
 template <int DP>
-struct DqDsSmem {
-  static constexpr int kStages = 3;
-  static constexpr int kDsBytes = 128 * 64 * 2;  // [128 m][64 n]
-  static constexpr int kKBytes = 64 * DP * 2;    // [64 n][DP]
-  static constexpr int kStage = kDsBytes + kKBytes;
+struct FromDsSmem {
+  static constexpr int kStages = DP == 256 ? 2 : 3;
+  static constexpr int kDsBytes = 128 * 64 * 2;  // [128 m][64 n], or two blocks [64 m][64 n]
+  static constexpr int kBBytes = 64 * DP * 2;    // [64 n][DP] of K, or [64 m][DP] of Q
+  static constexpr int kStage = kDsBytes + kBBytes;
   static constexpr int kTotal = kStages * kStage;
   static constexpr int kDynamic = kTotal + 1024;
 };
 
-template <int DP, typename T>
-__global__ void __launch_bounds__(192, 2) dq_from_ds_kernel(const __grid_constant__ DqParams p) {
-  using L = DqDsSmem<DP>;
+template <int DP, typename T, bool KEYS>
+__global__ void __launch_bounds__(192, 2) from_ds_kernel(const __grid_constant__ FromDsParams p) {
+  using L = FromDsSmem<DP>;
   using P2 = Pack2<T>;
   constexpr int KB = DP / 64;
-  constexpr uint32_t kTmemCols = DP;  // 64 or 128 accumulator columns
+  constexpr int kB64 = 64 * 128;        // bytes of a [64][64] block
+  constexpr uint32_t kTmemCols = DP;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -438,19 +455,21 @@ __global__ void __launch_bounds__(192, 2) dq_from_ds_kernel(const __grid_constan
   // warps then run converged and only elect a lane for the issue itself
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lane = tid & 31;
-  const int m_block = gridDim.x - 1 - blockIdx.x;
-  // the (batch, head) problems in reverse: the dS tiles written last by the dK/dV kernel are
-  // still in L2 when this kernel starts
-  const int bh = p.bh0 + gridDim.y - 1 - blockIdx.y;
+  // Longest causal blocks first: the last query rows, the first keys.
+  const int blk = KEYS ? blockIdx.x : gridDim.x - 1 - blockIdx.x;
+  // The (batch, head) problems against the order of the kernel before: the dS tiles it touched last
+  // are still in L2 when this kernel starts.
+  const int bh = p.bh0 + (p.ascending ? blockIdx.y : gridDim.y - 1 - blockIdx.y);
   const int b = bh / p.H;
   const int h = bh - b * p.H;
-  const int m0 = m_block * 128;
-  // 64-key steps; causal rows of this block see keys < m0 + 128
-  int n_end = p.N;
-  if (p.causal) n_end = min(n_end, m0 + 128);
-  const int nsteps = (n_end + 63) >> 6;
+  const int r0 = blk * 128;  // first output row
+  // 64-wide steps over keys (causal rows of this block see keys < r0 + 128) or over query rows (the
+  // causal dK/dV stage leaves dS of whole 128-row blocks from row r0 on)
+  const int s_end = KEYS ? (p.M + 63) >> 6 : ((p.causal ? min(p.N, r0 + 128) : p.N) + 63) >> 6;
+  const int s0 = KEYS && p.causal ? min(r0 >> 6, s_end) : 0;
+  const int nsteps = s_end - s0;
 
-  WaitCtx ctx{&abort_flag, p.status, 4};
+  WaitCtx ctx{&abort_flag, p.status, KEYS ? 6 : 4};
   if (tid == 0) {
     abort_flag = 0;
     for (int i = 0; i < L::kStages; ++i) {
@@ -475,7 +494,7 @@ __global__ void __launch_bounds__(192, 2) dq_from_ds_kernel(const __grid_constan
   if (warp == 4) {
     if (lane == 0 && live) {
       tma_prefetch_desc(&p.map_ds);
-      tma_prefetch_desc(&p.map_k);
+      tma_prefetch_desc(&p.map_b);
       const uint64_t pol_stream = policy_evict_first();
       const int ds_h = p.ds_flat ? bh - p.bh0 : h, ds_b = p.ds_flat ? 0 : b;
       bool ok = true;
@@ -485,17 +504,23 @@ __global__ void __launch_bounds__(192, 2) dq_from_ds_kernel(const __grid_constan
         if (use >= 1) ok = mbar_wait(&empty[st], (use - 1) & 1, ctx, kSiteStageEmpty, s);
         if (!ok) break;
         uint8_t* base = smem + st * L::kStage;
+        const int c0 = (s0 + s) * 64;
         mbar_expect_tx(&full[st], L::kStage);
-        tma_load_4d_hint(base, &p.map_ds, &full[st], s * 64, m0, ds_h, ds_b, pol_stream);
+        if (KEYS) {
+          // the second block lies past the last key for a short edge: zeros
+          tma_load_4d(base, &p.map_ds, &full[st], r0, c0, ds_h, ds_b);
+          tma_load_4d(base + kB64, &p.map_ds, &full[st], r0 + 64, c0, ds_h, ds_b);
+        } else {
+          tma_load_4d_hint(base, &p.map_ds, &full[st], c0, r0, ds_h, ds_b, pol_stream);
+        }
         for (int kb = 0; kb < KB; ++kb)
-          tma_load_4d(base + L::kDsBytes + kb * (64 * 128), &p.map_k, &full[st], kb * 64, h, s * 64,
-                      b);
+          tma_load_4d(base + L::kDsBytes + kb * kB64, &p.map_b, &full[st], kb * 64, h, c0, b);
       }
     }
   } else if (warp == 5) {
     // (whole warp converged, one elected lane issues)
     if (live) {
-      constexpr uint32_t idesc = make_idesc(P2::kIsBf16, false, true, 128, DP);
+      constexpr uint32_t idesc = make_idesc(P2::kIsBf16, KEYS, true, 128, DP);
       bool ok = true;
       for (int s = 0; s < nsteps && ok; ++s) {
         const int st = s % L::kStages;
@@ -505,8 +530,8 @@ __global__ void __launch_bounds__(192, 2) dq_from_ds_kernel(const __grid_constan
         const uint32_t a_addr = smem_u32(smem + st * L::kStage);
         const uint32_t b_addr = a_addr + L::kDsBytes;
         if (elect_one()) {
-          issue_gemm_ss<4, false, true>(tmem, make_sdesc(a_addr, 0, 1024),
-                                        make_sdesc(b_addr, 64 * 128, 1024), 0, 0, idesc, s > 0);
+          issue_gemm_ss<4, KEYS, true>(tmem, make_sdesc(a_addr, KEYS ? kB64 : 0, 1024), make_sdesc(b_addr, kB64, 1024), 0,
+                                       0, idesc, s > 0);
           mma_commit(&empty[st]);
         }
         __syncwarp();
@@ -515,24 +540,28 @@ __global__ void __launch_bounds__(192, 2) dq_from_ds_kernel(const __grid_constan
     }
     __syncwarp();
   } else {
-    const int r = tid;
     const uint32_t lane_base = static_cast<uint32_t>(warp) * 32u;
-    const int m = m0 + r;
+    const int row = r0 + tid;
     bool ok = live;
     if (ok) ok = wait_warp(&acc_done, 0, ctx, kSiteEpilogue, 0);
     if (ok) {
       tc_fence_after();
-      T* row = reinterpret_cast<T*>(p.dq) + b * p.dq_sB + (int64_t)m * p.dq_sM + h * p.dq_sH;
+      T* out = reinterpret_cast<T*>(p.out) + b * p.out_sB + (int64_t)row * p.out_sR + h * p.out_sH;
 #pragma unroll
       for (int g = 0; g < DP / 32; ++g) {
         uint32_t a[32];
-        tmem_ld32(tmem_addr(tmem, lane_base, g * 32), a);
-        tmem_ld_wait();
-        if (m < p.M) {
+        if (nsteps > 0) {
+          tmem_ld32(tmem_addr(tmem, lane_base, g * 32), a);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) a[i] = 0;  // keys no query row sees
+        }
+        if (row < (KEYS ? p.N : p.M)) {
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
             const int d = g * 32 + c * 8;
-            if (d < p.D) *reinterpret_cast<uint4*>(row + d) = pack8<P2>(a + c * 8, p.sm_scale);
+            if (d < p.D) *reinterpret_cast<uint4*>(out + d) = pack8<P2>(a + c * 8, p.sm_scale);
           }
         }
       }
@@ -557,7 +586,7 @@ int configure(K kern, int smem_bytes, bool* configured) {
 }
 
 template <int DP, typename T, int BIAS>
-int launch_recompute(const DqParams& kp, dim3 /*tile_grid*/, cudaStream_t stream) {
+int launch_recompute(const DqParams& kp, cudaStream_t stream) {
   const dim3 grid(persistent_grid(kp.causal ? (kp.n_tiles + 1) / 2 : kp.n_tiles));
   using L = DqSmem<DP>;
   static bool configured[64] = {};
@@ -566,67 +595,105 @@ int launch_recompute(const DqParams& kp, dim3 /*tile_grid*/, cudaStream_t stream
   return launch_overlapped(kern, grid, 608, L::kDynamic, stream, kp);
 }
 
-template <int DP, typename T>
-int launch_from_ds(const DqParams& kp, dim3 grid, cudaStream_t stream) {
-  using L = DqDsSmem<DP>;
+template <int DP, typename T, bool KEYS>
+int launch_from_ds_inst(const FromDsParams& kp, dim3 grid, cudaStream_t stream) {
+  using L = FromDsSmem<DP>;
   static bool configured[64] = {};
-  auto kern = dq_from_ds_kernel<DP, T>;
+  auto kern = from_ds_kernel<DP, T, KEYS>;
   if (int r = configure(kern, L::kDynamic, configured)) return r;
   return launch_overlapped(kern, grid, 192, L::kDynamic, stream, kp);
 }
 
+// dQ, or (keys: at head dimension 256) dK, from the 16-bit dS that the dK/dV stage has left in the slab, in
+// the bias gradient or in the ds16 scratch.
+int launch_from_ds(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab, bool keys) {
+  const bool f32 = p.bias_kind == FA_BIAS_F32;
+  const int64_t* ds_stride = f32 ? p.ds16_stride : p.dbias_stride;
+  const void* ds = f32 ? p.ds16 : p.dbias;
+  if (!slab && p.D == 256) ds = d256_ds_tensor(p, &ds_stride);
+  if (!slab && !ds) return FA_ERR_NULL;
+  FromDsParams kp;
+  int r;
+  if (slab) {
+    r = make_tmap_slab(&kp.map_ds, *slab, p.M, p.N, keys ? 64 : 128);
+  } else {
+    int bm, hm;
+    r = make_tmap_bhmn(&kp.map_ds, ds, 2, p.B, p.H, p.M, p.N, ds_stride, 64, keys ? 64 : 128, &bm, &hm);
+    if (!r && (!bm || !hm)) r = FA_ERR_ALIGN;  // must be a real (B, H, M, N) tensor
+  }
+  if (r) return r;
+  r = keys ? make_tmap_bshd(&kp.map_b, p.q, p.B, p.M, p.H, p.D, p.q_stride, 64)
+           : make_tmap_bshd(&kp.map_b, p.k, p.B, p.N, p.H, p.D, p.k_stride, 64);
+  if (r) return r;
+  auto bad = [](const void* ptr, const int64_t s[3]) {
+    return reinterpret_cast<uintptr_t>(ptr) % 16 != 0 || s[0] % 8 || s[1] % 8 || s[2] % 8;
+  };
+  // q, v and do are asked of every backward call, whether this stage reads them or not
+  if (bad(p.q, p.q_stride) || bad(p.v, p.v_stride) || bad(p.d_o, p.do_stride)) return FA_ERR_ALIGN;
+  const int64_t* out_stride = keys ? p.dk_stride : p.dq_stride;
+  kp.out = keys ? p.dk : p.dq;
+  if (bad(kp.out, out_stride)) return FA_ERR_ALIGN;
+  kp.status = status;
+  kp.out_sB = out_stride[0], kp.out_sR = out_stride[1], kp.out_sH = out_stride[2];
+  kp.H = p.H, kp.M = p.M, kp.N = p.N, kp.D = p.D;
+  kp.bh0 = slab ? slab->bh0 : 0;
+  kp.ds_flat = slab != nullptr;
+  kp.ascending = p.D == 256 && !keys;  // there the dK product, in descending order, came before
+  kp.causal = p.causal ? 1 : 0;
+  kp.sm_scale = p.sm_scale;
+  const dim3 grid(((keys ? p.N : p.M) + 127) / 128, slab ? slab->n_bh : p.B * p.H);  // one CTA per tile
+  const bool bf = p.dtype == FA_BF16;
+  const int dp = padded_head_dim(p.D);
+  if (keys)  // D = 256 only
+    return bf ? launch_from_ds_inst<256, __nv_bfloat16, true>(kp, grid, stream)
+              : launch_from_ds_inst<256, __half, true>(kp, grid, stream);
+  if (dp == 256)
+    return bf ? launch_from_ds_inst<256, __nv_bfloat16, false>(kp, grid, stream)
+              : launch_from_ds_inst<256, __half, false>(kp, grid, stream);
+  if (dp == 128)
+    return bf ? launch_from_ds_inst<128, __nv_bfloat16, false>(kp, grid, stream)
+              : launch_from_ds_inst<128, __half, false>(kp, grid, stream);
+  return bf ? launch_from_ds_inst<64, __nv_bfloat16, false>(kp, grid, stream)
+            : launch_from_ds_inst<64, __half, false>(kp, grid, stream);
+}
+
 template <int DP, typename T>
-int launch_bias(const DqParams& kp, int bias_kind, bool from_ds, dim3 grid, cudaStream_t stream) {
-  if (from_ds) return launch_from_ds<DP, T>(kp, grid, stream);
+int launch_bias(const DqParams& kp, int bias_kind, cudaStream_t stream) {
   switch (bias_kind) {
-    case FA_BIAS_NONE: return launch_recompute<DP, T, 0>(kp, grid, stream);
-    case FA_BIAS_SAME: return launch_recompute<DP, T, 1>(kp, grid, stream);
-    case FA_BIAS_BOOL: return launch_recompute<DP, T, 2>(kp, grid, stream);
+    case FA_BIAS_NONE: return launch_recompute<DP, T, 0>(kp, stream);
+    case FA_BIAS_SAME: return launch_recompute<DP, T, 1>(kp, stream);
+    case FA_BIAS_BOOL: return launch_recompute<DP, T, 2>(kp, stream);
     default: return FA_ERR_UNSUPPORTED;
   }
 }
 
 }  // namespace
 
+int launch_bwd_dk_from_ds(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab) {
+  return launch_from_ds(p, stream, status, slab, true);
+}
+
 int launch_bwd_dq(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab) {
-  DqParams kp;
   // When the dK/dV stage has just left dS in a 16-bit tensor (the bias gradient itself, or
   // scratch) the streamed GEMM variant is used, otherwise the general kernel.
   // At head dimension 256 only the streamed variant exists: its dK/dV kernel always leaves dS.
   const bool f32 = p.bias_kind == FA_BIAS_F32;
-  const bool d256 = p.D == 256;
   if (f32 && !p.ds16 && !slab) return FA_ERR_NULL;
-  const bool from_ds = slab || d256 || f32 || (p.write_dbias && p.bias_kind == FA_BIAS_SAME);
-  kp.bh0 = slab ? slab->bh0 : 0;
-  kp.ds_flat = slab != nullptr;
-  const int64_t* ds_stride = f32 ? p.ds16_stride : p.dbias_stride;
-  const void* ds = f32 ? p.ds16 : p.dbias;
-  if (slab) ds = slab->base;
-  else if (d256) ds = d256_ds_tensor(p, &ds_stride);
-  if (from_ds && !ds) return FA_ERR_NULL;
+  if (slab || p.D == 256 || f32 || (p.write_dbias && p.bias_kind == FA_BIAS_SAME))
+    return launch_from_ds(p, stream, status, slab, false);
+  DqParams kp;
   int r = make_tmap_bshd(&kp.map_q, p.q, p.B, p.M, p.H, p.D, p.q_stride, 128);
   if (r) return r;
-  r = make_tmap_bshd(&kp.map_k, p.k, p.B, p.N, p.H, p.D, p.k_stride, from_ds ? 64 : 128);
+  r = make_tmap_bshd(&kp.map_k, p.k, p.B, p.N, p.H, p.D, p.k_stride, 128);
   if (r) return r;
   r = make_tmap_bshd(&kp.map_v, p.v, p.B, p.N, p.H, p.D, p.v_stride, 128);
   if (r) return r;
   r = make_tmap_bshd(&kp.map_do, p.d_o, p.B, p.M, p.H, p.D, p.do_stride, 128);
   if (r) return r;
-  if (slab) {
-    r = make_tmap_slab(&kp.map_ds, *slab, p.M, p.N);
-    if (r) return r;
-  } else if (from_ds) {
-    int bm, hm;
-    r = make_tmap_bhmn(&kp.map_ds, ds, 2, p.B, p.H, p.M, p.N, ds_stride, 64, 128, &bm, &hm);
-    if (r) return r;
-    if (!bm || !hm) return FA_ERR_ALIGN;
-  } else {
-    kp.map_ds = kp.map_q;
-  }
   if (reinterpret_cast<uintptr_t>(p.dq) % 16 != 0 || p.dq_stride[0] % 8 || p.dq_stride[1] % 8 ||
       p.dq_stride[2] % 8)
     return FA_ERR_ALIGN;
-  if (p.bias_kind != FA_BIAS_NONE && !from_ds) {
+  if (p.bias_kind != FA_BIAS_NONE) {
     const int eb = p.bias_kind == FA_BIAS_BOOL ? 1 : 2;
     if (reinterpret_cast<uintptr_t>(p.bias) % 16 != 0 || (p.bias_stride[0] * eb) % 16 ||
         (p.bias_stride[1] * eb) % 16 || (p.bias_stride[2] * eb) % 16)
@@ -658,17 +725,13 @@ int launch_bwd_dq(const fa_params& p, cudaStream_t stream, int* status, const Ds
   kp.sm_scale = p.sm_scale;
   kp.n_mblk = (p.M + 127) / 128;
   kp.n_tiles = kp.n_mblk * p.B * p.H;
-  const dim3 grid((p.M + 127) / 128, slab ? slab->n_bh : p.B * p.H);  // streamed-dS variant: one CTA per tile
   const int dp = padded_head_dim(p.D);
-  if (dp == 256)
-    return p.dtype == FA_BF16 ? launch_from_ds<256, __nv_bfloat16>(kp, grid, stream)
-                              : launch_from_ds<256, __half>(kp, grid, stream);
   if (p.dtype == FA_BF16) {
-    return dp == 64 ? launch_bias<64, __nv_bfloat16>(kp, p.bias_kind, from_ds, grid, stream)
-                    : launch_bias<128, __nv_bfloat16>(kp, p.bias_kind, from_ds, grid, stream);
+    return dp == 64 ? launch_bias<64, __nv_bfloat16>(kp, p.bias_kind, stream)
+                    : launch_bias<128, __nv_bfloat16>(kp, p.bias_kind, stream);
   }
-  return dp == 64 ? launch_bias<64, __half>(kp, p.bias_kind, from_ds, grid, stream)
-                  : launch_bias<128, __half>(kp, p.bias_kind, from_ds, grid, stream);
+  return dp == 64 ? launch_bias<64, __half>(kp, p.bias_kind, stream)
+                  : launch_bias<128, __half>(kp, p.bias_kind, stream);
 }
 
 }  // namespace fa

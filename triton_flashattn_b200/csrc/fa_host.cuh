@@ -44,10 +44,11 @@ int launch_bwd_pre(const fa_params& p, cudaStream_t stream, int* status);
 // Without a slab: all problems, dS going where the parameters say (dbias, ds16 or nowhere).
 int launch_bwd_dkdv(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab = nullptr);
 int launch_bwd_dq(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab = nullptr);
-// Head dimension 256: its own dK/dV kernel, which always leaves the 16-bit dS in global
-// memory (in dbias for a 16-bit bias that wants its gradient, else in the ds16 scratch);
-// d256_ds_tensor names that tensor, the dQ stage streams it.
+// Head dimension 256: its own dV kernel, which always leaves the 16-bit dS in global
+// memory (in dbias for a 16-bit bias that wants its gradient, else in the ds16 scratch;
+// d256_ds_tensor names that tensor), and dK and dQ as products that stream it.
 int launch_bwd_dkdv_d256(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab);
+int launch_bwd_dk_from_ds(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab);
 const void* d256_ds_tensor(const fa_params& p, const int64_t** stride);
 int launch_selftest(int mode, int dtype, const void* a, const void* b, void* c, cudaStream_t stream,
                     int* status);
@@ -84,12 +85,12 @@ inline int launch_overlapped(Kern kern, dim3 grid, int threads, size_t smem, cud
   return FA_OK;
 }
 
-// Tile map for the slabs of a DsSlab: dims {N, M, problems, 1}, box {64, 128}.
-inline int make_tmap_slab(CUtensorMap* out, const DsSlab& slab, int M, int N) {
+// Tile map for the slabs of a DsSlab: dims {N, M, problems, 1}, box {64, box_rows}.
+inline int make_tmap_slab(CUtensorMap* out, const DsSlab& slab, int M, int N, int box_rows = 128) {
   const uint64_t dims[4] = {(uint64_t)N, (uint64_t)M, (uint64_t)slab.n_bh, 1};
   const uint64_t row = (uint64_t)slab.pitch * 2;
   const uint64_t sb[3] = {row, row * M, row * M * (uint64_t)slab.n_bh};
-  const uint32_t box[4] = {64, 128, 1, 1};
+  const uint32_t box[4] = {64, (uint32_t)box_rows, 1, 1};
   return make_tmap_4d(out, slab.base, 2, dims, sb, box);
 }
 
