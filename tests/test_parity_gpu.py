@@ -61,7 +61,7 @@ def test_ragged_lengths(M, N, causal, bias_kind, device_ok):
 @pytest.mark.parametrize("bias_kind,trainable", [(None, False), ("float", True), ("float", False), ("bool", False)])
 def test_head_dim_256(dtype, M, N, causal, bias_kind, trainable, device_ok):
     """Head dimension 256 (flash_attention.py line 776 accepts it): one query tile per CTA in the
-    forward, the transposed 64-key dK/dV kernel and the streamed dQ in the backward.
+    forward, the transposed dV kernel and the streamed dK and dQ in the backward.
 
     delta = rowsum(o * do) is formed from the 16-bit output, and two correct 16-bit roundings of
     o differ by one unit in some of a row's elements; that difference, summed over D = 256

@@ -8,30 +8,36 @@
 //   fa_bwd_dq.cu    dK = sm_scale * dS^T Q, then dQ = sm_scale * dS K
 // Persistent, one CTA per SM.  A tile is 128 keys of one (batch, head); a CTA walks its tiles and,
 // inside a tile, the 128-row query blocks that see its keys.  K and V stay in shared memory for a
-// tile (64 KB each); Q and dO pass through a ring of two 32 KB stages, each [128 rows][128 head-dim
-// columns], in the order the products take them:
-//   Q(0) | Q(1) dO(0) | Q(2) dO(1) | ...
-// so S of the next step is computed while the row threads form P of this one.  The last 32 KB are P;
-// a 16-bit bias tile lands there by TMA first, each thread reads the chunks it overwrites with P.
+// tile (64 KB each); Q and dO pass through a ring of three 32 KB stages, each [128 rows][128 head-dim
+// columns].  Everything is kept TRANSPOSED, keys as tensor-memory lanes:
+//   S^T = K Q^T, dP^T = V dO^T     (both operands in shared memory)
+//   dV += P^T dO                   (P^T in tensor memory, over the columns of S^T it was formed from)
+// so P needs no shared memory and the third ring stage has room.  The row threads own a key: a bias
+// row, a mask row or a row of dS is then 32 neighbouring keys per warp access (64 bytes), and -LSE2 and
+// -delta of the query rows come from shared memory.
 // Roles (640 threads):
-//   warps 0-15  row threads: tensor-memory lanes 32*(w&3).. (query rows), 32-key column quarter w>>2
+//   warps 0-15  row threads: lanes 32*(w&3).. (keys), 32-query column quarter w>>2
 //   warps 16/17 TMA producers: each brings one of the two 16 KB boxes of every stage and half of K
 //               and V (one thread's stream of boxes reaches 24 bytes per cycle, a step needs 30)
-//   warp 18     MMA issuer, tensor-memory owner
-//   warp 19     TMA loads of the 16-bit bias tiles
+//   warp 18     MMA issuer, tensor-memory owner: per step S, dP, dV
+//   warp 19     -LSE2 and -delta of a step into shared memory
 // The control warps walk their loops converged and elect a lane for the issue.
 // Rule kept by every barrier here: the next completion of a barrier needs progress of every thread
 // that waits on it, so a parity wait can never be two phases behind.
 //
-// What bounds it: a step is 128 KB of Q / dO against 3072 cycles of products, with one ring turn
-// (product, hand-back, load) exposed per step.  The version before kept dV^T and dK^T of 64 keys in
-// one kernel with everything single-staged: 11,900 cycles a step of half the keys.
-// B4 H8 S2048, 16-bit bias: 0.33 ms and 0.075 ms for dK; the training pass 957 -> 731 us.
+// What bounds it: a step takes 6400 cycles against 3072 of products; the issuer's looks at barriers
+// (about 280 cycles each, so they are combined) and the wait for P make up most of the rest.  (A second
+// issuer for dP changed nothing: 0.245 / 0.251 ms.)  B4 H8 S2048, 16-bit bias: 0.245 ms; with the query
+// rows as lanes, P in shared memory and two ring stages 0.330 ms (9800 cycles: each stage was waited for,
+// and a row of bias or dS per thread is 32 sectors per warp access), with four 16 KB stages 0.379 ms
+// (N = 64 products of 16-wide slices take 48 cycles, not 32, and twice the looks).
 //
 // Query blocks above the causal diagonal are not visited: the caller zero-fills dbias.
 //
 // Replaces _attn_bwd_dkdv / _attn_bwd_dkdv_inner of the reference (flash_attention.py
 // 237-454) at BLOCK_HEADDIM = 256: same P, dS, dbias = dS, dK scaled by sm_scale.
+#include <type_traits>
+
 #include "fa_common.cuh"
 #include "fa_host.cuh"
 
@@ -43,7 +49,7 @@ struct Dkdv256Params {
   CUtensorMap map_k;
   CUtensorMap map_v;
   CUtensorMap map_do;
-  CUtensorMap map_bias;
+  CUtensorMap map_bias;  // only used to pull bias tiles into L2
   const void* bias;
   void* dv;
   void* ds16;        // (B, H, M, N) 16-bit dS out; rows 16-byte aligned
@@ -59,19 +65,19 @@ struct Dkdv256Params {
   int n_nblk, n_tiles;  // key blocks per (batch, head); tiles of this launch
   int bh0;              // first (batch, head) of this launch
   int ds_flat;          // ds16 holds slabs numbered from bh0 (ds_sH apart) instead of a (B, H, M, N) tensor
-  int causal, bias_vec32, bias_b_mul, bias_h_mul;
-  int ds_vec32, dv_vec32;  // bases and strides are multiples of 32 bytes
+  int causal, bias_b_mul, bias_h_mul;
+  int dv_vec32;  // base and strides are multiples of 32 bytes
   float scale_log2;        // sm_scale * log2(e)
 };
 
 enum Dkdv256Site { kSiteKFull = 1, kSiteKEmpty, kSiteVFull, kSiteVEmpty, kSiteFull, kSiteEmpty, kSiteSFull,
-                   kSiteSFree, kSitePReady, kSiteDpFull, kSiteDvDone, kSiteBiasFull, kSiteEpilogue };
+                   kSiteStatFull, kSitePReady, kSiteDpFull, kSiteDpFree, kSiteAccDone };
 
 constexpr int kTile256 = 128 * 256 * 2;  // K or V: four [128][64] blocks
 constexpr int kStage256 = 2 * kBlk;      // [128 rows][128 columns] of Q or dO
+constexpr uint32_t kStages256 = 3;
 constexpr int kOffK = 0, kOffV = kOffK + kTile256, kOffRing = kOffV + kTile256;
-constexpr int kOffP = kOffRing + 2 * kStage256;
-constexpr int kSmem256 = kOffP + 2 * kBlk + 1024;  // + slack for 1024-byte alignment
+constexpr int kSmem256 = kOffRing + kStages256 * kStage256 + 1024;  // + slack for 1024-byte alignment
 
 // 32 bytes: one sector store, or two halves where the address is only 16-byte aligned
 __device__ __forceinline__ void store32(void* dst, const uint32_t* w, bool vec32) {
@@ -94,8 +100,9 @@ __global__ void __launch_bounds__(640, 1) dkdv256_kernel(const __grid_constant__
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  __shared__ uint64_t k_full, k_empty, v_full, v_empty, full[2], empty[2];
-  __shared__ uint64_t s_full, s_free, p_ready, dp_full, dv_done, bias_full;
+  __shared__ uint64_t k_full, k_empty, v_full, v_empty, full[kStages256], empty[kStages256];
+  __shared__ uint64_t s_full, stat_full, p_ready, dp_full, dp_free, acc_done;
+  __shared__ __align__(16) float s_nlse[128], s_ndelta[128];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
@@ -146,16 +153,16 @@ __global__ void __launch_bounds__(640, 1) dkdv256_kernel(const __grid_constant__
     mbar_init(&k_empty, 1);
     mbar_init(&v_full, 2);
     mbar_init(&v_empty, 1);
-    for (int i = 0; i < 2; ++i) {
+    for (uint32_t i = 0; i < kStages256; ++i) {
       mbar_init(&full[i], 2);
       mbar_init(&empty[i], 1);
     }
     mbar_init(&s_full, 1);
-    mbar_init(&s_free, 16);
+    mbar_init(&stat_full, 1);
     mbar_init(&p_ready, 16);
     mbar_init(&dp_full, 1);
-    mbar_init(&dv_done, 1);
-    mbar_init(&bias_full, 1);
+    mbar_init(&dp_free, 16);
+    mbar_init(&acc_done, 1);
     mbar_fence_init();
   }
   if (warp == 18) {
@@ -197,8 +204,8 @@ __global__ void __launch_bounds__(640, 1) dkdv256_kernel(const __grid_constant__
       auto ring_load = [&](const CUtensorMap* map, const Step& s) -> bool {
         const int b = s.bh / p.H, h = s.bh - b * p.H;
         for (int c = 0; c < 2; ++c, ++use) {
-          const uint32_t st = use & 1;
-          if (use >= 2 && !wait_warp(&empty[st], ((use >> 1) - 1) & 1, ctx, kSiteEmpty, s.mb)) return false;
+          const uint32_t st = use % kStages256, round = use / kStages256;
+          if (round >= 1 && !wait_warp(&empty[st], (round - 1) & 1, ctx, kSiteEmpty, s.mb)) return false;
           if (elect_one()) {
             mbar_expect_tx(&full[st], kBlk);
             tma_load_4d(smem + kOffRing + st * kStage256 + half * kBlk, map, &full[st], c * 128 + half * 64, h,
@@ -208,43 +215,35 @@ __global__ void __launch_bounds__(640, 1) dkdv256_kernel(const __grid_constant__
         }
         return true;
       };
-      Step cur, prev;
-      prev.valid = false;
-      next_step(cur);
-      while (ok && (cur.valid || prev.valid)) {
-        if (cur.valid) {
-          if (cur.first) {
-            if (nk >= 1) ok = wait_warp(&k_empty, (nk - 1) & 1, ctx, kSiteKEmpty, cur.it);
-            if (!ok) break;
-            ++nk;
-            tile_load(&p.map_k, kOffK, &k_full, cur);
-          }
-          if (BIAS != 0 && half == 0) {
-            // the bias tile of this step is pulled into L2, about a step before it is read
-            constexpr int kBox = BIAS == 1 ? 64 : (BIAS == 3 ? 32 : 128);  // keys per box of map_bias
-            const int b = cur.bh / p.H, h = cur.bh - b * p.H;
-            if (elect_one()) {
-#pragma unroll
-              for (int c = 0; c < 128; c += kBox)
-                if (cur.nb * 128 + c < p.N)
-                  tma_prefetch_l2_4d(&p.map_bias, cur.nb * 128 + c, cur.mb * 128, h * p.bias_h_mul, b * p.bias_b_mul);
-            }
-            __syncwarp();
-          }
-          ok = ring_load(&p.map_q, cur);
+      Step s;
+      for (next_step(s); ok && s.valid; next_step(s)) {
+        if (s.first) {
+          if (nk >= 1) ok = wait_warp(&k_empty, (nk - 1) & 1, ctx, kSiteKEmpty, s.it);
           if (!ok) break;
+          ++nk;
+          tile_load(&p.map_k, kOffK, &k_full, s);
         }
-        if (prev.valid) {
-          if (prev.first) {
-            if (nv >= 1) ok = wait_warp(&v_empty, (nv - 1) & 1, ctx, kSiteVEmpty, prev.it);
-            if (!ok) break;
-            ++nv;
-            tile_load(&p.map_v, kOffV, &v_full, prev);
+        if (BIAS != 0 && half == 0) {
+          // the bias tile of this step is pulled into L2, about a step before it is read
+          constexpr int kBox = BIAS == 1 ? 64 : (BIAS == 3 ? 32 : 128);  // keys per box of map_bias
+          const int b = s.bh / p.H, h = s.bh - b * p.H;
+          if (elect_one()) {
+#pragma unroll
+            for (int c = 0; c < 128; c += kBox)
+              if (c == 0 || s.nb * 128 + c < p.N)
+                tma_prefetch_l2_4d(&p.map_bias, s.nb * 128 + c, s.mb * 128, h * p.bias_h_mul, b * p.bias_b_mul);
           }
-          ok = ring_load(&p.map_do, prev);
+          __syncwarp();
         }
-        prev = cur;
-        if (cur.valid) next_step(cur);
+        ok = ring_load(&p.map_q, s);
+        if (!ok) break;
+        if (s.first) {
+          if (nv >= 1) ok = wait_warp(&v_empty, (nv - 1) & 1, ctx, kSiteVEmpty, s.it);
+          if (!ok) break;
+          ++nv;
+          tile_load(&p.map_v, kOffV, &v_full, s);
+        }
+        ok = ring_load(&p.map_do, s);
       }
     }
   } else if (warp == 18) {
@@ -252,229 +251,216 @@ __global__ void __launch_bounds__(640, 1) dkdv256_kernel(const __grid_constant__
     if (live) {
       constexpr bool bf = P2::kIsBf16;
       constexpr uint32_t idesc_s = make_idesc(bf, false, false, 128, 128);
-      constexpr uint32_t idesc_g = make_idesc(bf, true, true, 128, 128);
+      constexpr uint32_t idesc_g = make_idesc(bf, false, true, 128, 128);
       const uint64_t k_km = make_sdesc(smem_u32(smem + kOffK), 0, 1024), v_km = make_sdesc(smem_u32(smem + kOffV), 0, 1024);
-      const uint64_t p_mn = make_sdesc(smem_u32(smem + kOffP), kBlk, 1024);
       const uint32_t ring = smem_u32(smem + kOffRing);
       constexpr uint64_t kHalfTile = static_cast<uint64_t>(2 * kBlk) >> 4;  // two blocks, in descriptor units
       bool ok = true;
-      uint32_t use = 0;         // ring stages taken so far
-      uint32_t nk = 0, nv = 0;  // K / V tiles taken so far
-      uint32_t g = 0;           // steps whose S was issued
-      Step cur, prev;
-      prev.valid = false;
-      next_step(cur);
-      while (ok && (cur.valid || prev.valid)) {
-        const Step here = cur;
-        if (cur.valid) next_step(cur);
-        if (here.valid) {
-          // S of step g: its columns are free once the row threads hold S of step g-1
-          if (here.first) {
-            ok = wait_warp(&k_full, nk & 1, ctx, kSiteKFull, here.it);
-            ++nk;
-          }
-          if (ok && g >= 1) ok = wait_warp_hot(&s_free, (g - 1) & 1, ctx, kSiteSFree, here.mb);
-          for (int c = 0; c < 2 && ok; ++c, ++use) {
-            const uint32_t st = use & 1;
-            ok = wait_warp_hot(&full[st], (use >> 1) & 1, ctx, kSiteFull, here.mb);
-            if (!ok) break;
-            tc_fence_after();
-            if (elect_one()) {
-              issue_gemm_ss<8, false, false>(tmem + kColS, make_sdesc(ring + st * kStage256, 0, 1024),
-                                             k_km + c * kHalfTile, kBlk, kBlk, idesc_s, c > 0);
-              mma_commit(&empty[st]);
-              if (c == 1) {
-                mma_commit(&s_full);
-                if (cur.valid && cur.first) mma_commit(&k_empty);  // last step of its tile: K may be replaced
-              }
-            }
-            __syncwarp();
-          }
-          if (!ok) break;
-          ++g;
-        }
-        if (prev.valid) {
-          // dP and dV of the step before.  All sixteen row warps announce P after they have read dP of
-          // the step before that and, at the start of a tile, the finished dV of the last one.
-          const uint32_t gp = here.valid ? g - 2 : g - 1;
-          if (prev.first) {
-            ok = wait_warp(&v_full, nv & 1, ctx, kSiteVFull, prev.it);
-            ++nv;
-          }
-          if (ok) ok = wait_warp_hot(&p_ready, gp & 1, ctx, kSitePReady, prev.mb);
-          for (int c = 0; c < 2 && ok; ++c) {
-            const uint32_t st = (use + c) & 1;
-            ok = wait_warp_hot(&full[st], ((use + c) >> 1) & 1, ctx, kSiteFull, prev.mb);
-            if (!ok) break;
-            tc_fence_after();
-            if (elect_one()) {
-              issue_gemm_ss<8, false, false>(tmem + kColDp, make_sdesc(ring + st * kStage256, 0, 1024),
-                                             v_km + c * kHalfTile, kBlk, kBlk, idesc_s, c > 0);
-              if (c == 1) {
-                mma_commit(&dp_full);
-                if (!here.valid || here.first) mma_commit(&v_empty);  // last step of its tile
-              }
-            }
-            __syncwarp();
-          }
-          if (!ok) break;
-          if (elect_one()) {
+      uint32_t use = 0;   // ring stages taken so far
+      uint32_t tile = 0;  // K / V tiles taken so far
+      uint32_t g = 0;     // steps done
+      Step s;
+      next_step(s);
+      while (ok && s.valid) {
+        const Step here = s;
+        next_step(s);
+        const bool last = !s.valid || s.first;  // last step of its tile
+        uint32_t st[4], par[4];                 // Q and dO of this step: ring stage, parity
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              const uint32_t st = (use + c) & 1;
-              issue_gemm_ss<8, true, true>(tmem + kColDv + c * 128, p_mn, make_sdesc(ring + st * kStage256, kBlk, 1024),
-                                           kBlk, kBlk, idesc_g, !prev.first);
-              mma_commit(&empty[st]);
+        for (int c = 0; c < 4; ++c) {
+          st[c] = (use + c) % kStages256;
+          par[c] = ((use + c) / kStages256) & 1;
+        }
+        use += 4;
+        // S^T: its columns hold P of the step before, whose dV this thread has issued already
+        if (here.first) ok = wait_warp(&k_full, tile & 1, ctx, kSiteKFull, here.it);
+        uint32_t seen0, seen1;
+        mbar_poll2(&full[st[0]], par[0], &full[st[1]], par[1], seen0, seen1);
+        for (int c = 0; c < 2 && ok; ++c) {
+          ok = wait_warp_polled(c ? seen1 : seen0, &full[st[c]], par[c], ctx, kSiteFull, here.mb);
+          if (!ok) break;
+          tc_fence_after();
+          if (elect_one()) {
+            issue_gemm_ss<8, false, false>(tmem + kColS, k_km + c * kHalfTile, make_sdesc(ring + st[c] * kStage256, 0, 1024),
+                                           kBlk, kBlk, idesc_s, c > 0);
+            mma_commit(&empty[st[c]]);
+            if (c == 1) {
+              mma_commit(&s_full);
+              if (last) mma_commit(&k_empty);  // K may be replaced
             }
-            mma_commit(&dv_done);
           }
           __syncwarp();
-          use += 2;
         }
-        prev = here;
+        if (!ok) break;
+        // dP^T: its columns are free once the row threads hold dP of the step before
+        if (here.first) ok = wait_warp(&v_full, tile & 1, ctx, kSiteVFull, here.it);
+        uint32_t seen2 = 1;
+        // (full[st[3]] is the stage of Q's first half: only asked about once S has been issued, and a
+        // parity look is right then because this warp has seen that stage's completion before)
+        if (g >= 1)
+          mbar_poll3(&full[st[2]], par[2], &full[st[3]], par[3], &dp_free, (g - 1) & 1, seen0, seen1, seen2);
+        else
+          mbar_poll2(&full[st[2]], par[2], &full[st[3]], par[3], seen0, seen1);
+        if (ok && g >= 1) ok = wait_warp_polled(seen2, &dp_free, (g - 1) & 1, ctx, kSiteDpFree, here.mb);
+        for (int c = 0; c < 2 && ok; ++c) {
+          ok = wait_warp_polled(c ? seen1 : seen0, &full[st[2 + c]], par[2 + c], ctx, kSiteFull, here.mb);
+          if (!ok) break;
+          tc_fence_after();
+          if (elect_one()) {
+            issue_gemm_ss<8, false, false>(tmem + kColDp, v_km + c * kHalfTile,
+                                           make_sdesc(ring + st[2 + c] * kStage256, 0, 1024), kBlk, kBlk, idesc_s, c > 0);
+            if (c == 1) {
+              mma_commit(&dp_full);
+              if (last) mma_commit(&v_empty);
+            }
+          }
+          __syncwarp();
+        }
+        if (!ok) break;
+        // dV.  The first product of a tile overwrites the accumulator: P is only announced by all sixteen
+        // row warps after they have read it.
+        ok = wait_warp_hot(&p_ready, g & 1, ctx, kSitePReady, here.mb);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const uint64_t do_mn = make_sdesc(ring + st[2 + c] * kStage256, kBlk, 1024);
+#pragma unroll
+            for (int ks = 0; ks < 8; ++ks)  // 16 query rows: two slices per quarter of the columns
+              mma_ts(tmem + kColDv + c * 128, tmem + kColS + (ks >> 1) * 32 + (ks & 1) * 8, do_mn + mnmajor_step(ks),
+                     idesc_g, !here.first || ks > 0);
+            mma_commit(&empty[st[2 + c]]);
+          }
+          if (last) mma_commit(&acc_done);
+        }
+        __syncwarp();
+        ++g;
+        if (last) ++tile;
       }
     }
     __syncwarp();
   } else if (warp == 19) {
-    // ----------------------------------------------------------- bias tile loads
-    if (BIAS == 1 && live) {
-      if (lane == 0) tma_prefetch_desc(&p.map_bias);
-      bool ok = true;
+    // ---------------------------------------------- -LSE2 and -delta of a step's query rows
+    if (live) {
+      uint32_t g = 0;
       Step s;
-      next_step(s);
-      for (uint32_t gs = 0; s.valid; ++gs, next_step(s)) {
-        // the P tile is free once dV of the previous step has read it
-        if (gs >= 1) ok = wait_warp_hot(&dv_done, (gs - 1) & 1, ctx, kSiteDvDone, s.mb);
-        if (!ok) break;
-        const int b = s.bh / p.H, h = s.bh - b * p.H, n0 = s.nb * 128;
-        const bool two = n0 + 64 < p.N;
-        if (elect_one()) {
-          mbar_expect_tx(&bias_full, two ? 2 * kBlk : kBlk);
-          tma_load_4d(smem + kOffP, &p.map_bias, &bias_full, n0, s.mb * 128, h * p.bias_h_mul, b * p.bias_b_mul);
-          if (two)
-            tma_load_4d(smem + kOffP + kBlk, &p.map_bias, &bias_full, n0 + 64, s.mb * 128, h * p.bias_h_mul,
-                        b * p.bias_b_mul);
+      for (next_step(s); s.valid; next_step(s), ++g) {
+        float nl[4], nd[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          // rows beyond M get -inf / 0, which makes their P and dS zero
+          const int m = s.mb * 128 + j * 32 + lane;
+          const int64_t idx = static_cast<int64_t>(s.bh) * p.M + m;
+          nl[j] = m < p.M ? -__ldcg(p.lse + idx) : -INFINITY;
+          nd[j] = m < p.M ? -__ldcg(p.delta + idx) : 0.f;
+        }
+        if (g >= 1 && !wait_warp(&dp_free, (g - 1) & 1, ctx, kSiteDpFree, s.mb)) break;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          s_nlse[j * 32 + lane] = nl[j];
+          s_ndelta[j * 32 + lane] = nd[j];
         }
         __syncwarp();
+        if (lane == 0) mbar_arrive(&stat_full);
       }
     }
     __syncwarp();
   } else {
     // --------------------------------------------------------------- row threads
-    const int r = (warp & 3) * 32 + lane;  // query row inside the block = tensor-memory lane
-    const int qt = warp >> 2;              // column quarter: keys n0 + 32*qt .. +31
+    const int r = (warp & 3) * 32 + lane;  // key inside the tile = tensor-memory lane
+    const int qt = warp >> 2;              // column quarter: query rows 32*qt .. +31 of the block
     const uint32_t lane_base = static_cast<uint32_t>(warp & 3) * 32u;
     bool ok = live;
-    // this thread's four 16-byte chunks of P: chunk c at sp_row + ((chunk0 + c) ^ (r & 7)) * 16
-    const uint32_t sp_row = smem_u32(smem + kOffP + (qt >> 1) * kBlk) + static_cast<uint32_t>(r) * 128u;
-    const uint32_t chunk0 = (qt & 1) * 4;
     const uint32_t tm_sc = tmem_addr(tmem, lane_base, kColS + qt * 32);
-
-    constexpr int BR = BIAS == 2 ? 2 : 0;  // the byte mask is read one step ahead
-    BiasRegs<BR> bnext;
-    // -LSE2 and delta of the coming step's row, as loaded: looked at when that step starts
-    float lse_next = 0.f, delta_next = 0.f;
-    auto prefetch = [&](int bh_, int c0, int mblk) {
-      const int m = mblk * 128 + r;
-      if constexpr (BR == 2) {
-        const int b_ = bh_ / p.H, h_ = bh_ - b_ * p.H;
-        load_bias_row<2>(bnext, p.bias, b_ * p.bias_sB + h_ * p.bias_sH + (int64_t)m * p.bias_sM, m < p.M, c0, p.N,
-                         p.bias_vec32 != 0);
-      }
-      const int64_t idx = (int64_t)bh_ * p.M + min(m, p.M - 1);
-      lse_next = __ldcg(p.lse + idx);
-      delta_next = __ldcg(p.delta + idx);
-    };
-    uint32_t gs = 0;  // steps done so far, over all tiles
+    const uint32_t nlse_a = smem_u32(s_nlse + qt * 32), ndelta_a = smem_u32(s_ndelta + qt * 32);
+    uint32_t gs = 0;     // steps done so far, over all tiles
+    uint32_t tiles = 0;  // tiles with at least one step so far
     int bh, nb, i_start;
-    if (ok && tile_at(0, bh, nb, i_start) && i_start < n_mblk) prefetch(bh, nb * 128 + qt * 32, i_start);
 #pragma unroll 1
     for (int it = 0; ok && tile_at(it, bh, nb, i_start); ++it) {
-      const int col0 = nb * 128 + qt * 32;
+      const int n = nb * 128 + r;
       const int b = bh / p.H, h = bh - b * p.H;
-      const int64_t ds_bh = p.ds_flat ? (bh - p.bh0) * p.ds_sH : b * p.ds_sB + h * p.ds_sH;
+      const bool key_ok = n < p.N;
+      // Keys beyond N compute on zero rows of K and V and what they read as bias is key N-1's; nothing of
+      // theirs is stored, and no other key's result depends on them.
+      const int64_t bias_off = b * p.bias_sB + h * p.bias_sH + min(n, p.N - 1);
+      const int64_t ds_off = (p.ds_flat ? (bh - p.bh0) * p.ds_sH : b * p.ds_sB + h * p.ds_sH) + n;
+      const int64_t dbf_off = b * p.dbf_sB + h * p.dbf_sH + n;
 #pragma unroll 1
       for (int mb = i_start; mb < n_mblk && ok; ++mb, ++gs) {
-        const int m0 = mb * 128;
-        const bool row_ok = m0 + r < p.M;
-        BiasRegs<BR> bcur = bnext;
-        BiasRegs<BIAS == 3 ? 3 : 0> bf32;
-        // fp32 bias row of this step: asked for now, used once S has arrived
-        if constexpr (BIAS == 3)
-          load_bias_row<3>(bf32, p.bias, b * p.bias_sB + h * p.bias_sH + (int64_t)(m0 + r) * p.bias_sM, row_ok, col0, p.N,
-                           p.bias_vec32 != 0);
-        // rows beyond M get -inf / 0, which makes their P and dS zero
-        const float neg_lse = row_ok ? -lse_next : -INFINITY, delta_r = row_ok ? delta_next : 0.f;
-        if (mb + 1 < n_mblk) prefetch(bh, col0, mb + 1);
+        const int m0 = mb * 128 + qt * 32;  // this thread's first query row
+        const int rows = p.M - m0;          // of its 32 query rows the first `rows` exist
+        // The bias of this step travels while S is computed.  (Whole blocks without a test per row: with
+        // one the loads went out one after the other, 8200 cycles a step.)
+        uint32_t w[BIAS != 0 ? 32 : 1];
+        if constexpr (BIAS != 0) {
+          using E = std::conditional_t<BIAS == 1, uint16_t, std::conditional_t<BIAS == 2, uint8_t, uint32_t>>;
+          const E* src = static_cast<const E*>(p.bias) + bias_off;
+          if (rows >= 32) {
+            src += static_cast<int64_t>(m0) * p.bias_sM;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              w[i] = __ldcg(src);
+              src += p.bias_sM;
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              w[i] = __ldcg(src + static_cast<int64_t>(min(m0 + i, p.M - 1)) * p.bias_sM);
+              if (i >= rows) w[i] = 0;
+            }
+          }
+        }
 
-        // ---- P
-        ok = wait_warp(&s_full, gs & 1, ctx, kSiteSFull, mb);
+        // ---- P^T
+        uint32_t ps, pstat;
+        mbar_poll2(&s_full, gs & 1, &stat_full, gs & 1, ps, pstat);
+        ok = wait_warp_polled(pstat, &stat_full, gs & 1, ctx, kSiteStatFull, mb);
+        if (ok) ok = wait_warp_polled(ps, &s_full, gs & 1, ctx, kSiteSFull, mb);
         if (!ok) break;
         tc_fence_after();
         float pr[32];
         tmem_ld32(tm_sc, reinterpret_cast<uint32_t*>(pr));
         tmem_ld_wait();
-        // S now lives in registers: hand its columns back for the next S
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&s_free);
         // P = exp2(S * scale * log2e + bias * log2e - LSE2)
-        if constexpr (BIAS == 1) {
+        const f32x2 sc2 = f2(p.scale_log2, p.scale_log2);
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const f32x2 x = ffma2(f2(pr[i], pr[i + 1]), f2(p.scale_log2, p.scale_log2), f2(neg_lse, neg_lse));
-            pr[i] = f2_lo(x);
-            pr[i + 1] = f2_hi(x);
-          }
-          ok = wait_warp(&bias_full, gs & 1, ctx, kSiteBiasFull, mb);
-          if (!ok) break;
+        for (int c = 0; c < 8; ++c) {
+          const uint4 v = lds128(nlse_a + c * 16);
+          const f32x2 nl[2] = {f2(__uint_as_float(v.x), __uint_as_float(v.y)), f2(__uint_as_float(v.z), __uint_as_float(v.w))};
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const uint4 v = lds128(sp_row + (((chunk0 + c) ^ (r & 7)) << 4));
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float2 f = P2::unpack(w[e]);
-              const int i = c * 8 + e * 2;
-              const f32x2 a = ffma2(f2(f.x, f.y), f2(kLog2e, kLog2e), f2(pr[i], pr[i + 1]));
-              pr[i] = ex2(f2_lo(a));
-              pr[i + 1] = ex2(f2_hi(a));
+          for (int e = 0; e < 2; ++e) {
+            const int i = c * 4 + e * 2;
+            f32x2 a = ffma2(f2(pr[i], pr[i + 1]), sc2, nl[e]);
+            if constexpr (BIAS == 1) {
+              const float2 f = P2::unpack(w[i] | (w[i + 1] << 16));
+              a = ffma2(f2(f.x, f.y), f2(kLog2e, kLog2e), a);
+            } else if constexpr (BIAS == 3) {
+              a = ffma2(f2(__uint_as_float(w[i]), __uint_as_float(w[i + 1])), f2(kLog2e, kLog2e), a);
             }
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            f32x2 a = ffma2(f2(pr[i], pr[i + 1]), f2(p.scale_log2, p.scale_log2), f2(neg_lse, neg_lse));
-            if constexpr (BIAS == 3)
-              a = ffma2(f2(__uint_as_float(bf32.w[i]), __uint_as_float(bf32.w[i + 1])), f2(kLog2e, kLog2e), a);
-            float e0 = ex2(f2_lo(a)), e1 = ex2(f2_hi(a));
+            pr[i] = ex2(f2_lo(a));
+            pr[i + 1] = ex2(f2_hi(a));
             if constexpr (BIAS == 2) {
-              const uint32_t m2 = bcur.w[i >> 2] >> (8 * (i & 3));
-              e0 = (m2 & 0xFFu) != 0 ? e0 : 0.f;
-              e1 = (m2 & 0xFF00u) != 0 ? e1 : 0.f;
+              pr[i] = w[i] != 0 ? pr[i] : 0.f;
+              pr[i + 1] = w[i + 1] != 0 ? pr[i + 1] : 0.f;
             }
-            pr[i] = e0;
-            pr[i + 1] = e1;
           }
         }
-        if ((col0 + 32 > p.N) || (p.causal && col0 + 31 > m0)) {
-          int limit = p.N - col0;
-          if (p.causal) limit = min(limit, m0 + r - col0 + 1);
+        if (p.causal && nb * 128 + 127 > m0) {
+          const int hidden = n - m0;  // the first query rows do not see this key
 #pragma unroll
           for (int i = 0; i < 32; ++i)
-            if (i >= limit) pr[i] = 0.f;
+            if (i < hidden) pr[i] = 0.f;
         }
-        // dV of the previous step has read P (the first step of a tile: seen in the epilogue)
-        if (mb > i_start) {
-          ok = wait_warp(&dv_done, (gs - 1) & 1, ctx, kSiteDvDone, mb);
-          if (!ok) break;
-        }
+        {
+          uint32_t pk[16];
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
-          sts128(sp_row + (((chunk0 + c) ^ (r & 7)) << 4), P2::pack(pr[c * 8 + 0], pr[c * 8 + 1]),
-                 P2::pack(pr[c * 8 + 2], pr[c * 8 + 3]), P2::pack(pr[c * 8 + 4], pr[c * 8 + 5]),
-                 P2::pack(pr[c * 8 + 6], pr[c * 8 + 7]));
-        fence_proxy_async_smem();
+          for (int i = 0; i < 16; ++i) pk[i] = P2::pack(pr[2 * i], pr[2 * i + 1]);
+          tmem_st16(tm_sc, pk);  // over this thread's own scores
+          tmem_st_wait();
+        }
+        tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&p_ready);
 
@@ -482,68 +468,69 @@ __global__ void __launch_bounds__(640, 1) dkdv256_kernel(const __grid_constant__
         ok = wait_warp(&dp_full, gs & 1, ctx, kSiteDpFull, mb);
         if (!ok) break;
         tc_fence_after();
-        T* drow = reinterpret_cast<T*>(p.ds16) + ds_bh + (int64_t)(m0 + r) * p.ds_sM + col0;
+        uint32_t all = 0xffffffffu;
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
           uint32_t dp[16];
           tmem_ld16(tm_sc + (kColDp - kColS) + hf * 16, dp);
           tmem_ld_wait();
-          if (hf == 1) tc_fence_before();  // the next arrival on p_ready hands the dP columns back
-          uint32_t dsu[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int e = hf * 16 + 2 * i;
-            const f32x2 d = fmul2(f2(pr[e], pr[e + 1]),
-                                  fadd2(f2(__uint_as_float(dp[2 * i]), __uint_as_float(dp[2 * i + 1])),
-                                        f2(-delta_r, -delta_r)));
-            dsu[i] = P2::pack(f2_lo(d), f2_hi(d));
-            if (BIAS == 3) {
-              dp[2 * i] = __float_as_uint(f2_lo(d));
-              dp[2 * i + 1] = __float_as_uint(f2_hi(d));
+          for (int c = 0; c < 4; ++c) {
+            const uint4 v = lds128(ndelta_a + hf * 64 + c * 16);
+            const f32x2 nd[2] = {f2(__uint_as_float(v.x), __uint_as_float(v.y)), f2(__uint_as_float(v.z), __uint_as_float(v.w))};
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int k = c * 4 + e * 2, i = hf * 16 + k;
+              const f32x2 d = fmul2(f2(pr[i], pr[i + 1]),
+                                    fadd2(f2(__uint_as_float(dp[k]), __uint_as_float(dp[k + 1])), nd[e]));
+              pr[i] = f2_lo(d);
+              pr[i + 1] = f2_hi(d);
+              all &= __float_as_uint(pr[i]) & __float_as_uint(pr[i + 1]);
             }
           }
-          const int c0 = col0 + hf * 16;
-          if (row_ok && c0 < p.N) {
-            if (c0 + 16 <= p.N) {
-              store32(drow + hf * 16, dsu, p.ds_vec32 != 0);
-            } else {
-              const uint16_t* e16 = reinterpret_cast<const uint16_t*>(dsu);
+        }
+        // dP and the row statistics go back only once every lane has used them (the vote needs them all)
+        if (__all_sync(0xffffffffu, all == 0xffffffffu)) tc_fence_after();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&dp_free);
+        if (key_ok) {
+          uint16_t* drow = static_cast<uint16_t*>(p.ds16) + ds_off + static_cast<int64_t>(m0) * p.ds_sM;
+          if (rows >= 32) {
 #pragma unroll
-              for (int k = 0; k < 16; ++k)
-                if (c0 + k < p.N) reinterpret_cast<uint16_t*>(drow)[hf * 16 + k] = e16[k];
+            for (int i = 0; i < 32; i += 2) {
+              const uint32_t d2 = P2::pack(pr[i], pr[i + 1]);
+              drow[0] = static_cast<uint16_t>(d2);
+              drow[p.ds_sM] = static_cast<uint16_t>(d2 >> 16);
+              drow += 2 * p.ds_sM;
             }
-            if (BIAS == 3 && p.dbias_f32 != nullptr) {
-              // the fp32 bias gradient goes out unrounded
-              float* frow = p.dbias_f32 + b * p.dbf_sB + h * p.dbf_sH + (int64_t)(m0 + r) * p.dbf_sM + c0;
-              if (c0 + 16 <= p.N) {
+          } else {
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                  *reinterpret_cast<uint4*>(frow + 4 * k) = make_uint4(dp[4 * k], dp[4 * k + 1], dp[4 * k + 2], dp[4 * k + 3]);
-              } else {
-#pragma unroll
-                for (int k = 0; k < 16; ++k)
-                  if (c0 + k < p.N) frow[k] = __uint_as_float(dp[k]);
-              }
+            for (int i = 0; i < 32; i += 2) {
+              const uint32_t d2 = P2::pack(pr[i], pr[i + 1]);
+              if (i < rows) drow[i * p.ds_sM] = static_cast<uint16_t>(d2);
+              if (i + 1 < rows) drow[(i + 1) * p.ds_sM] = static_cast<uint16_t>(d2 >> 16);
             }
+          }
+          if (BIAS == 3 && p.dbias_f32 != nullptr) {
+            // the fp32 bias gradient goes out unrounded
+            float* frow = p.dbias_f32 + dbf_off + static_cast<int64_t>(m0) * p.dbf_sM;
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (i < rows) frow[i * p.dbf_sM] = pr[i];
           }
         }
       }
       if (!ok) break;
 
-      // the next tile's first rows travel while this tile's result is stored
-      {
-        int bh2, nb2, is2;
-        if (tile_at(it + 1, bh2, nb2, is2) && is2 < n_mblk) prefetch(bh2, nb2 * 128 + qt * 32, is2);
-      }
-
       // ---- epilogue: dV (rows = keys) -> global, 64 head-dim columns per thread
       const bool any = i_start < n_mblk;
       if (any) {
-        ok = wait_warp(&dv_done, (gs - 1) & 1, ctx, kSiteEpilogue, 0);
+        ok = wait_warp(&acc_done, tiles & 1, ctx, kSiteAccDone, it);
         if (!ok) break;
+        ++tiles;
       }
       tc_fence_after();
-      const int n = nb * 128 + r;
       T* row = reinterpret_cast<T*>(p.dv) + b * p.dv_sB + (int64_t)n * p.dv_sN + h * p.dv_sH + qt * 64;
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
@@ -555,7 +542,7 @@ __global__ void __launch_bounds__(640, 1) dkdv256_kernel(const __grid_constant__
 #pragma unroll
           for (int i = 0; i < 32; ++i) a[i] = 0;  // keys no query row sees
         }
-        if (n < p.N) {
+        if (key_ok) {
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             const uint4 lo = pack8<P2>(a + c * 16, 1.f), hi = pack8<P2>(a + c * 16 + 8, 1.f);
@@ -664,13 +651,9 @@ int launch_bwd_dkdv_d256(const fa_params& p, cudaStream_t stream, int* status, c
                        &kp.bias_h_mul);
     if (r) return r;
   }
-  kp.bias_vec32 = p.bias_kind != FA_BIAS_NONE && reinterpret_cast<uintptr_t>(p.bias) % 32 == 0 &&
-                  (p.bias_stride[0] * eb) % 32 == 0 && (p.bias_stride[1] * eb) % 32 == 0 &&
-                  (p.bias_stride[2] * eb) % 32 == 0;
   auto al32 = [](const void* ptr, const int64_t s[3]) {
     return reinterpret_cast<uintptr_t>(ptr) % 32 == 0 && s[0] % 16 == 0 && s[1] % 16 == 0 && s[2] % 16 == 0;
   };
-  kp.ds_vec32 = al32(ds, ds_stride);
   kp.dv_vec32 = al32(p.dv, p.dv_stride);
   kp.bias = p.bias;
   kp.dv = p.dv;
