@@ -225,3 +225,21 @@ def test_backward_through_slabs_of_any_size(D, M, N, causal, bias_kind, device_o
         assert torch.equal(dq, results[1][0]), room
         ref = results[0][0].float()
         assert bool(((dq.float() - ref).abs() <= 2.0 ** -7 * ref.abs() + flips + 1e-6).all()), room
+
+
+@pytest.mark.parametrize("which", ["q", "v", "bias", "qkv"])
+def test_forward_mode_is_refused(which, device_ok):
+    """No forward-mode rule exists: a dual tensor raises instead of losing its tangent."""
+    import torch.autograd.forward_ad as fwad
+    from triton_flashattn_b200 import flash_attention_fn, flash_attention_qkvpacked_fn
+
+    x = {n: torch.randn(1, 64, 2, 64, dtype=torch.float16, device="cuda") for n in ("q", "k", "v")}
+    x["bias"] = torch.randn(1, 2, 64, 64, dtype=torch.float16, device="cuda")
+    qkv = torch.stack([x["q"], x["k"], x["v"]], dim=2)
+    with fwad.dual_level(), pytest.raises(NotImplementedError, match="jvp"):
+        if which == "qkv":
+            flash_attention_qkvpacked_fn(fwad.make_dual(qkv, torch.ones_like(qkv)))
+        else:
+            x[which] = fwad.make_dual(x[which], torch.ones_like(x[which]))
+            flash_attention_fn(x["q"], x["k"], x["v"], x["bias"])
+    assert flash_attention_fn(x["q"], x["k"], x["v"]).shape == (1, 64, 2, 64)  # outside the level: as ever

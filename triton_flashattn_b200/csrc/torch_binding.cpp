@@ -419,6 +419,10 @@ Tensor attention(const Tensor& a, const Tensor& k, const Tensor& v, const Tensor
   const bool packed = !k.defined();
   const bool train_bias = bias.defined() && bias.requires_grad();
   if (train_bias && bias.scalar_type() == at::kBool) fail(PyExc_TypeError, "a bool mask cannot require grad");
+  // The node has no forward-mode rule; without this the tangents would be dropped silently.
+  for (const Tensor* t : {&a, &k, &v, &bias})
+    if (t->defined() && t->_fw_grad(0).defined())
+      fail(PyExc_NotImplementedError, "attention has no forward-mode derivative (jvp)");
   const Shape s = packed ? check_packed(a, bias) : check_inputs(a, k, v, bias);
   const double scale = scale_of(scale_obj, s.D);
   require_health_words(s.device);
