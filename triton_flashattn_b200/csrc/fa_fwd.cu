@@ -296,6 +296,11 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
     // (the whole warp walks the loop converged, one elected lane issues)
     if (live) {
       const int t = warp == 9 ? 0 : 1;
+      // A look at a barrier takes about 280 cycles.  Without a bias the issuer is on the critical path, so it
+      // looks at the loads, which have landed by then as a rule, while the row threads still form P or
+      // read S (causal B2 H32 S4096 D128: 342 -> 328 us).  With a bias the row threads are behind anyway,
+      // and a late load would hold up what could be issued: 16-bit bias, D = 64, 44 us against 47.
+      constexpr bool kLoadsFirst = BIAS == 0 || BIAS == 2;
       constexpr bool bf = P2::kIsBf16;
       constexpr uint32_t idesc_qk = make_idesc(bf, false, false, 128, 64);
       constexpr uint32_t idesc_pv = make_idesc(bf, false, true, 128, DP);
@@ -342,8 +347,9 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
             const uint32_t gh = gv + 2 * j + h;
             const uint32_t vs = gh % VS, v_par = (gh / VS) & 1;
             if (mine) {
-              ok = wait_warp_hot(&p_full[t][h], cs & 1, ctx, kSitePFull, j);
-              if (ok) ok = wait_warp(&v_full[vs], v_par, ctx, kSiteVFull, j);
+              if (kLoadsFirst) ok = wait_warp(&v_full[vs], v_par, ctx, kSiteVFull, j);
+              if (ok) ok = wait_warp_hot(&p_full[t][h], cs & 1, ctx, kSitePFull, j);
+              if (ok && !kLoadsFirst) ok = wait_warp(&v_full[vs], v_par, ctx, kSiteVFull, j);
               if (!ok) break;
               tc_fence_after();
               if (elect_one()) {
@@ -363,8 +369,9 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
               // Keys 0-63 of block j+1 go into the column half whose scores (keys 64-127 of
               // block j) the row threads have just taken into registers: this product runs
               // under the second half of this step's softmax.
-              if (mine) ok = wait_warp_hot(&s_read[t], cs & 1, ctx, kSiteSRead, j);
-              if (ok && more) ok = wait_warp(&k_full[kn], kn_par, ctx, kSiteKFull, j + 1);
+              if (kLoadsFirst && more) ok = wait_warp(&k_full[kn], kn_par, ctx, kSiteKFull, j + 1);
+              if (ok && mine) ok = wait_warp_hot(&s_read[t], cs & 1, ctx, kSiteSRead, j);
+              if (ok && !kLoadsFirst && more) ok = wait_warp(&k_full[kn], kn_par, ctx, kSiteKFull, j + 1);
               if (!ok) break;
               if (mine_next) {
                 tc_fence_after();
