@@ -14,7 +14,7 @@
 // The S and dP columns are handed back to the MMA issuer as soon as they sit in
 // registers, so the next block's products run while the row threads compute.
 //
-// (2) dq_from_ds_kernel -- used when the dK/dV kernel has just written dS as 16-bit
+// (2) from_ds_kernel -- used when the dK/dV kernel has just written dS as 16-bit
 // values, either as dbias or into scratch slabs: dQ = sm_scale * dS . K is then a plain
 // streamed GEMM whose A operand is loaded by TMA from that tensor
 // (64-key stages, two CTAs per SM).  The reference itself rounds dS to the
