@@ -124,6 +124,32 @@ def test_few_query_rows(M, N, D, dtype, bias_kind, causal, device_ok):
             verbose=False)
 
 
+@pytest.mark.parametrize("M", [1, 16, 17])
+@pytest.mark.parametrize("where", ["q", "key", "bias", "inf bias"])
+def test_nan_scores_reach_the_output(M, where, device_ok):
+    """A NaN score (or an infinite one: inf - inf) makes its row NaN, by the kernel for few rows (M <= 16) as by
+    the tile kernel, and no other row or head; the log-sum-exp of such a row is +inf."""
+    from triton_flashattn_b200 import flash_attention as fa
+
+    q, k, v, bias, _ = make_inputs(1, M, 300, 2, 128, BF, "float", 23)
+    clean, lse = fa._flash_attn_fwd(q, k, v, bias, False, 0.1)
+    rows = slice(0, M) if where == "key" else slice(0, 1)
+    if where == "q":
+        q[0, 0, 0, 3] = float("nan")
+    elif where == "key":
+        k[0, 200, 0, 3] = float("nan")
+    else:
+        bias[0, 0, 0, 5] = float("nan" if where == "bias" else "inf")
+    out, lse_nan = fa._flash_attn_fwd(q, k, v, bias, False, 0.1)
+    assert out[0, rows, 0].isnan().all() and lse_nan[0, 0, rows].isposinf().all()
+    assert torch.equal(out[:, :, 1], clean[:, :, 1]) and torch.equal(lse_nan[:, 1], lse[:, 1])
+    if where != "key":
+        # the head's other rows: P may be rounded against another running maximum (2^-9 of each probability, twice)
+        bound = 2.0 ** -8 * (v[0, :, 0].float().abs().max() + clean[0, 1:, 0].float().abs())
+        assert bool(((out[0, 1:, 0].float() - clean[0, 1:, 0].float()).abs() <= bound).all())
+        assert torch.allclose(lse_nan[0, 0, 1:], lse[0, 0, 1:], rtol=0, atol=1e-4)
+
+
 @pytest.mark.parametrize("D", [16, 32])
 @pytest.mark.parametrize("bias_kind", [None, "float"])
 def test_small_head_dims(D, bias_kind, device_ok):

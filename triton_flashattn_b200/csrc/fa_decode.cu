@@ -300,10 +300,11 @@ __global__ void __launch_bounds__(W * 32) decode_kernel(const DecodeParams p) {
       acc += f * (parts > 1 ? *cluster.map_shared_rank(&c_o[m][d], c) : c_o[m][d]);
       sum += f * (parts > 1 ? *cluster.map_shared_rank(&c_l[m], c) : c_l[m]);
     }
-    // a row whose keys are all masked out: output 0, log-sum-exp +inf
+    // A row whose keys are all masked out: output 0, log-sum-exp +inf.  A NaN sum ends here too, and the product
+    // with zero lets the NaN of its accumulators through (the tile kernel does the same).
     const bool any_key = m_all != -INFINITY && sum > 0.f;
     if (d < p.D)
-      (static_cast<T*>(p.o) + b * p.o_sB + m * p.o_sM + h * p.o_sH)[d] = static_cast<T>(any_key ? acc / sum : 0.f);
+      (static_cast<T*>(p.o) + b * p.o_sB + m * p.o_sM + h * p.o_sH)[d] = static_cast<T>(any_key ? acc / sum : acc * 0.f);
     if (d == 0) p.lse[static_cast<int64_t>(bh) * p.M + m] = any_key ? m_all + log2f(sum) : INFINITY;
   }
   if (parts > 1) cluster.sync();  // no CTA leaves while another still reads its shared memory
