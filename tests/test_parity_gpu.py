@@ -150,6 +150,21 @@ def test_nan_scores_reach_the_output(M, where, device_ok):
         assert torch.allclose(lse_nan[0, 0, 1:], lse[0, 0, 1:], rtol=0, atol=1e-4)
 
 
+@pytest.mark.parametrize("M", [1, 16, 17])
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+def test_masked_key_with_a_bad_score_takes_no_part(M, bad, device_ok):
+    """Keys that the mask hides may hold anything (an unwritten cache slot): their scores are ignored.  (Their
+    values may not: 0 * inf in the product with V.)"""
+    from triton_flashattn_b200 import flash_attention_fn
+
+    q, k, v, mask, _ = make_inputs(1, M, 300, 2, 128, BF, "bool", 24)
+    mask[..., 200] = False
+    k[0, 200, :, 3] = 0
+    clean = flash_attention_fn(q, k, v, mask)
+    k[0, 200, :, 3] = bad
+    assert torch.equal(flash_attention_fn(q, k, v, mask), clean)
+
+
 @pytest.mark.parametrize("D", [16, 32])
 @pytest.mark.parametrize("bias_kind", [None, "float"])
 def test_small_head_dims(D, bias_kind, device_ok):

@@ -83,10 +83,11 @@ __device__ __forceinline__ uint32_t transpose8x8(uint32_t x) {
   return y;
 }
 
+// The bias of one score; a mask as 1 (seen) or 0.
 template <int BIAS, typename T>
 __device__ __forceinline__ float load_bias(const DecodeParams& p, int64_t off) {
   if constexpr (BIAS == 1) return static_cast<float>(static_cast<const T*>(p.bias)[off]);
-  if constexpr (BIAS == 2) return static_cast<const uint8_t*>(p.bias)[off] ? 0.f : -INFINITY;
+  if constexpr (BIAS == 2) return static_cast<const uint8_t*>(p.bias)[off] ? 1.f : 0.f;
   if constexpr (BIAS == 3) return static_cast<const float*>(p.bias)[off];
   return 0.f;
 }
@@ -200,7 +201,9 @@ __global__ void __launch_bounds__(W * 32) decode_kernel(const DecodeParams p) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         float x = s[n][i] * p.sm_scale;
-        if (BIAS != 0) x += bf[n][i];
+        // a mask selects: whatever the score of a masked key is (infinite, NaN), it takes no part
+        if (BIAS == 2) x = bf[n][i] != 0.f ? x : -INFINITY;
+        else if (BIAS != 0) x += bf[n][i];
         const int key = tile * 16 + r + 8 * (i >> 1);
         if (key >= p.n_keys || (p.causal && key > n * 8 + 2 * t + (i & 1))) x = -INFINITY;
         s[n][i] = x * kLog2e;
