@@ -124,6 +124,30 @@ def test_few_query_rows(M, N, D, dtype, bias_kind, causal, device_ok):
             verbose=False)
 
 
+@pytest.mark.parametrize("M", [1, 4, 16, 17])
+@pytest.mark.parametrize("bias_dtype", [torch.float64, HF, torch.float32])
+@pytest.mark.parametrize("trainable,packed", [(True, False), (False, False), (True, True), (False, True)])
+def test_few_rows_train_with_a_bias_of_another_dtype(M, bias_dtype, trainable, packed, device_ok):
+    """The kernel for few rows reads a converted bias with any row pitch, the backward's do not.  (Packed: M keys.)"""
+    from triton_flashattn_b200 import flash_attention_qkvpacked_fn
+
+    N = M if packed else 77
+    q, k, v, bias, do = make_inputs(2, M, N, 3, 64, BF, "float", 25)
+    bias = bias.to(bias_dtype)
+    if packed:
+        qkv = torch.stack([q, k, v], dim=2).requires_grad_()
+        b = bias.clone().requires_grad_(trainable)
+        out = flash_attention_qkvpacked_fn(qkv, b)
+        out.backward(do)
+        ours = {"out": out.detach(), "dq": qkv.grad[:, :, 0], "dk": qkv.grad[:, :, 1], "dv": qkv.grad[:, :, 2]}
+        if trainable:
+            ours["dbias"] = b.grad
+    else:
+        ours = run_ours(q, k, v, bias, False, None, do, trainable)
+    assert not trainable or ours["dbias"].dtype == bias_dtype
+    compare(ours, q, k, v, bias, False, None, do, BF, label=f"M{M} {bias_dtype}: ", verbose=False)
+
+
 @pytest.mark.parametrize("M", [1, 16, 17])
 @pytest.mark.parametrize("where", ["q", "key", "bias", "inf bias"])
 def test_nan_scores_reach_the_output(M, where, device_ok):

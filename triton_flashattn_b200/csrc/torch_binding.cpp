@@ -120,18 +120,23 @@ Tensor pitched_empty(const Tensor& like, at::IntArrayRef size, at::ScalarType dt
   return n_pad == size[3] ? buf : buf.narrow(3, 0, size[3]);
 }
 
+// What the tile kernels need of a bias: unit inner stride, 16-byte aligned pitches and address.
+bool bias_ok(const Tensor& bias) {
+  const int64_t eb = static_cast<int64_t>(bias.element_size());
+  const auto st = bias.strides();
+  return st[3] == 1 && st[2] > 0 && (st[0] * eb) % 16 == 0 && (st[1] * eb) % 16 == 0 && (st[2] * eb) % 16 == 0 &&
+         reinterpret_cast<uintptr_t>(bias.const_data_ptr()) % 16 == 0;
+}
+
 // Bias / mask with unit inner stride and 16-byte aligned pitches.  Expanded views (stride 0 over B
 // or H) pass through untouched.  Otherwise a copy is made, with its rows padded to 32 bytes (the
 // kernels then fetch whole sectors) and its expanded B and H dimensions kept folded: a key-padding
 // mask (B, 1, 1, N) expanded over heads and rows is written once per batch element, not per head.
 Tensor bias_ready(const Tensor& bias) {
-  const int64_t eb = static_cast<int64_t>(bias.element_size());
+  if (bias_ok(bias)) return bias;
   const auto st = bias.strides();
   const auto sz = bias.sizes();
-  if (st[3] == 1 && st[2] > 0 && (st[0] * eb) % 16 == 0 && (st[1] * eb) % 16 == 0 && (st[2] * eb) % 16 == 0 &&
-      reinterpret_cast<uintptr_t>(bias.const_data_ptr()) % 16 == 0)
-    return bias;
-  const int64_t align = 32 / eb;
+  const int64_t align = 32 / static_cast<int64_t>(bias.element_size());
   const int64_t n_pad = (sz[3] + align - 1) / align * align;
   const int64_t b = st[0] == 0 ? 1 : sz[0], h = st[1] == 0 ? 1 : sz[1];
   Tensor out = empty_on(bias, {b, h, sz[2], n_pad}, bias.scalar_type()).narrow(3, 0, sz[3]);
@@ -462,7 +467,8 @@ Tensor attention(const Tensor& a, const Tensor& k, const Tensor& v, const Tensor
   }
   if (bias.defined()) {
     node->bias_ = SavedVariable(bias, false);
-    if (!b.t.is_same(bias) && static_cast<int64_t>(b.t.storage().nbytes()) <= kKeepBiasCopyBytes)
+    // (a converted bias that only the kernel for few rows can read is made again for the backward)
+    if (!b.t.is_same(bias) && bias_ok(b.t) && static_cast<int64_t>(b.t.storage().nbytes()) <= kKeepBiasCopyBytes)
       node->bias_copy_ = std::move(b.t);
   }
   node->lse_ = SavedVariable(lse, false);
