@@ -243,3 +243,28 @@ def test_forward_mode_is_refused(which, device_ok):
             x[which] = fwad.make_dual(x[which], torch.ones_like(x[which]))
             flash_attention_fn(x["q"], x["k"], x["v"], x["bias"])
     assert flash_attention_fn(x["q"], x["k"], x["v"]).shape == (1, 64, 2, 64)  # outside the level: as ever
+
+
+@pytest.mark.parametrize("use", ["offload", "checkpoint"])
+def test_nothing_bypasses_saved_tensor_hooks(use, device_ok):
+    """A padding mask over 777 keys is copied into padded rows for the kernels; with hooks that take the saved
+    tensors away, or under checkpointing, no such copy stays on the device between forward and backward."""
+    from torch.utils.checkpoint import checkpoint
+    from triton_flashattn_b200 import flash_attention_fn
+
+    q, k, v, _, do = make_inputs(2, 1000, 777, 4, 64, BF, None, 61)
+    lens = torch.tensor([[500], [700]], device="cuda")
+    mask = (torch.arange(777, device="cuda")[None] < lens)[:, None, None].expand(2, 4, 1000, 777)
+    inputs = [t.requires_grad_() for t in (q, k, v)]
+    want = torch.autograd.grad(flash_attention_fn(*inputs, mask), inputs, do)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    if use == "offload":
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t.cpu(), lambda t: t.cuda()):
+            out = flash_attention_fn(*inputs, mask)
+    else:
+        out = checkpoint(lambda *a: flash_attention_fn(*a), *inputs, mask, use_reentrant=False)
+    assert torch.cuda.memory_allocated() - before == out.numel() * 2
+    got = torch.autograd.grad(out, inputs, do)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)

@@ -9,6 +9,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/SavedTensorHooks.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -348,7 +349,8 @@ Tensor finish_dbias(const Tensor& dbias, at::ScalarType dtype) {
 
 // ---------------------------------------------------------------------------- autograd
 // A copy of the bias that the forward had to make is kept for the backward up to this size; a larger
-// one is made again there, so that many layers do not hold two copies of a big bias each.
+// one is made again there, so that many layers do not hold two copies of a big bias each.  Under
+// saved-tensor hooks (checkpointing, offloading) none is kept: what the hooks see is all that stays.
 constexpr int64_t kKeepBiasCopyBytes = 64ll << 20;
 
 // Backward node of one attention call: inputs (q, k, v, bias), or (qkv, bias) when packed.
@@ -468,7 +470,8 @@ Tensor attention(const Tensor& a, const Tensor& k, const Tensor& v, const Tensor
   if (bias.defined()) {
     node->bias_ = SavedVariable(bias, false);
     // (a converted bias that only the kernel for few rows can read is made again for the backward)
-    if (!b.t.is_same(bias) && bias_ok(b.t) && static_cast<int64_t>(b.t.storage().nbytes()) <= kKeepBiasCopyBytes)
+    if (!b.t.is_same(bias) && bias_ok(b.t) && static_cast<int64_t>(b.t.storage().nbytes()) <= kKeepBiasCopyBytes &&
+        !at::SavedTensorDefaultHooks::get_hooks().has_value())
       node->bias_copy_ = std::move(b.t);
   }
   node->lse_ = SavedVariable(lse, false);
