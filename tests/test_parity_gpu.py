@@ -124,6 +124,30 @@ def test_few_query_rows(M, N, D, dtype, bias_kind, causal, device_ok):
             verbose=False)
 
 
+@pytest.mark.parametrize("S", [4, 100])
+@pytest.mark.parametrize("layout", ["one element off", "padded head dim", "heads first"])
+def test_packed_qkv_in_other_layouts(S, layout, device_ok):
+    """Packed projections whose slices the kernels cannot read in place are copied: same results, gradients too."""
+    from triton_flashattn_b200 import flash_attention_qkvpacked_fn
+
+    x = torch.randn(2, S, 3, 2, 64, generator=torch.Generator().manual_seed(26)).to(BF).cuda()
+    do = torch.randn(2, S, 2, 64, generator=torch.Generator().manual_seed(27)).to(BF).cuda()
+    if layout == "one element off":
+        y = torch.empty(x.numel() + 1, dtype=BF, device="cuda")[1:].view(x.shape)
+        y.copy_(x)
+    elif layout == "padded head dim":
+        y = torch.nn.functional.pad(x, (0, 3))[..., :64]
+    else:
+        y = x.permute(0, 3, 1, 2, 4).contiguous().permute(0, 2, 3, 1, 4)
+    res = []
+    for t in (x, y):
+        t = t.detach().requires_grad_()
+        out = flash_attention_qkvpacked_fn(t, None, True)
+        res.append((out, *torch.autograd.grad(out, t, do)))
+    for a, b in zip(*res):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("M", [1, 4, 16, 17])
 @pytest.mark.parametrize("bias_dtype", [torch.float64, HF, torch.float32])
 @pytest.mark.parametrize("trainable,packed", [(True, False), (False, False), (True, True), (False, True)])

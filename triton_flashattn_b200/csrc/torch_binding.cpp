@@ -226,10 +226,12 @@ Shape check_packed(const Tensor& qkv, const Tensor& bias) {
   return s;
 }
 
-// qkv such that its three slices are tile ready
+// qkv such that its three slices are tile ready.  (A copy and not contiguous(): a dense tensor may lie at an address
+// that is no multiple of 16 bytes.)
 Tensor packed_ready(const Tensor& qkv) {
   const auto st = qkv.strides();
-  return strides_ok(st[0], st[1], st[3], st[4], qkv.const_data_ptr()) && st[2] % 8 == 0 ? qkv : qkv.contiguous();
+  if (strides_ok(st[0], st[1], st[3], st[4], qkv.const_data_ptr()) && st[2] % 8 == 0) return qkv;
+  return qkv.clone(at::MemoryFormat::Contiguous);
 }
 
 // ---------------------------------------------------------------------------- C ABI calls
