@@ -268,3 +268,26 @@ def test_nothing_bypasses_saved_tensor_hooks(use, device_ok):
     got = torch.autograd.grad(out, inputs, do)
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("packed", [False, True])
+def test_no_upstream_gradient_counts_as_zeros(packed, device_ok):
+    """A function behind the attention that returns None for its gradient: every input gets zeros, not None."""
+    from triton_flashattn_b200 import flash_attention_fn, flash_attention_qkvpacked_fn
+
+    class Stop(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, x):
+            return x.clone()
+
+        @staticmethod
+        def backward(ctx, grad):
+            return None
+
+    q, k, v, bias, _ = make_inputs(2, 96, 96, 2, 64, BF, "float", 62)
+    inputs = [torch.stack([q, k, v], dim=2), bias] if packed else [q, k, v, bias]
+    for t in inputs:
+        t.requires_grad_()
+    Stop.apply((flash_attention_qkvpacked_fn if packed else flash_attention_fn)(*inputs)).sum().backward()
+    for t in inputs:
+        assert t.grad is not None and t.grad.shape == t.shape and not t.grad.any()

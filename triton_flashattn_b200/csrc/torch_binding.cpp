@@ -378,10 +378,11 @@ struct AttentionBackward : public torch::autograd::Node {
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
     variable_list res(packed_ ? 2 : 4);
-    if (!grads[0].defined()) return res;
     const Tensor a0 = a_.unpack(), out = out_.unpack(shared_from_this()), lse = lse_.unpack();
     const Tensor bias = has_bias_ ? bias_.unpack() : Tensor();
     at::AutoDispatchBelowADInplaceOrView guard;
+    // an upstream function that returned no gradient counts as zeros, as for a Python autograd function
+    const Tensor grad = grads[0].defined() ? grads[0] : at::zeros_like(out);
     const auto bias_for = [&](at::ScalarType dt) {
       return bias_copy_.defined() ? Bias{bias_copy_, bias.scalar_type() == at::kBool ? FA_BIAS_BOOL
                                                      : bias.scalar_type() == dt      ? FA_BIAS_SAME
@@ -394,7 +395,7 @@ struct AttentionBackward : public torch::autograd::Node {
       const Tensor qkv = packed_ready(a0);
       Tensor dqkv = empty_on(qkv, qkv.sizes(), s.dtype);
       Tensor dbias = train_bias_ ? new_dbias(s, bias, causal_) : Tensor();
-      backward(s, grads[0], slice_of(qkv, 0), slice_of(qkv, 1), slice_of(qkv, 2), out, lse, bias_for(s.dtype), causal_,
+      backward(s, grad, slice_of(qkv, 0), slice_of(qkv, 1), slice_of(qkv, 2), out, lse, bias_for(s.dtype), causal_,
                scale_, slice_of(dqkv, 0), slice_of(dqkv, 1), slice_of(dqkv, 2), dbias);
       res[0] = std::move(dqkv);
       if (train_bias_) res[1] = finish_dbias(dbias, bias.scalar_type());
@@ -406,7 +407,7 @@ struct AttentionBackward : public torch::autograd::Node {
     const Tensor q = tile_ready(a0), k = tile_ready(k0), v = tile_ready(v0);
     Tensor dq = grad_like(a0), dk = grad_like(k0), dv = grad_like(v0);
     Tensor dbias = train_bias_ ? new_dbias(s, bias, causal_) : Tensor();
-    backward(s, grads[0], view_of(q), view_of(k), view_of(v), out, lse, bias_for(s.dtype), causal_, scale_, view_of(dq),
+    backward(s, grad, view_of(q), view_of(k), view_of(v), out, lse, bias_for(s.dtype), causal_, scale_, view_of(dq),
              view_of(dk), view_of(dv), dbias);
     res[0] = std::move(dq);
     res[1] = std::move(dk);
