@@ -93,3 +93,29 @@ def test_public_api_rejects_cpu_tensors_loudly():
     q = torch.randn(1, 16, 1, 16, dtype=torch.float16)
     with pytest.raises(ValueError, match="no CPU path"):
         flash_attention_fn(q, q, q)
+
+
+@pytest.mark.parametrize("transform", ["vmap", "grad", "jvp", "captured"])
+@pytest.mark.parametrize("packed", [False, True])
+def test_func_transforms_are_refused(transform, packed):
+    """There are no rules for torch.func transforms: any call under one raises, also one whose tensors are only
+    captured by the transformed function, whatever their device."""
+    import torch
+    from triton_flashattn_b200 import flash_attention_fn, flash_attention_qkvpacked_fn
+
+    x = torch.zeros(2, 4, 3, 1, 16) if packed else torch.zeros(2, 4, 1, 16)
+
+    def f(t):
+        return flash_attention_qkvpacked_fn(t) if packed else flash_attention_fn(t, t, t)
+
+    with pytest.raises(RuntimeError, match="functorch transforms"):
+        if transform == "vmap":
+            torch.func.vmap(f)(x)
+        elif transform == "grad":
+            torch.func.grad(lambda t: f(t).sum())(x)
+        elif transform == "jvp":
+            torch.func.jvp(f, (x,), (x,))
+        else:
+            torch.func.vmap(lambda s: f(x) * s)(torch.ones(3))
+    with pytest.raises((ValueError, TypeError)):  # outside the transform: the ordinary complaint
+        f(x)

@@ -9,6 +9,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/FuncTorchTLS.h>
 #include <ATen/SavedTensorHooks.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -426,6 +427,9 @@ double scale_of(PyObject* obj, int64_t D) {
 
 // One attention call with its graph node when a gradient is wanted.  `k`, `v` undefined: packed.
 Tensor attention(const Tensor& a, const Tensor& k, const Tensor& v, const Tensor& bias, bool causal, PyObject* scale_obj) {
+  // No rule for torch.func transforms exists either (RuntimeError): under one, what looks like a plain tensor may be
+  // a batch or a differentiation level of its own.
+  if (const auto& transforms = at::functorch::functorchTLSAccessor()) transforms->checkSupportsCppAutogradFunction();
   const bool packed = !k.defined();
   const bool train_bias = bias.defined() && bias.requires_grad();
   if (train_bias && bias.scalar_type() == at::kBool) fail(PyExc_TypeError, "a bool mask cannot require grad");
