@@ -291,3 +291,17 @@ def test_no_upstream_gradient_counts_as_zeros(packed, device_ok):
     Stop.apply((flash_attention_qkvpacked_fn if packed else flash_attention_fn)(*inputs)).sum().backward()
     for t in inputs:
         assert t.grad is not None and t.grad.shape == t.shape and not t.grad.any()
+
+
+@pytest.mark.parametrize("kind", ["float", "0-d tensor", "tensor on the device", "text"])
+def test_scale_is_whatever_float_takes(kind, device_ok):
+    from triton_flashattn_b200 import flash_attention_fn
+
+    q, k, v, _, _ = make_inputs(1, 40, 40, 2, 64, BF, None, 63)
+    scale = {"float": 0.25, "0-d tensor": torch.tensor(0.25), "tensor on the device": torch.tensor(0.25, device="cuda"),
+             "text": "0.25"}[kind]
+    assert torch.equal(flash_attention_fn(q, k, v, None, False, scale), flash_attention_fn(q, k, v, None, False, 0.25))
+    with pytest.raises(TypeError):
+        flash_attention_fn(q, k, v, None, False, [0.25])
+    with pytest.raises(ValueError):
+        flash_attention_fn(q, k, v, None, False, "a quarter")

@@ -420,9 +420,9 @@ struct AttentionBackward : public torch::autograd::Node {
 
 double scale_of(PyObject* obj, int64_t D) {
   if (obj == Py_None) return 1.0 / std::sqrt(static_cast<double>(D));
-  const double v = PyFloat_AsDouble(obj);
-  if (v == -1.0 && PyErr_Occurred()) throw python_error();
-  return v;
+  THPObjectPtr number(PyNumber_Float(obj));  // whatever float() takes
+  if (!number) throw python_error();
+  return PyFloat_AsDouble(number.get());
 }
 
 // One attention call with its graph node when a gradient is wanted.  `k`, `v` undefined: packed.
