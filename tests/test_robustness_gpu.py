@@ -305,3 +305,31 @@ def test_scale_is_whatever_float_takes(kind, device_ok):
         flash_attention_fn(q, k, v, None, False, [0.25])
     with pytest.raises(ValueError):
         flash_attention_fn(q, k, v, None, False, "a quarter")
+
+
+@pytest.mark.parametrize("M", [1, 16, 17])
+def test_zero_strides_are_refused_by_every_kernel(M, device_ok):
+    """A stride of zero over B, S or H of q, k, v (or do) is an alignment error, whichever kernel a call goes to.
+    (All strides stay inside the tensors: a refusal that failed to come would read in bounds.)"""
+    from triton_flashattn_b200 import _cabi
+    from triton_flashattn_b200 import flash_attention as fa
+
+    lib = _cabi.load()
+    B, N, H, D = 2, 64, 2, 64
+    q, k, v, bias, do = make_inputs(B, M, N, H, D, BF, "float", 64)
+    o, lse = fa._flash_attn_fwd(q, k, v, bias, False, 0.1)
+    dq, dk, dv = (torch.empty_like(t) for t in (q, k, v))
+    dbias, delta = torch.zeros_like(bias), torch.empty_like(lse)
+    for which in ("q", "k", "v", "do"):
+        for i in range(3):
+            p, keep = _bwd_params(fa, q, k, v, o, lse, bias, False, 0.1, do, dq, dk, dv, dbias, delta)
+            st = list(getattr(p, which + "_stride"))
+            st[i] = 0
+            setattr(p, which + "_stride", _cabi._I64x3(*st))
+            if which != "do":
+                assert lib.fa_fwd(ctypes.byref(p), None) == 5, (which, i)  # FA_ERR_ALIGN
+            assert lib.fa_bwd_dkdv(ctypes.byref(p), None) == 5, (which, i)
+            assert lib.fa_bwd_dq(ctypes.byref(p), None) == 5, (which, i)
+    p, keep = _bwd_params(fa, q, k, v, o, lse, bias, False, 0.1, do, dq, dk, dv, dbias, delta)
+    assert lib.fa_fwd(ctypes.byref(p), None) == 0 and lib.fa_bwd(ctypes.byref(p), None) == 0
+    torch.cuda.synchronize()

@@ -629,7 +629,7 @@ int launch_from_ds(const fa_params& p, cudaStream_t stream, int* status, const D
     return reinterpret_cast<uintptr_t>(ptr) % 16 != 0 || s[0] % 8 || s[1] % 8 || s[2] % 8;
   };
   // q, v and do are asked of every backward call, whether this stage reads them or not
-  if (bad(p.q, p.q_stride) || bad(p.v, p.v_stride) || bad(p.d_o, p.do_stride)) return FA_ERR_ALIGN;
+  if (!operand_ok(p.q, p.q_stride) || !operand_ok(p.v, p.v_stride) || !operand_ok(p.d_o, p.do_stride)) return FA_ERR_ALIGN;
   const int64_t* out_stride = keys ? p.dk_stride : p.dq_stride;
   kp.out = keys ? p.dk : p.dq;
   if (bad(kp.out, out_stride)) return FA_ERR_ALIGN;

@@ -414,7 +414,8 @@ int launch_decode(const fa_params& p, cudaStream_t stream, int* status) {
   auto bad = [](const void* ptr, const int64_t s[3]) {
     return reinterpret_cast<uintptr_t>(ptr) % 16 != 0 || s[0] % 8 || s[1] % 8 || s[2] % 8;
   };
-  if (bad(p.q, p.q_stride) || bad(p.k, p.k_stride) || bad(p.v, p.v_stride) || bad(p.o, p.o_stride)) return FA_ERR_ALIGN;
+  if (!operand_ok(p.q, p.q_stride) || !operand_ok(p.k, p.k_stride) || !operand_ok(p.v, p.v_stride) || bad(p.o, p.o_stride))
+    return FA_ERR_ALIGN;
   DecodeParams d;
   d.q = p.q;
   d.k = p.k;

@@ -94,6 +94,12 @@ inline int make_tmap_slab(CUtensorMap* out, const DsSlab& slab, int M, int N, in
   return make_tmap_4d(out, slab.base, 2, dims, sb, box);
 }
 
+// What every entry point asks of a (B, S, H, D) operand, whether its kernel reads it through a tile map (whose
+// encoding refuses the rest) or with plain loads: 16-byte aligned base and strides, no stride of zero or less.
+inline bool operand_ok(const void* ptr, const int64_t s[3]) {
+  return reinterpret_cast<uintptr_t>(ptr) % 16 == 0 && s[0] > 0 && s[1] > 0 && s[2] > 0 && (s[0] | s[1] | s[2]) % 8 == 0;
+}
+
 // Head dims are computed on a padded width: 16/32/64 -> 64, 128 -> 128, 256 -> 256.
 inline int padded_head_dim(int d) { return d <= 64 ? 64 : d; }
 
