@@ -575,11 +575,14 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
             // every lane and so every value read from them.  (Right after the reads is too early: the
             // arrival may then take effect while reads of the warp are still under way, and the next
             // bulk load overwrote rows before they were read about once in ten full-size passes.)
+            // The vote's result picks the arriving lane, so that no schedule can put the arrival first
+            // (B16 S512 H12 D64 fp16 bias: 40.1 -> 40.8 us; the arrival behind the rescaling branch: 42.1).
+            const int handing_back = any_need ? 1 : 0;
             if (BIAS == 1 || (BIAS == 2 && h == 1)) {
               b_phase ^= 1u << bs;
-              if (lane == 0) mbar_arrive(&bias_empty[bs]);
-            } else if (BIAS == 3 && lane < 2) {
-              mbar_arrive(&bias_empty[(unit + lane) % NB]);
+              if (lane == handing_back) mbar_arrive(&bias_empty[bs]);
+            } else if (BIAS == 3 && (lane >> 1) == handing_back) {
+              mbar_arrive(&bias_empty[(unit + (lane & 1)) % NB]);
             }
             if (any_need) {
               const float m_new = need ? mx : m_used;
