@@ -324,13 +324,11 @@ __global__ void __launch_bounds__(608, 1) dq_recompute_kernel(const __grid_const
 
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          f32x2 a;
+          // the exponent in the dK/dV kernel's order, so that dS and with it dQ have the bits of the streamed variant
+          f32x2 a = ffma2(f2(pr[i], pr[i + 1]), f2(p.scale_log2, p.scale_log2), f2(neg_lse, neg_lse));
           if (BIAS == 1) {
             const float2 f = P2::unpack(bcur.w[i >> 1]);
-            a = ffma2(f2(pr[i], pr[i + 1]), f2(p.scale_log2, p.scale_log2),
-                      ffma2(f2(f.x, f.y), f2(kLog2e, kLog2e), f2(neg_lse, neg_lse)));
-          } else {
-            a = ffma2(f2(pr[i], pr[i + 1]), f2(p.scale_log2, p.scale_log2), f2(neg_lse, neg_lse));
+            a = ffma2(f2(f.x, f.y), f2(kLog2e, kLog2e), a);
           }
           const f32x2 pe = f2(ex2(f2_lo(a)), ex2(f2_hi(a)));
           if (BIAS == 2) {
