@@ -356,3 +356,43 @@ def test_full_size_forwards_repeat_bitwise(D, bias_kind, causal, device_ok):
         out, lse2 = fa._flash_attn_fwd(q, k, v, bias, causal, D ** -0.5)
         differing += not (torch.equal(out, first) and torch.equal(lse, lse2))
     assert differing == 0, f"{differing} of 40 passes differ"
+
+
+@pytest.mark.parametrize("bias_kind,D", [(0, 64), (2, 128), (0, 256), (3, 128)])
+def test_scratch_for_ds_is_bounded(bias_kind, D, device_ok):
+    """The scratch a backward asks for: at most 1.5 GiB, and nothing where that holds no problem or too few to fill
+    the SMs; only where no other dQ kernel exists (head dim 256, fp32 bias) more, but never more than all of dS."""
+    from triton_flashattn_b200 import _cabi
+    from triton_flashattn_b200 import flash_attention as fa
+
+    lib = _cabi.load()
+    t, lse = torch.empty(1, 1, 1, D, dtype=BF, device="cuda"), torch.empty(1, device="cuda")
+    p = fa._params(t, t, t, t, lse, t, bias_kind, True, 0.1)
+    seen = set()
+    for B, H, M, N in ((1, 1, 1, 1), (2, 16, 1000, 777), (4, 32, 4096, 4096), (1, 8, 16384, 16384), (1, 8, 20480, 20480),
+                       (1, 8, 27000, 27000), (1, 3, 32768, 32768), (1, 1, 131072, 131072), (8, 1, 17, 1 << 20)):
+        p.B, p.H, p.M, p.N = B, H, M, N
+        one, got = M * ((N + 7) // 8 * 8) * 2, lib.fa_bwd_workspace_bytes(ctypes.byref(p))
+        assert got % one == 0 and got <= one * B * H, (B, H, M, N)
+        if D == 256 or bias_kind == 3:
+            assert got >= one, (B, H, M, N)
+        else:
+            assert got <= 3 << 29, (B, H, M, N)
+            if one > 3 << 29:
+                assert got == 0, (B, H, M, N)
+        seen.add(got // one)
+    assert len(seen) > 2
+
+
+def test_a_long_plain_backward_needs_no_quadratic_memory(device_ok):
+    from triton_flashattn_b200 import flash_attention_fn
+
+    S = 32768
+    q, k, v = (torch.randn(1, S, 1, 64, device="cuda", dtype=BF, requires_grad=True) for _ in range(3))
+    out = flash_attention_fn(q, k, v, None, True)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    out.backward(torch.ones_like(out))
+    torch.cuda.synchronize()
+    assert torch.cuda.max_memory_allocated() - before < 64 << 20  # gradients, do and delta; dS would be 2 GiB

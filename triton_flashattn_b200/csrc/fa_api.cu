@@ -172,24 +172,27 @@ bool ds_is_dbias(const fa_params& p) { return p.write_dbias && p.bias_kind == FA
 int64_t slab_pitch(const fa_params& p) { return ((int64_t)p.N + 7) / 8 * 8; }
 uint64_t slab_bytes(const fa_params& p) { return (uint64_t)slab_pitch(p) * p.M * 2; }
 
-// Problems per part of the backward, at most `most`: the number that makes the persistent dK/dV
-// grids of all parts together need the fewest turns of one work unit per SM, where every part
-// costs about a third of a turn more for its two launches and its drained tail.
+// Turns of one work unit per SM that the persistent dK/dV grids need for all problems, n at a time.
+int64_t dkdv_turns(const fa_params& p, int n) {
+  const int total = p.B * p.H, tiles = (p.N + 127) / 128, sms = persistent_grid(1 << 30);
+  auto turns = [&](int problems) {
+    const int64_t k = (int64_t)problems * tiles;
+    const int64_t units = p.causal ? (k + 1) / 2 : k;  // a causal unit is a heavy and a light tile
+    return (units + sms - 1) / sms;
+  };
+  return total / n * turns(n) + turns(total % n);
+}
+
+// Problems per part of the backward, at most `most`: the number that makes the dK/dV grids of all
+// parts together need the fewest turns, where every part costs about a third of a turn more for
+// its two launches and its drained tail.
 int problems_per_part(const fa_params& p, int most) {
   const int total = p.B * p.H;
   if (most >= total) return total;
-  const int tiles = (p.N + 127) / 128;
-  const bool pairs = p.causal != 0;  // a causal unit is a heavy and a light tile
-  const int sms = persistent_grid(1 << 30);
-  auto turns = [&](int n) {
-    const int64_t units = pairs ? ((int64_t)n * tiles + 1) / 2 : (int64_t)n * tiles;
-    return (units + sms - 1) / sms;
-  };
   int best = most;
   int64_t best_cost = -1;
   for (int n = most; n >= 1 && n > most / 2; --n) {
-    const int parts = total / n, rest = total % n;
-    const int64_t cost = 3 * (parts * turns(n) + (rest ? turns(rest) : 0)) + parts + (rest ? 1 : 0);
+    const int64_t cost = 3 * dkdv_turns(p, n) + (total + n - 1) / n;
     if (best_cost < 0 || cost < best_cost) {
       best_cost = cost;
       best = n;
@@ -199,15 +202,28 @@ int problems_per_part(const fa_params& p, int most) {
 }
 
 // The scratch a backward works best with: room for the dS of all problems, or of as many as
-// kSlabCap holds.  Slabs of 1.5 GiB hold tens of long-sequence heads, enough work units to fill
-// the SMs several times, so more would not shorten the turns by more than a few per cent.
+// kSlabCap holds: 48 at a sequence length of 4096, 12 at 8192, 3 at 16384, none from 28 k on, where
+// the scratch would grow with the square of the length.
 constexpr uint64_t kSlabCap = 3ull << 29;
+
+// Whether parts of n problems lose no more in turns that are not full than the streamed dQ gains over
+// the recomputing one.  Causal training pass, D = 128, recomputing against slabs under kSlabCap:
+//   H8 S16384 4 turns / 4 in parts: 2415 / 2219 us      H8 S16384 not causal 7 / 8: 4242 / 4158
+//   H5 S27000 4 / 5: 4208 / 4365     H4 S24576 3 / 4: 2858 / 3177     H8 S20480 5 / 8: 3874 / 4890
+bool parts_pay(const fa_params& p, int n) { return 6 * dkdv_turns(p, n) <= 7 * dkdv_turns(p, p.B * p.H); }
 
 uint64_t bwd_workspace_bytes(const fa_params& p) {
   if (ds_is_dbias(p)) return 0;
-  const uint64_t one = slab_bytes(p);
-  const uint64_t fit = kSlabCap / one;
-  return one * (uint64_t)problems_per_part(p, fit < 1 ? 1 : (fit > 65535 ? 65535 : (int)fit));
+  const uint64_t one = slab_bytes(p), fit = kSlabCap / one;
+  const int total = p.B * p.H;
+  int n = fit < 1 ? 0 : problems_per_part(p, fit > (uint64_t)total ? total : (int)fit);
+  if (p.D == 256 || p.bias_kind == FA_BIAS_F32) {
+    // no other dQ kernel exists: as many more problems as fill the turns
+    if (n < 1) n = 1;
+    while (n < total && !parts_pay(p, n)) ++n;
+    return one * (uint64_t)n;
+  }
+  return n >= 1 && parts_pay(p, n) ? one * (uint64_t)n : 0;
 }
 
 int bwd_in_parts(const fa_params& p, void* ws, uint64_t bytes, cudaStream_t s, int* st) {
