@@ -119,3 +119,21 @@ def test_func_transforms_are_refused(transform, packed):
             torch.func.vmap(lambda s: f(x) * s)(torch.ones(3))
     with pytest.raises((ValueError, TypeError)):  # outside the transform: the ordinary complaint
         f(x)
+
+
+def test_launch_path_is_rebuilt_for_another_torch(tmp_path, monkeypatch):
+    """The launch path is compiled against the installed torch: one built for another torch, or of unknown
+    origin, is not up to date however new its file is."""
+    import torch
+    from triton_flashattn_b200 import build
+
+    lib, stamp = tmp_path / "_fa_torch.so", tmp_path / "stamp"
+    monkeypatch.setattr(build, "BINDING_PATH", str(lib))
+    monkeypatch.setattr(build, "BINDING_STAMP", str(stamp))
+    assert build._binding_stale()  # not there at all
+    lib.write_bytes(b"")
+    assert build._binding_stale()  # nothing says what it was built against
+    stamp.write_text(build._binding_key())
+    assert not build._binding_stale()
+    monkeypatch.setattr(torch, "__version__", torch.__version__ + ".post1")
+    assert build._binding_stale()

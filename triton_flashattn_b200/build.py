@@ -21,6 +21,7 @@ BUILD_DIR = os.path.join(PKG_DIR, "build")
 LIB_PATH = os.path.join(PKG_DIR, "libfa_sm100.so")
 BINDING_SRC = os.path.join(CSRC, "torch_binding.cpp")
 BINDING_PATH = os.path.join(PKG_DIR, "_fa_torch.so")
+BINDING_STAMP = os.path.join(BUILD_DIR, "_fa_torch.stamp")
 INCLUDE_DIR = os.path.join(os.path.dirname(PKG_DIR), "include")
 
 SOURCES = [
@@ -100,13 +101,30 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB_PATH
 
 
+def _binding_key() -> str:
+    """What the launch path is compiled against, besides its sources."""
+    import torch
+
+    return f"torch {torch.__version__} {torch.version.git_version} {sysconfig.get_config_var('SOABI')}\n"
+
+
+def _binding_stale() -> bool:
+    """Older than its sources, or built against another torch or Python than the running one."""
+    if _stale(BINDING_PATH, [BINDING_SRC] + [h for h in _headers() if h.endswith(".h")]):
+        return True
+    try:
+        with open(BINDING_STAMP) as f:
+            return f.read() != _binding_key()
+    except OSError:
+        return True
+
+
 def build_binding(force: bool = False) -> str:
     """Compile the PyTorch launch path against the installed torch and link it to libfa_sm100.so
     (found beside it at run time); returns its path."""
     import torch
 
-    deps = [BINDING_SRC] + [h for h in _headers() if h.endswith(".h")]
-    if not force and not _stale(BINDING_PATH, deps):
+    if not force and not _binding_stale():
         return BINDING_PATH
     root = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
@@ -122,6 +140,8 @@ def build_binding(force: bool = False) -> str:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed for {BINDING_SRC}:\n{r.stdout}\n{r.stderr}")
+    with open(BINDING_STAMP, "w") as f:
+        f.write(_binding_key())
     return BINDING_PATH
 
 
