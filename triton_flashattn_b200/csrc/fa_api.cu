@@ -183,21 +183,16 @@ int64_t dkdv_turns(const fa_params& p, int n) {
   return total / n * turns(n) + turns(total % n);
 }
 
-// Problems per part of the backward, at most `most`: the number that makes the dK/dV grids of all
-// parts together need the fewest turns, where every part costs about a third of a turn more for
-// its two launches and its drained tail.
+// A backward in parts of n problems, in thirds of a turn: every part costs about one more for its two
+// launches and its drained tail.
+int64_t parts_cost(const fa_params& p, int n) { return 3 * dkdv_turns(p, n) + (p.B * p.H + n - 1) / n; }
+
+// Problems per part of the backward, at most `most`: the number of least cost.
 int problems_per_part(const fa_params& p, int most) {
-  const int total = p.B * p.H;
-  if (most >= total) return total;
+  if (most >= p.B * p.H) return p.B * p.H;
   int best = most;
-  int64_t best_cost = -1;
-  for (int n = most; n >= 1 && n > most / 2; --n) {
-    const int64_t cost = 3 * dkdv_turns(p, n) + (total + n - 1) / n;
-    if (best_cost < 0 || cost < best_cost) {
-      best_cost = cost;
-      best = n;
-    }
-  }
+  for (int n = most; n >= 1 && n > most / 2; --n)
+    if (parts_cost(p, n) < parts_cost(p, best)) best = n;
   return best;
 }
 
@@ -206,11 +201,20 @@ int problems_per_part(const fa_params& p, int most) {
 // the scratch would grow with the square of the length.
 constexpr uint64_t kSlabCap = 3ull << 29;
 
-// Whether parts of n problems lose no more in turns that are not full than the streamed dQ gains over
-// the recomputing one.  Causal training pass, D = 128, recomputing against slabs under kSlabCap:
-//   H8 S16384 4 turns / 4 in parts: 2415 / 2219 us      H8 S16384 not causal 7 / 8: 4242 / 4158
-//   H5 S27000 4 / 5: 4208 / 4365     H4 S24576 3 / 4: 2858 / 3177     H8 S20480 5 / 8: 3874 / 4890
-bool parts_pay(const fa_params& p, int n) { return 6 * dkdv_turns(p, n) <= 7 * dkdv_turns(p, p.B * p.H); }
+// Whether a backward in parts of n problems is faster than one with the recomputing dQ kernel.  Without a turn
+// lost that kernel costs more than the streamed product by a share of the dK/dV time that depends on what it
+// recomputes: three products instead of one at D = 128, little more than the traffic of dS at D = 64, and the
+// bias or mask.  Backward alone, bf16, recomputing / in parts, us (turns / turns in parts, parts):
+//   D 128: H8 S16384 causal (4 / 4, 4) 1760 / 1580      H8 S16384 (7 / 8, 3) 3230 / 3250
+//          H8 S20480 causal (5 / 8, 8) 2900 / 3900      H5 S27000 causal (4 / 5, 5) 3200 / 3300
+//   D 64:  B16 H32 S2048 (56 / 56, 3) 2820 / 2759       the same causal (28 / 28, 3) 1657 / 1531
+//          B4 H32 S4096 (28 / 28, 3) 2692 / 2708        B2 H16 S8192 causal (7 / 8, 4) 1359 / 1467
+//          H16 S8192 (7 / 8, 2) 1312 / 1442             the same causal (4 / 4, 2) 773 / 741
+//          H32 S12288 causal (11 / 11, 11) 3057 / 3285  B2 H12 S8192 causal, mask (6 / 6, 2) 1337 / 1163
+bool parts_pay(const fa_params& p, int n) {
+  const int64_t percent = (p.D > 64 ? 25 : 2) + (p.causal ? 10 : 0) + (p.bias_kind != FA_BIAS_NONE ? 20 : 0);
+  return 100 * parts_cost(p, n) <= 3 * dkdv_turns(p, p.B * p.H) * (100 + percent) + 100;
+}
 
 uint64_t bwd_workspace_bytes(const fa_params& p) {
   if (ds_is_dbias(p)) return 0;
@@ -218,9 +222,10 @@ uint64_t bwd_workspace_bytes(const fa_params& p) {
   const int total = p.B * p.H;
   int n = fit < 1 ? 0 : problems_per_part(p, fit > (uint64_t)total ? total : (int)fit);
   if (p.D == 256 || p.bias_kind == FA_BIAS_F32) {
-    // no other dQ kernel exists: as many more problems as fill the turns
+    // no other dQ kernel exists: as many more problems as lose no more than a seventh in turns that are not full
+    // (H4 S20480 D256 causal in parts of one 4799 us a training pass, of all 3743)
     if (n < 1) n = 1;
-    while (n < total && !parts_pay(p, n)) ++n;
+    while (n < total && 6 * dkdv_turns(p, n) > 7 * dkdv_turns(p, total)) ++n;
     return one * (uint64_t)n;
   }
   return n >= 1 && parts_pay(p, n) ? one * (uint64_t)n : 0;
