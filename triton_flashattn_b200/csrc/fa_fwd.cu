@@ -298,9 +298,13 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
       const int t = warp == 9 ? 0 : 1;
       // A look at a barrier takes about 280 cycles.  Without a bias the issuer is on the critical path, so it
       // looks at the loads, which have landed by then as a rule, while the row threads still form P or
-      // read S (causal B2 H32 S4096 D128: 342 -> 328 us).  With a bias the row threads are behind anyway,
-      // and a late load would hold up what could be issued: 16-bit bias, D = 64, 44 us against 47.
-      constexpr bool kLoadsFirst = BIAS == 0 || BIAS == 2;
+      // read S (causal B2 H32 S4096 D128: 342 -> 328 us).  With a mask that gains where the products are long
+      // enough to matter and loses where they are not; with a float bias the row threads are behind anyway.
+      // us, B4 H16 S2048 (D = 256: B2 H8), loads last / first, then causal:
+      //   mask   D128 194.8 / 189.2, 121.0 / 119.7     D64 174.3 / 193.8, 102.9 / 107.1    D256 96.2 / 98.7
+      //   16 bit D128 198.4 / 198.2, 125.2 / 125.3     D64 180.8 / 181.8, 106.9 / 106.9    D256 97.1 / 100.3
+      //   fp32   D128 351.3 / 349.7, 210.4 / 209.4     D64 332.0 / 329.0, 186.4 / 185.3    D256 116.9 / 115.9
+      constexpr bool kLoadsFirst = BIAS == 0 || (BIAS == 2 && DP == 128);
       constexpr bool bf = P2::kIsBf16;
       constexpr uint32_t idesc_qk = make_idesc(bf, false, false, 128, 64);
       constexpr uint32_t idesc_pv = make_idesc(bf, false, true, 128, DP);
