@@ -480,6 +480,7 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
             // Without a bias (and a positive scale) the raw q.k is kept and the scale is
             // folded into the exponent below.
             float mul = kLog2e;  // exponent = s * mul - m
+            float mx = -INFINITY;  // row maximum of this half
             if (BIAS == 0) {
               if (fold_scale) {
                 mul = scale_log2;
@@ -516,7 +517,19 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
                     s[i + 2] = f2_lo(x1);
                     s[i + 3] = f2_hi(x1);
                   }
+                  // Each unit goes back by itself, behind a vote on the maximum of its 32 scores (see below): four
+                  // units a key block pass through this ring of three.
+                  float ma = max3(s[sub * 32], s[sub * 32 + 1], s[sub * 32 + 2]);
+                  float mb = max3(s[sub * 32 + 3], s[sub * 32 + 4], s[sub * 32 + 5]);
+#pragma unroll
+                  for (int i = sub * 32 + 6; i < sub * 32 + 30; i += 4) {
+                    ma = max3(ma, s[i], s[i + 1]);
+                    mb = max3(mb, s[i + 2], s[i + 3]);
+                  }
+                  mx = fmaxf(mx, fmaxf(max3(ma, s[sub * 32 + 30], s[sub * 32 + 31]), mb));
+                  const bool above = __any_sync(0xffffffffu, mx * kLog2e > m_used + 8.0f);
                   b_phase ^= 1u << bs;
+                  if (lane == (above ? 1 : 0)) mbar_arrive(&bias_empty[bs]);
                 }
                 if (!ok) break;
               } else if (BIAS == 1) {
@@ -553,7 +566,8 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
               }
             }
             // ---- bounds and causal masks (only on halves that need them)
-            if ((n0 + 64 > p.N) || (p.causal && n0 + 63 > m0)) {
+            const bool edge = (n0 + 64 > p.N) || (p.causal && n0 + 63 > m0);
+            if (edge) {
               int limit = p.N - n0;
               if (p.causal) limit = min(limit, m0 + r - n0 + 1);
 #pragma unroll
@@ -561,18 +575,21 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
                 if (i >= limit) s[i] = -INFINITY;
             }
             // ---- row maximum of this half
-            float mx0 = max3(s[0], s[1], s[2]), mx1 = max3(s[3], s[4], s[5]);
-            float mx2 = max3(s[6], s[7], s[8]), mx3 = max3(s[9], s[10], s[11]);
+            if (BIAS != 3 || edge) {  // (an fp32 bias has it already where nothing was masked since)
+              float mx0 = max3(s[0], s[1], s[2]), mx1 = max3(s[3], s[4], s[5]);
+              float mx2 = max3(s[6], s[7], s[8]), mx3 = max3(s[9], s[10], s[11]);
 #pragma unroll
-            for (int i = 12; i + 7 < 64; i += 8) {
-              mx0 = max3(mx0, s[i], s[i + 1]);
-              mx1 = max3(mx1, s[i + 2], s[i + 3]);
-              mx2 = max3(mx2, s[i + 4], s[i + 5]);
-              mx3 = max3(mx3, s[i + 6], s[i + 7]);
+              for (int i = 12; i + 7 < 64; i += 8) {
+                mx0 = max3(mx0, s[i], s[i + 1]);
+                mx1 = max3(mx1, s[i + 2], s[i + 3]);
+                mx2 = max3(mx2, s[i + 4], s[i + 5]);
+                mx3 = max3(mx3, s[i + 6], s[i + 7]);
+              }
+              mx0 = max3(mx0, s[60], s[61]);  // 12 + 6*8 = 60 consumed; 60..63 left
+              mx1 = max3(mx1, s[62], s[63]);
+              mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
             }
-            mx0 = max3(mx0, s[60], s[61]);  // 12 + 6*8 = 60 consumed; 60..63 left
-            mx1 = max3(mx1, s[62], s[63]);
-            const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * mul;  // log2 domain
+            mx *= mul;  // log2 domain
             const bool need = mx > m_used + 8.0f;
             const bool any_need = __any_sync(0xffffffffu, need);
             // The bias units go back to their producer only after the vote, which needs the maximum of
@@ -581,12 +598,9 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
             // bulk load overwrote rows before they were read about once in ten full-size passes.)
             // The vote's result picks the arriving lane, so that no schedule can put the arrival first
             // (B16 S512 H12 D64 fp16 bias: 40.1 -> 40.8 us; the arrival behind the rescaling branch: 42.1).
-            const int handing_back = any_need ? 1 : 0;
             if (BIAS == 1 || (BIAS == 2 && h == 1)) {
               b_phase ^= 1u << bs;
-              if (lane == handing_back) mbar_arrive(&bias_empty[bs]);
-            } else if (BIAS == 3 && (lane >> 1) == handing_back) {
-              mbar_arrive(&bias_empty[(unit + (lane & 1)) % NB]);
+              if (lane == (any_need ? 1 : 0)) mbar_arrive(&bias_empty[bs]);
             }
             if (any_need) {
               const float m_new = need ? mx : m_used;
