@@ -396,3 +396,22 @@ def test_a_long_plain_backward_needs_no_quadratic_memory(device_ok):
     out.backward(torch.ones_like(out))
     torch.cuda.synchronize()
     assert torch.cuda.max_memory_allocated() - before < 64 << 20  # gradients, do and delta; dS would be 2 GiB
+
+
+def test_scratch_size_is_cheap_to_ask_for(device_ok):
+    """Every backward asks for the scratch size on the host; with tens of thousands of small problems too."""
+    import time
+
+    from triton_flashattn_b200 import _cabi
+    from triton_flashattn_b200 import flash_attention as fa
+
+    lib = _cabi.load()
+    t, lse = torch.empty(1, 1, 1, 64, dtype=BF, device="cuda"), torch.empty(1, device="cuda")
+    p = fa._params(t, t, t, t, lse, None, 0, True, 0.1)
+    for p.B, p.H, p.M, p.N in ((4096, 15, 160, 160), (8192, 7, 180, 180), (1, 65535, 120, 120), (4, 32, 4096, 4096)):
+        best = 1.0
+        for _ in range(20):
+            start = time.perf_counter()
+            lib.fa_bwd_workspace_bytes(ctypes.byref(p))
+            best = min(best, time.perf_counter() - start)
+        assert best < 40e-6, f"B{p.B} H{p.H} M{p.M}: {best * 1e6:.0f} us"

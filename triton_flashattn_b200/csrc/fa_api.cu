@@ -172,29 +172,34 @@ bool ds_is_dbias(const fa_params& p) { return p.write_dbias && p.bias_kind == FA
 int64_t slab_pitch(const fa_params& p) { return ((int64_t)p.N + 7) / 8 * 8; }
 uint64_t slab_bytes(const fa_params& p) { return (uint64_t)slab_pitch(p) * p.M * 2; }
 
-// Turns of one work unit per SM that the persistent dK/dV grids need for all problems, n at a time.
-int64_t dkdv_turns(const fa_params& p, int n) {
-  const int total = p.B * p.H, tiles = (p.N + 127) / 128, sms = persistent_grid(1 << 30);
-  auto turns = [&](int problems) {
-    const int64_t k = (int64_t)problems * tiles;
-    const int64_t units = p.causal ? (k + 1) / 2 : k;  // a causal unit is a heavy and a light tile
-    return (units + sms - 1) / sms;
-  };
-  return total / n * turns(n) + turns(total % n);
-}
-
-// A backward in parts of n problems, in thirds of a turn: every part costs about one more for its two
-// launches and its drained tail.
-int64_t parts_cost(const fa_params& p, int n) { return 3 * dkdv_turns(p, n) + (p.B * p.H + n - 1) / n; }
-
-// Problems per part of the backward, at most `most`: the number of least cost.
-int problems_per_part(const fa_params& p, int most) {
-  if (most >= p.B * p.H) return p.B * p.H;
-  int best = most;
-  for (int n = most; n >= 1 && n > most / 2; --n)
-    if (parts_cost(p, n) < parts_cost(p, best)) best = n;
-  return best;
-}
+// What a backward in parts of n problems costs in the dK/dV stage.
+struct PartsCost {
+  int total, tiles, sms;
+  bool pairs;  // a causal unit is a heavy and a light tile
+  explicit PartsCost(const fa_params& p)
+      : total(p.B * p.H), tiles((p.N + 127) / 128), sms(persistent_grid(1 << 30)), pairs(p.causal != 0) {}
+  // Turns of one work unit per SM that the persistent grids need for all problems, n at a time.
+  int64_t turns(int n) const {
+    auto of = [&](int problems) {
+      const int64_t k = (int64_t)problems * tiles;
+      return ((pairs ? (k + 1) / 2 : k) + sms - 1) / sms;
+    };
+    return total / n * of(n) + of(total % n);
+  }
+  // In thirds of a turn: every part costs about one more for its two launches and its drained tail.
+  int64_t cost(int n) const { return 3 * turns(n) + (total + n - 1) / n; }
+  // Problems per part, at most `most`: the number of least cost.  Among thousands of small problems one more
+  // or less changes little, and a few hundred numbers are looked at (all of them took up to 0.1 ms a call).
+  int best(int most) const {
+    if (most >= total) return total;
+    int n = most;
+    int64_t least = cost(most);
+    const int step = most / 512 + 1;
+    for (int k = most - step; k > most / 2; k -= step)
+      if (const int64_t c = cost(k); c < least) least = c, n = k;
+    return n;
+  }
+};
 
 // The scratch a backward works best with: room for the dS of all problems, or of as many as
 // kSlabCap holds: 48 at a sequence length of 4096, 12 at 8192, 3 at 16384, none from 28 k on, where
@@ -211,30 +216,32 @@ constexpr uint64_t kSlabCap = 3ull << 29;
 //          B4 H32 S4096 (28 / 28, 3) 2692 / 2708        B2 H16 S8192 causal (7 / 8, 4) 1359 / 1467
 //          H16 S8192 (7 / 8, 2) 1312 / 1442             the same causal (4 / 4, 2) 773 / 741
 //          H32 S12288 causal (11 / 11, 11) 3057 / 3285  B2 H12 S8192 causal, mask (6 / 6, 2) 1337 / 1163
-bool parts_pay(const fa_params& p, int n) {
+bool parts_pay(const fa_params& p, const PartsCost& parts, int n) {
   const int64_t percent = (p.D > 64 ? 25 : 2) + (p.causal ? 10 : 0) + (p.bias_kind != FA_BIAS_NONE ? 20 : 0);
-  return 100 * parts_cost(p, n) <= 3 * dkdv_turns(p, p.B * p.H) * (100 + percent) + 100;
+  return 100 * parts.cost(n) <= 3 * parts.turns(parts.total) * (100 + percent) + 100;
 }
 
 uint64_t bwd_workspace_bytes(const fa_params& p) {
   if (ds_is_dbias(p)) return 0;
   const uint64_t one = slab_bytes(p), fit = kSlabCap / one;
-  const int total = p.B * p.H;
-  int n = fit < 1 ? 0 : problems_per_part(p, fit > (uint64_t)total ? total : (int)fit);
+  const PartsCost parts(p);
+  const int total = parts.total;
+  int n = fit < 1 ? 0 : parts.best(fit > (uint64_t)total ? total : (int)fit);
   if (p.D == 256 || p.bias_kind == FA_BIAS_F32) {
     // no other dQ kernel exists: as many more problems as lose no more than a seventh in turns that are not full
     // (H4 S20480 D256 causal in parts of one 4799 us a training pass, of all 3743)
     if (n < 1) n = 1;
-    while (n < total && 6 * dkdv_turns(p, n) > 7 * dkdv_turns(p, total)) ++n;
+    const int64_t full = parts.turns(total);
+    while (n < total && 6 * parts.turns(n) > 7 * full) ++n;
     return one * (uint64_t)n;
   }
-  return n >= 1 && parts_pay(p, n) ? one * (uint64_t)n : 0;
+  return n >= 1 && parts_pay(p, parts, n) ? one * (uint64_t)n : 0;
 }
 
 int bwd_in_parts(const fa_params& p, void* ws, uint64_t bytes, cudaStream_t s, int* st) {
   const uint64_t fit = bytes / slab_bytes(p);
   const int total = p.B * p.H;
-  const int n = problems_per_part(p, fit > (uint64_t)total ? total : (int)fit);
+  const int n = PartsCost(p).best(fit > (uint64_t)total ? total : (int)fit);
   for (int bh0 = 0; bh0 < total; bh0 += n) {
     const DsSlab slab = {ws, slab_pitch(p), bh0, n < total - bh0 ? n : total - bh0};
     if (int e = launch_bwd_dkdv(p, s, st, &slab)) return e;
