@@ -124,6 +124,27 @@ def test_few_query_rows(M, N, D, dtype, bias_kind, causal, device_ok):
             verbose=False)
 
 
+@pytest.mark.parametrize("M", [1, 2, 4, 7, 8, 16])
+@pytest.mark.parametrize("N,D", [(1, 128), (33, 64), (600, 128), (1023, 32), (1920, 64), (2049, 128), (4096, 128), (9000, 64), (20011, 128)])
+def test_few_rows_result_does_not_depend_on_the_other_heads(M, N, D, device_ok):
+    """How the keys of a head are split over warps and CTAs depends on how many heads the call has; the result
+    does not: one head alone, a batch element alone and a shard of four heads have the bits of the whole call.
+    (Key counts around two and four tiles a leaf and on both sides of the largest number of leaves.)"""
+    from triton_flashattn_b200 import flash_attention as fa
+
+    B, H = 8, 32
+    g = torch.Generator(device="cuda").manual_seed(28)
+    q, k, v = (torch.randn(B, S, H, D, generator=g, device="cuda").to(BF) for S in (M, N, N))
+    out, lse = fa._flash_attn_fwd(q, k, v, None, False, D ** -0.5)
+    for b, h in ((slice(0, 1), slice(0, 1)), (slice(3, 4), slice(0, 32)), (slice(2, 6), slice(8, 12)), (slice(0, 8), slice(5, 21))):
+        o, l = fa._flash_attn_fwd(q[b, :, h], k[b, :, h], v[b, :, h], None, False, D ** -0.5)
+        assert torch.equal(o, out[b, :, h]) and torch.equal(l, lse[b, h]), (b, h)
+    ref = oracle.attention_backward(q[:1], k[:1], v[:1], None, False, None, torch.zeros_like(q[:1]))["out"] \
+        if N <= 2049 else torch.nn.functional.scaled_dot_product_attention(
+            *(t[:1].float().transpose(1, 2) for t in (q, k, v))).transpose(1, 2)
+    assert (out[:1].float() - ref).abs().max().item() <= TOL[BF]
+
+
 @pytest.mark.parametrize("S", [4, 100])
 @pytest.mark.parametrize("layout", ["one element off", "padded head dim", "heads first"])
 def test_packed_qkv_in_other_layouts(S, layout, device_ok):

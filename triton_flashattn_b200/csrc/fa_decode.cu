@@ -9,8 +9,8 @@
 // of CTAs, so that even a few heads fill the chip.  (The tile kernel gives each head to one CTA.)
 // The warp-level matrix instruction is enough: at the HBM rate an SM has 350 cycles for the 32 products
 // of a tile, and tcgen05 would want the operands in shared memory and 128 rows of queries.
-//   B8 H32 N4096 D128, M=1, bf16:  119 -> 89 us (6.0 TB/s);  B1 H32 N20011:  277 -> 61 us;
-//   B64 H32 N2048: 316 us (6.8 TB/s).  A ring of asynchronous copies in shared memory in place of the
+//   tile kernel -> here, bf16, us:  B8 H32 N4096 D128, M=1 120 -> 93 (5.8 TB/s), M=16 119 -> 115;  B1 H32 N20011
+//   277 -> 60;  B64 H32 N2048 407 -> 325 (6.6 TB/s);  B32 H32 N1000 D64 92 -> 57.  A ring of asynchronous copies in shared memory in place of the
 //   register tiles, two or three tiles deep, was slower (109 and 71 us for the first two).
 //
 // Per warp and tile of 16 keys (r = lane / 4, t = lane % 4):
@@ -22,8 +22,12 @@
 //        (eight lanes: 128 contiguous bytes) and pairs the keys with byte permutes.
 // The running maximum is raised only when some score passes it by more than 8 (log2 units), so the
 // common tile needs one vote and no shuffles; row sums stay per lane until the end.
-// Partial results are merged in shared memory, then over the cluster through distributed shared
-// memory; every merge runs in a fixed order, so results do not vary from run to run.
+// A result must not depend on how many heads a call has, although the split over warps and CTAs does.  So the
+// keys of a head are cut into leaves of a few tiles, by their number alone: a leaf has its own running maximum
+// and starts from zero, four leaves in a row are folded from left to right into a group, and the groups (at most
+// 32) are summed in order.  Whoever computes or folds a leaf, the operations and their order are the same.  A warp
+// keeps its partial results in shared memory, whole groups or, where the heads are too few for that, leaves;
+// the CTA folds those, and the cluster sums the groups through distributed shared memory.
 //
 // Replaces _attn_fwd of the reference (flash_attention.py 12-194) for short queries: same masks,
 // bias, base-2 softmax and log-sum-exp as the tile kernel.
@@ -51,6 +55,9 @@ struct DecodeParams {
   int64_t bias_sB, bias_sH, bias_sM;
   int H, M, N, D;
   int n_keys;  // keys some row sees: N, or min(N, M) when causal
+  int leaf;    // tiles of 16 keys in a leaf
+  int fold;    // leaves in a partial result that a warp keeps: 1 or kGroup
+  int own;     // partial results of a warp
   int causal;
   float sm_scale;
 };
@@ -92,19 +99,49 @@ __device__ __forceinline__ float load_bias(const DecodeParams& p, int64_t off) {
   return 0.f;
 }
 
+constexpr int kGroup = 4;       // leaves in a group
+constexpr int kMaxGroups = 32;  // of a head
+constexpr int kMaxLeaves = kGroup * kMaxGroups;
+
+// The shared memory of a CTA: room for the partial results of its warps, 16 rows for each group of 8 query rows a warp.
+// What is not shared memory buffers the loads in flight, as much again: with twice the room B8 H32 N4096 D128 took
+// 174 us instead of 90.
+template <int DP, int NQ, int W>
+struct DecodeSmem {
+  static constexpr int kRows = 16 * NQ;   // query rows of partial results that a warp has room for
+  static constexpr int kRow = DP + 8;     // accumulators of a row, and its sum in eight parts (one per lane that has it)
+  float o[W * kRows * kRow];              // [partial result][query row][kRow]
+  float m[W * kRows], gm[W * kRows];      // maximum of a partial result's row; the same of a group, at its first leaf
+  float weight[NQ * 8][kMaxGroups];
+  float m_all[NQ * 8], l_all[NQ * 8];
+  const float* group[kMaxGroups];  // accumulators of a group, wherever in the cluster they are
+  // partial results that a warp has room for; more than 8 would not make a better split
+  static constexpr int slots(int rows) { return kRows / rows < 8 ? kRows / rows : 8; }
+};
+
+// What a partial result with maximum m counts in one with maximum m_all >= m; 0 where it has no key (its accumulators
+// are zero then, or NaN, which stays).
+__device__ __forceinline__ float weight_of(float m, float m_all) { return m == -INFINITY ? 0.f : ex2(m - m_all); }
+
+// acc, of weight fa, followed by x, of weight fx.  (Spelled out, so that every place that folds rounds alike.)
+__device__ __forceinline__ float fold2(float fa, float acc, float fx, float x) {
+  return __fmaf_rn(fx, x, __fmul_rn(fa, acc));
+}
+
+// CTAs per SM: what the registers of the tile loop allow (a few words spill with a bias).
+constexpr int decode_ctas(int DP, int NQ, int W) { return (DP == 64 ? (NQ == 1 ? 20 : 16) : (NQ == 1 ? 12 : 8)) / W; }
+
 // DP: head dim rounded up to 64 or 128; NQ: groups of 8 query rows; W: warps per CTA.
 // Grid: (cluster size, B * H).  The CTAs of a cluster share one (batch, head).
 template <int DP, int NQ, int W, typename T, int BIAS>
-__global__ void __launch_bounds__(W * 32) decode_kernel(const DecodeParams p) {
+__global__ void __launch_bounds__(W * 32, decode_ctas(DP, NQ, W)) decode_kernel(const DecodeParams p) {
   using P2 = Pack2<T>;
+  using Smem = DecodeSmem<DP, NQ, W>;
   constexpr int KG = DP / 32;  // 16-byte loads per lane and key row of K
   constexpr int VG = DP / 64;  // ... of V
-  constexpr int QR = NQ * 8;
 
-  __shared__ float s_o[W][QR][DP + 4];  // +4: rows a few banks apart
-  __shared__ float s_m[W][QR], s_l[W][QR];
-  __shared__ float c_o[QR][DP];  // this CTA's partial result, read by the whole cluster
-  __shared__ float c_m[QR], c_l[QR];
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int r = lane >> 2, t = lane & 3;
@@ -114,8 +151,8 @@ __global__ void __launch_bounds__(W * 32) decode_kernel(const DecodeParams p) {
   const bool live = *reinterpret_cast<volatile int*>(p.status) == 0;
 
   const int n_tiles = live ? (p.n_keys + 15) >> 4 : 0;
-  const int stride = static_cast<int>(gridDim.x) * W;
-  const int first = static_cast<int>(blockIdx.x) * W + warp;
+  const int first = (static_cast<int>(blockIdx.x) * W + warp) * p.own * p.fold * p.leaf;
+  const int last = min(first + p.own * p.fold * p.leaf, n_tiles);
 
   // Q as the B operand: row = query, the same 16-byte pieces of the head dim as a key's
   uint4 q[NQ][KG];
@@ -175,13 +212,64 @@ __global__ void __launch_bounds__(W * 32) decode_kernel(const DecodeParams p) {
 #pragma unroll
   for (int n = 0; n < NQ; ++n) mx[n][0] = mx[n][1] = -INFINITY, l[n][0] = l[n][1] = 0.f;
 
-  if (first < n_tiles) {
+  // The leaf in the accumulators is complete: into the warp's partial result `slot`, which it starts or follows.
+  auto close_leaf = [&](int slot, bool starts) {
+    float m_new[NQ][2];
+#pragma unroll
+    for (int n = 0; n < NQ; ++n)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int m = n * 8 + 2 * t + j, at = slot * p.M + m;
+        m_new[n][j] = mx[n][j];
+        if (m < p.M) {
+          // lane (r, t) holds head-dim elements 64 g + 8 r .. + 7 of its query rows, and part r of their sums
+          float* row = sm.o + at * Smem::kRow;
+          float fa = 0.f, fx = 1.f;
+          if (!starts) {
+            const float m_old = sm.m[at];
+            m_new[n][j] = fmaxf(m_old, mx[n][j]);
+            fa = weight_of(m_old, m_new[n][j]);
+            fx = weight_of(mx[n][j], m_new[n][j]);
+            l[n][j] = fold2(fa, row[DP + r], fx, l[n][j]);
+          }
+          row[DP + r] = l[n][j];
+#pragma unroll
+          for (int i = 0; i < VG * 4; i += 2) {
+            float4 v = make_float4(o[n][i][j], o[n][i][j + 2], o[n][i + 1][j], o[n][i + 1][j + 2]);
+            float4& dst = *reinterpret_cast<float4*>(row + (i >> 2) * 64 + r * 8 + (i & 3) * 2);
+            if (!starts) {
+              const float4 a = dst;
+              v = make_float4(fold2(fa, a.x, fx, v.x), fold2(fa, a.y, fx, v.y), fold2(fa, a.z, fx, v.z),
+                              fold2(fa, a.w, fx, v.w));
+            }
+            dst = v;
+          }
+        }
+        mx[n][j] = -INFINITY;
+        l[n][j] = 0.f;
+      }
+    __syncwarp();
+#pragma unroll
+    for (int n = 0; n < NQ; ++n) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        if (r == 0 && n * 8 + 2 * t + j < p.M) sm.m[slot * p.M + n * 8 + 2 * t + j] = m_new[n][j];
+#pragma unroll
+      for (int i = 0; i < VG * 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[n][i][e] = 0.f;
+    }
+    __syncwarp();
+  };
+
+  if (first < last) {
     load_k(first);
     load_b(first);
     load_v(first);
   }
+  int left = p.leaf, leaf = 0;  // tiles left of the running leaf; leaves closed so far
 #pragma unroll 1
-  for (int tile = first; tile < n_tiles; tile += stride) {
+  for (int tile = first; tile < last; ++tile) {
     float s[NQ][4];
 #pragma unroll
     for (int n = 0; n < NQ; ++n) {
@@ -192,8 +280,8 @@ __global__ void __launch_bounds__(W * 32) decode_kernel(const DecodeParams p) {
         mma16816<T>(s[n], kf[0][g].z, kf[1][g].z, kf[0][g].w, kf[1][g].w, q[n][g].z, q[n][g].w);
       }
     }
-    const bool more = tile + stride < n_tiles;
-    if (more) load_k(tile + stride);
+    const bool more = tile + 1 < last;
+    if (more) load_k(tile + 1);
     // scores in log2 units, -inf where masked
     bool need = false;
 #pragma unroll
@@ -209,7 +297,7 @@ __global__ void __launch_bounds__(W * 32) decode_kernel(const DecodeParams p) {
         s[n][i] = x * kLog2e;
         need = need || s[n][i] > mx[n][i & 1] + 8.f;
       }
-    if (more) load_b(tile + stride);
+    if (more) load_b(tile + 1);
     if (__any_sync(0xffffffffu, need)) {
 #pragma unroll
       for (int n = 0; n < NQ; ++n)
@@ -248,63 +336,72 @@ __global__ void __launch_bounds__(W * 32) decode_kernel(const DecodeParams p) {
         for (int n = 0; n < NQ; ++n) mma16816<T>(o[n][g * 4 + i], a0, a1, a2, a3, pb[n][0], pb[n][1]);
       }
     }
-    if (more) load_v(tile + stride);
+    if (more) load_v(tile + 1);
+    if (--left == 0 || !more) {
+      close_leaf(warp * p.own + (p.fold == 1 ? leaf : leaf / kGroup), p.fold == 1 || leaf % kGroup == 0);
+      ++leaf;
+      left = p.leaf;
+    }
   }
 
-  // ---- this warp's part: maximum and sum per query, O^T with lane (r, t) holding head-dim rows
-  // 64 g + 8 r + 2 i (+1) of queries 2t, 2t+1
-#pragma unroll
-  for (int n = 0; n < NQ; ++n)
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      for (int off = 4; off < 32; off <<= 1) l[n][j] += __shfl_xor_sync(0xffffffffu, l[n][j], off);
-      const int m = n * 8 + 2 * t + j;
-      if (r == 0) s_m[warp][m] = mx[n][j], s_l[warp][m] = l[n][j];
-#pragma unroll
-      for (int g = 0; g < VG; ++g)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          s_o[warp][m][g * 64 + r * 8 + 2 * i] = o[n][g * 4 + i][j];
-          s_o[warp][m][g * 64 + r * 8 + 2 * i + 1] = o[n][g * 4 + i][j + 2];
-        }
-    }
   __syncthreads();
-  // ---- this CTA's part
-  for (int e = tid; e < QR * DP; e += W * 32) {
-    const int m = e / DP, d = e - m * DP;
-    float m_all = s_m[0][m];
-#pragma unroll
-    for (int w = 1; w < W; ++w) m_all = fmaxf(m_all, s_m[w][m]);
-    float acc = 0.f, sum = 0.f;
-#pragma unroll
-    for (int w = 0; w < W; ++w) {
-      const float f = m_all == -INFINITY ? 0.f : ex2(s_m[w][m] - m_all);
-      acc += f * s_o[w][m][d];
-      sum += f * s_l[w][m];
+  const int n_leaves = (n_tiles + p.leaf - 1) / p.leaf;
+  const int n_groups = (n_leaves + kGroup - 1) / kGroup;
+  const int cta_groups = W * p.own * p.fold / kGroup;
+  if (p.fold == 1) {
+    // ---- this CTA's leaves into groups, in the place of each group's first leaf
+    const int here = min(n_leaves - static_cast<int>(blockIdx.x) * W * p.own, W * p.own);
+    const int size = p.M * Smem::kRow;
+    for (int e = tid; e < (here + kGroup - 1) / kGroup * size; e += W * 32) {
+      const int g = e / size, at = e - g * size, m = at / Smem::kRow;
+      const int s0 = g * kGroup;
+      float acc = sm.o[s0 * size + at], m_acc = sm.m[s0 * p.M + m];
+      for (int sx = s0 + 1; sx < min(here, s0 + kGroup); ++sx) {
+        const float m_x = sm.m[sx * p.M + m], m_new = fmaxf(m_acc, m_x);
+        acc = fold2(weight_of(m_acc, m_new), acc, weight_of(m_x, m_new), sm.o[sx * size + at]);
+        m_acc = m_new;
+      }
+      sm.o[s0 * size + at] = acc;
+      if (at == m * Smem::kRow) sm.gm[s0 * p.M + m] = m_acc;
     }
-    c_o[m][d] = acc;
-    if (d == 0) c_m[m] = m_all, c_l[m] = sum;
   }
-  // ---- the cluster's result: each CTA finishes a share of the elements
+  // ---- the head's result: each CTA finishes a share of the elements
   const int parts = static_cast<int>(gridDim.x);
   cg::cluster_group cluster = cg::this_cluster();
   if (parts > 1)
     cluster.sync();
   else
     __syncthreads();
+  // a group: the CTA that has it, and its (first) place there
+  const int rank = lane / cta_groups, place = lane % cta_groups * (kGroup / p.fold);
+  auto of_group = [&](float* mine) -> float* { return parts > 1 ? cluster.map_shared_rank(mine, rank) : mine; };
+  if (warp == 0 && lane < n_groups) sm.group[lane] = of_group(sm.o + place * p.M * Smem::kRow);
+  for (int m = warp; live && m < p.M; m += W) {  // a warp per row, a lane per group
+    float gm = -INFINITY, gl = 0.f;
+    if (lane < n_groups) {
+      gm = *of_group((p.fold == 1 ? sm.gm : sm.m) + place * p.M + m);
+      const float4* part = reinterpret_cast<const float4*>(of_group(sm.o + (place * p.M + m) * Smem::kRow + DP));
+      const float4 a = part[0], b4 = part[1];
+      gl = ((a.x + a.y) + (a.z + a.w)) + ((b4.x + b4.y) + (b4.z + b4.w));
+    }
+    float m_all = gm;
+    for (int off = 1; off < 32; off <<= 1) m_all = fmaxf(m_all, __shfl_xor_sync(0xffffffffu, m_all, off));
+    const float f = weight_of(gm, m_all);
+    float sum = __fmul_rn(f, gl);
+    for (int off = 1; off < 32; off <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    sm.weight[m][lane] = f;
+    if (lane == 0) sm.m_all[m] = m_all, sm.l_all[m] = sum;
+  }
+  __syncthreads();
   for (int e = static_cast<int>(blockIdx.x) * W * 32 + tid; live && e < p.M * DP; e += parts * W * 32) {
     const int m = e / DP, d = e - m * DP;
-    float m_all = -INFINITY;
-    for (int c = 0; c < parts; ++c) m_all = fmaxf(m_all, parts > 1 ? *cluster.map_shared_rank(&c_m[m], c) : c_m[m]);
-    float acc = 0.f, sum = 0.f;
-    for (int c = 0; c < parts; ++c) {
-      const float mc = parts > 1 ? *cluster.map_shared_rank(&c_m[m], c) : c_m[m];
-      const float f = m_all == -INFINITY ? 0.f : ex2(mc - m_all);
-      acc += f * (parts > 1 ? *cluster.map_shared_rank(&c_o[m][d], c) : c_o[m][d]);
-      sum += f * (parts > 1 ? *cluster.map_shared_rank(&c_l[m], c) : c_l[m]);
-    }
+    float acc = 0.f;
+#pragma unroll 8
+    for (int g = 0; g < n_groups; ++g)
+      acc = __fmaf_rn(sm.weight[m][g], sm.group[g][m * Smem::kRow + d], acc);
     // A row whose keys are all masked out: output 0, log-sum-exp +inf.  A NaN sum ends here too, and the product
     // with zero lets the NaN of its accumulators through (the tile kernel does the same).
+    const float m_all = sm.m_all[m], sum = sm.l_all[m];
     const bool any_key = m_all != -INFINITY && sum > 0.f;
     if (d < p.D)
       (static_cast<T*>(p.o) + b * p.o_sB + m * p.o_sM + h * p.o_sH)[d] = static_cast<T>(any_key ? acc / sum : acc * 0.f);
@@ -316,7 +413,7 @@ __global__ void __launch_bounds__(W * 32) decode_kernel(const DecodeParams p) {
 // How many clusters of 1 .. 16 CTAs of a kernel the current device holds at once (asked once).
 constexpr int kMaxParts = 16;
 template <auto kern>  // one table per kernel
-const int* resident_clusters(int warps) {
+const int* resident_clusters(int warps, int smem) {
   static int table[64][kMaxParts + 1] = {};
   static std::mutex mu;
   int dev = 0;
@@ -326,10 +423,12 @@ const int* resident_clusters(int warps) {
   int* t = table[dev];
   if (t[0] == 0) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return nullptr;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return nullptr;
     for (int parts = 1; parts <= kMaxParts; ++parts) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(parts, 1);
       cfg.blockDim = dim3(warps * 32);
+      cfg.dynamicSmemBytes = smem;
       cudaLaunchAttribute attr;
       attr.id = cudaLaunchAttributeClusterDimension;
       attr.val.clusterDim.x = parts;
@@ -348,38 +447,58 @@ const int* resident_clusters(int warps) {
   return t;
 }
 
-// The split of a (batch, head)'s key tiles over `parts` CTAs of `warps` warps: the one with the least
+// Tiles in a leaf: a function of the number of keys and query rows alone.  Closing a leaf takes a quarter of a
+// tile's instructions, more with many rows, so a leaf has a few tiles where there are enough; and there are no
+// more leaves than the warps of a cluster can use - fewer for many rows, of which a warp can keep only two.
+int leaf_tiles(int tiles, int rows) {
+  const int most = rows <= 4 ? 120 : 64;
+  static_assert(120 <= kMaxLeaves);
+  const int least = tiles < 64 ? 2 : (rows <= 8 || tiles < 128 ? 4 : 8);
+  return tiles <= least * most ? least : (tiles + most - 1) / most;
+}
+
+// The split of a (batch, head)'s leaves over the warps of `parts` CTAs: the one with the least
 // (turns of the resident clusters) x (tiles per warp + the start and the merge of a CTA, which take
 // about as long as six tiles).  A single turn that fills the SMs wins where there are few heads,
-// several turns of longer CTAs where there are many.  B1 H32 N20011 D128: 10 CTAs a head 61 us,
-// 8: 70, 11 (no longer one turn): 95; B8 H32 N4096: 3 a head 90 us, 1: 108, 2: 117, 4: 99.
+// several turns of longer CTAs where there are many.  (With a split free of leaves, and so results that depend on the
+// number of heads: B8 H32 N4096 90 us, B1 H32 N20011 61, B64 H32 N2048 319, B32 H32 N1000 D64 50.)
 struct Split {
-  int parts = 0, warps = 0;
+  int parts = 0, warps = 0, fold = 0, own = 0;
   int64_t cost = -1;
 };
-void consider(Split& best, const int* resident, int warps, int bh, int tiles) {
+void consider(Split& best, const int* resident, int warps, int slots, int bh, int tiles, int leaf) {
   if (!resident) return;
-  for (int parts = 1; parts <= kMaxParts; ++parts) {
-    if (resident[parts] < 1 || (parts > 1 && (parts - 1) * warps >= tiles)) continue;
-    const int64_t turns = (bh + resident[parts] - 1) / resident[parts];
-    const int64_t cost = turns * ((tiles + parts * warps - 1) / (parts * warps) + 6);
-    if (best.cost < 0 || cost < best.cost) best = {parts, warps, cost};
-  }
+  const int leaves = (tiles + leaf - 1) / leaf;
+  for (int fold = 1; fold <= kGroup; fold += kGroup - 1)
+    for (int own = 1; own <= slots; ++own) {
+      const int parts = (leaves + warps * own * fold - 1) / (warps * own * fold);
+      if (parts > kMaxParts || resident[parts] < 1) continue;
+      const int64_t turns = (bh + resident[parts] - 1) / resident[parts];
+      const int per_warp = own * fold * leaf;
+      const int64_t cost = turns * ((per_warp < tiles ? per_warp : tiles) + 6);
+      if (best.cost < 0 || cost < best.cost) best = {parts, warps, fold, own, cost};
+    }
 }
 
 template <int DP, int NQ, typename T, int BIAS>
-int launch_inst(const DecodeParams& dp, int bh, cudaStream_t stream) {
+int launch_inst(DecodeParams dp, int bh, cudaStream_t stream) {
   const int tiles = (dp.n_keys + 15) / 16;
+  dp.leaf = leaf_tiles(tiles, dp.M);
+  constexpr int kSmem4 = sizeof(DecodeSmem<DP, NQ, 4>);
   Split s;
-  consider(s, resident_clusters<decode_kernel<DP, NQ, 4, T, BIAS>>(4), 4, bh, tiles);
-  // twice the warps per head where even 16 CTAs leave SMs idle (one group of rows only: two groups
-  // of partial results would not fit the static shared memory)
-  if constexpr (NQ == 1) consider(s, resident_clusters<decode_kernel<DP, NQ, 8, T, BIAS>>(8), 8, bh, tiles);
+  consider(s, resident_clusters<decode_kernel<DP, NQ, 4, T, BIAS>>(4, kSmem4), 4, DecodeSmem<DP, NQ, 4>::slots(dp.M), bh, tiles, dp.leaf);
+  // twice the warps per head where even 16 CTAs leave SMs idle (one group of rows only: with two the
+  // registers do not allow it)
+  constexpr int kSmem8 = sizeof(DecodeSmem<DP, 1, 8>);
+  if constexpr (NQ == 1)
+    consider(s, resident_clusters<decode_kernel<DP, NQ, 8, T, BIAS>>(8, kSmem8), 8, DecodeSmem<DP, NQ, 8>::slots(dp.M), bh, tiles, dp.leaf);
   if (s.cost < 0) return FA_ERR_CUDA;
+  dp.fold = s.fold;
+  dp.own = s.own;
   if constexpr (NQ == 1)
     if (s.warps == 8)
-      return launch_overlapped(decode_kernel<DP, NQ, 8, T, BIAS>, dim3(s.parts, bh), 256, 0, stream, dp, s.parts);
-  return launch_overlapped(decode_kernel<DP, NQ, 4, T, BIAS>, dim3(s.parts, bh), 128, 0, stream, dp, s.parts);
+      return launch_overlapped(decode_kernel<DP, NQ, 8, T, BIAS>, dim3(s.parts, bh), 256, kSmem8, stream, dp, s.parts);
+  return launch_overlapped(decode_kernel<DP, NQ, 4, T, BIAS>, dim3(s.parts, bh), 128, kSmem4, stream, dp, s.parts);
 }
 
 template <int DP, typename T, int BIAS>
