@@ -26,8 +26,9 @@ Rank 0 prints one JSON line:
   burst        the same for the fastest single step
   e2e          same metric with HOST (pinned) inputs and outputs: H2D of q,k,v,bias,do and D2H
                of out,dq,dk,dv,dbias inside the timed region
-  roofline     dominant kernel (dK/dV) against the measured peaks; "kernels" lists all four, each
-               timed alone through the C ABI in a short loop (full clock: held against the burst
+  roofline     dominant kernel (dK/dV; without a trained bias the whole backward, whose stages share
+               scratch) against the measured peaks; "kernels" lists them all, each timed alone
+               through the C ABI in a short loop (full clock: held against the burst
                tensor peak) and in a long one (held against the sustained tensor peak)
   cpu_baseline fp32 eager oracle on the host cores, on a bounded sample of (b,h) problems
 --impl reference times that CPU oracle alone (the reference project's CPU-runnable path is
@@ -106,7 +107,7 @@ def captured_dkdv_traffic():
 
 def flops(w, which):
     c = 0.5 if w["causal"] else 1.0
-    mult = {"fwd": 4, "bwd": 10, "fwd+bwd": 14, "dkdv": 8, "dq_recompute": 6, "dq_from_ds": 2}[which]
+    mult = {"fwd": 4, "bwd": 10, "fwd+bwd": 14, "dkdv": 8, "dq_from_ds": 2, "bwd_recompute": 14}[which]
     return mult * w["B"] * w["H"] * w["M"] * w["N"] * w["D"] * c
 
 
@@ -125,10 +126,12 @@ def kernel_bytes(w, which):
         return 2 * qd + 4 * B * H * M
     if which == "dkdv":
         return 2 * qd + 4 * kd + bhmn * b * c + (bhmn * 2 if trainable else 0) + 8 * B * H * M
-    if which == "dq":
-        if trainable:  # streams dS (written as dbias) instead of the bias
-            return qd + kd + bhmn * 2 * c
-        return 3 * qd + 2 * kd + bhmn * b * c + 8 * B * H * M
+    if which == "dq":  # streams dS (written as dbias) instead of the bias
+        return qd + kd + bhmn * 2 * c
+    if which == "bwd":  # the whole backward with dS in scratch, written once and read once
+        return (kernel_bytes(w, "pre") + kernel_bytes(w, "dkdv") + qd + kd + bhmn * 4 * c)
+    if which == "bwd_recompute":  # without scratch: dQ reads what dK/dV reads
+        return kernel_bytes(w, "pre") + kernel_bytes(w, "dkdv") + 3 * qd + 2 * kd + bhmn * b * c + 8 * B * H * M
     raise KeyError(which)
 
 
@@ -645,7 +648,9 @@ def verify_shards(w, w_local, shard, q, k, v, bias, do, attn, device, rank, worl
 
 def time_kernels(w, q, k, v, bias, do, trainable, peaks, fa_mod, _cabi, use_capture):
     """Each kernel alone through the C ABI: a short loop (20 launches, full clock; tensor side
-    held against the burst peak) and a long one (>= 0.4 s; held against the sustained peak)."""
+    held against the burst peak) and a long one (>= 0.4 s; held against the sustained peak).
+    Without a trained bias the stages of the backward share scratch for dS, in parts of the
+    problems, so there it is timed as a whole ("bwd"), by the call the public functions make."""
     kernels = {}
     with torch.no_grad():
         scale = w["D"] ** -0.5
@@ -665,15 +670,24 @@ def time_kernels(w, q, k, v, bias, do, trainable, peaks, fa_mod, _cabi, use_capt
             p.dbias, p.dbias_stride = dbias.data_ptr(), fa_mod._stride3(dbias)
         lib = _cabi.load()
         stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        dq_kind = "dq_from_ds" if trainable else "dq_recompute"
         hbm = peaks["hbm_gbs"] * 1e9
-        for name, fn, fl in (("fwd", lib.fa_fwd, flops(w, "fwd")), ("pre", lib.fa_bwd_pre, 0.0),
-                             ("dkdv", lib.fa_bwd_dkdv, flops(w, "dkdv")),
-                             ("dq", lib.fa_bwd_dq, flops(w, dq_kind))):
+        rows = [("fwd", lib.fa_fwd, flops(w, "fwd"), kernel_bytes(w, "fwd"))]
+        if trainable:
+            main_kernel, main_row = "dkdv_kernel", "dkdv"
+            rows += [("pre", lib.fa_bwd_pre, 0.0, kernel_bytes(w, "pre")),
+                     ("dkdv", lib.fa_bwd_dkdv, flops(w, "dkdv"), kernel_bytes(w, "dkdv")),
+                     ("dq", lib.fa_bwd_dq, flops(w, "dq_from_ds"), kernel_bytes(w, "dq"))]
+        else:
+            main_kernel, main_row = "fa_bwd_workspace (pre, dK/dV, dQ)", "bwd"
+            room = lib.fa_bwd_workspace_bytes(ctypes.byref(p))
+            ws = torch.empty(max(room, 16), dtype=torch.uint8, device=q.device)
+            kind = "bwd" if room else "bwd_recompute"
+            rows += [("bwd", lambda params, st: lib.fa_bwd_workspace(params, ws.data_ptr(), room, st), flops(w, kind),
+                      kernel_bytes(w, kind))]
+        for name, fn, fl, nbytes in rows:
             call = lambda fn=fn: _cabi.check(fn(ctypes.byref(p), stream), name)
             for _ in range(3):
                 call()
-            nbytes = kernel_bytes(w, name)
             # a pause first: right after a long loop the GPU still sits at the clock its power
             # cap forced, and a "short loop" number taken then is not a full-clock number
             torch.cuda.synchronize()
@@ -689,17 +703,17 @@ def time_kernels(w, q, k, v, bias, do, trainable, peaks, fa_mod, _cabi, use_capt
                 "long": {"ms": round(t_long, 4), "tflops": round(fl / t_long / 1e9, 1),
                          "gbs": round(nbytes / t_long / 1e6, 1), "roof_ms": round(roof_s, 4),
                          "frac": round(roof_s / t_long, 3)}}
-        kd = kernels["dkdv"]
-        fl, nbytes = flops(w, "dkdv"), kernel_bytes(w, "dkdv")
+        kd = kernels[main_row]
+        fl, nbytes = next(row[2:] for row in rows if row[0] == main_row)
         tensor_bound = fl / (peaks["tflops"] * 1e12) >= nbytes / hbm
         # the dominant kernel in the long loop (the regime of `value`), against the sustained peaks
         if tensor_bound:
-            roofline = {"kernel": "dkdv_kernel", "bound": "tensor", "achieved": kd["long"]["tflops"],
+            roofline = {"kernel": main_kernel, "bound": "tensor", "achieved": kd["long"]["tflops"],
                         "peak": peaks["tflops"], "unit": "TFLOP/s",
                         "frac": round(kd["long"]["tflops"] / peaks["tflops"], 3),
                         "peak_source": peaks["source"] + " sustained bf16"}
         else:
-            roofline = {"kernel": "dkdv_kernel", "bound": "hbm", "achieved": kd["long"]["gbs"],
+            roofline = {"kernel": main_kernel, "bound": "hbm", "achieved": kd["long"]["gbs"],
                         "peak": peaks["hbm_gbs"], "unit": "GB/s",
                         "frac": round(kd["long"]["gbs"] / peaks["hbm_gbs"], 3), "peak_source": peaks["source"]}
         roofline["burst"] = {"achieved_tflops": kd["tflops"], "achieved_gbs": kd["gbs"], "frac": kd["frac"]}

@@ -152,7 +152,9 @@ int fa_bwd(const fa_params* p, void* stream);
  * problems are worked through in parts that fit the workspace.
  *   workspace: 16-byte aligned device memory, contents unspecified before and after;
  *   bytes: any size; fa_bwd_workspace_bytes(p) is what the call works best with (0: it has no
- *     use for one).  Less than the dS of one problem (M rows of N 16-bit values, rows padded
+ *     use for one: dS has its own tensor, or recomputing is faster than parts of so few problems).
+ *     That is at most 1.5 GiB, except at D = 256 and with an fp32 bias, which have no other way to
+ *     dQ: as many problems as fill the SMs, at the most all.  Less than the dS of one problem (M rows of N 16-bit values, rows padded
  *     to 16 bytes), or a null workspace: the call is fa_bwd.
  */
 uint64_t fa_bwd_workspace_bytes(const fa_params* p);

@@ -1,6 +1,8 @@
 // dQ kernels for sm_100a.
 //
-// (1) dq_recompute_kernel -- general path (no bias, bool mask, float bias).
+// (1) dq_recompute_kernel -- where dS is in no memory (no bias, bool mask, frozen 16-bit bias): a backward without
+// scratch, or whose scratch would hold too few problems to pay (fa_api.cu has the rule).  Its dS has the bits of
+// the dK/dV kernel's, so dQ does not depend on which of the two it is.
 // Persistent, one CTA per SM, scheduled like the forward kernel: a tile is 128 query
 // rows of one (batch, head); a CTA walks its tiles and, inside a tile, the key blocks;
 // rings, tensor-memory buffers and barrier phases carry on from tile to tile.
