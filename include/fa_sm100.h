@@ -138,6 +138,16 @@ int fa_fwd(const fa_params* p, void* stream);
 int fa_fwd_takes_any_bias(int M, int D);
 
 /*
+ * Short sequences (fa_small_takes: M, N <= 64 and D <= 64).  fa_fwd, fa_bwd and fa_bwd_workspace use the same kernels
+ * for them and ask of the bias, its gradient and ds16 what they ask at any size.  These two take the bias and write its
+ * gradient at any naturally aligned address with any strides (the innermost is 1), use no ds16 and no scratch, and
+ * leave every element of a gradient of shape (B, H, M, N) written.  Other sizes: FA_ERR_UNSUPPORTED.
+ */
+int fa_small_takes(int M, int N, int D);
+int fa_small_fwd(const fa_params* p, void* stream);
+int fa_small_bwd(const fa_params* p, void* stream);
+
+/*
  * Backward, all three stages in order on `stream`.  Replaces _flash_attn_bwd
  * (FA:688-763): the eager pre-scaled copies of k and bias (FA:699-704) and the
  * zero fill of dbias (FA:799) are folded into the kernels.

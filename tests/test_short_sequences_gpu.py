@@ -1,0 +1,87 @@
+"""The kernels for short sequences (M, N, D <= 64): edges of their 16-row tiles against the fp32 oracle, biases in layouts
+the tile kernels do not take, and what the C entries refuse."""
+import ctypes
+
+import pytest
+import torch
+
+from tests._util import compare, make_inputs, run_ours
+
+pytestmark = pytest.mark.gpu
+BF, HF = torch.bfloat16, torch.float16
+
+
+@pytest.mark.parametrize("M,N", [(1, 1), (16, 64), (17, 1), (17, 17), (33, 47), (48, 49), (49, 49), (64, 16), (64, 64), (64, 65),
+                                 (65, 64)])
+@pytest.mark.parametrize("D,dtype,kind,causal", [(16, HF, "float", False), (32, BF, "float", True), (64, HF, "float", True),
+                                                 (32, HF, "bool", True), (64, BF, "bool", False), (16, BF, None, True),
+                                                 (64, HF, None, False)])
+def test_edges_against_oracle(M, N, D, dtype, kind, causal, device_ok):
+    q, k, v, bias, do = make_inputs(3, M, N, 3, D, dtype, kind, 100 + M + N)
+    ours = run_ours(q, k, v, bias, causal, None, do)
+    compare(ours, q, k, v, bias, causal, None, do, dtype, label=f"{M}x{N}: ")
+
+
+@pytest.mark.parametrize("layout", ["sliced", "heads_last", "expanded", "f32_sliced"])
+def test_bias_in_any_layout(layout, device_ok):
+    """A bias whose rows are not 16-byte aligned, in another order or expanded, gives what its padded copy gives."""
+    B, S, H, D = 3, 49, 4, 32
+    q, k, v, bias, do = make_inputs(B, S, S, H, D, HF, "float", 77)
+    if layout == "f32_sliced":
+        bias = bias.float()
+    if layout == "expanded":
+        bias = bias[:1].expand(B, H, S, S)
+        odd = bias
+    else:
+        shape = (B, S, H, S + 3) if layout == "heads_last" else (B, H, S, S + 3)
+        buf = torch.zeros(shape, dtype=bias.dtype, device="cuda")
+        odd = buf[..., 1:S + 1]
+        if layout == "heads_last":
+            odd = odd.transpose(1, 2)
+        odd.copy_(bias)
+    dense = bias.contiguous()
+    want, got = run_ours(q, k, v, dense, True, None, do), None
+    from triton_flashattn_b200 import flash_attention_fn
+
+    ins = [t.detach().clone().requires_grad_() for t in (q, k, v)]
+    b = odd.detach().requires_grad_()
+    out = flash_attention_fn(*ins, b, True)
+    got = dict(zip(("dq", "dk", "dv", "dbias"), torch.autograd.grad(out, [*ins, b], do)), out=out.detach())
+    for name in want:
+        assert torch.equal(want[name], got[name]), name
+
+
+def test_masked_rows_and_nan(device_ok):
+    """A row without a key gives zeros and zero gradients; a NaN score makes its row NaN."""
+    q, k, v, bias, do = make_inputs(2, 40, 50, 2, 32, BF, "bool", 5)
+    bias[0, 1, 7] = False
+    ours = run_ours(q, k, v, bias, False, None, do)
+    assert not ours["out"][0, 7, 1].any() and not ours["dq"][0, 7, 1].any()
+    assert all(torch.isfinite(t).all() for t in ours.values())
+    q[1, 3, 0, 0] = float("nan")
+    ours = run_ours(q, k, v, None, False, None, do)
+    assert torch.isnan(ours["out"][1, 3, 0]).all() and torch.isfinite(ours["out"][1, 4]).all()
+
+
+def test_c_entries_refuse_what_the_tile_kernels_refuse(device_ok):
+    from triton_flashattn_b200 import _cabi
+
+    lib = _cabi.load()
+    q, k, v, bias, _ = make_inputs(1, 49, 49, 2, 32, BF, "float", 3)
+    o, lse = torch.empty_like(q), torch.empty(1, 2, 49, device="cuda")
+    p = _cabi.FaParams()
+    p.struct_size = ctypes.sizeof(_cabi.FaParams)
+    p.B, p.H, p.M, p.N, p.D, p.dtype, p.bias_kind, p.sm_scale = 1, 2, 49, 49, 32, 1, 1, 0.2
+    for name, t in (("q", q), ("k", k), ("v", v), ("o", o)):
+        setattr(p, name, t.data_ptr())
+        st = t.stride()
+        setattr(p, name + "_stride", _cabi._I64x3(st[0], st[1], st[2]))
+    p.lse, p.bias = lse.data_ptr(), bias.data_ptr()
+    st = bias.stride()
+    p.bias_stride = _cabi._I64x3(st[0], st[1], st[2])
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert lib.fa_fwd(ctypes.byref(p), stream) == 5  # rows of 98 bytes
+    assert lib.fa_small_fwd(ctypes.byref(p), stream) == 0
+    p.M = 65
+    assert lib.fa_small_takes(65, 49, 32) == 0 and lib.fa_small_fwd(ctypes.byref(p), stream) == 8
+    torch.cuda.synchronize()

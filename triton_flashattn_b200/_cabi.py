@@ -68,6 +68,9 @@ EXPORTED_SYMBOLS = (
     "fa_status_string",
     "fa_fwd",
     "fa_fwd_takes_any_bias",
+    "fa_small_takes",
+    "fa_small_fwd",
+    "fa_small_bwd",
     "fa_bwd",
     "fa_bwd_workspace",
     "fa_bwd_workspace_bytes",

@@ -29,6 +29,7 @@ SOURCES = [
     "fa_selftest.cu",
     "fa_fwd.cu",
     "fa_decode.cu",
+    "fa_small.cu",
     "fa_bwd_pre.cu",
     "fa_bwd_dkdv.cu",
     "fa_bwd_dq.cu",

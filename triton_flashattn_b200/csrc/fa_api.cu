@@ -222,7 +222,7 @@ bool parts_pay(const fa_params& p, const PartsCost& parts, int n) {
 }
 
 uint64_t bwd_workspace_bytes(const fa_params& p) {
-  if (ds_is_dbias(p)) return 0;
+  if (ds_is_dbias(p) || (small_takes(p.M, p.N, p.D) && p.bias_kind != FA_BIAS_F32)) return 0;
   const uint64_t one = slab_bytes(p), fit = kSlabCap / one;
   const PartsCost parts(p);
   const int total = parts.total;
@@ -248,6 +248,17 @@ int bwd_in_parts(const fa_params& p, void* ws, uint64_t bytes, cudaStream_t s, i
     if (int e = launch_bwd_dq(p, s, st, &slab)) return e;
   }
   return FA_OK;
+}
+
+// All stages of a backward without scratch.
+int bwd_whole(const fa_params& p, cudaStream_t s, int* st) {
+  if (small_takes(p.M, p.N, p.D)) {
+    if (int e = check_tiled_bias(p, true)) return e;
+    return launch_small(p, true, s, st);
+  }
+  if (int e = launch_bwd_pre(p, s, st)) return e;
+  if (int e = launch_bwd_dkdv(p, s, st)) return e;
+  return launch_bwd_dq(p, s, st);
 }
 
 template <typename F>
@@ -295,6 +306,22 @@ int fa_fwd(const fa_params* p, void* stream) {
 
 int fa_fwd_takes_any_bias(int M, int D) { return decode_takes(M, D) ? 1 : 0; }
 
+int fa_small_takes(int M, int N, int D) { return small_takes(M, N, D) ? 1 : 0; }
+
+int fa_small_fwd(const fa_params* p, void* stream) {
+  int r = validate_common(p);
+  if (r) return r;
+  if (!small_takes(p->M, p->N, p->D)) return FA_ERR_UNSUPPORTED;
+  return with_device(p->device, [&](int* st) { return launch_small(*p, false, static_cast<cudaStream_t>(stream), st); });
+}
+
+int fa_small_bwd(const fa_params* p, void* stream) {
+  int r = validate_bwd(p, true);
+  if (r) return r;
+  if (!small_takes(p->M, p->N, p->D)) return FA_ERR_UNSUPPORTED;
+  return with_device(p->device, [&](int* st) { return launch_small(*p, true, static_cast<cudaStream_t>(stream), st); });
+}
+
 int fa_bwd_pre(const fa_params* p, void* stream) {
   int r = validate_bwd(p);
   if (r) return r;
@@ -322,14 +349,7 @@ int fa_bwd_dq(const fa_params* p, void* stream) {
 int fa_bwd(const fa_params* p, void* stream) {
   int r = validate_bwd(p);
   if (r) return r;
-  return with_device(p->device, [&](int* st) {
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    int e = launch_bwd_pre(*p, s, st);
-    if (e) return e;
-    e = launch_bwd_dkdv(*p, s, st);
-    if (e) return e;
-    return launch_bwd_dq(*p, s, st);
-  });
+  return with_device(p->device, [&](int* st) { return bwd_whole(*p, static_cast<cudaStream_t>(stream), st); });
 }
 
 uint64_t fa_bwd_workspace_bytes(const fa_params* p) {
@@ -350,6 +370,7 @@ int fa_bwd_workspace(const fa_params* p, void* workspace, uint64_t bytes, void* 
   if (reinterpret_cast<uintptr_t>(workspace) % 16 != 0) return FA_ERR_ALIGN;
   return with_device(p->device, [&](int* st) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (small_takes(p->M, p->N, p->D)) return bwd_whole(*p, s, st);
     if (int e = launch_bwd_pre(*p, s, st)) return e;
     return bwd_in_parts(*p, workspace, bytes, s, st);
   });

@@ -736,6 +736,10 @@ int launch_bias(const FwdParams& fp, int bias_kind, dim3 grid, cudaStream_t stre
 
 int launch_fwd(const fa_params& p, cudaStream_t stream, int* status) {
   if (decode_takes(p.M, p.D)) return launch_decode(p, stream, status);
+  if (small_takes(p.M, p.N, p.D)) {
+    if (int e = check_tiled_bias(p, false)) return e;
+    return launch_small(p, false, stream, status);
+  }
   FwdParams fp;
   int r = make_tmap_bshd(&fp.map_q, p.q, p.B, p.M, p.H, p.D, p.q_stride, 128);
   if (r) return r;

@@ -40,6 +40,11 @@ int launch_fwd(const fa_params& p, cudaStream_t stream, int* status);
 // element by element, so that needs no alignment there.
 bool decode_takes(int M, int D);
 int launch_decode(const fa_params& p, cudaStream_t stream, int* status);
+// Short sequences: whether the kernels of fa_small.cu take the problem, and their launch.  They read the bias and write its
+// gradient at any address, with any strides but the innermost; `check_tiled_bias` has what the tile kernels ask of them.
+bool small_takes(int M, int N, int D);
+int launch_small(const fa_params& p, bool bwd, cudaStream_t stream, int* status);
+int check_tiled_bias(const fa_params& p, bool bwd);
 int launch_bwd_pre(const fa_params& p, cudaStream_t stream, int* status);
 // Without a slab: all problems, dS going where the parameters say (dbias, ds16 or nowhere).
 int launch_bwd_dkdv(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab = nullptr);

@@ -170,9 +170,12 @@ Bias classify_bias(const Tensor& bias, at::ScalarType q_dtype, bool any_layout =
   // flash_attention.py 52, 292): nothing is rounded to 16 bits, the gradient comes back in fp32.
   return {ready(dt == at::kFloat ? bias : bias.to(at::kFloat)), FA_BIAS_F32};
 }
-Bias forward_bias(const Shape& s, const Tensor& bias) {
-  return classify_bias(bias, s.dtype, fa_fwd_takes_any_bias(static_cast<int>(s.M), static_cast<int>(s.D)) != 0);
+// Short sequences: the kernels read the bias and write its gradient in any layout.
+bool is_small(const Shape& s) {
+  return fa_small_takes(static_cast<int>(s.M), static_cast<int>(s.N), static_cast<int>(s.D)) != 0;
 }
+bool few_rows(const Shape& s) { return fa_fwd_takes_any_bias(static_cast<int>(s.M), static_cast<int>(s.D)) != 0; }
+Bias forward_bias(const Shape& s, const Tensor& bias) { return classify_bias(bias, s.dtype, few_rows(s) || is_small(s)); }
 
 // ---------------------------------------------------------------------------- argument checks
 std::string shape_text(at::IntArrayRef s) {
@@ -280,15 +283,16 @@ std::tuple<Tensor, Tensor> forward(const Shape& s, const Tensor& like, const Vie
   Tensor o = empty_on(like, {s.B, s.M, s.H, s.D}, s.dtype);
   Tensor lse = empty_on(like, {s.B, s.H, s.M}, at::kFloat);
   const fa_params p = common_params(s, q, k, v, view_of(o), lse, bias, causal, scale);
-  check_code(fa_fwd(&p, stream_of(s.device)), "fa_fwd");
+  check_code(!few_rows(s) && is_small(s) ? fa_small_fwd(&p, stream_of(s.device)) : fa_fwd(&p, stream_of(s.device)), "fa_fwd");
   return {std::move(o), std::move(lse)};
 }
 
 // Backward launches; fills dq, dk, dv and - when defined - dbias.  Replaces _flash_attn_bwd of the
-// reference (flash_attention.py 688-763).
+// reference (flash_attention.py 688-763).  `any_layout`: the bias and dbias may be laid out as only the kernels for
+// short sequences take them (these sequences are).
 void backward(const Shape& s, const Tensor& grad, const View& q, const View& k, const View& v, const Tensor& out,
               const Tensor& lse, const Bias& bias, bool causal, double scale, const View& dq, const View& dk,
-              const View& dv, const Tensor& dbias) {
+              const View& dv, const Tensor& dbias, bool any_layout) {
   raise_if_unhealthy(s.device);
   const Tensor o = tile_ready(out), g = tile_ready(grad);
   Tensor delta = empty_on(o, {s.B, s.H, s.M}, at::kFloat);
@@ -307,6 +311,10 @@ void backward(const Shape& s, const Tensor& grad, const View& q, const View& k, 
     p.write_dbias = 1;
     p.dbias = dbias.mutable_data_ptr();
     set_stride(p.dbias_stride, dbias.strides().data());
+  }
+  if (any_layout) {
+    check_code(fa_small_bwd(&p, stream_of(s.device)), "fa_bwd");
+    return;
   }
   // Scratch for dS where it has no tensor of its own.  Without the memory for all the library asks
   // for, one problem's share; without that, the scores are recomputed where the kernels can.
@@ -342,6 +350,7 @@ Tensor grad_like(const Tensor& t) {
 // gradients; every gradient at head dim 256).
 Tensor new_dbias(const Shape& s, const Tensor& bias, bool causal) {
   const bool same = bias.scalar_type() == s.dtype;
+  if (is_small(s)) return empty_on(bias, {s.B, s.H, s.M, s.N}, same ? s.dtype : at::kFloat);  // dense, all of it is written
   return pitched_empty(bias, {s.B, s.H, s.M, s.N}, same ? s.dtype : at::kFloat, causal && (!same || s.D == 256));
 }
 // Gradient as the reference returns it (flash_attention.py 799): dense, in the bias's own dtype.
@@ -384,11 +393,11 @@ struct AttentionBackward : public torch::autograd::Node {
     at::AutoDispatchBelowADInplaceOrView guard;
     // an upstream function that returned no gradient counts as zeros, as for a Python autograd function
     const Tensor grad = grads[0].defined() ? grads[0] : at::zeros_like(out);
-    const auto bias_for = [&](at::ScalarType dt) {
+    const auto bias_for = [&](at::ScalarType dt, bool any_layout) {
       return bias_copy_.defined() ? Bias{bias_copy_, bias.scalar_type() == at::kBool ? FA_BIAS_BOOL
                                                      : bias.scalar_type() == dt      ? FA_BIAS_SAME
                                                                                      : FA_BIAS_F32}
-                                  : classify_bias(bias, dt);
+                                  : classify_bias(bias, dt, any_layout);
     };
     if (packed_) {
       const Shape s = check_packed(a0, bias);
@@ -396,8 +405,8 @@ struct AttentionBackward : public torch::autograd::Node {
       const Tensor qkv = packed_ready(a0);
       Tensor dqkv = empty_on(qkv, qkv.sizes(), s.dtype);
       Tensor dbias = train_bias_ ? new_dbias(s, bias, causal_) : Tensor();
-      backward(s, grad, slice_of(qkv, 0), slice_of(qkv, 1), slice_of(qkv, 2), out, lse, bias_for(s.dtype), causal_,
-               scale_, slice_of(dqkv, 0), slice_of(dqkv, 1), slice_of(dqkv, 2), dbias);
+      backward(s, grad, slice_of(qkv, 0), slice_of(qkv, 1), slice_of(qkv, 2), out, lse, bias_for(s.dtype, is_small(s)),
+               causal_, scale_, slice_of(dqkv, 0), slice_of(dqkv, 1), slice_of(dqkv, 2), dbias, is_small(s));
       res[0] = std::move(dqkv);
       if (train_bias_) res[1] = finish_dbias(dbias, bias.scalar_type());
       return res;
@@ -408,8 +417,8 @@ struct AttentionBackward : public torch::autograd::Node {
     const Tensor q = tile_ready(a0), k = tile_ready(k0), v = tile_ready(v0);
     Tensor dq = grad_like(a0), dk = grad_like(k0), dv = grad_like(v0);
     Tensor dbias = train_bias_ ? new_dbias(s, bias, causal_) : Tensor();
-    backward(s, grad, view_of(q), view_of(k), view_of(v), out, lse, bias_for(s.dtype), causal_, scale_, view_of(dq),
-             view_of(dk), view_of(dv), dbias);
+    backward(s, grad, view_of(q), view_of(k), view_of(v), out, lse, bias_for(s.dtype, is_small(s)), causal_, scale_,
+             view_of(dq), view_of(dk), view_of(dv), dbias, is_small(s));
     res[0] = std::move(dq);
     res[1] = std::move(dk);
     res[2] = std::move(dv);
@@ -578,7 +587,7 @@ PyObject* py_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
     at::AutoDispatchBelowADInplaceOrView guard;
     const Tensor q = tile_ready(q0), k = tile_ready(k0), v = tile_ready(v0);
     backward(s, g, view_of(q), view_of(k), view_of(v), o, lse, classify_bias(bias, s.dtype), causal, scale,
-             view_of(dq), view_of(dk), view_of(dv), dbias);
+             view_of(dq), view_of(dk), view_of(dv), dbias, false);
     Py_RETURN_NONE;
   });
 }
