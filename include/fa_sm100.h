@@ -148,6 +148,16 @@ int fa_small_fwd(const fa_params* p, void* stream);
 int fa_small_bwd(const fa_params* p, void* stream);
 
 /*
+ * Copies for callers whose bias does not meet the 16-byte rule, in elements of elem_bytes (1, 2, 4; strides and pitch in
+ * elements, the innermost is 1).  fa_pad_rows: a (B, H, M, N) tensor of any strides (0 included) into rows that start at
+ * multiples of 16 bytes; the last 16-byte unit of each row is filled up with zeros.  fa_pack_rows (2 or 4 bytes): rows of
+ * one pitch into a dense, 16-byte aligned tensor.
+ */
+int fa_pad_rows(void* dst, const int64_t dst_stride[3], const void* src, const int64_t src_stride[3], int elem_bytes, int B, int H,
+                int M, int N, int device, void* stream);
+int fa_pack_rows(void* dst, const void* src, int64_t pitch, int elem_bytes, int64_t rows, int N, int device, void* stream);
+
+/*
  * Backward, all three stages in order on `stream`.  Replaces _flash_attn_bwd
  * (FA:688-763): the eager pre-scaled copies of k and bias (FA:699-704) and the
  * zero fill of dbias (FA:799) are folded into the kernels.

@@ -71,6 +71,8 @@ EXPORTED_SYMBOLS = (
     "fa_small_takes",
     "fa_small_fwd",
     "fa_small_bwd",
+    "fa_pad_rows",
+    "fa_pack_rows",
     "fa_bwd",
     "fa_bwd_workspace",
     "fa_bwd_workspace_bytes",

@@ -30,6 +30,7 @@ SOURCES = [
     "fa_fwd.cu",
     "fa_decode.cu",
     "fa_small.cu",
+    "fa_copy.cu",
     "fa_bwd_pre.cu",
     "fa_bwd_dkdv.cu",
     "fa_bwd_dq.cu",

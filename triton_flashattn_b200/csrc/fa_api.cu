@@ -322,6 +322,25 @@ int fa_small_bwd(const fa_params* p, void* stream) {
   return with_device(p->device, [&](int* st) { return launch_small(*p, true, static_cast<cudaStream_t>(stream), st); });
 }
 
+int fa_pad_rows(void* dst, const int64_t dst_stride[3], const void* src, const int64_t src_stride[3], int elem_bytes, int B, int H,
+                int M, int N, int device, void* stream) {
+  if (!dst || !src || !dst_stride || !src_stride) return FA_ERR_NULL;
+  if (B < 1 || H < 1 || M < 1 || N < 1) return FA_ERR_SHAPE;
+  if (elem_bytes != 1 && elem_bytes != 2 && elem_bytes != 4) return FA_ERR_DTYPE;
+  return with_device(device, [&](int*) {
+    return launch_pad_rows(dst, dst_stride, src, src_stride, elem_bytes, B, H, M, N, static_cast<cudaStream_t>(stream));
+  });
+}
+
+int fa_pack_rows(void* dst, const void* src, int64_t pitch, int elem_bytes, int64_t rows, int N, int device, void* stream) {
+  if (!dst || !src) return FA_ERR_NULL;
+  if (rows < 1 || N < 1 || pitch < N) return FA_ERR_SHAPE;
+  if (elem_bytes != 2 && elem_bytes != 4) return FA_ERR_DTYPE;
+  return with_device(device, [&](int*) {
+    return launch_pack_rows(dst, src, pitch, elem_bytes, rows, N, static_cast<cudaStream_t>(stream));
+  });
+}
+
 int fa_bwd_pre(const fa_params* p, void* stream) {
   int r = validate_bwd(p);
   if (r) return r;

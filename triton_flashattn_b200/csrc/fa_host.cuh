@@ -45,6 +45,10 @@ int launch_decode(const fa_params& p, cudaStream_t stream, int* status);
 bool small_takes(int M, int N, int D);
 int launch_small(const fa_params& p, bool bwd, cudaStream_t stream, int* status);
 int check_tiled_bias(const fa_params& p, bool bwd);
+// Row copies (fa_copy.cu); strides and pitch in elements of `eb` bytes.
+int launch_pad_rows(void* dst, const int64_t dst_stride[3], const void* src, const int64_t src_stride[3], int eb, int B, int H, int M,
+                    int N, cudaStream_t stream);
+int launch_pack_rows(void* dst, const void* src, int64_t pitch, int eb, int64_t rows, int N, cudaStream_t stream);
 int launch_bwd_pre(const fa_params& p, cudaStream_t stream, int* status);
 // Without a slab: all problems, dS going where the parameters say (dbias, ds16 or nowhere).
 int launch_bwd_dkdv(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab = nullptr);

@@ -108,6 +108,8 @@ View slice_of(const Tensor& qkv, int i) {
   return View{static_cast<char*>(const_cast<void*>(qkv.const_data_ptr())) + i * st[2] * 2, {st[0], st[1], st[3]}};
 }
 
+void* stream_of(int device) { return c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream(); }
+
 Tensor empty_on(const Tensor& like, at::IntArrayRef size, at::ScalarType dtype) {
   return at::detail::empty_cuda(size, dtype, like.device(), std::nullopt);
 }
@@ -142,7 +144,12 @@ Tensor bias_ready(const Tensor& bias) {
   const int64_t n_pad = (sz[3] + align - 1) / align * align;
   const int64_t b = st[0] == 0 ? 1 : sz[0], h = st[1] == 0 ? 1 : sz[1];
   Tensor out = empty_on(bias, {b, h, sz[2], n_pad}, bias.scalar_type()).narrow(3, 0, sz[3]);
-  out.copy_(bias.narrow(0, 0, b).narrow(1, 0, h));
+  const int eb = static_cast<int>(bias.element_size());
+  if (st[3] != 1 || eb > 4 ||
+      fa_pad_rows(out.mutable_data_ptr(), out.strides().data(), bias.const_data_ptr(), st.data(), eb, static_cast<int>(b),
+                  static_cast<int>(h), static_cast<int>(sz[2]), static_cast<int>(sz[3]), bias.get_device(),
+                  stream_of(bias.get_device())) != FA_OK)
+    out.copy_(bias.narrow(0, 0, b).narrow(1, 0, h));  // another inner stride, or too large for it
   return out.expand(sz);
 }
 
@@ -273,8 +280,6 @@ fa_params common_params(const Shape& s, const View& q, const View& k, const View
   return p;
 }
 
-void* stream_of(int device) { return c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream(); }
-
 // Forward launch: (out (B, M, H, D), log2-domain log-sum-exp (B, H, M) fp32).  Replaces
 // _flash_attn_fwd of the reference (flash_attention.py 649-685).
 std::tuple<Tensor, Tensor> forward(const Shape& s, const Tensor& like, const View& q, const View& k, const View& v,
@@ -356,7 +361,13 @@ Tensor new_dbias(const Shape& s, const Tensor& bias, bool causal) {
 // Gradient as the reference returns it (flash_attention.py 799): dense, in the bias's own dtype.
 Tensor finish_dbias(const Tensor& dbias, at::ScalarType dtype) {
   if (dbias.scalar_type() != dtype) return dbias.to(dtype);  // also compacts a padded buffer
-  return dbias.contiguous();
+  if (dbias.is_contiguous()) return dbias;
+  const auto sz = dbias.sizes();
+  Tensor out = empty_on(dbias, sz, dtype);
+  if (fa_pack_rows(out.mutable_data_ptr(), dbias.const_data_ptr(), dbias.stride(2), static_cast<int>(dbias.element_size()),
+                   sz[0] * sz[1] * sz[2], static_cast<int>(sz[3]), dbias.get_device(), stream_of(dbias.get_device())) != FA_OK)
+    out.copy_(dbias);
+  return out;
 }
 
 // ---------------------------------------------------------------------------- autograd
