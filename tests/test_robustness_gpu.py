@@ -415,3 +415,16 @@ def test_scratch_size_is_cheap_to_ask_for(device_ok):
             lib.fa_bwd_workspace_bytes(ctypes.byref(p))
             best = min(best, time.perf_counter() - start)
         assert best < 40e-6, f"B{p.B} H{p.H} M{p.M}: {best * 1e6:.0f} us"
+
+
+@pytest.mark.parametrize("M,N", [(1024, 1024), (300, 700), (700, 300)])
+@pytest.mark.parametrize("bias_kind", [None, "float", "bool"])
+def test_causal_gradients_do_not_depend_on_the_schedule(M, N, bias_kind, device_ok, monkeypatch):
+    """Few causal key blocks per CTA go longest first, many in pairs of a long and a short one: the same bits."""
+    q, k, v, bias, do = make_inputs(2, M, N, 3, 64, BF, bias_kind, 71)
+    want = run_ours(q, k, v, bias, True, None, do)
+    for ctas in (1, 7):
+        monkeypatch.setenv("FA_MAX_CTAS", str(ctas))
+        got = run_ours(q, k, v, bias, True, None, do)
+        for name in want:
+            assert torch.equal(want[name], got[name]), (name, ctas)
