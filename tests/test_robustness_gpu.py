@@ -8,7 +8,7 @@ import pytest
 import torch
 
 from oracle import eager_oracle as oracle
-from tests._util import accept, account, make_inputs
+from tests._util import accept, account, make_inputs, run_ours
 
 pytestmark = pytest.mark.gpu
 
