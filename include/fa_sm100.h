@@ -151,7 +151,8 @@ int fa_small_bwd(const fa_params* p, void* stream);
  * Copies for callers whose bias does not meet the 16-byte rule, in elements of elem_bytes (1, 2, 4; strides and pitch in
  * elements, the innermost is 1).  fa_pad_rows: a (B, H, M, N) tensor of any strides (0 included) into rows that start at
  * multiples of 16 bytes; the last 16-byte unit of each row is filled up with zeros.  fa_pack_rows (2 or 4 bytes): rows of
- * one pitch into a dense, 16-byte aligned tensor.
+ * one pitch into a dense, 16-byte aligned tensor.  A row of more than 2^31 - 17 bytes is FA_ERR_TOO_LARGE, as are more than
+ * 65535 (batch, head) pairs or 16 GiB a pair in fa_pad_rows.
  */
 int fa_pad_rows(void* dst, const int64_t dst_stride[3], const void* src, const int64_t src_stride[3], int elem_bytes, int B, int H,
                 int M, int N, int device, void* stream);

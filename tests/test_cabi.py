@@ -86,6 +86,22 @@ def test_selftest_entry_validates_arguments():
     assert lib.fa_last_device_status(0, None) == 2
 
 
+@pytest.mark.parametrize("elem_bytes", [1, 2, 4])
+def test_row_copies_refuse_rows_that_32_bits_cannot_count(elem_bytes):
+    """Before any CUDA call: such a row would be taken for an empty or a negative one.  The longest row that fits gets as far as
+    the device (-1, an error of its own)."""
+    lib = _cabi.load()
+    buf = ctypes.create_string_buffer(64)
+    at = ctypes.c_void_p(ctypes.addressof(buf))
+    st = (ctypes.c_int64 * 3)(0, 0, 0)
+    longest = (2**31 - 17) // elem_bytes
+    for n in (longest + 1, 2**31 // elem_bytes - 1, 2**31 - 1):
+        assert lib.fa_pad_rows(at, st, at, st, elem_bytes, 1, 1, 1, n, -1, None) == 9  # FA_ERR_TOO_LARGE
+        if elem_bytes > 1:
+            assert lib.fa_pack_rows(at, at, ctypes.c_int64(n), elem_bytes, ctypes.c_int64(1), n, -1, None) == 9
+    assert lib.fa_pad_rows(at, st, at, st, elem_bytes, 1, 1, 1, longest, -1, None) == 6  # FA_ERR_CUDA
+
+
 def test_public_api_rejects_cpu_tensors_loudly():
     import torch
     from triton_flashattn_b200 import flash_attention_fn

@@ -261,6 +261,9 @@ int bwd_whole(const fa_params& p, cudaStream_t s, int* st) {
   return launch_bwd_dq(p, s, st);
 }
 
+// The row copies count the bytes of a row, and places up to 16 bytes behind its end, in 32 bits.
+bool row_fits_copy(int N, int elem_bytes) { return static_cast<int64_t>(N) * elem_bytes <= INT32_MAX - 16; }
+
 template <typename F>
 int with_device(int device, F&& f) {
   DeviceGuard g(device);
@@ -327,6 +330,7 @@ int fa_pad_rows(void* dst, const int64_t dst_stride[3], const void* src, const i
   if (!dst || !src || !dst_stride || !src_stride) return FA_ERR_NULL;
   if (B < 1 || H < 1 || M < 1 || N < 1) return FA_ERR_SHAPE;
   if (elem_bytes != 1 && elem_bytes != 2 && elem_bytes != 4) return FA_ERR_DTYPE;
+  if (!row_fits_copy(N, elem_bytes)) return FA_ERR_TOO_LARGE;
   return with_device(device, [&](int*) {
     return launch_pad_rows(dst, dst_stride, src, src_stride, elem_bytes, B, H, M, N, static_cast<cudaStream_t>(stream));
   });
@@ -336,6 +340,7 @@ int fa_pack_rows(void* dst, const void* src, int64_t pitch, int elem_bytes, int6
   if (!dst || !src) return FA_ERR_NULL;
   if (rows < 1 || N < 1 || pitch < N) return FA_ERR_SHAPE;
   if (elem_bytes != 2 && elem_bytes != 4) return FA_ERR_DTYPE;
+  if (!row_fits_copy(N, elem_bytes)) return FA_ERR_TOO_LARGE;
   return with_device(device, [&](int*) {
     return launch_pack_rows(dst, src, pitch, elem_bytes, rows, N, static_cast<cudaStream_t>(stream));
   });

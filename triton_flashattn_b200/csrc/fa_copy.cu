@@ -35,7 +35,7 @@ struct RowsParams {
   const uint8_t* src;
   uint8_t* dst;
   int64_t s_sB, s_sH, s_sM, d_sB, d_sH, d_sM;  // bytes
-  int H, M, row_bytes, chunks;
+  int H, M, row_bytes, chunks;  // (row_bytes + 16 fits, see row_fits_copy)
 };
 // Into rows whose starts are multiples of 16 bytes; the last unit of a row is filled up with zeros.
 __global__ void __launch_bounds__(256) pad_rows_kernel(const RowsParams p) {

@@ -145,7 +145,7 @@ Tensor bias_ready(const Tensor& bias) {
   const int64_t b = st[0] == 0 ? 1 : sz[0], h = st[1] == 0 ? 1 : sz[1];
   Tensor out = empty_on(bias, {b, h, sz[2], n_pad}, bias.scalar_type()).narrow(3, 0, sz[3]);
   const int eb = static_cast<int>(bias.element_size());
-  if (st[3] != 1 || eb > 4 ||
+  if (st[3] != 1 || eb > 4 || sz[2] > INT32_MAX || sz[3] > INT32_MAX ||
       fa_pad_rows(out.mutable_data_ptr(), out.strides().data(), bias.const_data_ptr(), st.data(), eb, static_cast<int>(b),
                   static_cast<int>(h), static_cast<int>(sz[2]), static_cast<int>(sz[3]), bias.get_device(),
                   stream_of(bias.get_device())) != FA_OK)
@@ -364,7 +364,8 @@ Tensor finish_dbias(const Tensor& dbias, at::ScalarType dtype) {
   if (dbias.is_contiguous()) return dbias;
   const auto sz = dbias.sizes();
   Tensor out = empty_on(dbias, sz, dtype);
-  if (fa_pack_rows(out.mutable_data_ptr(), dbias.const_data_ptr(), dbias.stride(2), static_cast<int>(dbias.element_size()),
+  if (sz[3] > INT32_MAX ||
+      fa_pack_rows(out.mutable_data_ptr(), dbias.const_data_ptr(), dbias.stride(2), static_cast<int>(dbias.element_size()),
                    sz[0] * sz[1] * sz[2], static_cast<int>(sz[3]), dbias.get_device(), stream_of(dbias.get_device())) != FA_OK)
     out.copy_(dbias);
   return out;
