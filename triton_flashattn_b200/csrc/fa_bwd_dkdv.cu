@@ -63,8 +63,6 @@ struct DkdvParams {
   int n_nblk, n_tiles;  // key blocks per (batch, head); tiles of this launch
   int bh0;              // first (batch, head) of this launch
   int ds_flat;          // dS goes to slabs numbered from bh0 instead of a (B, H, M, N) tensor
-  int n_bh;             // problems of this launch
-  int longest_first;    // schedule: see tile_at
   int causal, bias_vec32, bias_b_mul, bias_h_mul;
   int dkv_vec32;  // dk / dv bases and strides are multiples of 32 bytes
   int store_ds;    // the 16-bit dS tiles go out through map_dbias (as dbias, or as scratch for dQ)
@@ -73,6 +71,7 @@ struct DkdvParams {
   int64_t dbf_sB, dbf_sH, dbf_sM;
   float scale_log2;  // sm_scale * log2(e)
   float sm_scale;
+  int n_bh;  // problems of this launch
 };
 
 enum DkdvSite { kSiteKV = 1, kSiteQFull, kSiteQEmpty, kSiteDoFull, kSiteDoEmpty, kSiteSFull,
@@ -93,7 +92,7 @@ struct DkdvSmem {
   static constexpr int kDynamic = kTotal + 1024;
 };
 
-template <int DP, typename T, int BIAS>
+template <int DP, typename T, int BIAS, bool LONGEST_FIRST>
 __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ DkdvParams p) {
   using L = DkdvSmem<DP>;
   using P2 = Pack2<T>;
@@ -127,11 +126,13 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
   // that CTAs running at the same time work on neighbouring tiles and share Q / dO in L2.  A
   // unit is one tile, or - causal - two consecutive entries of the per-(batch, head) order
   // [first, last, first+1, last-1, ...]: a heavy and a light key block.
-  // With longest_first (causal, few tiles a CTA) the tiles are numbered by length instead, and the CTAs take them in rows,
-  // every second row from the other end: what a CTA has too much of in one row it has too little of in the next.
+  // With LONGEST_FIRST (causal, few tiles a CTA) the tiles are numbered by length instead, and the CTAs take them in rows,
+  // every second row from the other end: what a CTA has too much of in one row it has too little of in the next.  It is a
+  // variant of its own because every role walks the schedule: chosen at run time it cost every short tile of the others
+  // (trained bias shared by the batch, 72 x 72, B539 H3 D16 44.4 -> 49.0 us, 100 x 100, B600 H4 D64 69.0 -> 74.3).
   const int sched_sh = p.causal ? 1 : 0;
   auto tile_at = [&](int it, int& bh, int& nb, int& i_start, int& T_steps) -> bool {
-    if (p.longest_first) {
+    if constexpr (LONGEST_FIRST) {
       const int G = static_cast<int>(gridDim.x), c = static_cast<int>(blockIdx.x);
       const int k = it * G + ((it & 1) ? G - 1 - c : c);
       if (k >= p.n_tiles) return false;
@@ -762,10 +763,10 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
   if (warp == 17) tmem_dealloc(tmem, kTmemCols);
 }
 
-template <int DP, typename T, int BIAS>
+template <int DP, typename T, int BIAS, bool LONGEST_FIRST>
 int launch_inst(const DkdvParams& kp, dim3 grid, cudaStream_t stream) {
   using L = DkdvSmem<DP>;
-  auto kern = dkdv_kernel<DP, T, BIAS>;
+  auto kern = dkdv_kernel<DP, T, BIAS, LONGEST_FIRST>;
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -778,15 +779,24 @@ int launch_inst(const DkdvParams& kp, dim3 grid, cudaStream_t stream) {
   return launch_overlapped(kern, grid, 640, L::kDynamic, stream, kp);
 }
 
-template <int DP, typename T>
+template <int DP, typename T, bool LONGEST_FIRST>
 int launch_bias(const DkdvParams& kp, int bias_kind, dim3 grid, cudaStream_t stream) {
   switch (bias_kind) {
-    case FA_BIAS_NONE: return launch_inst<DP, T, 0>(kp, grid, stream);
-    case FA_BIAS_SAME: return launch_inst<DP, T, 1>(kp, grid, stream);
-    case FA_BIAS_BOOL: return launch_inst<DP, T, 2>(kp, grid, stream);
-    case FA_BIAS_F32: return launch_inst<DP, T, 3>(kp, grid, stream);
+    case FA_BIAS_NONE: return launch_inst<DP, T, 0, LONGEST_FIRST>(kp, grid, stream);
+    case FA_BIAS_SAME: return launch_inst<DP, T, 1, LONGEST_FIRST>(kp, grid, stream);
+    case FA_BIAS_BOOL: return launch_inst<DP, T, 2, LONGEST_FIRST>(kp, grid, stream);
+    case FA_BIAS_F32: return launch_inst<DP, T, 3, LONGEST_FIRST>(kp, grid, stream);
     default: return FA_ERR_UNSUPPORTED;
   }
+}
+template <bool LONGEST_FIRST>
+int launch_dim(const DkdvParams& kp, int dtype, int bias_kind, dim3 grid, cudaStream_t stream) {
+  const bool dp64 = padded_head_dim(kp.D) == 64;
+  if (dtype == FA_BF16)
+    return dp64 ? launch_bias<64, __nv_bfloat16, LONGEST_FIRST>(kp, bias_kind, grid, stream)
+                : launch_bias<128, __nv_bfloat16, LONGEST_FIRST>(kp, bias_kind, grid, stream);
+  return dp64 ? launch_bias<64, __half, LONGEST_FIRST>(kp, bias_kind, grid, stream)
+              : launch_bias<128, __half, LONGEST_FIRST>(kp, bias_kind, grid, stream);
 }
 
 }  // namespace
@@ -901,15 +911,10 @@ int launch_bwd_dkdv(const fa_params& p, cudaStream_t stream, int* status, const 
   // 71.9 / 70.4, 16-bit bias 91.4 / 92.2, mask 76.9 / 75.5; H8 S8192 D128, bias (0.86) 571 / 544; B2 H8 S2048 D64 (0.86)
   // 62.7 / 59.1; B8 H12 S512 D64 (0.65) 45.3 / 38.2; H12 S2048 D128, mask (0.65) 76.5 / 71.5; B2 H16 S512 D64 (0.43) 27.1 / 24.6.
   const int sms = persistent_grid(1 << 30), turns = (units + sms - 1) / sms;
-  kp.longest_first = p.causal && kp.n_tiles <= 4 * sms && 8 * units < 7 * turns * sms;
-  const dim3 grid(persistent_grid(kp.longest_first ? kp.n_tiles : units));
-  const int dp = padded_head_dim(p.D);
-  if (p.dtype == FA_BF16) {
-    return dp == 64 ? launch_bias<64, __nv_bfloat16>(kp, p.bias_kind, grid, stream)
-                    : launch_bias<128, __nv_bfloat16>(kp, p.bias_kind, grid, stream);
-  }
-  return dp == 64 ? launch_bias<64, __half>(kp, p.bias_kind, grid, stream)
-                  : launch_bias<128, __half>(kp, p.bias_kind, grid, stream);
+  const bool longest_first = p.causal && kp.n_tiles <= 4 * sms && 8 * units < 7 * turns * sms;
+  const dim3 grid(persistent_grid(longest_first ? kp.n_tiles : units));
+  return longest_first ? launch_dim<true>(kp, p.dtype, p.bias_kind, grid, stream)
+                       : launch_dim<false>(kp, p.dtype, p.bias_kind, grid, stream);
 }
 
 }  // namespace fa
