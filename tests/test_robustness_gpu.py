@@ -417,14 +417,48 @@ def test_scratch_size_is_cheap_to_ask_for(device_ok):
         assert best < 40e-6, f"B{p.B} H{p.H} M{p.M}: {best * 1e6:.0f} us"
 
 
-@pytest.mark.parametrize("M,N", [(1024, 1024), (300, 700), (700, 300)])
-@pytest.mark.parametrize("bias_kind", [None, "float", "bool"])
-def test_causal_gradients_do_not_depend_on_the_schedule(M, N, bias_kind, device_ok, monkeypatch):
-    """Few causal key blocks per CTA go longest first, many in pairs of a long and a short one: the same bits."""
-    q, k, v, bias, do = make_inputs(2, M, N, 3, 64, BF, bias_kind, 71)
+# Caps on the grid at which a causal dK/dV of six problems goes longest first in three or four rows of tiles, in two, and in
+# one (a quarter of the tiles a CTA, or more, is the most it takes; one CTA always goes by pairs).
+@pytest.mark.parametrize("M,N,caps", [(1024, 1024, (15, 17, 30)), (300, 700, (9, 11, 25)), (700, 300, (6, 7, 10)), (640, 640, (8, 13, 20))])
+@pytest.mark.parametrize("D,bias_kind", [(64, None), (64, "float"), (64, "bool"), (64, "f32"), (128, None), (128, "float"),
+                                         (128, "bool"), (128, "f32")])
+def test_causal_gradients_do_not_depend_on_the_schedule(M, N, caps, D, bias_kind, device_ok, monkeypatch):
+    """Few causal key blocks per CTA go longest first, many in pairs of a long and a short one: the same bits, also with key
+    blocks that no query sees (M < N) and with several rows of tiles, every second one from the other end."""
+    q, k, v, bias, do = make_inputs(2, M, N, 3, D, BF, "float" if bias_kind == "f32" else bias_kind, 71)
+    if bias_kind == "f32":
+        bias = bias.float()
+    monkeypatch.setenv("FA_MAX_CTAS", "1")
     want = run_ours(q, k, v, bias, True, None, do)
-    for ctas in (1, 7):
+    for ctas in (*caps, 148):
         monkeypatch.setenv("FA_MAX_CTAS", str(ctas))
         got = run_ours(q, k, v, bias, True, None, do)
         for name in want:
             assert torch.equal(want[name], got[name]), (name, ctas)
+
+
+@pytest.mark.parametrize("D,M,N,bias_kind,ctas", [(64, 300, 700, None, 5), (128, 1024, 1024, None, 5), (128, 700, 300, "bool", 2),
+                                                  (64, 1024, 1024, "bool", 5)])
+def test_longest_first_over_slabs(D, M, N, bias_kind, ctas, device_ok, monkeypatch):
+    """The same with dS in slabs, two of six problems at a time (parts that begin behind the first problem), each part
+    longest first in three or four rows of tiles: the bits of one CTA that goes by pairs."""
+    from triton_flashattn_b200 import _cabi
+    from triton_flashattn_b200 import flash_attention as fa
+
+    lib = _cabi.load()
+    q, k, v, bias, do = make_inputs(2, M, N, 3, D, BF, bias_kind, 72)
+    o, lse = fa._flash_attn_fwd(q, k, v, bias, True, 0.1)
+    delta = torch.empty_like(lse)
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    one = M * ((N + 7) // 8 * 8) * 2
+    ws = torch.empty(2 * one, dtype=torch.uint8, device="cuda")
+    results = []
+    for cap, room in ((1, 0), (ctas, 2), (1, 2)):
+        monkeypatch.setenv("FA_MAX_CTAS", str(cap))
+        grads = [torch.full_like(t, 7.0) for t in (q, k, v)]
+        p, keep = _bwd_params(fa, q, k, v, o, lse, bias, True, 0.1, do, *grads, None, delta)
+        _cabi.check(lib.fa_bwd_workspace(ctypes.byref(p), ws.data_ptr() if room else None, ctypes.c_uint64(room * one), stream), "bwd")
+        results.append(grads)
+    for grads in results[1:]:
+        for name, a, b in zip(("dq", "dk", "dv"), grads, results[0]):
+            assert torch.equal(a, b), name

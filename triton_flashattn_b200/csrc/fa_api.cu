@@ -174,20 +174,26 @@ uint64_t slab_bytes(const fa_params& p) { return (uint64_t)slab_pitch(p) * p.M *
 
 // What a backward in parts of n problems costs in the dK/dV stage.
 struct PartsCost {
-  int total, tiles, sms;
-  bool pairs;  // a causal unit is a heavy and a light tile
+  static constexpr int kTurn = 48;  // the unit: a 48th of a turn of one work unit per SM
+  const fa_params& p;
+  int total, tiles, sms, pair;
   explicit PartsCost(const fa_params& p)
-      : total(p.B * p.H), tiles((p.N + 127) / 128), sms(persistent_grid(1 << 30)), pairs(p.causal != 0) {}
-  // Turns of one work unit per SM that the persistent grids need for all problems, n at a time.
+      : p(p), total(p.B * p.H), tiles((p.N + 127) / 128), sms(persistent_grid(1 << 30)), pair(dkdv_pair_work(p)) {}
+  // Time the persistent grids need for all problems, n at a time: full turns, or what the longest CTA does where a
+  // causal launch goes longest first.  (A causal unit is a heavy and a light tile.)
   int64_t turns(int n) const {
-    auto of = [&](int problems) {
+    auto of = [&](int problems) -> int64_t {
+      if (problems == 0) return 0;
+      if (p.causal && p.D <= 128)
+        if (const DkdvPlan plan = plan_dkdv(p, problems, sms, false); plan.longest_first)
+          return (static_cast<int64_t>(kTurn) * plan.span + pair - 1) / pair;
       const int64_t k = (int64_t)problems * tiles;
-      return ((pairs ? (k + 1) / 2 : k) + sms - 1) / sms;
+      return kTurn * (((p.causal ? (k + 1) / 2 : k) + sms - 1) / sms);
     };
     return total / n * of(n) + of(total % n);
   }
-  // In thirds of a turn: every part costs about one more for its two launches and its drained tail.
-  int64_t cost(int n) const { return 3 * turns(n) + (total + n - 1) / n; }
+  // Every part costs about a third of a turn more for its two launches and its drained tail.
+  int64_t cost(int n) const { return turns(n) + kTurn / 3 * ((total + n - 1) / n); }
   // Problems per part, at most `most`: the number of least cost.  Among thousands of small problems one more
   // or less changes little, and a few hundred numbers are looked at (all of them took up to 0.1 ms a call).
   int best(int most) const {
@@ -209,16 +215,18 @@ constexpr uint64_t kSlabCap = 3ull << 29;
 // Whether a backward in parts of n problems is faster than one with the recomputing dQ kernel.  Without a turn
 // lost that kernel costs more than the streamed product by a share of the dK/dV time that depends on what it
 // recomputes: three products instead of one at D = 128, little more than the traffic of dS at D = 64, and the
-// bias or mask.  Backward alone, bf16, recomputing / in parts, us (turns / turns in parts, parts):
-//   D 128: H8 S16384 causal (4 / 4, 4) 1760 / 1580      H8 S16384 (7 / 8, 3) 3230 / 3250
-//          H8 S20480 causal (5 / 8, 8) 2900 / 3900      H5 S27000 causal (4 / 5, 5) 3200 / 3300
-//   D 64:  B16 H32 S2048 (56 / 56, 3) 2820 / 2759       the same causal (28 / 28, 3) 1657 / 1531
-//          B4 H32 S4096 (28 / 28, 3) 2692 / 2708        B2 H16 S8192 causal (7 / 8, 4) 1359 / 1467
-//          H16 S8192 (7 / 8, 2) 1312 / 1442             the same causal (4 / 4, 2) 773 / 741
-//          H32 S12288 causal (11 / 11, 11) 3057 / 3285  B2 H12 S8192 causal, mask (6 / 6, 2) 1337 / 1163
+// bias or mask.  Backward alone, bf16, recomputing / in parts, us (problems per part; "no": the rule refuses it):
+//   D 128: H8 S16384 causal 1790 / 1723 (3)          H8 S16384 3230 / 3250 (3)
+//          H8 S20480 causal 2960 / 4040 (1, no)      H5 S27000 causal 3400 / 3740 (1, no)
+//          H6 S16384 causal 1383 / 1289 (3)          H14 S8192 causal, mask 1117 / 790 (9; 12 in pairs 952)
+//   D 64:  B16 H32 S2048 2820 / 2759 (192)           the same causal 1838 / 1601 (185)
+//          B4 H32 S4096 2692 / 2708 (46, no)         B2 H16 S8192 causal 1466 / 1403 (8, no)
+//          H16 S8192 1312 / 1442 (12, no)            the same causal 817 / 710 (8; 12 in pairs 743)
+//          H32 S12288 causal 3052 / 3271 (3, no)     B2 H12 S8192 causal, mask 1388 / 1160 (9; 12 in pairs 1193)
 bool parts_pay(const fa_params& p, const PartsCost& parts, int n) {
+  if (n >= parts.total) return true;  // the same launches as without slabs
   const int64_t percent = (p.D > 64 ? 25 : 2) + (p.causal ? 10 : 0) + (p.bias_kind != FA_BIAS_NONE ? 20 : 0);
-  return 100 * parts.cost(n) <= 3 * parts.turns(parts.total) * (100 + percent) + 100;
+  return 100 * parts.cost(n) <= parts.turns(parts.total) * (100 + percent) + 100 * PartsCost::kTurn / 3;
 }
 
 uint64_t bwd_workspace_bytes(const fa_params& p) {

@@ -799,8 +799,74 @@ int launch_dim(const DkdvParams& kp, int dtype, int bias_kind, dim3 grid, cudaSt
               : launch_bias<128, __half, LONGEST_FIRST>(kp, bias_kind, grid, stream);
 }
 
+// Work of key block `nb` of a causal problem, in quarters of a step: four a step, six for the tile's boundary and `zeros`
+// for each zero tile that a 16-bit bias gradient gets above the diagonal.  A block that no query sees only stores zeros.
+int tile_work(int nb, int n_mblk, int zeros) {
+  const int steps = n_mblk - nb;
+  return steps > 0 ? 4 * steps + 6 + zeros * nb : 3 + zeros * n_mblk;
+}
+
 }  // namespace
 
+int dkdv_pair_work(const fa_params& p) {
+  const int n_mblk = (p.M + 127) / 128;
+  return tile_work(0, n_mblk, 0) + tile_work((p.N + 127) / 128 - 1, n_mblk, 0);
+}
+
+// Causal pairs of a heavy and a light tile leave CTAs idle in their last turn, with an odd number of key blocks also
+// before it, and one pair a CTA leaves half of the CTAs without one.  Longest first the tiles spread better, but a head's
+// tiles no longer run side by side: only up to four a CTA, so that all operands stay in L2 without an order by head.
+// The longest CTA of both orders decides, with 3 % for the pairs, and 6 % where a bias is read in more than two rows of
+// tiles (its sectors are shared by neighbouring key blocks).
+// Measured over 1382 calls (whole backward; D 64 and 128, four kinds of bias, 512 to 8192 keys, M = N and not): of the 1132
+// taken 10 lose more than 1.5 % (at most 5 %, 25 us calls of 1024 x 2048), of those left to the pairs 7 would have gained as
+// much (at most 2.4 %); the mean gain over all is 8.9 %.  Pairs / longest first, us (estimate, measured):
+//   S1024 D64: H45 63.9 / 51.0 (1.45, 1.25)   H64 71.9 / 69.6 (1.09, 1.03)   H72 74.6 / 77.1 (1.00, 0.97: pairs)
+//   the same, 16-bit bias, H64: 91.4 / 91.3 (1.06, 1.00)   S1000, 16-bit bias, H60: 95.5 / 98.8 (1.06, 0.97: pairs)
+//   S1032 D64 H22, nine key blocks: 52.2 / 41.4 (1.62, 1.26)   S4096 D128 H9: 129.8 / 128.3 (1.00, 1.01: pairs)
+//   S8192 D128: H2, 16-bit bias 271 / 235 (1.28, 1.15)   H3, fp32 bias 473 / 485 (1.04, 0.98)
+DkdvPlan plan_dkdv(const fa_params& p, int n_bh, int sms, bool writes_zeros) {
+  const int n_mblk = (p.M + 127) / 128, n_nblk = (p.N + 127) / 128;
+  const int64_t all = static_cast<int64_t>(n_nblk) * n_bh;
+  if (!p.causal || all > 4 * sms) return {false, 0};
+  const int n = static_cast<int>(all), zeros = writes_zeros ? 1 : 0;
+  const auto more = [](int& most, int load) { most = load > most ? load : most; };
+
+  // Pairs: a CTA has units c and c + G at most, and their work repeats every n_nblk units (half of that where it is
+  // even), so the first CTAs of those with two units and of those with one stand for all.
+  const int units = (n + 1) / 2, g_pairs = units < sms ? units : sms, period = n_nblk & 1 ? n_nblk : n_nblk / 2;
+  const auto unit_work = [&](int u) {
+    int work = 0;
+    for (int k = 2 * u, pos = k % n_nblk; k < 2 * u + 2 && k < n; ++k, pos = pos + 1 == n_nblk ? 0 : pos + 1)
+      work += tile_work(pos & 1 ? n_nblk - 1 - (pos >> 1) : pos >> 1, n_mblk, zeros);
+    return work;
+  };
+  int pairs = 0;
+  const int with_two = units - g_pairs;
+  for (int c = 0; c < with_two && c < period; ++c) more(pairs, unit_work(c) + unit_work(c + g_pairs));
+  for (int c = with_two; c < g_pairs && c < with_two + period; ++c) more(pairs, unit_work(c));
+
+  // Longest first: along the CTAs the work of even rows falls and that of odd rows rises, so the longest CTA is the first
+  // one, or one at which an odd row comes to a longer key block.
+  const int g = n < sms ? n : sms;
+  const auto load_of = [&](int c) {
+    int load = 0;
+    for (int at = 0, r = 0; at < n; at += g, ++r)
+      if (const int k = at + (r & 1 ? g - 1 - c : c); k < n) load += tile_work(k / n_bh, n_mblk, zeros);
+    return load;
+  };
+  int longest = load_of(0);
+  for (int at = g; at < n; at += 2 * g) {
+    const int last = at + g < n ? at + g - 1 : n - 1;
+    for (int nb = at / n_bh; nb <= last / n_bh; ++nb) {
+      const int k = (nb + 1) * n_bh - 1;
+      more(longest, load_of(at + g - 1 - (k < last ? k : last)));
+    }
+  }
+  const int margin = p.bias_kind != FA_BIAS_NONE && n > 2 * sms ? 106 : 103;
+  const bool longest_first = 100 * static_cast<int64_t>(pairs) >= margin * static_cast<int64_t>(longest);
+  return {longest_first, longest_first ? longest : pairs};
+}
 
 int launch_bwd_dkdv(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab) {
   if (p.D == 256) return launch_bwd_dkdv_d256(p, stream, status, slab);
@@ -904,15 +970,10 @@ int launch_bwd_dkdv(const fa_params& p, cudaStream_t stream, int* status, const 
   kp.n_nblk = (p.N + 127) / 128;
   kp.n_bh = slab ? slab->n_bh : p.B * p.H;
   kp.n_tiles = kp.n_nblk * kp.n_bh;
-  const int units = p.causal ? (kp.n_tiles + 1) / 2 : kp.n_tiles;
-  // Causal pairs of a heavy and a light tile leave CTAs idle in their last turn.  Where that costs more than an eighth,
-  // tiles go longest first one by one; only up to four a CTA, so that all operands stay in L2 without an order by head.
-  // Whole backward, causal, us (share of the pairs' turns that is filled), pairs / longest first: B4 H16 S1024 D64 (0.86)
-  // 71.9 / 70.4, 16-bit bias 91.4 / 92.2, mask 76.9 / 75.5; H8 S8192 D128, bias (0.86) 571 / 544; B2 H8 S2048 D64 (0.86)
-  // 62.7 / 59.1; B8 H12 S512 D64 (0.65) 45.3 / 38.2; H12 S2048 D128, mask (0.65) 76.5 / 71.5; B2 H16 S512 D64 (0.43) 27.1 / 24.6.
-  const int sms = persistent_grid(1 << 30), turns = (units + sms - 1) / sms;
-  const bool longest_first = p.causal && kp.n_tiles <= 4 * sms && 8 * units < 7 * turns * sms;
-  const dim3 grid(persistent_grid(longest_first ? kp.n_tiles : units));
+  const int sms = persistent_grid(1 << 30);
+  const bool longest_first = plan_dkdv(p, kp.n_bh, sms, kp.zero_tiles != 0).longest_first;
+  const int units = p.causal && !longest_first ? (kp.n_tiles + 1) / 2 : kp.n_tiles;
+  const dim3 grid(units < sms ? units : sms);
   return longest_first ? launch_dim<true>(kp, p.dtype, p.bias_kind, grid, stream)
                        : launch_dim<false>(kp, p.dtype, p.bias_kind, grid, stream);
 }

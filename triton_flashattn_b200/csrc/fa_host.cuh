@@ -50,6 +50,15 @@ int launch_pad_rows(void* dst, const int64_t dst_stride[3], const void* src, con
                     int N, cudaStream_t stream);
 int launch_pack_rows(void* dst, const void* src, int64_t pitch, int eb, int64_t rows, int N, cudaStream_t stream);
 int launch_bwd_pre(const fa_params& p, cudaStream_t stream, int* status);
+// How a causal dK/dV launch of head dims up to 128 over `n_bh` problems walks its tiles (see plan_dkdv), and how long its
+// longest CTA works then, in quarters of a step; 0 where that was not looked at (pairs, many tiles a CTA).
+struct DkdvPlan {
+  bool longest_first;
+  int span;
+};
+DkdvPlan plan_dkdv(const fa_params& p, int n_bh, int sms, bool writes_zeros);
+// Work of a pair of a heavy and a light tile in the same unit.
+int dkdv_pair_work(const fa_params& p);
 // Without a slab: all problems, dS going where the parameters say (dbias, ds16 or nowhere).
 int launch_bwd_dkdv(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab = nullptr);
 int launch_bwd_dq(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab = nullptr);
