@@ -133,15 +133,16 @@ int fa_fwd(const fa_params* p, void* stream);
 /*
  * Whether fa_fwd reads the bias of a problem with M query rows of head dim D element by element
  * (few rows: a decode step).  Such a bias needs a unit innermost stride and nothing else: any
- * address, any other strides, 0 for M included.
+ * naturally aligned address (else FA_ERR_ALIGN), any other strides, 0 for M included.
  */
 int fa_fwd_takes_any_bias(int M, int D);
 
 /*
  * Short sequences (fa_small_takes: M, N <= 64 and D <= 64).  fa_fwd, fa_bwd and fa_bwd_workspace use the same kernels
  * for them and ask of the bias, its gradient and ds16 what they ask at any size.  These two take the bias and write its
- * gradient at any naturally aligned address with any strides (the innermost is 1), use no ds16 and no scratch, and
- * leave every element of a gradient of shape (B, H, M, N) written.  Other sizes: FA_ERR_UNSUPPORTED.
+ * gradient at any naturally aligned address with any strides (the innermost is 1; those of the gradient are positive where
+ * the extent is more than 1), use no ds16 and no scratch, and leave every element of a gradient of shape (B, H, M, N)
+ * written.  Other sizes: FA_ERR_UNSUPPORTED.  An address or a stride that breaks this: FA_ERR_ALIGN.
  */
 int fa_small_takes(int M, int N, int D);
 int fa_small_fwd(const fa_params* p, void* stream);

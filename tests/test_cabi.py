@@ -86,6 +86,46 @@ def test_selftest_entry_validates_arguments():
     assert lib.fa_last_device_status(0, None) == 2
 
 
+def _small_params(**kw):
+    """A backward over a few rows whose pointers are never followed: the answer comes before any CUDA call, or (device -1) from
+    the first one."""
+    p = _params(B=2, H=2, M=16, N=16, D=32, device=-1, bias_kind=1, write_dbias=1)
+    for name in ("q", "k", "v", "o", "d_o", "dq", "dk", "dv", "bias", "dbias", "lse", "delta", "ds16"):
+        setattr(p, name, 4096)
+    for name in ("q", "k", "v", "o", "do", "dq", "dk", "dv", "bias", "dbias", "ds16"):
+        setattr(p, name + "_stride", (ctypes.c_int64 * 3)(1024, 512, 32))
+    for k, v in kw.items():
+        setattr(p, k, v)
+    return p
+
+
+@pytest.mark.parametrize("entry", ["fa_fwd", "fa_small_fwd", "fa_bwd", "fa_small_bwd"])
+@pytest.mark.parametrize("kind,offset", [(1, 1), (3, 2), (3, 1)])
+def test_a_bias_off_its_natural_alignment_is_refused(entry, kind, offset):
+    """The kernels for few rows and short sequences load a bias element by element: off its elements that would be a
+    misaligned access on the device."""
+    fn = getattr(_cabi.load(), entry)
+    assert fn(ctypes.byref(_small_params(bias_kind=kind)), None) == 6  # FA_ERR_CUDA: nothing to complain about before
+    assert fn(ctypes.byref(_small_params(bias_kind=kind, bias=4096 + offset)), None) == 5  # FA_ERR_ALIGN
+    assert fn(ctypes.byref(_small_params(bias_kind=2, write_dbias=0, bias=4096 + 1)), None) == 6  # bytes lie anywhere
+    if entry.endswith("bwd"):
+        assert fn(ctypes.byref(_small_params(bias_kind=kind, dbias=4096 + offset)), None) == 5
+
+
+def test_a_gradient_without_places_of_its_own_is_refused():
+    lib = _cabi.load()
+    for i in range(3):
+        st = [1024, 512, 32]
+        for bad in (0, -st[i]):
+            st[i] = bad
+            p = _small_params(dbias_stride=(ctypes.c_int64 * 3)(*st))
+            assert lib.fa_small_bwd(ctypes.byref(p), None) == 5
+        one = _small_params(dbias_stride=(ctypes.c_int64 * 3)(*st), **{"BHM"[i]: 1})
+        assert lib.fa_small_bwd(ctypes.byref(one), None) == 6  # a stride over one element says nothing
+    at, odd = ctypes.c_void_p(4096), ctypes.c_void_p(4097)
+    assert lib.fa_pack_rows(at, odd, ctypes.c_int64(16), 2, ctypes.c_int64(4), 16, -1, None) == 5
+
+
 @pytest.mark.parametrize("elem_bytes", [1, 2, 4])
 def test_row_copies_refuse_rows_that_32_bits_cannot_count(elem_bytes):
     """Before any CUDA call: such a row would be taken for an empty or a negative one.  The longest row that fits gets as far as

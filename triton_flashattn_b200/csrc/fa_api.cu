@@ -136,6 +136,13 @@ int* device_status_ptr(int device) {
 
 namespace {
 
+// Whether elements of a bias, a mask or a bias gradient can be loaded and stored one by one at this address: the kernels that
+// take any layout do that.
+bool element_aligned(const void* ptr, int bias_kind) {
+  const uintptr_t size = bias_kind == FA_BIAS_BOOL ? 1 : bias_kind == FA_BIAS_F32 ? 4 : 2;
+  return reinterpret_cast<uintptr_t>(ptr) % size == 0;
+}
+
 int validate_common(const fa_params* p) {
   if (!p) return FA_ERR_NULL;
   if (p->struct_size != sizeof(fa_params)) return FA_ERR_ABI;
@@ -146,6 +153,7 @@ int validate_common(const fa_params* p) {
   if (!p->q || !p->k || !p->v || !p->o || !p->lse) return FA_ERR_NULL;
   if (p->bias_kind != FA_BIAS_NONE && !p->bias) return FA_ERR_NULL;
   if ((int64_t)p->B * p->H > 65535) return FA_ERR_TOO_LARGE;
+  if (p->bias_kind != FA_BIAS_NONE && !element_aligned(p->bias, p->bias_kind)) return FA_ERR_ALIGN;
   return FA_OK;
 }
 
@@ -157,6 +165,7 @@ int validate_bwd(const fa_params* p, bool workspace = false) {
   if (p->write_dbias) {
     if (p->bias_kind != FA_BIAS_SAME && p->bias_kind != FA_BIAS_F32) return FA_ERR_DTYPE;
     if (!p->dbias) return FA_ERR_NULL;
+    if (!element_aligned(p->dbias, p->bias_kind)) return FA_ERR_ALIGN;
   }
   if (workspace) return FA_OK;
   if (p->bias_kind == FA_BIAS_F32 && !p->ds16) return FA_ERR_NULL;
@@ -330,6 +339,11 @@ int fa_small_bwd(const fa_params* p, void* stream) {
   int r = validate_bwd(p, true);
   if (r) return r;
   if (!small_takes(p->M, p->N, p->D)) return FA_ERR_UNSUPPORTED;
+  if (p->write_dbias) {  // every element has a place of its own
+    const int extent[3] = {p->B, p->H, p->M};
+    for (int i = 0; i < 3; ++i)
+      if (extent[i] > 1 && p->dbias_stride[i] <= 0) return FA_ERR_ALIGN;
+  }
   return with_device(p->device, [&](int* st) { return launch_small(*p, true, static_cast<cudaStream_t>(stream), st); });
 }
 
@@ -349,6 +363,7 @@ int fa_pack_rows(void* dst, const void* src, int64_t pitch, int elem_bytes, int6
   if (rows < 1 || N < 1 || pitch < N) return FA_ERR_SHAPE;
   if (elem_bytes != 2 && elem_bytes != 4) return FA_ERR_DTYPE;
   if (!row_fits_copy(N, elem_bytes)) return FA_ERR_TOO_LARGE;
+  if (reinterpret_cast<uintptr_t>(src) % 2 != 0) return FA_ERR_ALIGN;
   return with_device(device, [&](int*) {
     return launch_pack_rows(dst, src, pitch, elem_bytes, rows, N, static_cast<cudaStream_t>(stream));
   });
