@@ -59,3 +59,25 @@ def test_pack_rows(dtype, N, rows, device_ok):
                                   src.element_size(), ctypes.c_int64(rows), N, 0, _stream())
     assert r == 0
     assert torch.equal(out[:rows * N].view(rows, N), src) and (out[rows * N:] == 0x55).all()
+
+
+def test_an_earlier_error_is_not_taken_for_a_copys_own(device_ok):
+    """A call on a device that does not exist leaves an error behind in the runtime; the copies after it report their own."""
+    from triton_flashattn_b200 import _cabi
+
+    lib = _cabi.load()
+    src = _random((5, 9), torch.int16)
+    padded = torch.zeros((5, 16), dtype=torch.int16, device="cuda")
+    out = torch.zeros(5 * 9 + 3, dtype=torch.int16, device="cuda")
+
+    def pad(device):
+        return lib.fa_pad_rows(ctypes.c_void_p(padded.data_ptr()), _I64x3(80, 80, 16), ctypes.c_void_p(src.data_ptr()),
+                               _I64x3(45, 45, 9), 2, 1, 1, 5, 9, device, _stream())
+
+    def pack(device):
+        return lib.fa_pack_rows(ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(padded.data_ptr()), ctypes.c_int64(16), 2,
+                                ctypes.c_int64(5), 9, device, _stream())
+
+    assert pad(-1) == 6 and pad(0) == 0
+    assert pack(-1) == 6 and pack(0) == 0
+    assert torch.equal(out[:45].view(5, 9), src)

@@ -92,10 +92,7 @@ int launch_pad_rows(void* dst, const int64_t dst_stride[3], const void* src, con
   const int64_t row = static_cast<int64_t>(N) * eb, chunks = (row + 15) / 16;
   if (static_cast<int64_t>(B) * H > 65535 || chunks * M > (1ll << 30)) return FA_ERR_TOO_LARGE;
   p.H = H, p.M = M, p.row_bytes = static_cast<int>(row), p.chunks = static_cast<int>(chunks);
-  pad_rows_kernel<<<dim3(static_cast<unsigned>((chunks * M + 255) / 256), B * H), 256, 0, stream>>>(p);
-  if (cudaGetLastError() != cudaSuccess) return FA_ERR_CUDA;
-  g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-  return FA_OK;
+  return launch_ordered(pad_rows_kernel, dim3(static_cast<unsigned>((chunks * M + 255) / 256), B * H), 256, stream, p);
 }
 
 int launch_pack_rows(void* dst, const void* src, int64_t pitch, int eb, int64_t rows, int N, cudaStream_t stream) {
@@ -103,13 +100,9 @@ int launch_pack_rows(void* dst, const void* src, int64_t pitch, int eb, int64_t 
   if (reinterpret_cast<uintptr_t>(dst) % 16 || eb % 2) return FA_ERR_ALIGN;
   const int64_t total = rows * N * eb, blocks = (total + 4095) / 4096;
   if (blocks > (1ll << 30)) return FA_ERR_TOO_LARGE;
-  if (total < (1ll << 30))
-    pack_rows_kernel<uint32_t><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(p);
-  else
-    pack_rows_kernel<uint64_t><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(p);
-  if (cudaGetLastError() != cudaSuccess) return FA_ERR_CUDA;
-  g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-  return FA_OK;
+  const dim3 grid(static_cast<unsigned>(blocks));
+  return total < (1ll << 30) ? launch_ordered(pack_rows_kernel<uint32_t>, grid, 256, stream, p)
+                             : launch_ordered(pack_rows_kernel<uint64_t>, grid, 256, stream, p);
 }
 
 }  // namespace fa

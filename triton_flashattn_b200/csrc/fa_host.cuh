@@ -81,6 +81,24 @@ int persistent_grid(int n_tiles);
 // Kernels launched by this library since it was loaded (all devices, all threads).
 extern std::atomic<uint64_t> g_kernel_launches;
 
+// A launch answers with its own outcome: an error that an earlier call left behind is neither taken for it nor cleared.
+template <typename Kern, typename Params>
+inline int launch_counted(const cudaLaunchConfig_t& cfg, Kern kern, const Params& params) {
+  if (cudaLaunchKernelEx(&cfg, kern, params) != cudaSuccess) return FA_ERR_CUDA;
+  g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+  return FA_OK;
+}
+
+// Launch that starts when its predecessors on the stream are done.
+template <typename Kern, typename Params>
+inline int launch_ordered(Kern kern, dim3 grid, int threads, cudaStream_t stream, const Params& params) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.stream = stream;
+  return launch_counted(cfg, kern, params);
+}
+
 // Launch with the programmatic-stream-serialization attribute (see grid_dep_wait()).
 template <typename Kern, typename Params>
 inline int launch_overlapped(Kern kern, dim3 grid, int threads, size_t smem, cudaStream_t stream,
@@ -98,9 +116,7 @@ inline int launch_overlapped(Kern kern, dim3 grid, int threads, size_t smem, cud
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = cluster_x > 1 ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, kern, params) != cudaSuccess) return FA_ERR_CUDA;
-  g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-  return FA_OK;
+  return launch_counted(cfg, kern, params);
 }
 
 // Tile map for the slabs of a DsSlab: dims {N, M, problems, 1}, box {64, box_rows}.
