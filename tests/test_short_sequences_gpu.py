@@ -85,3 +85,22 @@ def test_c_entries_refuse_what_the_tile_kernels_refuse(device_ok):
     p.M = 65
     assert lib.fa_small_takes(65, 49, 32) == 0 and lib.fa_small_fwd(ctypes.byref(p), stream) == 8
     torch.cuda.synchronize()
+
+
+def test_a_converted_bias_is_kept_for_the_backward(device_ok):
+    """A bias of another dtype is converted once: between forward and backward its fp32 copy stays, beside the result and the
+    log-sum-exp, also where its rows (49 columns) are not 16-byte aligned."""
+    from triton_flashattn_b200 import flash_attention_fn
+
+    B, S, H, D = 16, 49, 4, 32
+    q, k, v, bias, do = make_inputs(B, S, S, H, D, HF, "float", 78)
+    bias = bias.to(BF)
+    inputs = [t.requires_grad_() for t in (q, k, v)]
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    out = flash_attention_fn(*inputs, bias)
+    held = torch.cuda.memory_allocated() - before
+    assert held >= out.numel() * 2 + B * H * S * 4 + bias.numel() * 4
+    want = torch.autograd.grad(flash_attention_fn(*inputs, bias.float()), inputs, do)
+    for a, b in zip(torch.autograd.grad(out, inputs, do), want):
+        assert torch.equal(a, b)

@@ -498,7 +498,7 @@ Tensor attention(const Tensor& a, const Tensor& k, const Tensor& v, const Tensor
   if (bias.defined()) {
     node->bias_ = SavedVariable(bias, false);
     // (a converted bias that only the kernel for few rows can read is made again for the backward)
-    if (!b.t.is_same(bias) && bias_ok(b.t) && static_cast<int64_t>(b.t.storage().nbytes()) <= kKeepBiasCopyBytes &&
+    if (!b.t.is_same(bias) && (bias_ok(b.t) || is_small(s)) && static_cast<int64_t>(b.t.storage().nbytes()) <= kKeepBiasCopyBytes &&
         !at::SavedTensorDefaultHooks::get_hooks().has_value())
       node->bias_copy_ = std::move(b.t);
   }
