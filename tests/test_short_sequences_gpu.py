@@ -104,3 +104,37 @@ def test_a_converted_bias_is_kept_for_the_backward(device_ok):
     want = torch.autograd.grad(flash_attention_fn(*inputs, bias.float()), inputs, do)
     for a, b in zip(torch.autograd.grad(out, inputs, do), want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("S", [48, 49])
+@pytest.mark.parametrize("kind", [None, "float", "bool", "f32"])
+def test_the_reference_classes_take_the_same_kernels(S, kind, device_ok):
+    """FlashAttentionFn and FlashAttentionQKVPackedFn give the bits of the functions, with as many launches, and ask for no scratch that these kernels do not use."""
+    from triton_flashattn_b200 import _cabi, flash_attention as fa
+
+    lib = _cabi.load()
+    q, k, v, bias, do = make_inputs(3, S, S, 4, 32, HF, "float" if kind == "f32" else kind, 79)
+    if kind == "f32":
+        bias = bias.float()
+    train = kind in ("float", "f32")
+
+    def grads(fn, *tensors):
+        ins = [t.detach().clone().requires_grad_() for t in tensors]
+        b = bias.detach().clone().requires_grad_(train) if kind else None
+        n = lib.fa_launch_count()
+        out = fn(*ins, b, True)
+        return [out.detach(), *torch.autograd.grad(out, ins + ([b] if train else []), do)], lib.fa_launch_count() - n
+
+    want, n = grads(fa.flash_attention_fn, q, k, v)
+    got, m = grads(lambda *a: fa.FlashAttentionFn.apply(*a), q, k, v)
+    assert n == m == 2 and all(torch.equal(a, b) for a, b in zip(want, got))
+    qkv = torch.stack([q, k, v], dim=2)
+    got, m = grads(lambda *a: fa.FlashAttentionQKVPackedFn.apply(*a), qkv)
+    packed = torch.stack(want[1:4], dim=2)
+    assert m == 2 and torch.equal(got[0], want[0]) and torch.equal(got[1], packed)
+    if train:
+        assert torch.equal(got[2], want[4])
+        if kind == "f32":
+            b, bias_kind = fa._classify_bias(bias, q)
+            p = fa._params(q, k, v, want[0], want[0], b, bias_kind, True, 0.1)
+            assert lib.fa_bwd_workspace_bytes(ctypes.byref(p)) == S * ((S + 7) // 8 * 8) * 2

@@ -239,8 +239,10 @@ bool parts_pay(const fa_params& p, const PartsCost& parts, int n) {
 }
 
 uint64_t bwd_workspace_bytes(const fa_params& p) {
-  if (ds_is_dbias(p) || (small_takes(p.M, p.N, p.D) && p.bias_kind != FA_BIAS_F32)) return 0;
   const uint64_t one = slab_bytes(p), fit = kSlabCap / one;
+  if (ds_is_dbias(p)) return 0;
+  // short sequences use none; with an fp32 bias some workspace is what stands for ds16 in the checks
+  if (small_takes(p.M, p.N, p.D)) return p.bias_kind == FA_BIAS_F32 ? one : 0;
   const PartsCost parts(p);
   const int total = parts.total;
   int n = fit < 1 ? 0 : parts.best(fit > (uint64_t)total ? total : (int)fit);

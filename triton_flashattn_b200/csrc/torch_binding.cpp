@@ -598,8 +598,10 @@ PyObject* py_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const c10::cuda::CUDAGuard device(static_cast<c10::DeviceIndex>(s.device));
     at::AutoDispatchBelowADInplaceOrView guard;
     const Tensor q = tile_ready(q0), k = tile_ready(k0), v = tile_ready(v0);
-    backward(s, g, view_of(q), view_of(k), view_of(v), o, lse, classify_bias(bias, s.dtype), causal, scale,
-             view_of(dq), view_of(dk), view_of(dv), dbias, false);
+    // (the caller's gradient has to meet the tile kernels' rule at any size)
+    const bool any_layout = is_small(s) && (!dbias.defined() || bias_ok(dbias));
+    backward(s, g, view_of(q), view_of(k), view_of(v), o, lse, classify_bias(bias, s.dtype, any_layout), causal, scale,
+             view_of(dq), view_of(dk), view_of(dv), dbias, any_layout);
     Py_RETURN_NONE;
   });
 }
