@@ -69,6 +69,7 @@ def test_abandoned_wait_is_reported_and_service_resumes_after_reset():
 
 
 SENT16 = 0x7B7B  # bit pattern written around every output (a large finite 16-bit float)
+SENT32 = 0x7B7B7B7B
 
 
 def _guarded(shape, dtype, pad_elems=4096):
@@ -79,12 +80,12 @@ def _guarded(shape, dtype, pad_elems=4096):
         n *= s
     buf = torch.empty(n + 2 * pad_elems, dtype=dtype, device="cuda")
     raw = buf.view(torch.int16 if dtype.itemsize == 2 else torch.int32)
-    raw.fill_(SENT16 if dtype.itemsize == 2 else 0x7B7B7B7B)
+    raw.fill_(SENT16 if dtype.itemsize == 2 else SENT32)
     return buf[pad_elems:pad_elems + n].view(shape), raw, slice(pad_elems, pad_elems + n)
 
 
 def _guards_intact(raw, payload):
-    sent = SENT16 if raw.dtype == torch.int16 else 0x7B7B7B7B
+    sent = SENT16 if raw.dtype == torch.int16 else SENT32
     return bool(torch.all(raw[:payload.start] == sent)) and bool(torch.all(raw[payload.stop:] == sent))
 
 
@@ -121,7 +122,7 @@ def test_stores_stay_inside_their_tensors(M, N, D, causal, bias_kind, device_ok)
     for name, raw, pl in (("o", o_raw, o_pl), ("lse", lse_raw, lse_pl), ("delta", delta_raw, delta_pl),
                           ("dq", dq_raw, dq_pl), ("dk", dk_raw, dk_pl), ("dv", dv_raw, dv_pl)):
         assert _guards_intact(raw, pl), f"{name}: a store landed outside the tensor"
-        sent = SENT16 if raw.dtype == torch.int16 else 0x7B7B7B7B
+        sent = SENT16 if raw.dtype == torch.int16 else SENT32
         assert not bool(torch.any(raw[pl] == sent)), f"{name}: an element was never written"
     if dbias is not None:
         assert _guards_intact(db_raw, db_pl), "dbias: a store landed outside the buffer"
@@ -329,8 +330,10 @@ def test_zero_strides_are_refused_by_every_kernel(M, device_ok):
             setattr(p, which + "_stride", _cabi._I64x3(*st))
             if which != "do":
                 assert lib.fa_fwd(ctypes.byref(p), None) == 5, (which, i)  # FA_ERR_ALIGN
+                assert lib.fa_small_fwd(ctypes.byref(p), None) == 5, (which, i)
             assert lib.fa_bwd_dkdv(ctypes.byref(p), None) == 5, (which, i)
             assert lib.fa_bwd_dq(ctypes.byref(p), None) == 5, (which, i)
+            assert lib.fa_bwd(ctypes.byref(p), None) == 5 and lib.fa_small_bwd(ctypes.byref(p), None) == 5, (which, i)
     p, keep = _bwd_params(fa, q, k, v, o, lse, bias, False, 0.1, do, dq, dk, dv, dbias, delta)
     assert lib.fa_fwd(ctypes.byref(p), None) == 0 and lib.fa_bwd(ctypes.byref(p), None) == 0
     torch.cuda.synchronize()
@@ -430,7 +433,7 @@ def test_causal_gradients_do_not_depend_on_the_schedule(M, N, caps, D, bias_kind
         bias = bias.float()
     monkeypatch.setenv("FA_MAX_CTAS", "1")
     want = run_ours(q, k, v, bias, True, None, do)
-    for ctas in (*caps, 148):
+    for ctas in (*caps, 7, 148):
         monkeypatch.setenv("FA_MAX_CTAS", str(ctas))
         got = run_ours(q, k, v, bias, True, None, do)
         for name in want:

@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from tests._util import compare, make_inputs, run_ours
+from tests.test_robustness_gpu import SENT16, SENT32, _guarded, _guards_intact
 
 pytestmark = pytest.mark.gpu
 BF, HF = torch.bfloat16, torch.float16
@@ -22,33 +23,82 @@ def test_edges_against_oracle(M, N, D, dtype, kind, causal, device_ok):
     compare(ours, q, k, v, bias, causal, None, do, dtype, label=f"{M}x{N}: ")
 
 
+@pytest.mark.parametrize("S", [48, 49])
 @pytest.mark.parametrize("layout", ["sliced", "heads_last", "expanded", "f32_sliced"])
-def test_bias_in_any_layout(layout, device_ok):
-    """A bias whose rows are not 16-byte aligned, in another order or expanded, gives what its padded copy gives."""
-    B, S, H, D = 3, 49, 4, 32
+def test_bias_in_any_layout(layout, S, device_ok):
+    """A bias whose rows are not 16-byte aligned, in another order or expanded, gives what its copy into padded rows gives
+    (48 columns: there pairs of elements are accessed at once), and that is right."""
+    from triton_flashattn_b200 import flash_attention_fn
+
+    B, H, D = 3, 4, 32
     q, k, v, bias, do = make_inputs(B, S, S, H, D, HF, "float", 77)
     if layout == "f32_sliced":
         bias = bias.float()
     if layout == "expanded":
-        bias = bias[:1].expand(B, H, S, S)
-        odd = bias
+        odd = bias = bias[:1].expand(B, H, S, S)
     else:
         shape = (B, S, H, S + 3) if layout == "heads_last" else (B, H, S, S + 3)
-        buf = torch.zeros(shape, dtype=bias.dtype, device="cuda")
-        odd = buf[..., 1:S + 1]
+        odd = torch.zeros(shape, dtype=bias.dtype, device="cuda")[..., 1:S + 1]
         if layout == "heads_last":
             odd = odd.transpose(1, 2)
         odd.copy_(bias)
-    dense = bias.contiguous()
-    want, got = run_ours(q, k, v, dense, True, None, do), None
-    from triton_flashattn_b200 import flash_attention_fn
+    padded = torch.zeros((B, H, S, 64), dtype=bias.dtype, device="cuda")[..., :S]
+    padded.copy_(bias)
 
-    ins = [t.detach().clone().requires_grad_() for t in (q, k, v)]
-    b = odd.detach().requires_grad_()
-    out = flash_attention_fn(*ins, b, True)
-    got = dict(zip(("dq", "dk", "dv", "dbias"), torch.autograd.grad(out, [*ins, b], do)), out=out.detach())
+    def run(b):
+        ins = [t.detach().clone().requires_grad_() for t in (q, k, v)]
+        b = b.detach().requires_grad_()
+        out = flash_attention_fn(*ins, b, True)
+        return dict(zip(("dq", "dk", "dv", "dbias"), torch.autograd.grad(out, [*ins, b], do)), out=out.detach())
+
+    want, got = run(padded), run(odd)
     for name in want:
         assert torch.equal(want[name], got[name]), name
+    compare(want, q, k, v, bias.contiguous(), True, None, do, HF, label=f"{layout} {S}: ")
+
+
+@pytest.mark.parametrize("M,N,D", [(49, 49, 32), (17, 64, 16), (64, 17, 64), (48, 48, 32), (1, 64, 64), (33, 1, 16)])
+@pytest.mark.parametrize("dtype,causal", [(BF, False), (torch.float32, True)])
+@pytest.mark.parametrize("layout", ["dense", "pitched", "odd", "heads_last"])
+def test_stores_stay_inside_their_tensors(M, N, D, dtype, causal, layout, device_ok):
+    """As for the tile kernels: every output lies in a sentinel-filled buffer; after fa_small_fwd and fa_small_bwd all of it has
+    been written and nothing around it, the columns between the rows of a pitched gradient included.  "odd": an element
+    beyond a pair, with an odd pitch, so that pairs cannot be accessed at once."""
+    from triton_flashattn_b200 import _cabi
+    from triton_flashattn_b200 import flash_attention as fa
+
+    lib = _cabi.load()
+    B, H = 2, 3
+    q, k, v, bias, do = make_inputs(B, M, N, H, D, BF, "float", 80)
+    bias = bias.to(dtype)
+    o, lse, delta = (_guarded(s, t) for s, t in (((B, M, H, D), BF), ((B, H, M), torch.float32), ((B, H, M), torch.float32)))
+    dq, dk, dv = (_guarded(t.shape, BF) for t in (q, k, v))
+    cols = {"dense": N, "pitched": (N + 15) // 8 * 8 + 8, "odd": N + 4 + N % 2 + 1, "heads_last": N}[layout]
+    shape = (B, M, H, cols) if layout == "heads_last" else (B, H, M, cols)
+    first = 1 if layout == "odd" else 0
+    whole, bias_whole = _guarded(shape, dtype), torch.zeros(shape, dtype=dtype, device="cuda")
+    cut = [t[..., first:first + N] for t in (whole[0], bias_whole)]
+    dbias, b = (t.transpose(1, 2) for t in cut) if layout == "heads_last" else cut
+    b.copy_(bias)
+    p = fa._params(q, k, v, o[0], lse[0], b, _cabi.FA_BIAS_SAME if dtype == BF else _cabi.FA_BIAS_F32, causal, D ** -0.5)
+    for name, t in (("d_o", do), ("dq", dq[0]), ("dk", dk[0]), ("dv", dv[0]), ("dbias", dbias)):
+        setattr(p, name, t.data_ptr())
+        setattr(p, ("do" if name == "d_o" else name) + "_stride", fa._stride3(t))
+    p.delta, p.write_dbias = delta[0].data_ptr(), 1
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    _cabi.check(lib.fa_small_fwd(ctypes.byref(p), stream), "fa_small_fwd")
+    _cabi.check(lib.fa_small_bwd(ctypes.byref(p), stream), "fa_small_bwd")
+    torch.cuda.synchronize()
+    for name, (_, raw, payload) in dict(o=o, lse=lse, delta=delta, dq=dq, dk=dk, dv=dv).items():
+        assert _guards_intact(raw, payload), f"{name}: a store landed outside the tensor"
+        assert not bool(torch.any(raw[payload] == (SENT16 if raw.dtype == torch.int16 else SENT32))), f"{name}: never written"
+    assert _guards_intact(whole[1], whole[2]), "dbias: a store landed outside the buffer"
+    sent = SENT16 if dtype == BF else SENT32
+    words = whole[1][whole[2]].view(shape)
+    assert bool(torch.all(words[..., :first] == sent)) and bool(torch.all(words[..., first + N:] == sent)), "dbias: between rows"
+    assert not bool(torch.any(words[..., first:first + N] == sent)), "dbias: never written"
+    ours = {"out": o[0], "dq": dq[0], "dk": dk[0], "dv": dv[0], "dbias": dbias}
+    compare(ours, q, k, v, bias, causal, None, do, BF, label=f"{M}x{N} D{D} {layout}: ")
 
 
 def test_masked_rows_and_nan(device_ok):
