@@ -113,8 +113,8 @@ typedef struct fa_params {
 int fa_version(void);
 
 /*
- * Number of attention kernels this library has launched since it was loaded (forward 1 per
- * call; backward 3: preprocess, dK/dV, dQ).  For benchmarks and tests that must show the
+ * Number of kernels this library has launched since it was loaded (forward 1 per call; backward 3:
+ * preprocess, dK/dV, dQ, with more parts two more each; short sequences 1; a row copy 1).  For benchmarks and tests that must show the
  * work ran here.  No counterpart in the reference.
  */
 uint64_t fa_launch_count(void);

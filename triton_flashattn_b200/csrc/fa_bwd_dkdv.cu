@@ -15,7 +15,7 @@
 //   warp 19    TMA loads of the 16-bit bias tiles
 // The four control warps walk their loops with all lanes converged and elect a lane only
 // for the TMA / MMA / commit instructions, whose operands are then warp-uniform values.
-// A barrier operation answers after ~200 cycles on this GPU, so two issuers keep
+// A wait takes 200 - 235 cycles here even on a completed barrier, so two issuers keep
 // the tensor pipe fed while the other one waits, and every role polls the
 // barriers it will need before it starts a stretch of independent work.
 // Per query block t:

@@ -26,7 +26,7 @@
 // that waits on it, so a parity wait can never be two phases behind.
 //
 // What bounds it: a step takes 6400 cycles against 3072 of products; the issuer's looks at barriers
-// (about 280 cycles each, so they are combined) and the wait for P make up most of the rest.  (A second
+// (200 - 235 cycles each, so they are combined) and the wait for P make up most of the rest.  (A second
 // issuer for dP changed nothing: 0.245 / 0.251 ms.)  B4 H8 S2048, 16-bit bias: 0.245 ms; with the query
 // rows as lanes, P in shared memory and two ring stages 0.330 ms (9800 cycles: each stage was waited for,
 // and a row of bias or dS per thread is 32 sectors per warp access), with four 16 KB stages 0.379 ms

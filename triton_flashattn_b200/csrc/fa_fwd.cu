@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
     // (the whole warp walks the loop converged, one elected lane issues)
     if (live) {
       const int t = warp == 9 ? 0 : 1;
-      // A look at a barrier takes about 280 cycles.  Without a bias the issuer is on the critical path, so it
+      // A wait on a completed barrier takes 200 - 235 cycles.  Without a bias the issuer is on the critical path, so it
       // looks at the loads, which have landed by then as a rule, while the row threads still form P or
       // read S (causal B2 H32 S4096 D128: 342 -> 328 us).  With a mask that gains where the products are long
       // enough to matter and loses where they are not; with a float bias the row threads are behind anyway.

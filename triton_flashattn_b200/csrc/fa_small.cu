@@ -4,12 +4,14 @@
 // and an epilogue that nothing overlaps, and a backward of three launches with dS going through memory.  Here a CTA loads
 // the whole problem into shared memory once, a warp takes 16 query rows, and the backward is one launch: delta, P and dS
 // of all keys, dQ from the warp's own dS, then dK and dV by 16 keys a warp from P and dS in shared memory.  What bounds
-// it is latency (loads, then a chain of a few hundred instructions), so many small CTAs per SM: four warps and 26 KB
-// for a window of 49 x 49 and D = 32.  The warp-level matrix instruction is enough for that: a window has 16 rows a warp
+// it is latency (loads, then a chain of a few hundred instructions), so many small CTAs per SM: four warps and 15 KB
+// (forward) or 38 KB (backward) for a window of 49 x 49 and D = 32.  The warp-level matrix instruction is enough for that: a window has 16 rows a warp
 // where tcgen05 wants 128, and a chain of its products would cost a round trip through tensor memory each.
 // fp16, us, tile kernels -> here, forward and whole backward (without the copies of padded biases and gradients):
 //   B256 H6 49 x 49 D32       no bias 32 -> 11, 52 -> 19     trained bias 41 -> 15, 58 -> 32     mask 42 -> 14, 60 -> 22
-//   B256 H6 64 x 64 D64       no bias 31 -> 16, 60 -> 44     B1024 H12, trained bias 328 -> 128, 439 -> 458
+//   B256 H6 64 x 64 D64       no bias 31 -> 16, 60 -> 44     B1024 H12, trained bias 321 -> 127, 438 -> 453
+//   (the one kind whose backward alone loses, up to 5 %: a trained 16-bit bias of each problem's own at D 64, 49 to 64 rows, thousands of
+//   problems; forward and backward 1.3 times as fast.  1536 problems of 64 x 64: 40 -> 19, 65.0 -> 65.2; of 56 x 56: 41 -> 17, 64 -> 55)
 //   B1024 H8 17 x 17 D16      trained bias 186 -> 24, 254 -> 51
 // The limit is 64: with up to 128 rows and keys and eight warps the same kernels lost as soon as the problems fill the
 // chip (B256 H12 128 x 128 D64: 57 -> 95, 152 -> 242; 96 x 96 D32, mask: 77 -> 74, 118 -> 159; 64 x 128: 53 -> 52,
