@@ -642,6 +642,47 @@ __device__ __forceinline__ bool wait_warp_hot(uint64_t* bar, uint32_t parity, co
   return __all_sync(0xffffffffu, ok);
 }
 
+// One to three phases at once for a converged control warp, with one vote: where they have all completed, as loads
+// have as a rule, this takes one round of looks instead of one after the other.  SPIN: every lane polls without suspending
+// (a suspended wait wakes up some hundred cycles late, polling takes issue slots from the row warps); otherwise the wait
+// for the first one, which should be the one that comes last, suspends.
+template <bool SPIN>
+__device__ __forceinline__ bool wait_all1(uint64_t* b0, uint32_t p0, const WaitCtx& ctx, int site, int iter) {
+  return SPIN ? wait_warp_hot(b0, p0, ctx, site, iter) : wait_warp(b0, p0, ctx, site, iter);
+}
+template <bool SPIN>
+__device__ __forceinline__ bool wait_all2(uint64_t* b0, uint32_t p0, uint64_t* b1, uint32_t p1, const WaitCtx& ctx, int site,
+                                          int iter) {
+  if (SPIN) {
+#pragma unroll 1
+    for (int i = 0; i < 2048; ++i) {
+      uint32_t r0, r1;
+      mbar_poll2(b0, p0, b1, p1, r0, r1);
+      if (__all_sync(0xffffffffu, (r0 & r1) != 0)) return true;
+    }
+  }
+  const uint32_t r1 = mbar_poll(b1, p1);
+  const bool ok = mbar_wait(b0, p0, ctx, site, iter) && (r1 || mbar_wait(b1, p1, ctx, site, iter));
+  return __all_sync(0xffffffffu, ok);
+}
+template <bool SPIN>
+__device__ __forceinline__ bool wait_all3(uint64_t* b0, uint32_t p0, uint64_t* b1, uint32_t p1, uint64_t* b2, uint32_t p2,
+                                          const WaitCtx& ctx, int site, int iter) {
+  if (SPIN) {
+#pragma unroll 1
+    for (int i = 0; i < 2048; ++i) {
+      uint32_t r0, r1, r2;
+      mbar_poll3(b0, p0, b1, p1, b2, p2, r0, r1, r2);
+      if (__all_sync(0xffffffffu, (r0 & r1 & r2) != 0)) return true;
+    }
+  }
+  uint32_t r1, r2;
+  mbar_poll2(b1, p1, b2, p2, r1, r2);
+  const bool ok = mbar_wait(b0, p0, ctx, site, iter) && (r1 || mbar_wait(b1, p1, ctx, site, iter)) &&
+                  (r2 || mbar_wait(b2, p2, ctx, site, iter));
+  return __all_sync(0xffffffffu, ok);
+}
+
 // Finish a wait whose phase was polled earlier: no further barrier traffic when the
 // poll had already seen the phase complete.
 __device__ __forceinline__ bool wait_polled(uint32_t polled, uint64_t* bar, uint32_t parity,

@@ -80,15 +80,21 @@ struct FwdSmem {
   static constexpr int kQTile = 128 * DP * 2;   // one query tile
   static constexpr int kKStage = 128 * DP * 2;  // 128 keys
   static constexpr int kVHalf = 64 * DP * 2;    // 64 keys
-  // Head dim 256: one query tile per unit, single K stage, two V half stages, two bias units
-  // (64 + 64 + 64 + 32 KB); otherwise two tiles, 2 / 3 / 3 stages (64 + 64 + 48 + 48 KB at 128).
+  // Head dim 256: one query tile per unit, K and V in two half stages each, two bias units (64 + 64 + 64 + 32 KB);
+  // otherwise two tiles, two K stages, and with a float bias a fourth bias unit rather than a third V half (64 + 64 + 32
+  // + 64 KB at 128).  us, V halves x bias units 3 x 3 / 2 x 4: 16 bit B1 H37 S4096 D128 397 / 388, causal H32 220 / 209,
+  // fp32 600 / 533 (and 525 / 640 without a bias, which keeps three halves); D64, 16 bit, 3 x 3 / 2 x 6 / 3 x 6 / 4 x 4:
+  // 358 / 349 / 348 / 328.
   static constexpr int kTiles = DP == 256 ? 1 : 2;
-  static constexpr int kKStages = DP == 256 ? 1 : 2;
-  static constexpr int kVStages = DP == 256 ? 2 : 3;
-  static constexpr int kBiasStages = BIAS == 0 ? 0 : (DP == 256 ? 2 : 3);  // 16 KB units
+  static constexpr bool kKHalves = DP == 256;  // K passes through its ring in 64-key halves
+  static constexpr int kKUnit = kKHalves ? kKStage / 2 : kKStage;
+  static constexpr int kKStages = 2;
+  static constexpr bool kFloatBias = BIAS == 1 || BIAS == 3;
+  static constexpr int kVStages = DP == 256 ? 2 : (!kFloatBias ? 3 : (DP == 64 ? 4 : 2));
+  static constexpr int kBiasStages = BIAS == 0 ? 0 : (DP == 256 ? 2 : (kFloatBias ? 4 : 3));  // 16 KB units
   static constexpr int kQ = 0;
   static constexpr int kK = kQ + kTiles * kQTile;
-  static constexpr int kV = kK + kKStages * kKStage;
+  static constexpr int kV = kK + kKStages * kKUnit;
   static constexpr int kBias = kV + kVStages * kVHalf;
   static constexpr int kTotal = kBias + kBiasStages * kBlk;
   static constexpr int kDynamic = kTotal + 1024;  // slack for 1024-byte alignment
@@ -190,9 +196,9 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  __shared__ uint64_t q_full, q_empty, k_full[2], k_empty[2], v_full[3], v_empty[3];  // rings: up to 2 / 3 stages
+  __shared__ uint64_t q_full, q_empty, k_full[2], k_empty[2], v_full[4], v_empty[4];  // rings: up to 2 / 4 stages
   __shared__ uint64_t s_full[2][2], s_read[2], p_full[2][2], pv_done[2][2];
-  __shared__ uint64_t bias_full[2][3], bias_empty[3];  // full: one set per consuming group
+  __shared__ uint64_t bias_full[2][4], bias_empty[4];  // full: one set per consuming group
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
@@ -217,7 +223,7 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
         mbar_init(&pv_done[i][h], 1);
       }
     }
-    for (int i = 0; i < 3; ++i) {
+    for (int i = 0; i < 4; ++i) {
       mbar_init(&v_full[i], 1);
       mbar_init(&v_empty[i], 2);
       mbar_init(&bias_full[0][i], 1);
@@ -264,29 +270,47 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
                           (u.mb0 + t) * 128, b);
         }
         __syncwarp();
-        for (int j = 0; j < u.nmax && ok; ++j, ++gk) {
-          const uint32_t ks = gk % KST;
-          const int n0 = j * 128;
-          if (gk >= KST) ok = wait_warp(&k_empty[ks], (gk / KST - 1) & 1, ctx, kSiteKEmpty, j);
-          if (!ok) break;
-          if (elect_one()) {
-            mbar_expect_tx(&k_full[ks], L::kKStage);
+        auto load_v = [&](int j, int hf) {
+          const uint32_t vs = gv % VS, use = gv / VS;
+          ++gv;
+          if (use >= 1) ok = wait_warp(&v_empty[vs], (use - 1) & 1, ctx, kSiteVEmpty, j);
+          if (ok && elect_one()) {
+            mbar_expect_tx(&v_full[vs], L::kVHalf);
             for (int kb = 0; kb < KB; ++kb)
-              tma_load_4d(smem + L::kK + ks * L::kKStage + kb * kBlk, &p.map_k, &k_full[ks], kb * 64, h,
-                          n0, b);
+              tma_load_4d(smem + L::kV + vs * L::kVHalf + kb * kVBlk, &p.map_v, &v_full[vs], kb * 64, h,
+                          j * 128 + hf * 64, b);
           }
           __syncwarp();
-          for (int hf = 0; hf < 2 && ok; ++hf, ++gv) {
-            const uint32_t vs = gv % VS, use = gv / VS;
-            if (use >= 1) ok = wait_warp(&v_empty[vs], (use - 1) & 1, ctx, kSiteVEmpty, j);
-            if (!ok) break;
-            if (elect_one()) {
-              mbar_expect_tx(&v_full[vs], L::kVHalf);
-              for (int kb = 0; kb < KB; ++kb)
-                tma_load_4d(smem + L::kV + vs * L::kVHalf + kb * kVBlk, &p.map_v, &v_full[vs], kb * 64, h,
-                            n0 + hf * 64, b);
+        };
+        auto load_k = [&](int j, int hf) {  // a block, or one half of it
+          constexpr int kBox = L::kKHalves ? kVBlk : kBlk;
+          const uint32_t ks = gk % KST, use = gk / KST;
+          ++gk;
+          if (use >= 1) ok = wait_warp(&k_empty[ks], (use - 1) & 1, ctx, kSiteKEmpty, j);
+          if (ok && elect_one()) {
+            mbar_expect_tx(&k_full[ks], L::kKUnit);
+            for (int kb = 0; kb < KB; ++kb)
+              tma_load_4d(smem + L::kK + ks * L::kKUnit + kb * kBox, &p.map_k, &k_full[ks], kb * 64, h,
+                          j * 128 + hf * 64, b);
+          }
+          __syncwarp();
+        };
+        if constexpr (L::kKHalves) {
+          // in the order in which the stages are handed back
+          load_k(0, 0);
+          if (ok) load_k(0, 1);
+          for (int j = 0; j < u.nmax && ok; ++j)
+            for (int hf = 0; hf < 2 && ok; ++hf) {
+              load_v(j, hf);
+              if (ok && j + 1 < u.nmax) load_k(j + 1, hf);
             }
-            __syncwarp();
+        } else {
+          // K of the next block before V of this one: its stage is free earlier, and its scores are wanted first
+          // (behind V a tile that runs ahead of the other waited some 1000 cycles a step for K with a float bias)
+          load_k(0, 0);
+          for (int j = 0; j < u.nmax && ok; ++j) {
+            if (j + 1 < u.nmax) load_k(j + 1, 0);
+            for (int hf = 0; hf < 2 && ok; ++hf) load_v(j, hf);
           }
         }
       }
@@ -296,15 +320,16 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
     // (the whole warp walks the loop converged, one elected lane issues)
     if (live) {
       const int t = warp == 9 ? 0 : 1;
-      // A wait on a completed barrier takes 200 - 235 cycles.  Without a bias the issuer is on the critical path, so it
-      // looks at the loads, which have landed by then as a rule, while the row threads still form P or
-      // read S (causal B2 H32 S4096 D128: 342 -> 328 us).  With a mask that gains where the products are long
-      // enough to matter and loses where they are not; with a float bias the row threads are behind anyway.
-      // us, B4 H16 S2048 (D = 256: B2 H8), loads last / first, then causal:
-      //   mask   D128 194.8 / 189.2, 121.0 / 119.7     D64 174.3 / 193.8, 102.9 / 107.1    D256 96.2 / 98.7
-      //   16 bit D128 198.4 / 198.2, 125.2 / 125.3     D64 180.8 / 181.8, 106.9 / 106.9    D256 97.1 / 100.3
-      //   fp32   D128 351.3 / 349.7, 210.4 / 209.4     D64 332.0 / 329.0, 186.4 / 185.3    D256 116.9 / 115.9
-      constexpr bool kLoadsFirst = BIAS == 0 || (BIAS == 2 && DP == 128);
+      // The issuer is on the critical path, and a wait takes some 200 cycles even on a completed barrier, an elect with
+      // its reconvergence another 100.  So the three groups of products of a step (P V of the first half, scores of the
+      // next block's first half, P V of the second half with the scores of the next block's second half) have one
+      // combined look and one elected stretch each, ring stages handed back included: 3500 -> 3060 cycles a step
+      // without a bias at D128.  us, before / after: B2 H37 S4096 D128 549 / 530, causal H32 307 / 284; B1 H37 S4096 with a
+      // mask D128 371 / 349, D64 334 / 311; B1 H37 S2048 D256 197 / 150 (with the K halves).
+      // It polls without suspending at D128 and D256 (D256 149.5, suspended 155.6); at D64 the row threads need the issue
+      // slots more (mask 324, suspended 311).  The producers wait suspended for the same reason (mask D128 373 polling,
+      // 346 suspended).
+      constexpr bool kSpin = DP > 64;
       constexpr bool bf = P2::kIsBf16;
       constexpr uint32_t idesc_qk = make_idesc(bf, false, false, 128, 64);
       constexpr uint32_t idesc_pv = make_idesc(bf, false, true, 128, DP);
@@ -315,80 +340,96 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
       uint32_t cs = 0;          // steps done by this tile slot, over all units
       uint32_t gk = 0, gv = 0;  // key blocks / V halves consumed before this unit
       Unit u;
-      // scores of one 64-key half of the block in ring stage `kslot` -> column half `ch`
-      auto issue_qk = [&](uint32_t kslot, int keys, uint32_t ch) {
-        if (elect_one()) {
-          issue_gemm_ss<KS_QK, false, false>(tm_s + ch * 64, make_sdesc(q_addr, 0, 1024),
-                                             make_sdesc(k_addr + kslot * L::kKStage + keys * (64 * 128), 0, 1024),
-                                             kBlk, kBlk, idesc_qk, false);
-          mma_commit(&s_full[t][keys]);
-        }
-        __syncwarp();
+      // What an elected lane issues: the scores of one 64-key half of key block `kb` -> column half `ch`,
+      auto qk = [&](uint32_t kb, int half, uint32_t ch) {
+        const uint32_t ka = L::kKHalves ? k_addr + half * L::kKUnit : k_addr + (kb % KST) * L::kKUnit + half * (64 * 128);
+        constexpr uint32_t kKBlk = L::kKHalves ? kVBlk : kBlk;
+        issue_gemm_ss<KS_QK, false, false>(tm_s + ch * 64, make_sdesc(q_addr, 0, 1024), make_sdesc(ka, 0, 1024), kBlk,
+                                           kKBlk, idesc_qk, false);
+        mma_commit(&s_full[t][half]);
       };
-      auto commit = [&](uint64_t* bar) {
-        if (elect_one()) mma_commit(bar);
-        __syncwarp();
+      // ... and O += P V of half `half`
+      auto pv = [&](uint32_t vs, int half, uint32_t f, bool first) {
+        issue_gemm_ts<4, true>(tm_o, tm_s + f * 64 + half * 32, make_sdesc(v_addr + vs * L::kVHalf, kVBlk, 1024), kVBlk,
+                               idesc_pv, !first);
+        mma_commit(&pv_done[t][half]);
       };
+      // K ring stage and parity that a half of key block `kb` (counted over all units) is in
+      auto k_stage = [&](uint32_t kb, int half) { return L::kKHalves ? static_cast<uint32_t>(half) : kb % KST; };
+      auto k_par = [&](uint32_t kb) { return (L::kKHalves ? kb : kb / KST) & 1; };
       for (int it = 0; ok && unit_at<L::kTiles>(p, it, u); ++it) {
         if (u.nmax == 0) continue;
         const int nblk = u.nb(t);
-        ok = wait_warp(&q_full, it & 1, ctx, kSiteQFull, it);
-        if (ok) ok = wait_warp(&k_full[gk % KST], (gk / KST) & 1, ctx, kSiteKFull, 0);
+        ok = wait_all2<kSpin>(&q_full, it & 1, &k_full[k_stage(gk, 0)], k_par(gk), ctx, kSiteQFull, it);
+        if (ok && L::kKHalves) ok = wait_all1<kSpin>(&k_full[1], k_par(gk), ctx, kSiteKFull, 0);
         if (!ok) break;
         tc_fence_after();
-        if (nblk > 0) {
-          issue_qk(gk % KST, 0, cs & 1);
-          issue_qk(gk % KST, 1, (cs & 1) ^ 1);
+        if (elect_one()) {
+          if (nblk > 0) {
+            qk(gk, 0, cs & 1);
+            if (L::kKHalves) mma_commit(&k_empty[0]);
+            qk(gk, 1, (cs & 1) ^ 1);
+          } else if (L::kKHalves) {
+            mma_commit(&k_empty[0]);
+          }
+          mma_commit(&k_empty[k_stage(gk, 1)]);
+          if (u.nmax == 1) mma_commit(&q_empty);
         }
-        commit(&k_empty[gk % KST]);
-        if (u.nmax == 1) commit(&q_empty);
         for (int j = 0; j < u.nmax && ok; ++j) {
-          const uint32_t kn = (gk + j + 1) % KST, kn_par = ((gk + j + 1) / KST) & 1;
+          const uint32_t kn = gk + j + 1;
           const bool more = j + 1 < u.nmax;  // the unit has a block j+1 (this tile may not visit it)
           const bool mine = j < nblk, mine_next = j + 1 < nblk;
           const uint32_t f = cs & 1;  // column half that holds keys 0-63 of this step, and P
-          for (int h = 0; h < 2 && ok; ++h) {
-            const uint32_t gh = gv + 2 * j + h;
-            const uint32_t vs = gh % VS, v_par = (gh / VS) & 1;
-            if (mine) {
-              if (kLoadsFirst) ok = wait_warp(&v_full[vs], v_par, ctx, kSiteVFull, j);
-              if (ok) ok = wait_warp_hot(&p_full[t][h], cs & 1, ctx, kSitePFull, j);
-              if (ok && !kLoadsFirst) ok = wait_warp(&v_full[vs], v_par, ctx, kSiteVFull, j);
-              if (!ok) break;
-              tc_fence_after();
-              if (elect_one()) {
-                issue_gemm_ts<4, true>(tm_o, tm_s + f * 64 + h * 32,
-                                       make_sdesc(v_addr + vs * L::kVHalf, kVBlk, 1024), kVBlk, idesc_pv,
-                                       j > 0 || h > 0);
-                mma_commit(&pv_done[t][h]);
-              }
-              __syncwarp();
-            } else {
-              // a block only the other tile visits: keep the ring counters in step
-              ok = wait_warp(&v_full[vs], v_par, ctx, kSiteVFull, j);
-              if (!ok) break;
-            }
-            commit(&v_empty[vs]);
-            if (h == 0) {
-              // Keys 0-63 of block j+1 go into the column half whose scores (keys 64-127 of
-              // block j) the row threads have just taken into registers: this product runs
-              // under the second half of this step's softmax.
-              if (kLoadsFirst && more) ok = wait_warp(&k_full[kn], kn_par, ctx, kSiteKFull, j + 1);
-              if (ok && mine) ok = wait_warp_hot(&s_read[t], cs & 1, ctx, kSiteSRead, j);
-              if (ok && !kLoadsFirst && more) ok = wait_warp(&k_full[kn], kn_par, ctx, kSiteKFull, j + 1);
-              if (!ok) break;
-              if (mine_next) {
-                tc_fence_after();
-                issue_qk(kn, 0, f ^ 1);
-              }
-            } else {
-              // Keys 64-127 of block j+1 go over the columns P of block j is read from: same
-              // issuing thread, so it executes after the products just issued.
-              if (mine_next) issue_qk(kn, 1, f);
-              if (more) {
-                commit(&k_empty[kn]);
-                if (j + 2 >= u.nmax) commit(&q_empty);
-              }
+          const uint32_t g0 = gv + 2 * j, v0 = g0 % VS, v1 = (g0 + 1) % VS;
+          uint64_t* const vb0 = &v_full[v0];
+          uint64_t* const vb1 = &v_full[v1];
+          const uint32_t vp0 = (g0 / VS) & 1, vp1 = ((g0 + 1) / VS) & 1;
+          // One combined look before each of the three groups of products.  A block only the other tile visits:
+          // the loads are waited for all the same, so that the ring counters stay in step.
+          uint64_t* const kb0 = more ? &k_full[k_stage(kn, 0)] : vb0;
+          const uint32_t kp0 = more ? k_par(kn) : vp0;
+          if (mine)
+            ok = L::kKHalves ? wait_all2<kSpin>(&p_full[t][0], cs & 1, vb0, vp0, ctx, kSitePFull, j)
+                             : wait_all3<kSpin>(&p_full[t][0], cs & 1, vb0, vp0, kb0, kp0, ctx, kSitePFull, j);
+          else
+            ok = wait_all2<kSpin>(vb0, vp0, kb0, kp0, ctx, kSiteVFull, j);
+          if (!ok) break;
+          tc_fence_after();
+          if (elect_one()) {
+            if (mine) pv(v0, 0, f, j == 0);
+            mma_commit(&v_empty[v0]);
+          }
+          // Keys 0-63 of block j+1 go into the column half whose scores (keys 64-127 of
+          // block j) the row threads have just taken into registers: this product runs
+          // under the second half of this step's softmax.
+          if (mine) {
+            ok = L::kKHalves ? wait_all2<kSpin>(&s_read[t], cs & 1, kb0, kp0, ctx, kSiteSRead, j)
+                             : wait_all1<kSpin>(&s_read[t], cs & 1, ctx, kSiteSRead, j);
+            if (!ok) break;
+            tc_fence_after();
+          }
+          if (elect_one()) {
+            if (mine_next) qk(kn, 0, f ^ 1);
+            if (L::kKHalves && more) mma_commit(&k_empty[0]);
+          }
+          // Keys 64-127 of block j+1 go over the columns P of block j is read from: same
+          // issuing thread, so it executes after the products just issued.
+          uint64_t* const kb1 = L::kKHalves && more ? &k_full[1] : vb1;
+          const uint32_t kp1 = L::kKHalves && more ? k_par(kn) : vp1;
+          if (mine)
+            ok = L::kKHalves ? wait_all3<kSpin>(&p_full[t][1], cs & 1, vb1, vp1, kb1, kp1, ctx, kSitePFull, j)
+                             : wait_all2<kSpin>(&p_full[t][1], cs & 1, vb1, vp1, ctx, kSitePFull, j);
+          else
+            ok = wait_all2<kSpin>(vb1, vp1, kb1, kp1, ctx, kSiteVFull, j);
+          if (!ok) break;
+          tc_fence_after();
+          if (elect_one()) {
+            if (mine) pv(v1, 1, f, false);
+            mma_commit(&v_empty[v1]);
+            if (mine_next) qk(kn, 1, f);
+            if (more) {
+              mma_commit(&k_empty[k_stage(kn, 1)]);
+              if (j + 2 >= u.nmax) mma_commit(&q_empty);
             }
           }
           if (mine) ++cs;
@@ -481,14 +522,15 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
             // folded into the exponent below.
             float mul = kLog2e;  // exponent = s * mul - m
             float mx = -INFINITY;  // row maximum of this half
-            if (BIAS == 0) {
+            if (BIAS == 0 || BIAS == 2) {
               if (fold_scale) {
                 mul = scale_log2;
               } else {
 #pragma unroll
                 for (int i = 0; i < 64; ++i) s[i] *= p.sm_scale;
               }
-            } else {
+            }
+            if (BIAS != 0) {
               if (BIAS != 2 || h == 0) {
                 ok = wait_warp_polled(pbias, &bias_full[t][bs], b_par, ctx, kSiteBiasFull, j);
                 if (!ok) break;
@@ -559,7 +601,7 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
                     for (int k = 0; k < 4; ++k) {
                       const int i = c * 16 + e * 4 + k;
                       const bool keep = ((w[e] >> (8 * k)) & 0xFFu) != 0;
-                      s[i] = keep ? s[i] * p.sm_scale : -INFINITY;
+                      if (!keep) s[i] = -INFINITY;
                     }
                   }
                 }
@@ -743,7 +785,7 @@ int launch_fwd(const fa_params& p, cudaStream_t stream, int* status) {
   FwdParams fp;
   int r = make_tmap_bshd(&fp.map_q, p.q, p.B, p.M, p.H, p.D, p.q_stride, 128);
   if (r) return r;
-  r = make_tmap_bshd(&fp.map_k, p.k, p.B, p.N, p.H, p.D, p.k_stride, 128);
+  r = make_tmap_bshd(&fp.map_k, p.k, p.B, p.N, p.H, p.D, p.k_stride, p.D == 256 ? 64 : 128);
   if (r) return r;
   r = make_tmap_bshd(&fp.map_v, p.v, p.B, p.N, p.H, p.D, p.v_stride, 64);
   if (r) return r;
