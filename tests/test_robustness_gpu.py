@@ -361,6 +361,28 @@ def test_full_size_forwards_repeat_bitwise(D, bias_kind, causal, device_ok):
     assert differing == 0, f"{differing} of 40 passes differ"
 
 
+@pytest.mark.parametrize("D,bias_kind", [(256, "16bit"), (256, "none"), (256, "bool"), (128, "16bit"), (128, "none"), (64, "f32")])
+def test_causal_units_of_every_length_repeat_bitwise(D, bias_kind, device_ok):
+    """Units of one key block and longer ones in turn, several a CTA, a hundred passes: every wait ends and the bits stay.
+    (An issuer that looked again at the barrier of a ring stage it had already handed back found it a completion further
+    about once in some hundred launches and waited for good.)"""
+    from triton_flashattn_b200 import flash_attention as fa
+
+    B, S, H = 2, 1000, 40
+    g = torch.Generator(device="cuda").manual_seed(66)
+    q, k, v = (torch.randn(B, S, H, D, generator=g, device="cuda", dtype=torch.float32).to(BF) for _ in range(3))
+    bias = None
+    if bias_kind == "bool":
+        bias = torch.rand(B, H, S, S, generator=g, device="cuda") < 0.9
+    elif bias_kind != "none":
+        bias = torch.randn(B, H, S, S, generator=g, device="cuda", dtype=torch.float32 if bias_kind == "f32" else BF)
+    first, lse = fa._flash_attn_fwd(q, k, v, bias, True, D ** -0.5)
+    for _ in range(100):
+        out, lse2 = fa._flash_attn_fwd(q, k, v, bias, True, D ** -0.5)
+    torch.cuda.synchronize()
+    assert torch.equal(out, first) and torch.equal(lse, lse2)
+
+
 @pytest.mark.parametrize("bias_kind,D", [(0, 64), (2, 128), (0, 256), (3, 128)])
 def test_scratch_for_ds_is_bounded(bias_kind, D, device_ok):
     """The scratch a backward asks for: at most 1.5 GiB, and nothing where that holds no problem or too few to fill

@@ -403,8 +403,10 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
           // block j) the row threads have just taken into registers: this product runs
           // under the second half of this step's softmax.
           if (mine) {
-            ok = L::kKHalves ? wait_all2<kSpin>(&s_read[t], cs & 1, kb0, kp0, ctx, kSiteSRead, j)
-                             : wait_all1<kSpin>(&s_read[t], cs & 1, ctx, kSiteSRead, j);
+            // (Not with vb0 in the place of a block that does not exist: its stage has been handed back, so the barrier
+            // may be a completion further already and its parity another one.)
+            ok = L::kKHalves && more ? wait_all2<kSpin>(&s_read[t], cs & 1, kb0, kp0, ctx, kSiteSRead, j)
+                                     : wait_all1<kSpin>(&s_read[t], cs & 1, ctx, kSiteSRead, j);
             if (!ok) break;
             tc_fence_after();
           }
