@@ -383,6 +383,30 @@ def test_causal_units_of_every_length_repeat_bitwise(D, bias_kind, device_ok):
     assert torch.equal(out, first) and torch.equal(lse, lse2)
 
 
+@pytest.mark.parametrize("D,bias_kind,M,N", [(64, "none", 900, 900), (64, "f32", 1030, 300), (128, "16bit", 1100, 700),
+                                             (128, "bool", 520, 1304), (128, "none", 129, 129), (256, "16bit", 500, 500)])
+def test_causal_forward_order_does_not_change_bits(D, bias_kind, M, N, device_ok, monkeypatch):
+    """Pairs of a heavy and a light unit, or longest first: the number of CTAs decides, each row is the same work."""
+    from oracle import eager_oracle as oracle
+    from triton_flashattn_b200 import flash_attention as fa
+
+    g = torch.Generator(device="cuda").manual_seed(67)
+    q, k, v = (torch.randn(1, s, 5, D, generator=g, device="cuda", dtype=torch.float32).to(BF) for s in (M, N, N))
+    bias = None
+    if bias_kind == "bool":
+        bias = torch.rand(1, 5, M, N, generator=g, device="cuda") < 0.9
+    elif bias_kind != "none":
+        bias = torch.randn(1, 5, M, N, generator=g, device="cuda", dtype=torch.float32 if bias_kind == "f32" else BF)
+    first, lse = fa._flash_attn_fwd(q, k, v, bias, True, D ** -0.5)
+    ref = oracle.attention_forward(q, k, v, bias, True, D ** -0.5)[0]
+    seen = ref.abs().sum(-1, keepdim=True) > 0  # rows with no key at all are zeros here
+    assert ((first.float() - ref.float()) * seen).abs().max() <= 2e-2 + 2 ** -7 * ref.abs().max()
+    for cap in (1, 2, 3, 7, 11, 16, 19):
+        monkeypatch.setenv("FA_MAX_CTAS", str(cap))
+        out, lse2 = fa._flash_attn_fwd(q, k, v, bias, True, D ** -0.5)
+        assert torch.equal(out, first) and torch.equal(lse, lse2), cap
+
+
 @pytest.mark.parametrize("bias_kind,D", [(0, 64), (2, 128), (0, 256), (3, 128)])
 def test_scratch_for_ds_is_bounded(bias_kind, D, device_ok):
     """The scratch a backward asks for: at most 1.5 GiB, and nothing where that holds no problem or too few to fill

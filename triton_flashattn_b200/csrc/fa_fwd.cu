@@ -69,6 +69,7 @@ struct FwdParams {
   int o_vec32;  // o's base and strides are multiples of 32 bytes
   int bias_b_mul, bias_h_mul;
   int n_mblk, n_pairs, n_units;  // query blocks / block pairs per (batch, head); units = pairs * B * H
+  int n_bh;                      // B * H
   float sm_scale;
 };
 
@@ -104,21 +105,34 @@ struct FwdSmem {
 // (batch*head)-major; CTA c takes c, c+G, c+2G, ... so that CTAs running at the same time
 // share K / V in L2.  Causal: the entries of one (batch, head) are ordered [last, first,
 // last-1, first+1, ...] and a CTA takes two consecutive ones, a heavy and a light pair.
+// With LONGEST_FIRST (causal, see plan_fwd) the units are numbered by length instead, and the CTAs take them in rows, every
+// second row from the other end: what a CTA has too much of in one row it has too little of in the next.  It is a variant
+// of its own because every role walks the schedule: chosen at run time it made every other forward 0.5 - 1 % slower.
 struct Unit {
   int bh, mb0;   // (batch, head) and first query block of the pair
   int nb0, nb1;  // key blocks each tile visits (0: the tile does not exist)
   int nmax;
   __device__ __forceinline__ int nb(int t) const { return t ? nb1 : nb0; }
 };
-template <int TILES>  // query tiles per unit: 2, or 1 at head dim 256
+template <int TILES, bool LONGEST_FIRST>  // query tiles per unit: 2, or 1 at head dim 256
 __device__ __forceinline__ bool unit_at(const FwdParams& p, int it, Unit& u) {
-  const int sh = p.causal ? 1 : 0;
-  const int c = static_cast<int>(blockIdx.x) + (it >> sh) * static_cast<int>(gridDim.x);
-  const int k = (c << sh) + (it & sh);
-  if (k >= p.n_units) return false;
-  u.bh = k / p.n_pairs;
-  const int pos = k - u.bh * p.n_pairs;
-  const int pair = p.causal ? ((pos & 1) ? (pos >> 1) : p.n_pairs - 1 - (pos >> 1)) : pos;
+  int pair;
+  if constexpr (LONGEST_FIRST) {
+    const int G = static_cast<int>(gridDim.x), c = static_cast<int>(blockIdx.x);
+    const int k = it * G + ((it & 1) ? G - 1 - c : c);
+    if (k >= p.n_units) return false;
+    const int level = k / p.n_bh;
+    u.bh = k - level * p.n_bh;
+    pair = p.n_pairs - 1 - level;
+  } else {
+    const int sh = p.causal ? 1 : 0;
+    const int c = static_cast<int>(blockIdx.x) + (it >> sh) * static_cast<int>(gridDim.x);
+    const int k = (c << sh) + (it & sh);
+    if (k >= p.n_units) return false;
+    u.bh = k / p.n_pairs;
+    const int pos = k - u.bh * p.n_pairs;
+    pair = p.causal ? ((pos & 1) ? (pos >> 1) : p.n_pairs - 1 - (pos >> 1)) : pos;
+  }
   u.mb0 = pair * TILES;
   const int nblk_all = (p.N + 127) >> 7;
   u.nb0 = u.mb0 >= p.n_mblk ? 0 : (p.causal ? min(nblk_all, u.mb0 + 1) : nblk_all);
@@ -130,7 +144,7 @@ __device__ __forceinline__ bool unit_at(const FwdParams& p, int it, Unit& u) {
 // Walks the bias units of this CTA in the order the softmax groups consume them:
 // per unit, per key block j, per tile t (if it visits j): two 64-key halves (16-bit bias),
 // four 32-key quarters (fp32 bias) or one unit (byte mask, [128][128] bytes per block).
-template <int BIAS, int TILES>
+template <int BIAS, int TILES, bool LONGEST_FIRST>
 struct BiasWalk {
   static constexpr int kSub = BIAS == 1 ? 2 : (BIAS == 3 ? 4 : 1);  // units per (tile, block)
   int it = 0, j = 0, t = 0, h = 0;
@@ -143,7 +157,7 @@ struct BiasWalk {
         ++it;
         j = 0;
         t = 0;
-        valid = unit_at<TILES>(p, it, u);
+        valid = unit_at<TILES, LONGEST_FIRST>(p, it, u);
         continue;
       }
       if (t >= 2) {
@@ -159,7 +173,7 @@ struct BiasWalk {
     }
   }
   __device__ __forceinline__ void start(const FwdParams& p) {
-    valid = unit_at<TILES>(p, 0, u);
+    valid = unit_at<TILES, LONGEST_FIRST>(p, 0, u);
     settle(p);
   }
   __device__ __forceinline__ void next(const FwdParams& p) {
@@ -181,7 +195,7 @@ struct BiasWalk {
   }
 };
 
-template <int DP, typename T, int BIAS>
+template <int DP, typename T, int BIAS, bool LONGEST_FIRST>
 __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ FwdParams p) {
   using L = FwdSmem<DP, BIAS>;
   using P2 = Pack2<T>;
@@ -257,7 +271,7 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
       bool ok = true;
       uint32_t gk = 0, gv = 0;  // key blocks / V halves issued so far, over all units
       Unit u;
-      for (int it = 0; ok && unit_at<L::kTiles>(p, it, u); ++it) {
+      for (int it = 0; ok && unit_at<L::kTiles, LONGEST_FIRST>(p, it, u); ++it) {
         const int b = u.bh / p.H, h = u.bh - b * p.H;
         // the Q pair is free once every Q K^T product of the previous unit is through
         if (it >= 1) ok = wait_warp(&q_empty, (it - 1) & 1, ctx, kSiteQEmpty, it);
@@ -357,7 +371,7 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
       // K ring stage and parity that a half of key block `kb` (counted over all units) is in
       auto k_stage = [&](uint32_t kb, int half) { return L::kKHalves ? static_cast<uint32_t>(half) : kb % KST; };
       auto k_par = [&](uint32_t kb) { return (L::kKHalves ? kb : kb / KST) & 1; };
-      for (int it = 0; ok && unit_at<L::kTiles>(p, it, u); ++it) {
+      for (int it = 0; ok && unit_at<L::kTiles, LONGEST_FIRST>(p, it, u); ++it) {
         if (u.nmax == 0) continue;
         const int nblk = u.nb(t);
         ok = wait_all2<kSpin>(&q_full, it & 1, &k_full[k_stage(gk, 0)], k_par(gk), ctx, kSiteQFull, it);
@@ -447,7 +461,7 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
     if (BIAS != 0 && live) {
       if (lane == 0) tma_prefetch_desc(&p.map_bias);
       const uint64_t pol_stream = policy_evict_first();
-      BiasWalk<BIAS, L::kTiles> cur;
+      BiasWalk<BIAS, L::kTiles, LONGEST_FIRST> cur;
       cur.start(p);
       bool ok = true;
       for (uint32_t unit = 0; ok && cur.valid; ++unit) {
@@ -488,7 +502,7 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
     // b_phase is the parity of this group's next unit in slot s.
     uint32_t b_phase = 0;
     Unit u;
-    for (int it = 0; ok && unit_at<L::kTiles>(p, it, u); ++it) {
+    for (int it = 0; ok && unit_at<L::kTiles, LONGEST_FIRST>(p, it, u); ++it) {
       const int nblk = u.nb(t);
       const int m0 = (u.mb0 + t) * 128;
       float m_used = -INFINITY;  // running maximum, log2 domain
@@ -749,10 +763,10 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
   if (warp == 9) tmem_dealloc(tmem, kTmemCols);
 }
 
-template <int DP, typename T, int BIAS>
+template <int DP, typename T, int BIAS, bool LONGEST_FIRST>
 int launch_inst(const FwdParams& fp, dim3 grid, cudaStream_t stream) {
   using L = FwdSmem<DP, BIAS>;
-  auto kern = fwd_kernel<DP, T, BIAS>;
+  auto kern = fwd_kernel<DP, T, BIAS, LONGEST_FIRST>;
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -765,15 +779,83 @@ int launch_inst(const FwdParams& fp, dim3 grid, cudaStream_t stream) {
   return launch_overlapped(kern, grid, 384, L::kDynamic, stream, fp);
 }
 
-template <int DP, typename T>
+template <int DP, typename T, bool LONGEST_FIRST>
 int launch_bias(const FwdParams& fp, int bias_kind, dim3 grid, cudaStream_t stream) {
   switch (bias_kind) {
-    case FA_BIAS_NONE: return launch_inst<DP, T, 0>(fp, grid, stream);
-    case FA_BIAS_SAME: return launch_inst<DP, T, 1>(fp, grid, stream);
-    case FA_BIAS_BOOL: return launch_inst<DP, T, 2>(fp, grid, stream);
-    case FA_BIAS_F32: return launch_inst<DP, T, 3>(fp, grid, stream);
+    case FA_BIAS_NONE: return launch_inst<DP, T, 0, LONGEST_FIRST>(fp, grid, stream);
+    case FA_BIAS_SAME: return launch_inst<DP, T, 1, LONGEST_FIRST>(fp, grid, stream);
+    case FA_BIAS_BOOL: return launch_inst<DP, T, 2, LONGEST_FIRST>(fp, grid, stream);
+    case FA_BIAS_F32: return launch_inst<DP, T, 3, LONGEST_FIRST>(fp, grid, stream);
     default: return FA_ERR_UNSUPPORTED;
   }
+}
+template <bool LONGEST_FIRST>
+int launch_dim(const FwdParams& fp, int dtype, int bias_kind, dim3 grid, cudaStream_t stream) {
+  const int dp = padded_head_dim(fp.D);
+  if (dtype == FA_BF16)
+    return dp == 64    ? launch_bias<64, __nv_bfloat16, LONGEST_FIRST>(fp, bias_kind, grid, stream)
+           : dp == 128 ? launch_bias<128, __nv_bfloat16, LONGEST_FIRST>(fp, bias_kind, grid, stream)
+                       : launch_bias<256, __nv_bfloat16, LONGEST_FIRST>(fp, bias_kind, grid, stream);
+  return dp == 64    ? launch_bias<64, __half, LONGEST_FIRST>(fp, bias_kind, grid, stream)
+         : dp == 128 ? launch_bias<128, __half, LONGEST_FIRST>(fp, bias_kind, grid, stream)
+                     : launch_bias<256, __half, LONGEST_FIRST>(fp, bias_kind, grid, stream);
+}
+
+// Whether a causal forward goes longest first.  Pairs of a heavy and a light unit leave CTAs idle in their last turn, and
+// half of the CTAs without a unit where there are fewer units than SMs.  Longest first spreads better, but a head's units no
+// longer run side by side, so once K and V are past what L2 holds beside the rest they are read more often.  The longest
+// CTA of both orders decides, in quarters of a step (four a step, five for a unit's boundary), with a margin that grows
+// with the bytes of K and V; a bias, which passes through L2 as well, and very short units want more.
+// Measured over 13000 calls (D 64 to 256, 128 to 11000 rows, four kinds of bias, M = N and not), pairs / longest first, us:
+// one unit a CTA or less gains 1.41 on average and never loses; elsewhere by estimate,
+//   K + V below 40 MB   1.02-1.06 gains 1.04, 1.10-1.14 1.08        90-140 MB, no bias  1.06-1.10 1.01, 1.10-1.14 1.03
+//   40-90 MB            1.02-1.06 1.02, 1.06-1.10 1.04              90-140 MB, a bias   1.10-1.14 1.01, 1.18-1.25 1.04
+//   140-250 MB          1.10-1.14 0.96, 1.18-1.25 1.03              up to three units a head, some heads twice: 0.85-1.2
+// B2 H12 S4096 D128 140 / 105, B16 H12 S512 D64 28.9 / 21.1, B4 H8 S2048 D256 81 / 74, B2 H32 S4096 D128 266 / 254; left to
+// the pairs: B4 H32 S4096 D128 with a mask 651 / 725.
+bool longest_first(const FwdParams& fp, int tiles, int sms, bool bias) {
+  constexpr int kMostRows = 16;
+  if (!fp.causal || fp.n_units > kMostRows * sms) return false;
+  const int n = fp.n_units, np = fp.n_pairs, nblk = (fp.N + 127) >> 7;
+  if (n <= sms) return true;
+  const auto work = [&](int pair) {  // by the key blocks that its last tile visits
+    const int last = (pair + 1) * tiles < fp.n_mblk ? (pair + 1) * tiles : fp.n_mblk;
+    return 4 * (last < nblk ? last : nblk) + 5;
+  };
+  const auto more = [](int& most, int load) { most = load > most ? load : most; };
+  // Pairs: the work of a CTA's pairs repeats every np of them (half of that where np is even), so the first CTAs of those
+  // with the most turns and of those with one less stand for all.
+  const int pairs = (n + 1) / 2, g_pairs = pairs < sms ? pairs : sms, period = np & 1 ? np : np / 2;
+  const auto pairs_of = [&](int c) {
+    int load = 0;
+    for (int u = c; u < pairs; u += g_pairs)
+      for (int k = 2 * u, pos = k % np; k < 2 * u + 2 && k < n; ++k, pos = pos + 1 == np ? 0 : pos + 1)
+        load += work(pos & 1 ? pos >> 1 : np - 1 - (pos >> 1));
+    return load;
+  };
+  int by_pairs = 0;
+  const int most_turns = (pairs - 1) % g_pairs + 1;
+  for (int c = 0; c < most_turns && c < period; ++c) more(by_pairs, pairs_of(c));
+  for (int c = most_turns; c < g_pairs && c < most_turns + period; ++c) more(by_pairs, pairs_of(c));
+  // Longest first: along the CTAs the work of even rows falls and that of odd rows rises, so the longest CTA is the first
+  // one, or one at which an odd row comes to a longer unit.
+  const auto load_of = [&](int c) {
+    int load = 0;
+    for (int at = 0, r = 0; at < n; at += sms, ++r)
+      if (const int k = at + (r & 1 ? sms - 1 - c : c); k < n) load += work(np - 1 - k / fp.n_bh);
+    return load;
+  };
+  int longest = load_of(0);
+  for (int at = sms; at < n; at += 2 * sms) {
+    const int last = at + sms < n ? at + sms - 1 : n - 1;
+    for (int level = at / fp.n_bh; level <= last / fp.n_bh; ++level) {
+      const int k = (level + 1) * fp.n_bh - 1;  // the last unit of this length
+      more(longest, load_of(at + sms - 1 - (k < last ? k : last)));
+    }
+  }
+  const int64_t kv_mb = 4 * static_cast<int64_t>(fp.n_bh) * fp.N * fp.D / 1000000;
+  const int margin = np <= 3 || kv_mb >= 140 ? 125 : (kv_mb >= 90 ? (bias ? 118 : 110) : (kv_mb >= 40 ? 107 : 104));
+  return 100 * static_cast<int64_t>(by_pairs) >= margin * static_cast<int64_t>(longest);
 }
 
 }  // namespace
@@ -829,15 +911,13 @@ int launch_fwd(const fa_params& p, cudaStream_t stream, int* status) {
   const int tiles = dp == 256 ? 1 : 2;  // query tiles per unit (FwdSmem::kTiles)
   fp.n_pairs = (fp.n_mblk + tiles - 1) / tiles;
   fp.n_units = fp.n_pairs * p.B * p.H;
-  const dim3 grid(persistent_grid(p.causal ? (fp.n_units + 1) / 2 : fp.n_units));
-  if (p.dtype == FA_BF16) {
-    return dp == 64    ? launch_bias<64, __nv_bfloat16>(fp, p.bias_kind, grid, stream)
-           : dp == 128 ? launch_bias<128, __nv_bfloat16>(fp, p.bias_kind, grid, stream)
-                       : launch_bias<256, __nv_bfloat16>(fp, p.bias_kind, grid, stream);
-  }
-  return dp == 64    ? launch_bias<64, __half>(fp, p.bias_kind, grid, stream)
-         : dp == 128 ? launch_bias<128, __half>(fp, p.bias_kind, grid, stream)
-                     : launch_bias<256, __half>(fp, p.bias_kind, grid, stream);
+  fp.n_bh = p.B * p.H;
+  const int sms = persistent_grid(1 << 30);
+  const bool by_length = longest_first(fp, tiles, sms, p.bias_kind != FA_BIAS_NONE);
+  const int turns_of = p.causal && !by_length ? (fp.n_units + 1) / 2 : fp.n_units;
+  const dim3 grid(turns_of < sms ? turns_of : sms);
+  return by_length ? launch_dim<true>(fp, p.dtype, p.bias_kind, grid, stream)
+                   : launch_dim<false>(fp, p.dtype, p.bias_kind, grid, stream);
 }
 
 }  // namespace fa
