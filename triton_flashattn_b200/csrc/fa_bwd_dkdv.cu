@@ -5,19 +5,21 @@
 // (only those at or below the diagonal when causal).  Ring stages, tensor-memory buffers
 // and barrier phases run on from tile to tile, so the next tile's K / V / Q / dO loads,
 // its first S and dP products and its first bias rows overlap the current tile's
-// epilogue.  Roles (640 threads):
-//   warps 0-15 "row" threads: warp w works on tensor-memory lanes 32*(w&3)..+31
-//              (query rows of the block) and on the 32-key column quarter (w>>2)
-//   warp 16    TMA producer: K, V per tile; Q ring (2), dO ring; bias tiles are asked
+// epilogue.  Roles (384 threads):
+//   warps 0-7  "row" threads: warp w works on tensor-memory lanes 32*(w&3)..+31
+//              (query rows of the block) and on the 64-key half (w>>2)
+//   warp 8     TMA producer: K, V per tile; Q ring (2), dO ring; bias tiles, asked
 //              into L2 one step ahead
-//   warp 17    MMA issuer for S and dP, tensor-memory owner
-//   warp 18    MMA issuer for dV and dK, bulk tensor stores of dS into dbias
-//   warp 19    TMA loads of the 16-bit bias tiles
+//   warp 9     MMA issuer for S and dP, tensor-memory owner
+//   warp 10    MMA issuer for dV and dK
+//   warp 11    bulk tensor stores of dS (into dbias or scratch)
 // The four control warps walk their loops with all lanes converged and elect a lane only
 // for the TMA / MMA / commit instructions, whose operands are then warp-uniform values.
 // A wait takes 200 - 235 cycles here even on a completed barrier, so two issuers keep
-// the tensor pipe fed while the other one waits, and every role polls the
-// barriers it will need before it starts a stretch of independent work.
+// the tensor pipe fed while the other one waits, each looks at the barriers of a product together, and the row threads
+// ask for the barriers they will need before the fence that ends the stretch before.  Whole backward, us, before these
+// looks and a warp of their own for the stores (which held the dV / dK issuer up until dS was read) / after: no bias
+// B2 H16 S4096 D64 683 / 636, B4 H16 S2048 D128 411 / 400; 16 bit B8 H16 S2048 D64 758 / 728.
 // Per query block t:
 //   S  = Q_t K^T            (tensor memory, 128 columns)
 //   dP = dO_t V^T           (tensor memory, 128 columns)
@@ -26,11 +28,12 @@
 //   dV += P^T dO_t          (sP and dO_t consumed MN-major)
 //   dK += dS^T Q_t          (sDS and Q_t consumed MN-major)
 //   dbias[b,h,m-block,n-block] <- sDS  (one bulk tensor store of the same tile)
-// A 16-bit bias tile is brought in by TMA (warp 19) and lands exactly where the row threads
-// then write P: each thread reads the four 16-byte chunks it is about to overwrite, so the
-// bias needs no shared memory of its own (none is left at head dim 128); warp 18 then also
-// issues the dbias stores.  A byte mask is read by the row threads straight from global
-// memory, 32 contiguous bytes per thread, one query block ahead.
+// A 16-bit bias tile is brought in by TMA and lands exactly where the row threads
+// then write P: each thread reads the eight 16-byte chunks it is about to overwrite, so the
+// bias needs no shared memory of its own (none is left at head dim 128).  (Read by the row threads into registers a step
+// ahead it takes no part in the chain of a step, but a load of 32 rows costs 24 - 60 cycles to issue: 5 - 12 % slower.)
+// A byte mask is read by the row threads straight from global
+// memory, 64 contiguous bytes per thread, one query block ahead.
 // Causally skipped tiles of dbias are written as zeros by this kernel, so dbias
 // needs no prior fill.
 // Rule kept by every barrier here: the next completion of a barrier needs progress of
@@ -78,6 +81,14 @@ enum DkdvSite { kSiteKV = 1, kSiteQFull, kSiteQEmpty, kSiteDoFull, kSiteDoEmpty,
                 kSiteDpFull, kSitePReady, kSiteDsReady, kSiteDvDone, kSiteDkDone, kSiteStDone,
                 kSiteZeroReady, kSiteEpilogue, kSiteSFree, kSiteDpFree, kSiteKVEmpty, kSiteBiasFull };
 
+// Eight row warps, a thread with half a row of a step: what a step costs a warp besides its values (looks at nine
+// barriers, votes, fences, loop) is paid half as often as with sixteen warps and quarters of a row, and 168 registers
+// hold the rest.  Whole backward, us, quarters / halves: no bias B4 H16 S2048 D128 403 / 400, 16 bit B8 H16 S2048 D128 902 / 894,
+// D64 742 / 728, mask, causal, B4 H32 S4096 D128 1805 / 1754, fp32 B4 H16 S2048 D128 882 / 867.
+constexpr int kCW = 64;           // columns of a step that a row thread works on
+constexpr int kNG = kCW / 32;     // ... in groups of 32
+constexpr int kRW = 512 / kCW;    // row warps
+constexpr int kThreads = 32 * (kRW + 4);
 template <int DP>
 struct DkdvSmem {
   static constexpr int kTile = 128 * DP * 2;
@@ -93,7 +104,7 @@ struct DkdvSmem {
 };
 
 template <int DP, typename T, int BIAS, bool LONGEST_FIRST>
-__global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ DkdvParams p) {
+__global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant__ DkdvParams p) {
   using L = DkdvSmem<DP>;
   using P2 = Pack2<T>;
   constexpr int KB = DP / 64;
@@ -101,9 +112,8 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
   constexpr int kDoStages = L::kDoStages;
   constexpr uint32_t kColS = 0, kColDp = 128, kColDv = 256, kColDk = 384;
   constexpr uint32_t kTmemCols = 512;
-  // BIAS: 0 none; 1 16-bit bias, brought in by TMA (warp 19; the dbias stores then move to
-  // warp 18); 2 byte mask and 3 fp32 bias, read by the row threads from global memory (the mask
-  // one step ahead, the fp32 row - 32 registers - at the start of its own step)
+  // BIAS: 0 none; 1 16-bit bias, brought in by TMA; 2 byte mask and 3 fp32 bias, read by the row threads from global
+  // memory (the mask one step ahead, the fp32 row - 64 registers - at the start of its own step)
   constexpr int BK = BIAS;
 
   extern __shared__ uint8_t smem_raw[];
@@ -168,18 +178,18 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
     }
     mbar_init(&s_full, 1);
     mbar_init(&dp_full, 1);
-    mbar_init(&p_ready, 16);
-    mbar_init(&ds_ready, 16);
+    mbar_init(&p_ready, kRW);
+    mbar_init(&ds_ready, kRW);
     mbar_init(&dv_done, 1);
     mbar_init(&dk_done, 1);
     mbar_init(&st_done, 1);
-    mbar_init(&zero_ready, 16);
-    mbar_init(&s_free, 16);
-    mbar_init(&dp_free, 16);
+    mbar_init(&zero_ready, kRW);
+    mbar_init(&s_free, kRW);
+    mbar_init(&dp_free, kRW);
     mbar_init(&bias_full, 1);
     mbar_fence_init();
   }
-  if (warp == 17) {
+  if (warp == kRW + 1) {
     tmem_alloc(&tmem_slot, kTmemCols);
     tmem_relinquish();
   }
@@ -191,7 +201,7 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
   grid_dep_wait();  // the previous kernel's results (and its status word) are visible from here
   const bool live = *reinterpret_cast<volatile int*>(p.status) == 0;
 
-  if (warp == 16) {
+  if (warp == kRW) {
     // ------------------------------------------------------------------ producer
     // (whole warp converged, one elected lane issues)
     if (live) {
@@ -264,6 +274,25 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
                           m0, b);
           }
           __syncwarp();
+          // The [128 rows][128 keys] 16-bit bias tile of a step lands exactly where the row threads
+          // will then write P (same two swizzled blocks, every thread reads the 16-byte
+          // chunks it is about to overwrite): no extra shared memory.  sP is free for it once the
+          // dV product of the previous step has read P, which at head dim 128 also frees dO.
+          auto load_bias = [&]() {
+            if (gs >= 1) ok = wait_warp_hot(&dv_done, (gs - 1) & 1, ctx, kSiteDvDone, t);
+            if (!ok) return;
+            const bool two = n0 + 64 < p.N;
+            if (elect_one()) {
+              mbar_expect_tx(&bias_full, two ? 2 * kBlk : kBlk);
+              tma_load_4d(smem + L::kP, &p.map_bias, &bias_full, n0, m0, h * p.bias_h_mul, b * p.bias_b_mul);
+              if (two)
+                tma_load_4d(smem + L::kP + kBlk, &p.map_bias, &bias_full, n0 + 64, m0, h * p.bias_h_mul,
+                            b * p.bias_b_mul);
+            }
+            __syncwarp();
+          };
+          if (BIAS == 1 && kDoStages == 1) load_bias();
+          if (!ok) break;
           const int ds = gs % kDoStages;
           const uint32_t du = gs / kDoStages;
           if (du >= 1) ok = wait_warp(&do_empty[ds], (du - 1) & 1, ctx, kSiteDoEmpty, t);
@@ -275,11 +304,12 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
                           h, m0, b);
           }
           __syncwarp();
+          if (BIAS == 1 && kDoStages != 1) load_bias();
         }
         g += T_steps;
       }
     }
-  } else if (warp == 17) {
+  } else if (warp == kRW + 1) {
     // ------------------------------------------------------- MMA issuer: S and dP
     // The whole warp walks the loop (waits included) and one elected lane issues: the
     // descriptors are then warp-uniform values, which the tensor-core instructions take
@@ -287,6 +317,7 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
     if (live) {
       constexpr bool bf = P2::kIsBf16;
       constexpr uint32_t idesc_s = make_idesc(bf, false, false, 128, 128);
+      constexpr bool kSpin = false;
       const uint32_t k_addr = smem_u32(smem + L::kK), v_addr = smem_u32(smem + L::kV);
       const uint32_t q_addr = smem_u32(smem + L::kQ), do_addr = smem_u32(smem + L::kDo);
       const uint64_t k_km = make_sdesc(k_addr, 0, 1024), v_km = make_sdesc(v_addr, 0, 1024);
@@ -305,8 +336,8 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
           const int qs = gs & 1, ds = gs % kDoStages;
           const uint32_t q_par = (gs >> 1) & 1, do_par = (gs / kDoStages) & 1;
           // S_gs: its columns are free once the row threads hold S_{gs-1} in registers
-          if (gs >= 1) ok = wait_warp_hot(&s_free, (gs - 1) & 1, ctx, kSiteSFree, t);
-          if (ok) ok = wait_warp(&q_full[qs], q_par, ctx, kSiteQFull, t);
+          ok = gs >= 1 ? wait_all2<kSpin>(&s_free, (gs - 1) & 1, &q_full[qs], q_par, ctx, kSiteSFree, t)
+                       : wait_all1<kSpin>(&q_full[qs], q_par, ctx, kSiteQFull, t);
           if (!ok) break;
           tc_fence_after();
           if (elect_one()) {
@@ -315,11 +346,10 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
             mma_commit(&s_full);
             mma_commit(&q_empty[qs]);
           }
-          __syncwarp();
           // dP_gs: same for the dP columns; dO_gs replaces dO_{gs-1} after dV_{gs-1} when
           // single-staged
-          if (gs >= 1) ok = wait_warp_hot(&dp_free, (gs - 1) & 1, ctx, kSiteDpFree, t);
-          if (ok) ok = wait_warp(&do_full[ds], do_par, ctx, kSiteDoFull, t);
+          ok = gs >= 1 ? wait_all2<kSpin>(&dp_free, (gs - 1) & 1, &do_full[ds], do_par, ctx, kSiteDpFree, t)
+                       : wait_all1<kSpin>(&do_full[ds], do_par, ctx, kSiteDoFull, t);
           if (!ok) break;
           tc_fence_after();
           if (elect_one()) {
@@ -329,13 +359,12 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
             mma_commit(&do_empty[ds]);
             if (t == T_steps - 1) mma_commit(&kv_empty);  // K and V may be replaced
           }
-          __syncwarp();
         }
         g += T_steps;
       }
     }
     __syncwarp();
-  } else if (warp == 18) {
+  } else if (warp == kRW + 2) {
     // ------------------------------------------------------ MMA issuer: dV and dK
     // (whole warp converged, one elected lane issues: see the S / dP issuer)
     if (live) {
@@ -347,67 +376,29 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
       const uint64_t do_mn_0 = make_sdesc(do_addr, kBlk, 1024),
                      do_mn_1 = make_sdesc(do_addr + (kDoStages - 1) * L::kTile, kBlk, 1024);
       const uint64_t p_mn = make_sdesc(p_addr, kBlk, 1024), ds_mn = make_sdesc(ds_addr, kBlk, 1024);
-      // The elected lane also sends the dS tiles out as dbias (a bias gradient only exists for a
-      // 16-bit bias).  st_done completes once per step when the store of dS has finished
-      // reading sDS and - causal only - once per tile before that, when the zero tiles above
-      // the diagonal are out.  (Without the zero tiles there is no per-tile completion: two
-      // completions in a row that no row thread has to wait for in between would let a parity
-      // wait fall two phases behind.)  The wait for the store's read sits right after the
-      // store: the next thing this warp needs, P of the next step, is further away.
-      const bool stores_here = p.store_ds != 0;
-      bool zeros_in_flight = false;
+      constexpr bool kSpin = false;
       bool ok = true;
       uint32_t g = 0;
       int bh, nb, i_start, T_steps;
       for (int it = 0; ok && tile_at(it, bh, nb, i_start, T_steps); ++it) {
-        const int b = bh / p.H, h = bh - b * p.H, n0 = nb * 128;
-        const int ds_h = p.ds_flat ? bh - p.bh0 : h, ds_b = p.ds_flat ? 0 : b;
-        if (p.zero_tiles) {
-          ok = wait_warp(&zero_ready, it & 1, ctx, kSiteZeroReady, it);
-          if (!ok) break;
-          if (elect_one()) {
-            for (int i = 0; i < i_start; ++i) {
-              tma_store_4d(&p.map_dbias, smem + L::kDs, n0, i * 128, h, b);
-              if (n0 + 64 < p.N)
-                tma_store_4d(&p.map_dbias, smem + L::kDs + kBlk, n0 + 64, i * 128, h, b);
-            }
-            tma_store_commit();
-            if (T_steps <= 0) {
-              tma_store_wait_read<0>();
-              mbar_arrive(&st_done);
-            }
-          }
-          __syncwarp();
-          // the zero tiles are read out of sDS while P of the first step is formed and dV is
-          // issued; their completion is announced just before this warp needs dS
-          zeros_in_flight = T_steps > 0;
-        }
         for (int t = 0; t < T_steps && ok; ++t) {
           const uint32_t gs = g + t;
           const int qs = gs & 1;
           const int ds = gs % kDoStages;
           // dV += P^T dO  (dO must have landed: P only depends on S).  The first product of a
-          // tile overwrites dV / dK: P and dS of a new tile are only announced by all sixteen
+          // tile overwrites dV / dK: P and dS of a new tile are only announced by all eight
           // row warps after they have read the previous tile's accumulators.
-          ok = wait_warp_hot(&p_ready, gs & 1, ctx, kSitePReady, t);
-          if (ok) ok = wait_warp(&do_full[ds], (gs / kDoStages) & 1, ctx, kSiteDoFull, t);
+          ok = wait_all2<kSpin>(&p_ready, gs & 1, &do_full[ds], (gs / kDoStages) & 1, ctx, kSitePReady, t);
           if (!ok) break;
           tc_fence_after();
           if (elect_one()) {
             issue_gemm_ss<8, true, true>(tmem + kColDv, p_mn, ds ? do_mn_1 : do_mn_0, kBlk, kBlk, idesc_g,
                                          t > 0);
-            mma_commit(&do_empty[ds]);
             mma_commit(&dv_done);
-            if (zeros_in_flight) {
-              tma_store_wait_read<0>();
-              mbar_arrive(&st_done);
-            }
+            mma_commit(&do_empty[ds]);
           }
-          __syncwarp();
-          zeros_in_flight = false;
           // dK += dS^T Q
-          ok = wait_warp_hot(&ds_ready, gs & 1, ctx, kSiteDsReady, t);
-          if (ok) ok = wait_warp(&q_full[qs], (gs >> 1) & 1, ctx, kSiteQFull, t);
+          ok = wait_all2<kSpin>(&ds_ready, gs & 1, &q_full[qs], (gs >> 1) & 1, ctx, kSiteDsReady, t);
           if (!ok) break;
           tc_fence_after();
           if (elect_one()) {
@@ -415,71 +406,77 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
                                          t > 0);
             mma_commit(&q_empty[qs]);
             mma_commit(&dk_done);
-            if (stores_here) {
-              const int m0 = (i_start + t) * 128;
-              tma_store_4d(&p.map_dbias, smem + L::kDs, n0, m0, ds_h, ds_b);
-              if (n0 + 64 < p.N) tma_store_4d(&p.map_dbias, smem + L::kDs + kBlk, n0 + 64, m0, ds_h, ds_b);
-              tma_store_commit();
-              tma_store_wait_read<0>();
-              mbar_arrive(&st_done);
-            }
           }
-          __syncwarp();
         }
         g += T_steps;
       }
-      if (stores_here && elect_one()) tma_store_wait_all<0>();
     }
     __syncwarp();
-  } else if (warp == 19) {
-    // ----------------------------------------------------------- bias tile loads
-    // The [128 rows][128 keys] 16-bit bias tile of a step lands exactly where the row threads
-    // will then write P (same two swizzled blocks, every thread reads the four 16-byte
-    // chunks it is about to overwrite): no extra shared memory.  sP is free for it once the
-    // dV product of the previous step has read P.
-    // (whole warp converged, one elected lane issues: the load follows the barrier sooner)
-    if (BIAS == 1 && live) {
-      if (lane == 0) tma_prefetch_desc(&p.map_bias);
+  } else if (warp == kRW + 3) {
+    // ----------------------------------------------------------- stores of dS
+    // (whole warp converged, one elected lane issues)
+    // st_done completes once per step when the store of dS has finished reading sDS and - where there are zero tiles -
+    // once per tile before that, when those above the diagonal are out.  (Without the zero tiles there is no per-tile
+    // completion: two completions in a row that no row thread has to wait for in between would let a parity wait fall
+    // two phases behind.)
+    if (live && p.store_ds) {
+      if (lane == 0) tma_prefetch_desc(&p.map_dbias);
       bool ok = true;
       uint32_t g = 0;
       int bh, nb, i_start, T_steps;
       for (int it = 0; ok && tile_at(it, bh, nb, i_start, T_steps); ++it) {
         const int b = bh / p.H, h = bh - b * p.H, n0 = nb * 128;
+        const int ds_h = p.ds_flat ? bh - p.bh0 : h, ds_b = p.ds_flat ? 0 : b;
         const bool two = n0 + 64 < p.N;
+        if (p.zero_tiles) {
+          ok = wait_warp(&zero_ready, it & 1, ctx, kSiteZeroReady, it);
+          if (!ok) break;
+          if (elect_one()) {
+            for (int i = 0; i < i_start; ++i) {
+              tma_store_4d(&p.map_dbias, smem + L::kDs, n0, i * 128, h, b);
+              if (two) tma_store_4d(&p.map_dbias, smem + L::kDs + kBlk, n0 + 64, i * 128, h, b);
+            }
+            tma_store_commit();
+            tma_store_wait_read<0>();
+            mbar_arrive(&st_done);
+          }
+          __syncwarp();
+        }
         for (int t = 0; t < T_steps && ok; ++t) {
-          const uint32_t gs = g + t;
-          if (gs >= 1) ok = wait_warp_hot(&dv_done, (gs - 1) & 1, ctx, kSiteDvDone, t);
+          // (Right when dS is there the store competes with dK for shared memory: D128, mask, causal B4 H32 S4096 1764 ->
+          // 1893 us, 16-bit bias B8 H16 S2048 898 -> 910.)
+          ok = wait_warp(&dk_done, (g + t) & 1, ctx, kSiteDkDone, t);
           if (!ok) break;
           const int m0 = (i_start + t) * 128;
           if (elect_one()) {
-            mbar_expect_tx(&bias_full, two ? 2 * kBlk : kBlk);
-            tma_load_4d(smem + L::kP, &p.map_bias, &bias_full, n0, m0, h * p.bias_h_mul,
-                        b * p.bias_b_mul);
-            if (two)
-              tma_load_4d(smem + L::kP + kBlk, &p.map_bias, &bias_full, n0 + 64, m0, h * p.bias_h_mul,
-                          b * p.bias_b_mul);
+            tma_store_4d(&p.map_dbias, smem + L::kDs, n0, m0, ds_h, ds_b);
+            if (two) tma_store_4d(&p.map_dbias, smem + L::kDs + kBlk, n0 + 64, m0, ds_h, ds_b);
+            tma_store_commit();
+            tma_store_wait_read<0>();
+            mbar_arrive(&st_done);
           }
           __syncwarp();
         }
         g += T_steps;
       }
+      if (elect_one()) tma_store_wait_all<0>();
     }
     __syncwarp();
   } else {
     // --------------------------------------------------------------- row threads
     const int r = (warp & 3) * 32 + lane;  // query row inside the block = tensor-memory lane
-    const int qt = warp >> 2;              // column quarter: keys n0 + 32*qt .. +31
+    const int qt = warp >> 2;              // column group: keys n0 + kCW*qt .. + kCW-1
     const uint32_t lane_base = static_cast<uint32_t>(warp & 3) * 32u;
     bool ok = live;
     // this thread's four 16-byte chunks inside the [128][128] 16-bit tiles: chunk c of the
     // row lands at sp_row + ((chunk0 + c) ^ (r & 7)) * 16; the dS tile sits kDs - kP further
-    const uint32_t sp_row = smem_u32(smem + L::kP + (qt >> 1) * kBlk) + static_cast<uint32_t>(r) * 128u;
-    const uint32_t chunk0 = (qt & 1) * 4;
+    const uint32_t sp_row = smem_u32(smem + L::kP + (qt * kCW / 64) * kBlk) + static_cast<uint32_t>(r) * 128u;
+    const uint32_t chunk0 = (qt * kCW % 64) / 8;
     // tensor-memory address of this thread's 32 columns of S (dP: + kColDp)
-    const uint32_t tm_sc = tmem_addr(tmem, lane_base, kColS + qt * 32);
+    const uint32_t tm_sc = tmem_addr(tmem, lane_base, kColS + qt * kCW);
 
     constexpr int BR = BIAS == 1 ? 0 : BK;  // bias staged in registers only for kinds 2 and 3
-    BiasRegs<BR> bnext;
+    BiasRegs<BR> bnext[kNG];
     // LSE2 and delta of the coming step's row, as loaded: they are only looked at (negated,
     // replaced for rows beyond M) when that step starts, so the loads travel during this one
     float lse_next = 0.f, delta_next = 0.f;
@@ -491,8 +488,10 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
       const int m = mblk * 128 + r;
       const bool row_ok = m < p.M;
       if constexpr (BR == 2) {
-        load_bias_row<BK>(bnext, p.bias, bias_bh + (int64_t)m * p.bias_sM, row_ok, c0, p.N,
-                          p.bias_vec32 != 0);
+#pragma unroll
+        for (int g = 0; g < kNG; ++g)
+          load_bias_row<BK>(bnext[g], p.bias, bias_bh + (int64_t)m * p.bias_sM, row_ok, c0 + g * 32, p.N,
+                            p.bias_vec32 != 0);
       }
       const int64_t idx = (int64_t)bh_ * p.M + min(m, p.M - 1);
       lse_next = __ldcg(p.lse + idx);
@@ -504,10 +503,13 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
     // of a tile is recomputed from col0 where needed.
     uint32_t gs = 0;  // steps done so far, over all tiles
     int bh, nb, i_start, T_steps;
-    if (ok && tile_at(0, bh, nb, i_start, T_steps) && T_steps > 0) prefetch(bh, nb * 128 + qt * 32, i_start);
+    if (ok && tile_at(0, bh, nb, i_start, T_steps) && T_steps > 0) prefetch(bh, nb * 128 + qt * kCW, i_start);
+    // What the last look at the barriers of the coming step saw (nothing yet).  "dV of step -1 has read P" and "dK of step
+    // -1 has read dS" hold from the start: a fresh barrier answers the parity of the phase before its first with yes.
+    uint32_t ps = 0, pdv = 0, pb = 0;
 #pragma unroll 1
     for (int it = 0; ok && tile_at(it, bh, nb, i_start, T_steps); ++it) {
-      const int col0 = nb * 128 + qt * 32;
+      const int col0 = nb * 128 + qt * kCW;
       if (p.zero_tiles) {
         // sDS becomes the zero tile for the causally skipped part of dbias: the last dbias
         // store of the previous tile must have read it (the last dK product has: its barrier
@@ -515,8 +517,8 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
         // indices gs+it (zero tiles out) and gs+it+1+t (store of step t).
         if (it >= 1) ok = wait_warp(&st_done, (gs + it - 1) & 1, ctx, kSiteStDone, it);
         if (!ok) break;
-        const uint32_t z = sp_row - static_cast<uint32_t>(r) * 128u - (qt >> 1) * kBlk + (L::kDs - L::kP);
-        for (int i = tid; i < 2 * kBlk / 16; i += 512) sts128(z + i * 16, 0, 0, 0, 0);
+        const uint32_t z = sp_row - static_cast<uint32_t>(r) * 128u - (qt * kCW / 64) * kBlk + (L::kDs - L::kP);
+        for (int i = tid; i < 2 * kBlk / 16; i += 32 * kRW) sts128(z + i * 16, 0, 0, 0, 0);
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(&zero_ready);
@@ -527,33 +529,27 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
         const int i0 = p.causal ? min(col0 >> 7, n_mblk) : 0;  // first query block of the tile
         const int t = mb - i0;
         const int m0 = mb * 128;
-        BiasRegs<BR> bcur = bnext;
+        BiasRegs<BR> bcur[kNG];
+#pragma unroll
+        for (int g = 0; g < kNG; ++g) bcur[g] = bnext[g];
         if constexpr (BR == 3) {
           // fp32 bias row of this step: asked for now, used once S has arrived
           const int b_ = bh / p.H, h_ = bh - b_ * p.H;
-          load_bias_row<3>(bcur, p.bias, b_ * p.bias_sB + h_ * p.bias_sH + (int64_t)(m0 + r) * p.bias_sM,
-                           m0 + r < p.M, col0, p.N, p.bias_vec32 != 0);
+#pragma unroll
+          for (int g = 0; g < kNG; ++g)
+            load_bias_row<3>(bcur[g], p.bias, b_ * p.bias_sB + h_ * p.bias_sH + (int64_t)(m0 + r) * p.bias_sM,
+                             m0 + r < p.M, col0 + g * 32, p.N, p.bias_vec32 != 0);
         }
         // rows beyond M get -inf / 0, which makes their P and dS zero
         const float neg_lse = row_ok_next ? -lse_next : -INFINITY, delta_r = row_ok_next ? delta_next : 0.f;
         if (mb + 1 < n_mblk) prefetch(bh, col0, mb + 1);
-        // S and "dV of the previous step has read P" are usually true by now: one combined look
-        uint32_t ps = 0, pdv = 1, pb = 1;
-        if (BIAS == 1 && t >= 1)
-          mbar_poll3(&s_full, gs & 1, &dv_done, (gs - 1) & 1, &bias_full, gs & 1, ps, pdv, pb);
-        else if (BIAS == 1)
-          mbar_poll2(&s_full, gs & 1, &bias_full, gs & 1, ps, pb);
-        else if (t >= 1)
-          mbar_poll2(&s_full, gs & 1, &dv_done, (gs - 1) & 1, ps, pdv);
-        else
-          ps = mbar_poll(&s_full, gs & 1);
-
         // ---- P
         ok = wait_warp_polled(ps, &s_full, gs & 1, ctx, kSiteSFull, t);
         if (!ok) break;
         tc_fence_after();
-        float pr[32];
-        tmem_ld32(tm_sc, reinterpret_cast<uint32_t*>(pr));
+        float pr[kCW];
+#pragma unroll
+        for (int g = 0; g < kNG; ++g) tmem_ld32(tm_sc + g * 32, reinterpret_cast<uint32_t*>(pr) + g * 32);
         tmem_ld_wait();
         // S now lives in registers: hand its columns back for the next S
         tc_fence_before();
@@ -564,7 +560,7 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
           // the bias tile sits where this thread's P chunks go; what does not need it is
           // computed while it travels: x = S * scale * log2e - LSE2
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
+          for (int i = 0; i < kCW; i += 2) {
             const f32x2 x = ffma2(f2(pr[i], pr[i + 1]), f2(p.scale_log2, p.scale_log2), f2(neg_lse, neg_lse));
             pr[i] = f2_lo(x);
             pr[i + 1] = f2_hi(x);
@@ -572,7 +568,7 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
           ok = wait_warp_polled(pb, &bias_full, gs & 1, ctx, kSiteBiasFull, t);
           if (!ok) break;
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 0; c < kCW / 8; ++c) {
             const uint4 v = lds128(sp_row + (((chunk0 + c) ^ (r & 7)) << 4));
             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -587,13 +583,13 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
           }
         } else {
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
+        for (int i = 0; i < kCW; i += 2) {
           f32x2 a = ffma2(f2(pr[i], pr[i + 1]), f2(p.scale_log2, p.scale_log2), f2(neg_lse, neg_lse));
           if (BK == 3)
-            a = ffma2(f2(__uint_as_float(bcur.w[i]), __uint_as_float(bcur.w[i + 1])), f2(kLog2e, kLog2e), a);
+            a = ffma2(f2(__uint_as_float(bcur[i / 32].w[i % 32]), __uint_as_float(bcur[i / 32].w[i % 32 + 1])), f2(kLog2e, kLog2e), a);
           const f32x2 pe = f2(ex2(f2_lo(a)), ex2(f2_hi(a)));
           if (BK == 2) {
-            const uint32_t m2 = bcur.w[i >> 2] >> (8 * (i & 3));
+            const uint32_t m2 = bcur[i / 32].w[(i % 32) >> 2] >> (8 * (i & 3));
             pr[i] = (m2 & 0xFFu) != 0 ? f2_lo(pe) : 0.f;
             pr[i + 1] = (m2 & 0xFF00u) != 0 ? f2_hi(pe) : 0.f;
           } else {
@@ -602,52 +598,45 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
           }
         }
         }
-        if ((col0 + 32 > p.N) || (p.causal && col0 + 31 > m0)) {
+        if ((col0 + kCW > p.N) || (p.causal && col0 + kCW - 1 > m0)) {
           int limit = p.N - col0;
           if (p.causal) limit = min(limit, m0 + r - col0 + 1);
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
+          for (int i = 0; i < kCW; ++i)
             if (i >= limit) pr[i] = 0.f;
         }
-        if (t >= 1) {
+        if (BIAS != 1) {  // (a 16-bit bias tile lands after it)
           ok = wait_warp_polled(pdv, &dv_done, (gs - 1) & 1, ctx, kSiteDvDone, t);
           if (!ok) break;
         }
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+        for (int c = 0; c < kCW / 8; ++c)
           sts128(sp_row + (((chunk0 + c) ^ (r & 7)) << 4), P2::pack(pr[c * 8 + 0], pr[c * 8 + 1]),
                  P2::pack(pr[c * 8 + 2], pr[c * 8 + 3]), P2::pack(pr[c * 8 + 4], pr[c * 8 + 5]),
                  P2::pack(pr[c * 8 + 6], pr[c * 8 + 7]));
+        // dP, "dK of the previous step has read dS" and "its store has": one combined look, asked for before the fence.
+        // sDS may be rewritten once its previous store has read it: with zero tiles completion gs+it of st_done (see
+        // above); otherwise completion gs-1 (the store of step gs-1)
+        uint32_t pdp, pdk, pst;
+        uint64_t* const st_bar = p.store_ds ? &st_done : &dk_done;
+        const uint32_t st_par = (p.zero_tiles ? gs + it : gs - 1) & 1;
+        mbar_poll3(&dp_full, gs & 1, &dk_done, (gs - 1) & 1, st_bar, st_par, pdp, pdk, pst);
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(&p_ready);
 
         // ---- dS
-        // dP, "dK of the previous step has read dS" and "its dbias store has": one combined look
-        uint32_t pdp = 0, pdk = 1, pst = 1;
-        // sDS may be rewritten once its previous dbias store has read it: causal -> completion
-        // gs+it of st_done (see above); otherwise completion gs-1 (the store of step gs-1)
-        const uint32_t st_par = (p.zero_tiles ? gs + it : gs - 1) & 1;
-        const bool st_wait = p.store_ds && (p.zero_tiles || gs >= 1);
-        if (t >= 1 && st_wait)
-          mbar_poll3(&dp_full, gs & 1, &dk_done, (gs - 1) & 1, &st_done, st_par, pdp, pdk, pst);
-        else if (t >= 1)
-          mbar_poll2(&dp_full, gs & 1, &dk_done, (gs - 1) & 1, pdp, pdk);
-        else if (st_wait)
-          mbar_poll2(&dp_full, gs & 1, &st_done, st_par, pdp, pst);
-        else
-          pdp = mbar_poll(&dp_full, gs & 1);
         ok = wait_warp_polled(pdp, &dp_full, gs & 1, ctx, kSiteDpFull, t);
         if (!ok) break;
         tc_fence_after();
-        uint32_t dsu[16];
+        uint32_t dsu[kCW / 2];
         // dP is fetched in two halves: fewer registers are live at once
 #pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
+        for (int hf = 0; hf < kCW / 16; ++hf) {
           uint32_t dp[16];
           tmem_ld16(tm_sc + (kColDp - kColS) + hf * 16, dp);
           tmem_ld_wait();
-          if (hf == 1) {
+          if (hf == kCW / 16 - 1) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&dp_free);
@@ -680,18 +669,20 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
             }
           }
         }
-        if (t >= 1) {
-          ok = wait_warp_polled(pdk, &dk_done, (gs - 1) & 1, ctx, kSiteDkDone, t);
-          if (!ok) break;
-        }
-        if (st_wait) {
-          ok = wait_warp_polled(pst, &st_done, st_par, ctx, kSiteStDone, t);
+        if (!__all_sync(0xffffffffu, (pdk & pst) != 0)) {
+          ok = mbar_wait(&dk_done, (gs - 1) & 1, ctx, kSiteDkDone, t) && mbar_wait(st_bar, st_par, ctx, kSiteStDone, t);
+          ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
         }
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+        for (int c = 0; c < kCW / 8; ++c)
           sts128(sp_row + (L::kDs - L::kP) + (((chunk0 + c) ^ (r & 7)) << 4), dsu[c * 4 + 0],
                  dsu[c * 4 + 1], dsu[c * 4 + 2], dsu[c * 4 + 3]);
+        // the looks of the next step, of this tile or the next one, are asked for before the fence
+        if (BIAS == 1)
+          mbar_poll2(&s_full, (gs + 1) & 1, &bias_full, (gs + 1) & 1, ps, pb);
+        else
+          mbar_poll2(&s_full, (gs + 1) & 1, &dv_done, gs & 1, ps, pdv);
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(&ds_ready);
@@ -701,7 +692,7 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
       // the next tile's first bias / LSE / delta rows travel while this tile's result is stored
       {
         int bh2, nb2, is2, T2;
-        if (tile_at(it + 1, bh2, nb2, is2, T2) && T2 > 0) prefetch(bh2, nb2 * 128 + qt * 32, is2);
+        if (tile_at(it + 1, bh2, nb2, is2, T2) && T2 > 0) prefetch(bh2, nb2 * 128 + qt * kCW, is2);
       }
 
       // ---- epilogue: dV, dK (rows = keys) -> global
@@ -715,7 +706,8 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
         tc_fence_after();
         const int b = bh / p.H, h = bh - b * p.H;
         const int n = (col0 & ~127) + r;
-        constexpr int kQD = DP / 4;  // columns of the head dim this thread stores (16 or 32)
+        constexpr int kQD = DP * kCW / 128;  // columns of the head dim this thread stores
+        constexpr int kQL = kQD > 32 ? 32 : kQD;
         const int d0 = qt * kQD;
         T* dkrow = reinterpret_cast<T*>(p.dk) + b * p.dk_sB + (int64_t)n * p.dk_sN + h * p.dk_sH;
         T* dvrow = reinterpret_cast<T*>(p.dv) + b * p.dv_sB + (int64_t)n * p.dv_sN + h * p.dv_sH;
@@ -726,7 +718,8 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
           const float mul = which == 0 ? 1.0f : p.sm_scale;
           uint32_t a[kQD];
           if (steps_here > 0) {
-            tmem_ld_cols<kQD>(tm_sc - qt * 32 + colbase + d0, a);
+#pragma unroll
+            for (int c = 0; c < kQD; c += kQL) tmem_ld_cols<kQL>(tm_sc - qt * kCW + colbase + d0 + c, a + c);
             tmem_ld_wait();
           } else {
 #pragma unroll
@@ -760,7 +753,7 @@ __global__ void __launch_bounds__(640, 1) dkdv_kernel(const __grid_constant__ Dk
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 17) tmem_dealloc(tmem, kTmemCols);
+  if (warp == kRW + 1) tmem_dealloc(tmem, kTmemCols);
 }
 
 template <int DP, typename T, int BIAS, bool LONGEST_FIRST>
@@ -776,7 +769,7 @@ int launch_inst(const DkdvParams& kp, dim3 grid, cudaStream_t stream) {
       return FA_ERR_CUDA;
     configured[dev] = true;
   }
-  return launch_overlapped(kern, grid, 640, L::kDynamic, stream, kp);
+  return launch_overlapped(kern, grid, kThreads, L::kDynamic, stream, kp);
 }
 
 template <int DP, typename T, bool LONGEST_FIRST>
