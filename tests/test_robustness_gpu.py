@@ -407,6 +407,33 @@ def test_causal_forward_order_does_not_change_bits(D, bias_kind, M, N, device_ok
         assert torch.equal(out, first) and torch.equal(lse, lse2), cap
 
 
+@pytest.mark.parametrize("D,M", [(16, 100), (32, 257), (64, 70), (64, 1), (128, 130), (256, 95)])
+@pytest.mark.parametrize("layout", ["dense", "padded", "reversed batch"])
+def test_forward_result_in_any_layout(layout, D, M, device_ok):
+    """The result leaves by bulk stores of 32 rows where its layout can be encoded, by plain ones where it cannot: the same
+    bits, and nothing beside it is touched.  M up to 16 goes to the kernel for few rows."""
+    from triton_flashattn_b200 import _cabi
+    from triton_flashattn_b200 import flash_attention as fa
+
+    B, H, N = 2, 3, 150
+    g = torch.Generator(device="cuda").manual_seed(68)
+    q, k, v = (torch.randn(B, s, H, D, generator=g, device="cuda", dtype=torch.float32).to(BF) for s in (M, N, N))
+    want, lse = fa._flash_attn_fwd(q, k, v, None, False, D ** -0.5)
+    pad = 0 if layout == "dense" else 8
+    buf = torch.full((B, M + 3, H, D + pad), 7.0, dtype=BF, device="cuda")
+    view = buf[:, :M, :, :D]
+    lse2 = torch.empty_like(lse)
+    p = fa._params(q, k, v, view, lse2, None, 0, False, D ** -0.5)
+    if layout == "reversed batch":
+        p.o, p.o_stride[0] = view[1].data_ptr(), -view.stride(0)
+    lib = _cabi.load()
+    assert lib.fa_fwd(ctypes.byref(p), torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    got = view.flip(0) if layout == "reversed batch" else view
+    assert torch.equal(got, want) and torch.equal(lse, lse2)
+    assert (buf[:, M:] == 7).all() and (buf[..., D:] == 7).all()
+
+
 @pytest.mark.parametrize("bias_kind,D", [(0, 64), (2, 128), (0, 256), (3, 128)])
 def test_scratch_for_ds_is_bounded(bias_kind, D, device_ok):
     """The scratch a backward asks for: at most 1.5 GiB, and nothing where that holds no problem or too few to fill

@@ -60,6 +60,7 @@ struct FwdParams {
   CUtensorMap map_k;
   CUtensorMap map_v;  // box of 64 keys
   CUtensorMap map_bias;
+  CUtensorMap map_o;  // boxes of 32 rows
   void* o;
   float* lse;
   int* status;
@@ -67,6 +68,7 @@ struct FwdParams {
   int H, M, N, D;
   int causal;
   int o_vec32;  // o's base and strides are multiples of 32 bytes
+  int o_tma;    // o leaves by bulk tensor stores where there is shared memory for it
   int bias_b_mul, bias_h_mul;
   int n_mblk, n_pairs, n_units;  // query blocks / block pairs per (batch, head); units = pairs * B * H
   int n_bh;                      // B * H
@@ -97,7 +99,10 @@ struct FwdSmem {
   static constexpr int kK = kQ + kTiles * kQTile;
   static constexpr int kV = kK + kKStages * kKUnit;
   static constexpr int kBias = kV + kVStages * kVHalf;
-  static constexpr int kTotal = kBias + kBiasStages * kBlk;
+  // O on its way out, 64 columns at a time: 4 KB a row warp at head dim 64 and wherever no bias takes the space
+  static constexpr bool kStageO = DP == 64 || BIAS == 0;
+  static constexpr int kOut = kBias + kBiasStages * kBlk;
+  static constexpr int kTotal = kOut + (kStageO ? kTiles * kBlk : 0);
   static constexpr int kDynamic = kTotal + 1024;  // slack for 1024-byte alignment
 };
 
@@ -725,28 +730,58 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
       // a row whose keys are all masked out keeps m_used = -inf and l = 0: output 0, LSE +inf
       const bool any_key = m_used != -INFINITY && l > 0.f;
       const float inv = any_key ? 1.0f / l : 0.f;
-      T* orow = reinterpret_cast<T*>(p.o) + b * p.o_sB + static_cast<int64_t>(m) * p.o_sM + hd * p.o_sH;
+      // Where there is shared memory, a row warp puts its rows there and one lane sends them off.  (Stored from the
+      // registers, a row a thread, every store touches 32 lines: 2700 cycles a unit at D64 and 3800 at D128 without a
+      // bias, where a step is 3000.  us, before / after: 16 bit B16 S512 H12 D64 45.1 / 41.0, S4096 H37 332 / 303, mask B4
+      // H12 S1000 D64 76.9 / 71.7, causal B4 H16 S1024 38.9 / 35.5, no bias B8 H16 S512 D128 32.8 / 30.8.)
+      if (L::kStageO && p.o_tma) {
+        const int row0 = m0 + (warp & 3) * 32;
+        uint8_t* const stage = smem + L::kOut + warp * 4096;
+        const uint32_t srow = smem_u32(stage) + static_cast<uint32_t>(lane) * 128u;
 #pragma unroll
-      for (int c = 0; c < DP / 32; ++c) {
-        uint32_t o[32];
-        tmem_ld32(tm_o + c * 32, o);
-        tmem_ld_wait();
-        if (m < p.M) {
-          if (p.o_vec32 && c * 32 + 32 <= p.D) {
-            // whole 32-byte sectors per store: half as many transactions as 16-byte stores for
-            // these row-strided writes
+        for (int kb = 0; kb < KB; ++kb) {
+          uint32_t o[64];
+          tmem_ld32(tm_o + kb * 64, o);
+          tmem_ld32(tm_o + kb * 64 + 32, o + 32);
+          if (lane == 0) tma_store_wait_read<0>();
+          tmem_ld_wait();
+          __syncwarp();
 #pragma unroll
-            for (int q2 = 0; q2 < 2; ++q2) {
-              const uint4 lo = pack8<P2>(o + q2 * 16, inv), hi = pack8<P2>(o + q2 * 16 + 8, inv);
-              asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(orow + c * 32 + q2 * 16),
-                           "r"(lo.x), "r"(lo.y), "r"(lo.z), "r"(lo.w), "r"(hi.x), "r"(hi.y), "r"(hi.z), "r"(hi.w)
-                           : "memory");
-            }
-          } else {
+          for (int c = 0; c < 8; ++c) {
+            const uint4 v = pack8<P2>(o + c * 8, inv);
+            sts128(srow + (static_cast<uint32_t>(c ^ (lane & 7)) << 4), v.x, v.y, v.z, v.w);
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0 && row0 < p.M) {
+            tma_store_4d(&p.map_o, stage, kb * 64, hd, row0, b);
+            tma_store_commit();
+          }
+        }
+      } else {
+        T* orow = reinterpret_cast<T*>(p.o) + b * p.o_sB + static_cast<int64_t>(m) * p.o_sM + hd * p.o_sH;
 #pragma unroll
-            for (int q4 = 0; q4 < 4; ++q4) {
-              const int d = c * 32 + q4 * 8;
-              if (d < p.D) *reinterpret_cast<uint4*>(orow + d) = pack8<P2>(o + q4 * 8, inv);
+        for (int c = 0; c < DP / 32; ++c) {
+          uint32_t o[32];
+          tmem_ld32(tm_o + c * 32, o);
+          tmem_ld_wait();
+          if (m < p.M) {
+            if (p.o_vec32 && c * 32 + 32 <= p.D) {
+              // whole 32-byte sectors per store: half as many transactions as 16-byte stores for
+              // these row-strided writes
+#pragma unroll
+              for (int q2 = 0; q2 < 2; ++q2) {
+                const uint4 lo = pack8<P2>(o + q2 * 16, inv), hi = pack8<P2>(o + q2 * 16 + 8, inv);
+                asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(orow + c * 32 + q2 * 16),
+                             "r"(lo.x), "r"(lo.y), "r"(lo.z), "r"(lo.w), "r"(hi.x), "r"(hi.y), "r"(hi.z), "r"(hi.w)
+                             : "memory");
+              }
+            } else {
+#pragma unroll
+              for (int q4 = 0; q4 < 4; ++q4) {
+                const int d = c * 32 + q4 * 8;
+                if (d < p.D) *reinterpret_cast<uint4*>(orow + d) = pack8<P2>(o + q4 * 8, inv);
+              }
             }
           }
         }
@@ -756,6 +791,7 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
       tc_fence_before();
       if (m < p.M) p.lse[static_cast<int64_t>(u.bh) * p.M + m] = any_key ? m_used + log2f(l) : INFINITY;
     }
+    if (L::kStageO && lane == 0) tma_store_wait_all<0>();
   }
 
   tc_fence_before();
@@ -895,6 +931,7 @@ int launch_fwd(const fa_params& p, cudaStream_t stream, int* status) {
   fp.o = p.o;
   fp.o_vec32 = reinterpret_cast<uintptr_t>(p.o) % 32 == 0 && p.o_stride[0] % 16 == 0 && p.o_stride[1] % 16 == 0 &&
                p.o_stride[2] % 16 == 0;
+  fp.o_tma = make_tmap_result(&fp.map_o, p.o, p.B, p.M, p.H, p.D, p.o_stride);
   fp.lse = p.lse;
   fp.status = status;
   fp.o_sB = p.o_stride[0];

@@ -146,6 +146,19 @@ inline int make_tmap_bshd(CUtensorMap* out, const void* base, int B, int S, int 
   return make_tmap_4d(out, base, 2, dims, sb, box);
 }
 
+// Tile map for a (B, S, H, D) result that leaves by bulk tensor stores of 32 rows and 64 columns.  False where the layout
+// cannot be encoded, which plain stores can write to all the same (a stride of zero or less); the stride of a dimension of
+// extent one does not matter.
+inline bool make_tmap_result(CUtensorMap* out, const void* base, int B, int S, int H, int D, const int64_t stride[3]) {
+  const int extent[3] = {B, S, H};
+  int64_t s[3];
+  for (int i = 0; i < 3; ++i) {
+    s[i] = extent[i] == 1 ? 8 : stride[i];
+    if (s[i] <= 0) return false;
+  }
+  return make_tmap_bshd(out, base, B, S, H, D, s, 32) == FA_OK;
+}
+
 // Tile map for a (B, H, M, N) bias-like tensor: dims {N, M, H, B}; a zero stride
 // on B or H collapses that dimension to extent 1 (the kernel then passes
 // coordinate 0).  box {box_cols, box_rows, 1, 1}.
