@@ -86,7 +86,7 @@ typedef struct fa_params {
   const void* bias;
   void* dbias;
   float* lse;   /* forward out / backward in: log2-domain log-sum-exp      */
-  float* delta; /* backward scratch: rowsum(o * do), written by fa_bwd_pre */
+  float* delta; /* backward scratch: rowsum(o * do), written by fa_bwd_pre or, in one launch, fa_bwd */
 
   int64_t q_stride[3];
   int64_t k_stride[3];

@@ -188,3 +188,46 @@ def test_the_reference_classes_take_the_same_kernels(S, kind, device_ok):
             b, bias_kind = fa._classify_bias(bias, q)
             p = fa._params(q, k, v, want[0], want[0], b, bias_kind, True, 0.1)
             assert lib.fa_bwd_workspace_bytes(ctypes.byref(p)) == S * ((S + 7) // 8 * 8) * 2
+
+
+@pytest.mark.parametrize("B,H", [(1, 2), (3, 64)])
+@pytest.mark.parametrize("M,N,D,kind,causal,dtype", [
+    (65, 65, 64, "float", False, HF), (128, 128, 64, "float", True, BF), (129, 100, 32, "f32", True, HF), (256, 128, 64, "bool", False, BF),
+    (1, 128, 64, None, False, BF), (20, 65, 64, "float", True, BF), (200, 1, 64, None, True, HF), (72, 72, 16, "float", False, HF),
+    (255, 127, 32, "bool", True, HF), (128, 120, 64, "f32", False, BF), (130, 128, 64, None, True, BF)])
+def test_one_launch_backward_equals_the_stages(M, N, D, kind, causal, dtype, B, H, device_ok):
+    """One tile of keys: fa_bwd runs everything in one kernel, the three stage entries do it one by one; the same bits,
+    delta among them."""
+    from tests.test_robustness_gpu import _bwd_params
+    from triton_flashattn_b200 import _cabi
+    from triton_flashattn_b200 import flash_attention as fa
+
+    lib = _cabi.load()
+    g = torch.Generator(device="cuda").manual_seed(M * 1000 + N)
+    q, k, v, do = (torch.randn(B, s, H, D, generator=g, device="cuda", dtype=torch.float32).to(dtype) for s in (M, N, N, M))
+    bias = None
+    if kind == "bool":
+        bias = torch.rand(B, H, M, N, generator=g, device="cuda") < 0.9
+    elif kind is not None:
+        bias = torch.randn(B, H, M, N, generator=g, device="cuda", dtype=torch.float32).to(torch.float32 if kind == "f32" else dtype)
+    o, lse = fa._flash_attn_fwd(q, k, v, bias, causal, D ** -0.5)
+
+    def run(stages):
+        outs = [torch.full_like(t, 7.0) for t in (q, k, v)]
+        delta = torch.full_like(lse, 7.0)
+        dbias = fa._new_dbias(bias, q, causal) if kind in ("float", "f32") else None
+        p, keep = _bwd_params(fa, q, k, v, o, lse, bias, causal, D ** -0.5, do, *outs, dbias, delta)
+        ds16 = torch.empty(B, H, M, (N + 7) // 8 * 8, dtype=dtype, device="cuda")
+        if kind == "f32":
+            p.ds16, p.ds16_stride = ds16.data_ptr(), _cabi._I64x3(*ds16.stride()[:3])
+        before = lib.fa_launch_count()
+        for f in stages:
+            assert f(ctypes.byref(p), None) == 0
+        torch.cuda.synchronize()
+        return outs + [delta] + ([dbias] if dbias is not None else []), lib.fa_launch_count() - before
+
+    one, n_one = run([lib.fa_bwd])
+    stages, n_stages = run([lib.fa_bwd_pre, lib.fa_bwd_dkdv, lib.fa_bwd_dq])
+    assert (n_one, n_stages) == (1, 3)  # up to two heads a CTA
+    for a, b, name in zip(one, stages, ("dq", "dk", "dv", "delta", "dbias")):
+        assert torch.equal(a, b), name

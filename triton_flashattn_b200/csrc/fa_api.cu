@@ -241,8 +241,8 @@ bool parts_pay(const fa_params& p, const PartsCost& parts, int n) {
 uint64_t bwd_workspace_bytes(const fa_params& p) {
   const uint64_t one = slab_bytes(p), fit = kSlabCap / one;
   if (ds_is_dbias(p)) return 0;
-  // short sequences use none; with an fp32 bias some workspace is what stands for ds16 in the checks
-  if (small_takes(p.M, p.N, p.D)) return p.bias_kind == FA_BIAS_F32 ? one : 0;
+  // backwards in one launch use none; with an fp32 bias some workspace is what stands for ds16 in the checks
+  if (small_takes(p.M, p.N, p.D) || one_tile_takes(p)) return p.bias_kind == FA_BIAS_F32 ? one : 0;
   const PartsCost parts(p);
   const int total = parts.total;
   int n = fit < 1 ? 0 : parts.best(fit > (uint64_t)total ? total : (int)fit);
@@ -275,6 +275,7 @@ int bwd_whole(const fa_params& p, cudaStream_t s, int* st) {
     if (int e = check_tiled_bias(p, true)) return e;
     return launch_small(p, true, s, st);
   }
+  if (one_tile_takes(p)) return launch_bwd_one_tile(p, s, st);
   if (int e = launch_bwd_pre(p, s, st)) return e;
   if (int e = launch_bwd_dkdv(p, s, st)) return e;
   return launch_bwd_dq(p, s, st);
@@ -419,7 +420,7 @@ int fa_bwd_workspace(const fa_params* p, void* workspace, uint64_t bytes, void* 
   if (reinterpret_cast<uintptr_t>(workspace) % 16 != 0) return FA_ERR_ALIGN;
   return with_device(p->device, [&](int* st) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (small_takes(p->M, p->N, p->D)) return bwd_whole(*p, s, st);
+    if (small_takes(p->M, p->N, p->D) || one_tile_takes(*p)) return bwd_whole(*p, s, st);
     if (int e = launch_bwd_pre(*p, s, st)) return e;
     return bwd_in_parts(*p, workspace, bytes, s, st);
   });

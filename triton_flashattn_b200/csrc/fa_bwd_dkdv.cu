@@ -39,6 +39,12 @@
 // Rule kept by every barrier here: the next completion of a barrier needs progress of
 // every thread that waits on it, so a parity wait can never be two phases behind.
 //
+// With at most 128 keys one tile holds a whole row of dS, and the ONE_TILE variant (head dims up to 64, up to 256 queries)
+// is the whole backward in one launch: dQ = dS K over the tile of dS that dK reads, into 64 free columns of tensor memory,
+// and delta from the rows of o and dO, which the threads of that query row add up as fa_bwd_pre.cu does (the same bits).
+// It saves two launches, and with an fp32 bias the way of dS through memory, but a tile's chain is longer (see
+// one_tile_takes).
+//
 // Replaces _attn_bwd_dkdv / _attn_bwd_dkdv_inner of the reference
 // (flash_attention.py 237-454): same P, dS, dbias = dS, dK scaled by sm_scale.
 #include "fa_common.cuh"
@@ -75,6 +81,12 @@ struct DkdvParams {
   float scale_log2;  // sm_scale * log2(e)
   float sm_scale;
   int n_bh;  // problems of this launch
+  // one tile of keys: what dQ and delta need
+  const void* o;
+  const void* d_o;
+  void* dq;
+  float* delta_out;
+  int64_t o_sB, o_sM, o_sH, do_sB, do_sM, do_sH, dq_sB, dq_sM, dq_sH;
 };
 
 enum DkdvSite { kSiteKV = 1, kSiteQFull, kSiteQEmpty, kSiteDoFull, kSiteDoEmpty, kSiteSFull,
@@ -103,7 +115,7 @@ struct DkdvSmem {
   static constexpr int kDynamic = kTotal + 1024;
 };
 
-template <int DP, typename T, int BIAS, bool LONGEST_FIRST>
+template <int DP, typename T, int BIAS, bool LONGEST_FIRST, bool ONE_TILE = false>
 __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant__ DkdvParams p) {
   using L = DkdvSmem<DP>;
   using P2 = Pack2<T>;
@@ -111,6 +123,8 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
   constexpr int KS_D = DP / 16;  // K slices of the two "score" products
   constexpr int kDoStages = L::kDoStages;
   constexpr uint32_t kColS = 0, kColDp = 128, kColDv = 256, kColDk = 384;
+  constexpr uint32_t kColDq = 320;  // one tile of keys, head dims up to 64
+  static_assert(!ONE_TILE || (DP == 64 && !LONGEST_FIRST), "dQ has no columns");
   constexpr uint32_t kTmemCols = 512;
   // BIAS: 0 none; 1 16-bit bias, brought in by TMA; 2 byte mask and 3 fp32 bias, read by the row threads from global
   // memory (the mask one step ahead, the fp32 row - 64 registers - at the start of its own step)
@@ -140,7 +154,7 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
   // every second row from the other end: what a CTA has too much of in one row it has too little of in the next.  It is a
   // variant of its own because every role walks the schedule: chosen at run time it cost every short tile of the others
   // (trained bias shared by the batch, 72 x 72, B539 H3 D16 44.4 -> 49.0 us, 100 x 100, B600 H4 D64 69.0 -> 74.3).
-  const int sched_sh = p.causal ? 1 : 0;
+  const int sched_sh = p.causal && !ONE_TILE ? 1 : 0;
   auto tile_at = [&](int it, int& bh, int& nb, int& i_start, int& T_steps) -> bool {
     if constexpr (LONGEST_FIRST) {
       const int G = static_cast<int>(gridDim.x), c = static_cast<int>(blockIdx.x);
@@ -158,7 +172,7 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
     bh = k / p.n_nblk;
     const int pos = k - bh * p.n_nblk;
     bh += p.bh0;
-    nb = p.causal ? ((pos & 1) ? p.n_nblk - 1 - (pos >> 1) : (pos >> 1)) : pos;
+    nb = sched_sh ? ((pos & 1) ? p.n_nblk - 1 - (pos >> 1) : (pos >> 1)) : pos;
     i_start = p.causal ? min(nb, n_mblk) : 0;
     T_steps = n_mblk - i_start;
     return true;
@@ -169,7 +183,7 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
   if (tid == 0) {
     abort_flag = 0;
     mbar_init(&kv_full, 1);
-    mbar_init(&kv_empty, 1);
+    mbar_init(&kv_empty, ONE_TILE ? 2 : 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&q_full[i], 1);
       mbar_init(&q_empty[i], 2);
@@ -404,6 +418,12 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
           if (elect_one()) {
             issue_gemm_ss<8, true, true>(tmem + kColDk, ds_mn, qs ? q_mn_1 : q_mn_0, kBlk, kBlk, idesc_g,
                                          t > 0);
+            if constexpr (ONE_TILE) {
+              // its columns are free: dS is only announced by row warps that have read the dQ of the step before
+              issue_gemm_ss<8, false, true>(tmem + kColDq, make_sdesc(ds_addr, 0, 1024), make_sdesc(smem_u32(smem + L::kK), kBlk, 1024),
+                                            kBlk, kBlk, make_idesc(bf, false, true, 128, DP), false);
+              if (t == T_steps - 1) mma_commit(&kv_empty);
+            }
             mma_commit(&q_empty[qs]);
             mma_commit(&dk_done);
           }
@@ -468,11 +488,11 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
     const int qt = warp >> 2;              // column group: keys n0 + kCW*qt .. + kCW-1
     const uint32_t lane_base = static_cast<uint32_t>(warp & 3) * 32u;
     bool ok = live;
-    // this thread's four 16-byte chunks inside the [128][128] 16-bit tiles: chunk c of the
+    // this thread's eight 16-byte chunks inside the [128][128] 16-bit tiles: chunk c of the
     // row lands at sp_row + ((chunk0 + c) ^ (r & 7)) * 16; the dS tile sits kDs - kP further
     const uint32_t sp_row = smem_u32(smem + L::kP + (qt * kCW / 64) * kBlk) + static_cast<uint32_t>(r) * 128u;
     const uint32_t chunk0 = (qt * kCW % 64) / 8;
-    // tensor-memory address of this thread's 32 columns of S (dP: + kColDp)
+    // tensor-memory address of this thread's 64 columns of S (dP: + kColDp)
     const uint32_t tm_sc = tmem_addr(tmem, lane_base, kColS + qt * kCW);
 
     constexpr int BR = BIAS == 1 ? 0 : BK;  // bias staged in registers only for kinds 2 and 3
@@ -481,6 +501,7 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
     // replaced for rows beyond M) when that step starts, so the loads travel during this one
     float lse_next = 0.f, delta_next = 0.f;
     bool row_ok_next = false;
+    uint4 o_next[ONE_TILE ? 8 : 1], do_next[ONE_TILE ? 8 : 1];  // delta is formed from them instead
     // fetches bias / -LSE2 / delta of query block `mblk` for the tile (bh_, key column c0)
     auto prefetch = [&](int bh_, int c0, int mblk) {
       const int b_ = bh_ / p.H, h_ = bh_ - b_ * p.H;
@@ -495,8 +516,40 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
       }
       const int64_t idx = (int64_t)bh_ * p.M + min(m, p.M - 1);
       lse_next = __ldcg(p.lse + idx);
-      delta_next = __ldcg(p.delta + idx);
       row_ok_next = row_ok;
+      if constexpr (!ONE_TILE) {
+        delta_next = __ldcg(p.delta + idx);
+      } else {
+        const uint4* orow = reinterpret_cast<const uint4*>(static_cast<const T*>(p.o) + b_ * p.o_sB + (int64_t)min(m, p.M - 1) * p.o_sM +
+                                                           h_ * p.o_sH);
+        const uint4* grow = reinterpret_cast<const uint4*>(static_cast<const T*>(p.d_o) + b_ * p.do_sB +
+                                                           (int64_t)min(m, p.M - 1) * p.do_sM + h_ * p.do_sH);
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          if (c * 8 < p.D) {
+            o_next[c] = __ldcg(orow + c);
+            do_next[c] = __ldcg(grow + c);
+          }
+      }
+    };
+    // rowsum(o * dO) in the order of fa_bwd_pre.cu: eight columns one after the other, then pairs
+    auto delta_of_next = [&]() {
+      float part[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        part[c] = 0.f;
+        if (c * 8 < p.D) {
+          const uint32_t a[4] = {o_next[ONE_TILE ? c : 0].x, o_next[ONE_TILE ? c : 0].y, o_next[ONE_TILE ? c : 0].z, o_next[ONE_TILE ? c : 0].w};
+          const uint32_t g[4] = {do_next[ONE_TILE ? c : 0].x, do_next[ONE_TILE ? c : 0].y, do_next[ONE_TILE ? c : 0].z, do_next[ONE_TILE ? c : 0].w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float2 x = P2::unpack(a[i]), y = P2::unpack(g[i]);
+            part[c] = fmaf(x.x, y.x, part[c]);
+            part[c] = fmaf(x.y, y.y, part[c]);
+          }
+        }
+      }
+      return ((part[0] + part[4]) + (part[2] + part[6])) + ((part[1] + part[5]) + (part[3] + part[7]));
     };
     // Loop state is kept small on purpose (registers): the running step count gs, the tile
     // counter it, and per tile bh, col0 and the current query block mb; the first query block
@@ -529,6 +582,10 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
         const int i0 = p.causal ? min(col0 >> 7, n_mblk) : 0;  // first query block of the tile
         const int t = mb - i0;
         const int m0 = mb * 128;
+        if constexpr (ONE_TILE) {
+          delta_next = delta_of_next();
+          if (qt == 0 && row_ok_next) p.delta_out[(int64_t)bh * p.M + m0 + r] = delta_next;
+        }
         BiasRegs<BR> bcur[kNG];
 #pragma unroll
         for (int g = 0; g < kNG; ++g) bcur[g] = bnext[g];
@@ -542,7 +599,7 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
         }
         // rows beyond M get -inf / 0, which makes their P and dS zero
         const float neg_lse = row_ok_next ? -lse_next : -INFINITY, delta_r = row_ok_next ? delta_next : 0.f;
-        if (mb + 1 < n_mblk) prefetch(bh, col0, mb + 1);
+        if (!ONE_TILE && mb + 1 < n_mblk) prefetch(bh, col0, mb + 1);
         // ---- P
         ok = wait_warp_polled(ps, &s_full, gs & 1, ctx, kSiteSFull, t);
         if (!ok) break;
@@ -686,11 +743,37 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(&ds_ready);
+
+        if constexpr (ONE_TILE) {
+          // the rows of the next step travel while dQ is formed and stored
+          if (mb + 1 < n_mblk) {
+            prefetch(bh, col0, mb + 1);
+          } else {
+            int bh2, nb2, is2, T2;
+            if (tile_at(it + 1, bh2, nb2, is2, T2)) prefetch(bh2, nb2 * 128 + qt * kCW, is2);
+          }
+          ok = wait_warp(&dk_done, gs & 1, ctx, kSiteDkDone, mb);
+          if (!ok) break;
+          tc_fence_after();
+          uint32_t a[32];
+          tmem_ld32(tm_sc - qt * kCW + kColDq + qt * 32, a);
+          tmem_ld_wait();
+          tc_fence_before();
+          if (m0 + r < p.M) {
+            const int b_ = bh / p.H, h_ = bh - b_ * p.H;
+            T* row = static_cast<T*>(p.dq) + b_ * p.dq_sB + (int64_t)(m0 + r) * p.dq_sM + h_ * p.dq_sH;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const int d = qt * 32 + c * 8;
+              if (d < p.D) *reinterpret_cast<uint4*>(row + d) = pack8<P2>(a + c * 8, p.sm_scale);
+            }
+          }
+        }
       }
       if (!ok) break;
 
       // the next tile's first bias / LSE / delta rows travel while this tile's result is stored
-      {
+      if (!ONE_TILE) {
         int bh2, nb2, is2, T2;
         if (tile_at(it + 1, bh2, nb2, is2, T2) && T2 > 0) prefetch(bh2, nb2 * 128 + qt * kCW, is2);
       }
@@ -756,10 +839,10 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
   if (warp == kRW + 1) tmem_dealloc(tmem, kTmemCols);
 }
 
-template <int DP, typename T, int BIAS, bool LONGEST_FIRST>
+template <int DP, typename T, int BIAS, bool LONGEST_FIRST, bool ONE_TILE = false>
 int launch_inst(const DkdvParams& kp, dim3 grid, cudaStream_t stream) {
   using L = DkdvSmem<DP>;
-  auto kern = dkdv_kernel<DP, T, BIAS, LONGEST_FIRST>;
+  auto kern = dkdv_kernel<DP, T, BIAS, LONGEST_FIRST, ONE_TILE>;
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -779,6 +862,16 @@ int launch_bias(const DkdvParams& kp, int bias_kind, dim3 grid, cudaStream_t str
     case FA_BIAS_SAME: return launch_inst<DP, T, 1, LONGEST_FIRST>(kp, grid, stream);
     case FA_BIAS_BOOL: return launch_inst<DP, T, 2, LONGEST_FIRST>(kp, grid, stream);
     case FA_BIAS_F32: return launch_inst<DP, T, 3, LONGEST_FIRST>(kp, grid, stream);
+    default: return FA_ERR_UNSUPPORTED;
+  }
+}
+template <typename T>
+int launch_one_tile(const DkdvParams& kp, int bias_kind, dim3 grid, cudaStream_t stream) {
+  switch (bias_kind) {
+    case FA_BIAS_NONE: return launch_inst<64, T, 0, false, true>(kp, grid, stream);
+    case FA_BIAS_SAME: return launch_inst<64, T, 1, false, true>(kp, grid, stream);
+    case FA_BIAS_BOOL: return launch_inst<64, T, 2, false, true>(kp, grid, stream);
+    case FA_BIAS_F32: return launch_inst<64, T, 3, false, true>(kp, grid, stream);
     default: return FA_ERR_UNSUPPORTED;
   }
 }
@@ -861,8 +954,20 @@ DkdvPlan plan_dkdv(const fa_params& p, int n_bh, int sms, bool writes_zeros) {
   return {longest_first, longest_first ? longest : pairs};
 }
 
-int launch_bwd_dkdv(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab) {
-  if (p.D == 256) return launch_bwd_dkdv_d256(p, stream, status, slab);
+// One tile of keys and at most two blocks of queries: dQ joins the chain of a step, which a head walks alone (at B1 H8 M4096
+// N128 the streamed dQ kernel has 256 CTAs, this one 8).  Up to two heads a CTA the launches are what a pass waits for; with
+// more, three kernels that overlap their tiles are faster, except with an fp32 bias, whose dS would go to scratch and back.
+// Training pass, us, three launches / one: B2 S128 H4 D64, 16-bit trained bias 79.9 / 74.0; B4 H16 S128 causal 68.0 / 62.1; B16
+// H12 200 x 77, padding mask 76.5 / 69.9; B64 H3 S81 D16, trained table 100.4 / 95.8; fp32 trained bias B8 H4 256 x 128 74.4 / 68.4,
+// B500 H8 128 x 100 577 / 536; left to three: trained table B256 H6 S100 D32 143 / 159, B600 H4 S128 D64 210 / 277.
+bool one_tile_takes(const fa_params& p) {
+  return p.N <= 128 && p.M <= 256 && p.D <= 64 && !small_takes(p.M, p.N, p.D) &&
+         (p.bias_kind == FA_BIAS_F32 || p.B * p.H <= 2 * persistent_grid(1 << 30));
+}
+
+namespace {
+
+int launch_dkdv(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab, bool one_tile) {
   DkdvParams kp;
   int r = make_tmap_bshd(&kp.map_q, p.q, p.B, p.M, p.H, p.D, p.q_stride, 128);
   if (r) return r;
@@ -875,7 +980,7 @@ int launch_bwd_dkdv(const fa_params& p, cudaStream_t stream, int* status, const 
   const bool f32 = p.bias_kind == FA_BIAS_F32;
   kp.ds_flat = slab != nullptr;
   kp.bh0 = slab ? slab->bh0 : 0;
-  kp.store_ds = slab || f32 || p.write_dbias;
+  kp.store_ds = slab || (f32 && !one_tile) || (!f32 && p.write_dbias);
   kp.zero_tiles = !f32 && p.write_dbias && p.causal;
   kp.dbias_f32 = nullptr;
   kp.dbf_sB = kp.dbf_sH = kp.dbf_sM = 0;
@@ -964,11 +1069,32 @@ int launch_bwd_dkdv(const fa_params& p, cudaStream_t stream, int* status, const 
   kp.n_bh = slab ? slab->n_bh : p.B * p.H;
   kp.n_tiles = kp.n_nblk * kp.n_bh;
   const int sms = persistent_grid(1 << 30);
+  if (one_tile) {
+    if (bad(p.o, p.o_stride) || bad(p.d_o, p.do_stride) || bad(p.dq, p.dq_stride)) return FA_ERR_ALIGN;
+    kp.o = p.o, kp.d_o = p.d_o, kp.dq = p.dq, kp.delta_out = p.delta;
+    kp.o_sB = p.o_stride[0], kp.o_sM = p.o_stride[1], kp.o_sH = p.o_stride[2];
+    kp.do_sB = p.do_stride[0], kp.do_sM = p.do_stride[1], kp.do_sH = p.do_stride[2];
+    kp.dq_sB = p.dq_stride[0], kp.dq_sM = p.dq_stride[1], kp.dq_sH = p.dq_stride[2];
+    const dim3 grid(kp.n_tiles < sms ? kp.n_tiles : sms);
+    return p.dtype == FA_BF16 ? launch_one_tile<__nv_bfloat16>(kp, p.bias_kind, grid, stream)
+                              : launch_one_tile<__half>(kp, p.bias_kind, grid, stream);
+  }
   const bool longest_first = plan_dkdv(p, kp.n_bh, sms, kp.zero_tiles != 0).longest_first;
   const int units = p.causal && !longest_first ? (kp.n_tiles + 1) / 2 : kp.n_tiles;
   const dim3 grid(units < sms ? units : sms);
   return longest_first ? launch_dim<true>(kp, p.dtype, p.bias_kind, grid, stream)
                        : launch_dim<false>(kp, p.dtype, p.bias_kind, grid, stream);
+}
+
+}  // namespace
+
+int launch_bwd_dkdv(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab) {
+  return p.D == 256 ? launch_bwd_dkdv_d256(p, stream, status, slab) : launch_dkdv(p, stream, status, slab, false);
+}
+
+int launch_bwd_one_tile(const fa_params& p, cudaStream_t stream, int* status) {
+  if (int e = check_tiled_bias(p, true)) return e;
+  return launch_dkdv(p, stream, status, nullptr, true);
 }
 
 }  // namespace fa

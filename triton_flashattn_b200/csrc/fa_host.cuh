@@ -61,6 +61,9 @@ DkdvPlan plan_dkdv(const fa_params& p, int n_bh, int sms, bool writes_zeros);
 int dkdv_pair_work(const fa_params& p);
 // Without a slab: all problems, dS going where the parameters say (dbias, ds16 or nowhere).
 int launch_bwd_dkdv(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab = nullptr);
+// The whole backward in one launch where one tile holds all keys: whether it takes the problem, and its launch.
+bool one_tile_takes(const fa_params& p);
+int launch_bwd_one_tile(const fa_params& p, cudaStream_t stream, int* status);
 int launch_bwd_dq(const fa_params& p, cudaStream_t stream, int* status, const DsSlab* slab = nullptr);
 // Head dimension 256: its own dV kernel, which always leaves the 16-bit dS in global
 // memory (in dbias for a 16-bit bias that wants its gradient, else in the ds16 scratch;
