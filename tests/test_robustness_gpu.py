@@ -434,6 +434,31 @@ def test_forward_result_in_any_layout(layout, D, M, device_ok):
     assert (buf[:, M:] == 7).all() and (buf[..., D:] == 7).all()
 
 
+@pytest.mark.parametrize("M,N,D", [(40, 40, 32), (100, 90, 64), (10, 200, 64), (300, 300, 128), (130, 130, 256)])
+def test_first_cuda_call_of_a_thread(M, N, D, device_ok):
+    """A thread whose first CUDA call is one of this library's: no context is bound to it yet, which the encoding of tile
+    maps wants.  (The autograd engine's thread is one in a program's first backward.)"""
+    import threading
+
+    from triton_flashattn_b200 import _cabi
+    from triton_flashattn_b200 import flash_attention as fa
+
+    lib = _cabi.load()
+    q, k, v, bias, do = make_inputs(1, M, N, 2, D, BF, "float", 69)
+    o, lse = fa._flash_attn_fwd(q, k, v, bias, False, 0.1)
+    dq, dk, dv = (torch.empty_like(t) for t in (q, k, v))
+    dbias, delta = fa._new_dbias(bias, q, False), torch.empty_like(lse)
+    p, keep = _bwd_params(fa, q, k, v, o, lse, bias, False, 0.1, do, dq, dk, dv, dbias, delta)
+    torch.cuda.synchronize()
+    for f in (lib.fa_fwd, lib.fa_bwd, lib.fa_bwd_dkdv, lib.fa_bwd_dq):
+        got = []
+        t = threading.Thread(target=lambda: got.append(f(ctypes.byref(p), None)))
+        t.start()
+        t.join()
+        assert got == [0]
+    torch.cuda.synchronize()
+
+
 @pytest.mark.parametrize("bias_kind,D", [(0, 64), (2, 128), (0, 256), (3, 128)])
 def test_scratch_for_ds_is_bounded(bias_kind, D, device_ok):
     """The scratch a backward asks for: at most 1.5 GiB, and nothing where that holds no problem or too few to fill
