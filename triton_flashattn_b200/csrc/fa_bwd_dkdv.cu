@@ -782,7 +782,6 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
       const int steps_here = n_mblk - (p.causal ? min(col0 >> 7, n_mblk) : 0);
       if (steps_here > 0) {
         ok = wait_warp(&dv_done, (gs - 1) & 1, ctx, kSiteEpilogue, 0);
-        if (ok) ok = wait_warp(&dk_done, (gs - 1) & 1, ctx, kSiteEpilogue, 1);
         if (!ok) break;
       }
       {
@@ -796,6 +795,11 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
         T* dvrow = reinterpret_cast<T*>(p.dv) + b * p.dv_sB + (int64_t)n * p.dv_sN + h * p.dv_sH;
 #pragma unroll
         for (int which = 0; which < 2; ++which) {
+          if (which == 1 && steps_here > 0) {  // dV is on its way while the last dK product still runs
+            ok = wait_warp(&dk_done, (gs - 1) & 1, ctx, kSiteEpilogue, 1);
+            if (!ok) break;
+            tc_fence_after();
+          }
           T* row = which == 0 ? dvrow : dkrow;
           const uint32_t colbase = which == 0 ? kColDv : kColDk;
           const float mul = which == 0 ? 1.0f : p.sm_scale;
