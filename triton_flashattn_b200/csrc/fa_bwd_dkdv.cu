@@ -28,12 +28,11 @@
 //   dV += P^T dO_t          (sP and dO_t consumed MN-major)
 //   dK += dS^T Q_t          (sDS and Q_t consumed MN-major)
 //   dbias[b,h,m-block,n-block] <- sDS  (one bulk tensor store of the same tile)
-// A 16-bit bias tile is brought in by TMA and lands exactly where the row threads
-// then write P: each thread reads the eight 16-byte chunks it is about to overwrite, so the
-// bias needs no shared memory of its own (none is left at head dim 128).  (Read by the row threads into registers a step
-// ahead it takes no part in the chain of a step, but a load of 32 rows costs 24 - 60 cycles to issue: 5 - 12 % slower.)
-// A byte mask is read by the row threads straight from global
-// memory, 64 contiguous bytes per thread, one query block ahead.
+// Bias.  16 bit, and a mask at head dim 64: by TMA, at head dim 64 into two tiles of its own, at 128, where no shared memory
+// is left, exactly where the row threads then write P: each thread reads the eight 16-byte chunks it is about to
+// overwrite.  (Read by the row threads into registers a step ahead it takes no part in the chain of a step, but a load of 32
+// rows costs 24 - 60 cycles to issue: 5 - 12 % slower.)  A mask at head dim 128 and an fp32 bias are read by the row threads
+// straight from global memory, the mask 64 contiguous bytes per thread, one query block ahead.
 // Causally skipped tiles of dbias are written as zeros by this kernel, so dbias
 // needs no prior fill.
 // Rule kept by every barrier here: the next completion of a barrier needs progress of
@@ -91,7 +90,7 @@ struct DkdvParams {
 
 enum DkdvSite { kSiteKV = 1, kSiteQFull, kSiteQEmpty, kSiteDoFull, kSiteDoEmpty, kSiteSFull,
                 kSiteDpFull, kSitePReady, kSiteDsReady, kSiteDvDone, kSiteDkDone, kSiteStDone,
-                kSiteZeroReady, kSiteEpilogue, kSiteSFree, kSiteDpFree, kSiteKVEmpty, kSiteBiasFull };
+                kSiteZeroReady, kSiteEpilogue, kSiteSFree, kSiteDpFree, kSiteKVEmpty, kSiteBiasFull, kSiteBiasEmpty };
 
 // Eight row warps, a thread with half a row of a step: what a step costs a warp besides its values (looks at nine
 // barriers, votes, fences, loop) is paid half as often as with sixteen warps and quarters of a row, and 168 registers
@@ -101,7 +100,7 @@ constexpr int kCW = 64;           // columns of a step that a row thread works o
 constexpr int kNG = kCW / 32;     // ... in groups of 32
 constexpr int kRW = 512 / kCW;    // row warps
 constexpr int kThreads = 32 * (kRW + 4);
-template <int DP>
+template <int DP, int BIAS>
 struct DkdvSmem {
   static constexpr int kTile = 128 * DP * 2;
   static constexpr int kDoStages = DP == 128 ? 1 : 2;
@@ -111,13 +110,20 @@ struct DkdvSmem {
   static constexpr int kDo = kQ + 2 * kTile;
   static constexpr int kP = kDo + kDoStages * kTile;
   static constexpr int kDs = kP + 2 * kBlk;
-  static constexpr int kTotal = kDs + 2 * kBlk;
+  // At head dim 64 there is room for two tiles of a 16-bit bias or a mask of their own, which then land a step ahead and
+  // not between two steps (16 bit) or load by load through the row threads (mask).  Whole backward, us, before / after: 16
+  // bit, trained, B8 H16 S2048 722 / 687, causal 508 / 488, B32 H16 S512 239 / 226; mask B8 H12 S1000 227 / 203, B2 H16 S4096
+  // 654 / 638.
+  static constexpr bool kOwnBias = DP == 64 && (BIAS == 1 || BIAS == 2);
+  static constexpr int kBiasTile = BIAS == 1 ? 2 * kBlk : kBlk;
+  static constexpr int kBias = kDs + 2 * kBlk;
+  static constexpr int kTotal = kBias + (kOwnBias ? 2 * kBiasTile : 0);
   static constexpr int kDynamic = kTotal + 1024;
 };
 
 template <int DP, typename T, int BIAS, bool LONGEST_FIRST, bool ONE_TILE = false>
 __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant__ DkdvParams p) {
-  using L = DkdvSmem<DP>;
+  using L = DkdvSmem<DP, BIAS>;
   using P2 = Pack2<T>;
   constexpr int KB = DP / 64;
   constexpr int KS_D = DP / 16;  // K slices of the two "score" products
@@ -126,8 +132,7 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
   constexpr uint32_t kColDq = 320;  // one tile of keys, head dims up to 64
   static_assert(!ONE_TILE || (DP == 64 && !LONGEST_FIRST), "dQ has no columns");
   constexpr uint32_t kTmemCols = 512;
-  // BIAS: 0 none; 1 16-bit bias, brought in by TMA; 2 byte mask and 3 fp32 bias, read by the row threads from global
-  // memory (the mask one step ahead, the fp32 row - 64 registers - at the start of its own step)
+  // BIAS: 0 none; 1 16-bit bias; 2 byte mask; 3 fp32 bias (its row - 64 registers - is asked for at the start of its own step)
   constexpr int BK = BIAS;
 
   extern __shared__ uint8_t smem_raw[];
@@ -135,7 +140,7 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
                                              ~static_cast<uintptr_t>(1023));
   __shared__ uint64_t kv_full, kv_empty, q_full[2], q_empty[2], do_full[2], do_empty[2];
   __shared__ uint64_t s_full, dp_full, p_ready, ds_ready, dv_done, dk_done, st_done, zero_ready;
-  __shared__ uint64_t s_free, dp_free, bias_full;
+  __shared__ uint64_t s_free, dp_free, bias_full[2], bias_empty[2];  // bias: one tile (in sP), or two of its own
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
 
@@ -200,7 +205,10 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
     mbar_init(&zero_ready, kRW);
     mbar_init(&s_free, kRW);
     mbar_init(&dp_free, kRW);
-    mbar_init(&bias_full, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bias_full[i], 1);
+      mbar_init(&bias_empty[i], kRW);
+    }
     mbar_fence_init();
   }
   if (warp == kRW + 1) {
@@ -260,17 +268,18 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
           }
           __syncwarp();
         };
-        if (BIAS != 0) {
+        constexpr bool kAskL2 = BIAS != 0 && !L::kOwnBias;
+        if (kAskL2) {
           for (int t = pf_done; t < kBiasAhead && t < T_steps; ++t) bias_l2(b, h, n0, i_start + t);
           pf_done = 0;
         }
         int bh2 = 0, nb2 = 0, is2 = 0, T2 = 0;
-        if (BIAS != 0 && !tile_at(it + 1, bh2, nb2, is2, T2)) T2 = 0;
+        if (kAskL2 && !tile_at(it + 1, bh2, nb2, is2, T2)) T2 = 0;
         for (int t = 0; t < T_steps && ok; ++t) {
           const uint32_t gs = g + t;
           const int m0 = (i_start + t) * 128;
           const int qs = gs & 1;
-          if (BIAS != 0) {
+          if (kAskL2) {
             if (t + kBiasAhead < T_steps) {
               bias_l2(b, h, n0, i_start + t + kBiasAhead);
             } else if (t + kBiasAhead - T_steps < T2) {
@@ -278,6 +287,19 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
               bias_l2(b2, bh2 - b2 * p.H, nb2 * 128, is2 + t + kBiasAhead - T_steps);
               ++pf_done;
             }
+          }
+          if constexpr (L::kOwnBias) {
+            // two steps ahead of the row threads at the most
+            if (gs >= 2) ok = wait_warp(&bias_empty[qs], ((gs >> 1) - 1) & 1, ctx, kSiteBiasEmpty, t);
+            if (!ok) break;
+            const bool two = BIAS == 1 && n0 + 64 < p.N;
+            if (elect_one()) {
+              uint8_t* const dst = smem + L::kBias + qs * L::kBiasTile;
+              mbar_expect_tx(&bias_full[qs], two ? 2 * kBlk : kBlk);
+              tma_load_4d(dst, &p.map_bias, &bias_full[qs], n0, m0, h * p.bias_h_mul, b * p.bias_b_mul);
+              if (two) tma_load_4d(dst + kBlk, &p.map_bias, &bias_full[qs], n0 + 64, m0, h * p.bias_h_mul, b * p.bias_b_mul);
+            }
+            __syncwarp();
           }
           if (gs >= 2) ok = wait_warp(&q_empty[qs], ((gs >> 1) - 1) & 1, ctx, kSiteQEmpty, t);
           if (!ok) break;
@@ -297,15 +319,15 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
             if (!ok) return;
             const bool two = n0 + 64 < p.N;
             if (elect_one()) {
-              mbar_expect_tx(&bias_full, two ? 2 * kBlk : kBlk);
-              tma_load_4d(smem + L::kP, &p.map_bias, &bias_full, n0, m0, h * p.bias_h_mul, b * p.bias_b_mul);
+              mbar_expect_tx(&bias_full[0], two ? 2 * kBlk : kBlk);
+              tma_load_4d(smem + L::kP, &p.map_bias, &bias_full[0], n0, m0, h * p.bias_h_mul, b * p.bias_b_mul);
               if (two)
-                tma_load_4d(smem + L::kP + kBlk, &p.map_bias, &bias_full, n0 + 64, m0, h * p.bias_h_mul,
+                tma_load_4d(smem + L::kP + kBlk, &p.map_bias, &bias_full[0], n0 + 64, m0, h * p.bias_h_mul,
                             b * p.bias_b_mul);
             }
             __syncwarp();
           };
-          if (BIAS == 1 && kDoStages == 1) load_bias();
+          if (BIAS == 1 && !L::kOwnBias) load_bias();
           if (!ok) break;
           const int ds = gs % kDoStages;
           const uint32_t du = gs / kDoStages;
@@ -318,7 +340,6 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
                           h, m0, b);
           }
           __syncwarp();
-          if (BIAS == 1 && kDoStages != 1) load_bias();
         }
         g += T_steps;
       }
@@ -495,7 +516,9 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
     // tensor-memory address of this thread's 64 columns of S (dP: + kColDp)
     const uint32_t tm_sc = tmem_addr(tmem, lane_base, kColS + qt * kCW);
 
-    constexpr int BR = BIAS == 1 ? 0 : BK;  // bias staged in registers only for kinds 2 and 3
+    constexpr int BR = BIAS == 1 || L::kOwnBias ? 0 : BK;  // bias read by the row threads: fp32, and a mask without tiles of its own
+    constexpr bool kBiasTma = BIAS == 1 || L::kOwnBias;
+    constexpr bool kBiasInP = kBiasTma && !L::kOwnBias;
     BiasRegs<BR> bnext[kNG];
     // LSE2 and delta of the coming step's row, as loaded: they are only looked at (negated,
     // replaced for rows beyond M) when that step starts, so the loads travel during this one
@@ -613,20 +636,22 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
         __syncwarp();
         if (lane == 0) mbar_arrive(&s_free);
         // P = exp2(S * scale * log2e + bias * log2e - LSE2); rows beyond M have LSE2 = +inf
+        // the tile of a bias brought in by TMA: own shared memory, or where this thread's P chunks go
+        const uint32_t b_slot = L::kOwnBias ? gs & 1 : 0, b_par = (L::kOwnBias ? gs >> 1 : gs) & 1;
         if constexpr (BIAS == 1) {
-          // the bias tile sits where this thread's P chunks go; what does not need it is
-          // computed while it travels: x = S * scale * log2e - LSE2
+          // what does not need the bias is computed while it travels: x = S * scale * log2e - LSE2
+          const uint32_t b_row = L::kOwnBias ? sp_row + (L::kBias - L::kP) + b_slot * L::kBiasTile : sp_row;
 #pragma unroll
           for (int i = 0; i < kCW; i += 2) {
             const f32x2 x = ffma2(f2(pr[i], pr[i + 1]), f2(p.scale_log2, p.scale_log2), f2(neg_lse, neg_lse));
             pr[i] = f2_lo(x);
             pr[i + 1] = f2_hi(x);
           }
-          ok = wait_warp_polled(pb, &bias_full, gs & 1, ctx, kSiteBiasFull, t);
+          ok = wait_warp_polled(pb, &bias_full[b_slot], b_par, ctx, kSiteBiasFull, t);
           if (!ok) break;
 #pragma unroll
           for (int c = 0; c < kCW / 8; ++c) {
-            const uint4 v = lds128(sp_row + (((chunk0 + c) ^ (r & 7)) << 4));
+            const uint4 v = lds128(b_row + (((chunk0 + c) ^ (r & 7)) << 4));
             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
@@ -639,6 +664,25 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
             }
           }
         } else {
+        BiasRegs<2> mask[kNG];  // of a mask tile: [128 rows][128 bytes]
+        if constexpr (BIAS == 2) {
+          if constexpr (L::kOwnBias) {
+            ok = wait_warp_polled(pb, &bias_full[b_slot], b_par, ctx, kSiteBiasFull, t);
+            if (!ok) break;
+            const uint32_t m_row = smem_u32(smem + L::kBias) + b_slot * L::kBiasTile + static_cast<uint32_t>(r) * 128u;
+#pragma unroll
+            for (int c = 0; c < kCW / 16; ++c) {
+              const uint4 v = lds128(m_row + (static_cast<uint32_t>((qt * (kCW / 16) + c) ^ (r & 7)) << 4));
+              uint32_t* const w = mask[c / 2].w + (c & 1) * 4;
+              w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
+            }
+          } else {
+#pragma unroll
+            for (int g = 0; g < kNG; ++g)
+#pragma unroll
+              for (int i = 0; i < 8; ++i) mask[g].w[i] = bcur[g].w[i % (sizeof(bcur[g].w) / 4)];
+          }
+        }
 #pragma unroll
         for (int i = 0; i < kCW; i += 2) {
           f32x2 a = ffma2(f2(pr[i], pr[i + 1]), f2(p.scale_log2, p.scale_log2), f2(neg_lse, neg_lse));
@@ -646,7 +690,7 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
             a = ffma2(f2(__uint_as_float(bcur[i / 32].w[i % 32]), __uint_as_float(bcur[i / 32].w[i % 32 + 1])), f2(kLog2e, kLog2e), a);
           const f32x2 pe = f2(ex2(f2_lo(a)), ex2(f2_hi(a)));
           if (BK == 2) {
-            const uint32_t m2 = bcur[i / 32].w[(i % 32) >> 2] >> (8 * (i & 3));
+            const uint32_t m2 = mask[i / 32].w[(i % 32) >> 2] >> (8 * (i & 3));
             pr[i] = (m2 & 0xFFu) != 0 ? f2_lo(pe) : 0.f;
             pr[i + 1] = (m2 & 0xFF00u) != 0 ? f2_hi(pe) : 0.f;
           } else {
@@ -662,7 +706,7 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
           for (int i = 0; i < kCW; ++i)
             if (i >= limit) pr[i] = 0.f;
         }
-        if (BIAS != 1) {  // (a 16-bit bias tile lands after it)
+        if (!kBiasInP) {  // (a bias tile lands there after it)
           ok = wait_warp_polled(pdv, &dv_done, (gs - 1) & 1, ctx, kSiteDvDone, t);
           if (!ok) break;
         }
@@ -680,7 +724,10 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
         mbar_poll3(&dp_full, gs & 1, &dk_done, (gs - 1) & 1, st_bar, st_par, pdp, pdk, pst);
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&p_ready);
+        if (lane == 0) {
+          mbar_arrive(&p_ready);
+          if constexpr (L::kOwnBias) mbar_arrive(&bias_empty[b_slot]);  // all that was read from it has gone into P
+        }
 
         // ---- dS
         ok = wait_warp_polled(pdp, &dp_full, gs & 1, ctx, kSiteDpFull, t);
@@ -736,8 +783,10 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
           sts128(sp_row + (L::kDs - L::kP) + (((chunk0 + c) ^ (r & 7)) << 4), dsu[c * 4 + 0],
                  dsu[c * 4 + 1], dsu[c * 4 + 2], dsu[c * 4 + 3]);
         // the looks of the next step, of this tile or the next one, are asked for before the fence
-        if (BIAS == 1)
-          mbar_poll2(&s_full, (gs + 1) & 1, &bias_full, (gs + 1) & 1, ps, pb);
+        if (L::kOwnBias)
+          mbar_poll3(&s_full, (gs + 1) & 1, &dv_done, gs & 1, &bias_full[(gs + 1) & 1], ((gs + 1) >> 1) & 1, ps, pdv, pb);
+        else if (kBiasInP)
+          mbar_poll2(&s_full, (gs + 1) & 1, &bias_full[0], (gs + 1) & 1, ps, pb);
         else
           mbar_poll2(&s_full, (gs + 1) & 1, &dv_done, gs & 1, ps, pdv);
         fence_proxy_async_smem();
@@ -845,7 +894,7 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
 
 template <int DP, typename T, int BIAS, bool LONGEST_FIRST, bool ONE_TILE = false>
 int launch_inst(const DkdvParams& kp, dim3 grid, cudaStream_t stream) {
-  using L = DkdvSmem<DP>;
+  using L = DkdvSmem<DP, BIAS>;
   auto kern = dkdv_kernel<DP, T, BIAS, LONGEST_FIRST, ONE_TILE>;
   static bool configured[64] = {};
   int dev = 0;
