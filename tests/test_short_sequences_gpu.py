@@ -231,3 +231,45 @@ def test_one_launch_backward_equals_the_stages(M, N, D, kind, causal, dtype, B, 
     assert (n_one, n_stages) == (1, 3)  # up to two heads a CTA
     for a, b, name in zip(one, stages, ("dq", "dk", "dv", "delta", "dbias")):
         assert torch.equal(a, b), name
+
+
+def test_one_launch_backward_takes_and_refuses_what_the_stages_do(device_ok):
+    """An fp32 gradient whose stride over a batch of one is zero is taken; a ds16 off its alignment is refused by fa_bwd and
+    ignored beside a workspace; a dq, o or do off 16 bytes is refused."""
+    from tests.test_robustness_gpu import _bwd_params
+    from triton_flashattn_b200 import _cabi
+    from triton_flashattn_b200 import flash_attention as fa
+
+    lib = _cabi.load()
+    q, k, v, bias, do = make_inputs(1, 100, 96, 2, 64, BF, "float", 70)
+    bias = bias.float()
+    o, lse = fa._flash_attn_fwd(q, k, v, bias, False, 0.1)
+    outs = [torch.empty_like(t) for t in (q, k, v)]
+    delta, dbias = torch.empty_like(lse), torch.full_like(bias, 7.0)
+    ds16 = torch.empty(1, 2, 100, 96, dtype=BF, device="cuda")
+    ws = torch.empty(2 * 100 * 96 * 2, dtype=torch.uint8, device="cuda")
+
+    def params():
+        p, keep = _bwd_params(fa, q, k, v, o, lse, bias, False, 0.1, do, *outs, dbias, delta)
+        p.ds16, p.ds16_stride = ds16.data_ptr(), _cabi._I64x3(*ds16.stride()[:3])
+        return p, keep
+
+    p, keep = params()
+    p.dbias_stride[0] = 0
+    assert lib.fa_bwd(ctypes.byref(p), None) == 0
+    torch.cuda.synchronize()
+    got = dbias.clone()
+    dbias.fill_(7.0)
+    p, keep = params()
+    for f in (lib.fa_bwd_pre, lib.fa_bwd_dkdv, lib.fa_bwd_dq):
+        assert f(ctypes.byref(p), None) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(got, dbias)
+    p.ds16 = ds16.data_ptr() + 2
+    assert lib.fa_bwd(ctypes.byref(p), None) == 5  # FA_ERR_ALIGN
+    assert lib.fa_bwd_workspace(ctypes.byref(p), ws.data_ptr(), ws.numel(), None) == 0
+    torch.cuda.synchronize()
+    for name in ("dq", "dk", "dv", "o", "d_o"):
+        p, keep = params()
+        setattr(p, name, getattr(p, name) + 2)
+        assert lib.fa_bwd(ctypes.byref(p), None) == 5, name

@@ -428,7 +428,12 @@ int fa_bwd_workspace(const fa_params* p, void* workspace, uint64_t bytes, void* 
   if (reinterpret_cast<uintptr_t>(workspace) % 16 != 0) return FA_ERR_ALIGN;
   return with_device(p->device, [&](int* st) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (small_takes(p->M, p->N, p->D) || one_tile_takes(*p)) return bwd_whole(*p, s, st);
+    if (small_takes(p->M, p->N, p->D)) return bwd_whole(*p, s, st);
+    if (one_tile_takes(*p)) {
+      fa_params q = *p;
+      q.ds16 = nullptr;  // the workspace stands for it, whatever it says
+      return bwd_whole(q, s, st);
+    }
     if (int e = launch_bwd_pre(*p, s, st)) return e;
     return bwd_in_parts(*p, workspace, bytes, s, st);
   });
