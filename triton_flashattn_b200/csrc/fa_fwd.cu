@@ -110,7 +110,7 @@ struct FwdSmem {
 // (batch*head)-major; CTA c takes c, c+G, c+2G, ... so that CTAs running at the same time
 // share K / V in L2.  Causal: the entries of one (batch, head) are ordered [last, first,
 // last-1, first+1, ...] and a CTA takes two consecutive ones, a heavy and a light pair.
-// With LONGEST_FIRST (causal, see plan_fwd) the units are numbered by length instead, and the CTAs take them in rows, every
+// With LONGEST_FIRST (causal, see longest_first) the units are numbered by length instead, and the CTAs take them in rows, every
 // second row from the other end: what a CTA has too much of in one row it has too little of in the next.  It is a variant
 // of its own because every role walks the schedule: chosen at run time it made every other forward 0.5 - 1 % slower.
 struct Unit {
@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
                     s[i + 3] = f2_hi(x1);
                   }
                   // Each unit goes back by itself, behind a vote on the maximum of its 32 scores (see below): four
-                  // units a key block pass through this ring of three.
+                  // units a key block pass through the ring.
                   float ma = max3(s[sub * 32], s[sub * 32 + 1], s[sub * 32 + 2]);
                   float mb = max3(s[sub * 32 + 3], s[sub * 32 + 4], s[sub * 32 + 5]);
 #pragma unroll
