@@ -407,6 +407,23 @@ def test_causal_forward_order_does_not_change_bits(D, bias_kind, M, N, device_ok
         assert torch.equal(out, first) and torch.equal(lse, lse2), cap
 
 
+@pytest.mark.parametrize("D,M,N", [(64, 130, 200), (128, 300, 300), (256, 100, 390), (32, 257, 65)])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("dtype", [BF, HF])
+def test_a_mask_is_a_bias_of_zeros_and_minus_infinity(D, M, N, causal, dtype, device_ok):
+    """The forward scales a score before it masks it or adds a bias, so the two give the same bits; also with a row that sees
+    no key, and with a scale that is no power of two (so that a scale folded into the exponent would round differently)."""
+    from triton_flashattn_b200 import flash_attention as fa
+
+    q, k, v, mask, _ = make_inputs(2, M, N, 3, D, dtype, "bool", 71)
+    mask[1, 2, 5] = False
+    zeros = torch.zeros(mask.shape, dtype=dtype, device="cuda")
+    out, lse = fa._flash_attn_fwd(q, k, v, mask, causal, 0.11)
+    want, want_lse = fa._flash_attn_fwd(q, k, v, zeros.masked_fill_(~mask, float("-inf")), causal, 0.11)
+    assert torch.equal(out, want) and torch.equal(lse, want_lse)
+    assert not out[1, 5, 2].any() and lse[1, 2, 5] == float("inf")
+
+
 @pytest.mark.parametrize("D,M", [(16, 100), (32, 257), (64, 70), (64, 1), (128, 130), (256, 95)])
 @pytest.mark.parametrize("layout", ["dense", "padded", "reversed batch"])
 def test_forward_result_in_any_layout(layout, D, M, device_ok):

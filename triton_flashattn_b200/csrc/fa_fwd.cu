@@ -540,15 +540,20 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
             const int n0 = j * 128 + h * 64;  // first key of this half
             // ---- score in the natural domain: q.k * sm_scale (+ bias), -inf where masked.
             // Without a bias (and a positive scale) the raw q.k is kept and the scale is
-            // folded into the exponent below.
+            // folded into the exponent below.  A mask scales first, as a bias of zeros does, and so gives the bits of one
+            // (folded in as well it rounds once less, with other bits; us, folded / scaled first two at a time: B1 H37 S4096 D128
+            // 344 / 335, D64 318 / 313, causal B4 H32 S4096 D128 670 / 641; one by one 370, 333, 683).
             float mul = kLog2e;  // exponent = s * mul - m
             float mx = -INFINITY;  // row maximum of this half
-            if (BIAS == 0 || BIAS == 2) {
-              if (fold_scale) {
-                mul = scale_log2;
-              } else {
+            if (BIAS == 0 && fold_scale) {
+              mul = scale_log2;
+            } else if (BIAS == 0 || BIAS == 2) {
+              const f32x2 sc2 = f2(p.sm_scale, p.sm_scale);
 #pragma unroll
-                for (int i = 0; i < 64; ++i) s[i] *= p.sm_scale;
+              for (int i = 0; i < 64; i += 2) {
+                const f32x2 x = fmul2(f2(s[i], s[i + 1]), sc2);
+                s[i] = f2_lo(x);
+                s[i + 1] = f2_hi(x);
               }
             }
             if (BIAS != 0) {
