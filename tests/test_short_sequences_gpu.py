@@ -273,3 +273,45 @@ def test_one_launch_backward_takes_and_refuses_what_the_stages_do(device_ok):
         p, keep = params()
         setattr(p, name, getattr(p, name) + 2)
         assert lib.fa_bwd(ctypes.byref(p), None) == 5, name
+
+
+@pytest.mark.parametrize("M,N,D", [(65, 65, 64), (128, 100, 32), (256, 128, 64), (129, 1, 16), (200, 127, 64)])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("B", [1, 60])
+def test_one_launch_backward_leaves_ds_where_it_is_told_to(M, N, D, causal, B, device_ok):
+    """fa_bwd with an fp32 bias leaves dS rounded to 16 bits in ds16, trained bias or not, and nothing behind the 16-byte
+    unit in which a row ends; fa_bwd_workspace does not touch ds16."""
+    ds16_is_left(M, N, D, causal, B)
+
+
+def ds16_is_left(M, N, D, causal, B):
+    from tests.test_robustness_gpu import _bwd_params
+    from triton_flashattn_b200 import _cabi
+    from triton_flashattn_b200 import flash_attention as fa
+
+    lib, H = _cabi.load(), 3
+    q, k, v, bias, do = make_inputs(B, M, N, H, D, HF, "float", 72)
+    bias = bias.float()
+    o, lse = fa._flash_attn_fwd(q, k, v, bias, causal, 0.2)
+    pitch = (N + 7) // 8 * 8 + 8
+
+    def run(entry, train):
+        outs, delta = [torch.empty_like(t) for t in (q, k, v)], torch.empty_like(lse)
+        dbias = fa._new_dbias(bias, q, causal) if train else None
+        ds16 = torch.full((B, H, M, pitch), 7.0, dtype=HF, device="cuda")
+        p, keep = _bwd_params(fa, q, k, v, o, lse, bias, causal, 0.2, do, *outs, dbias, delta)
+        p.ds16, p.ds16_stride = ds16.data_ptr(), fa._stride3(ds16)
+        assert entry(ctypes.byref(p)) == 0
+        torch.cuda.synchronize()
+        return outs, dbias, ds16
+
+    ws = torch.empty(B * H * M * pitch * 2, dtype=torch.uint8, device="cuda")
+    outs, dbias, ds16 = run(lambda p: lib.fa_bwd(p, None), True)
+    visible = torch.ones(M, N, dtype=torch.bool, device="cuda")
+    visible = visible.tril() if causal else visible  # above the diagonal it may hold anything
+    assert torch.equal(ds16[..., :N][..., visible], dbias[..., :N].to(HF)[..., visible])
+    assert (ds16[..., (N + 7) // 8 * 8:] == 7).all()
+    outs2, _, untrained = run(lambda p: lib.fa_bwd(p, None), False)
+    assert torch.equal(untrained, ds16) and all(torch.equal(a, b) for a, b in zip(outs, outs2))
+    outs3, _, untouched = run(lambda p: lib.fa_bwd_workspace(p, ws.data_ptr(), ws.numel(), None), False)
+    assert (untouched == 7).all() and all(torch.equal(a, b) for a, b in zip(outs, outs3))

@@ -1033,7 +1033,8 @@ int launch_dkdv(const fa_params& p, cudaStream_t stream, int* status, const DsSl
   const bool f32 = p.bias_kind == FA_BIAS_F32;
   kp.ds_flat = slab != nullptr;
   kp.bh0 = slab ? slab->bh0 : 0;
-  kp.store_ds = slab || (f32 && !one_tile) || (!f32 && p.write_dbias);
+  // (one tile of keys: nothing reads dS back, but a caller that gives a ds16 finds it there all the same)
+  kp.store_ds = slab || (f32 && (!one_tile || p.ds16)) || (!f32 && p.write_dbias);
   kp.zero_tiles = !f32 && p.write_dbias && p.causal;
   kp.dbias_f32 = nullptr;
   kp.dbf_sB = kp.dbf_sH = kp.dbf_sM = 0;
@@ -1051,13 +1052,6 @@ int launch_dkdv(const fa_params& p, cudaStream_t stream, int* status, const DsSl
     if (!bm || !hm) return FA_ERR_ALIGN;  // must be a real (B,H,M,N) tensor
   } else {
     kp.map_dbias = kp.map_q;
-    if (one_tile && f32 && p.ds16) {  // not used, but what the three stages refuse of it is refused
-      CUtensorMap map;
-      int bm, hm;
-      r = make_tmap_bhmn(&map, p.ds16, 2, p.B, p.H, p.M, p.N, p.ds16_stride, 64, 128, &bm, &hm);
-      if (r) return r;
-      if (!bm || !hm) return FA_ERR_ALIGN;
-    }
   }
   if (f32 && p.write_dbias) {
     if (reinterpret_cast<uintptr_t>(p.dbias) % 16 != 0 || p.dbias_stride[0] % 4 || p.dbias_stride[1] % 4 ||
