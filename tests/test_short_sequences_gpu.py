@@ -313,5 +313,16 @@ def ds16_is_left(M, N, D, causal, B):
     assert (ds16[..., (N + 7) // 8 * 8:] == 7).all()
     outs2, _, untrained = run(lambda p: lib.fa_bwd(p, None), False)
     assert torch.equal(untrained, ds16) and all(torch.equal(a, b) for a, b in zip(outs, outs2))
-    outs3, _, untouched = run(lambda p: lib.fa_bwd_workspace(p, ws.data_ptr(), ws.numel(), None), False)
-    assert (untouched == 7).all() and all(torch.equal(a, b) for a, b in zip(outs, outs3))
+    others = [lambda p: lib.fa_bwd_workspace(p, ws.data_ptr(), ws.numel(), None)]
+    if lib.fa_small_takes(M, N, D):
+        others.append(lambda p: lib.fa_small_bwd(p, None))
+    for entry in others:
+        outs2, _, untouched = run(entry, False)
+        assert (untouched == 7).all() and all(torch.equal(a, b) for a, b in zip(outs, outs2))
+
+
+@pytest.mark.parametrize("M,N,D", [(64, 64, 64), (49, 49, 32), (1, 17, 16), (40, 33, 64), (33, 1, 16)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_short_backward_leaves_ds_where_it_is_told_to(M, N, D, causal, device_ok):
+    """The same for the kernels for short sequences, whose own entry does not touch ds16 either."""
+    ds16_is_left(M, N, D, causal, 2)

@@ -355,7 +355,9 @@ int fa_small_bwd(const fa_params* p, void* stream) {
     for (int i = 0; i < 3; ++i)
       if (extent[i] > 1 && p->dbias_stride[i] <= 0) return FA_ERR_ALIGN;
   }
-  return with_device(p->device, [&](int* st) { return launch_small(*p, true, static_cast<cudaStream_t>(stream), st); });
+  fa_params q = *p;
+  q.ds16 = nullptr;  // not used here, whatever it says
+  return with_device(p->device, [&](int* st) { return launch_small(q, true, static_cast<cudaStream_t>(stream), st); });
 }
 
 int fa_pad_rows(void* dst, const int64_t dst_stride[3], const void* src, const int64_t src_stride[3], int elem_bytes, int B, int H,
@@ -428,8 +430,7 @@ int fa_bwd_workspace(const fa_params* p, void* workspace, uint64_t bytes, void* 
   if (reinterpret_cast<uintptr_t>(workspace) % 16 != 0) return FA_ERR_ALIGN;
   return with_device(p->device, [&](int* st) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (small_takes(p->M, p->N, p->D)) return bwd_whole(*p, s, st);
-    if (one_tile_takes(*p)) {
+    if (small_takes(p->M, p->N, p->D) || one_tile_takes(*p)) {
       fa_params q = *p;
       q.ds16 = nullptr;  // the workspace stands for it, whatever it says
       return bwd_whole(q, s, st);
