@@ -425,22 +425,29 @@ def test_a_mask_is_a_bias_of_zeros_and_minus_infinity(D, M, N, causal, dtype, de
 
 
 @pytest.mark.parametrize("D,M", [(16, 100), (32, 257), (64, 70), (64, 1), (128, 130), (256, 95)])
+@pytest.mark.parametrize("kind", [None, "float", "bool"])
 @pytest.mark.parametrize("layout", ["dense", "padded", "reversed batch"])
-def test_forward_result_in_any_layout(layout, D, M, device_ok):
-    """The result leaves by bulk stores of 32 rows where its layout can be encoded, by plain ones where it cannot: the same
-    bits, and nothing beside it is touched.  M up to 16 goes to the kernel for few rows."""
+def test_forward_result_in_any_layout(layout, D, M, kind, device_ok):
+    """The result leaves by bulk stores of 32 rows where its layout can be encoded, by plain ones where it cannot, and where a bias
+    at head dims 128 and 256 leaves no shared memory for them: the same bits, and nothing beside it is touched.  M up to 16
+    goes to the kernel for few rows."""
     from triton_flashattn_b200 import _cabi
     from triton_flashattn_b200 import flash_attention as fa
 
     B, H, N = 2, 3, 150
     g = torch.Generator(device="cuda").manual_seed(68)
     q, k, v = (torch.randn(B, s, H, D, generator=g, device="cuda", dtype=torch.float32).to(BF) for s in (M, N, N))
-    want, lse = fa._flash_attn_fwd(q, k, v, None, False, D ** -0.5)
+    bias = None
+    if kind is not None:
+        bias = torch.randn(B, H, M, N + 10, generator=g, device="cuda", dtype=torch.float32)  # rows of 160
+        bias = (bias.to(BF) if kind == "float" else bias > -1)[..., :N]
+    want, lse = fa._flash_attn_fwd(q, k, v, bias, False, D ** -0.5)
     pad = 0 if layout == "dense" else 8
     buf = torch.full((B, M + 3, H, D + pad), 7.0, dtype=BF, device="cuda")
     view = buf[:, :M, :, :D]
     lse2 = torch.empty_like(lse)
-    p = fa._params(q, k, v, view, lse2, None, 0, False, D ** -0.5)
+    b, bias_kind = fa._classify_bias(bias, q)
+    p = fa._params(q, k, v, view, lse2, b, bias_kind, False, D ** -0.5)
     if layout == "reversed batch":
         p.o, p.o_stride[0] = view[1].data_ptr(), -view.stride(0)
     lib = _cabi.load()

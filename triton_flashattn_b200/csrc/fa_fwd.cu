@@ -78,6 +78,9 @@ struct FwdParams {
 enum FwdSite { kSiteQFull = 1, kSiteQEmpty, kSiteKFull, kSiteKEmpty, kSiteVFull, kSiteVEmpty,
                kSiteSFull, kSiteSRead, kSitePFull, kSitePvDone, kSiteBiasFull, kSiteBiasEmpty, kSiteEpilogue };
 
+// Whether a forward's results leave through shared memory: at head dim 64, and wherever no bias takes the space.
+constexpr bool stages_result(int dp, int bias_kind) { return dp == 64 || bias_kind == FA_BIAS_NONE; }
+
 template <int DP, int BIAS>
 struct FwdSmem {
   static constexpr int kQTile = 128 * DP * 2;   // one query tile
@@ -99,8 +102,7 @@ struct FwdSmem {
   static constexpr int kK = kQ + kTiles * kQTile;
   static constexpr int kV = kK + kKStages * kKUnit;
   static constexpr int kBias = kV + kVStages * kVHalf;
-  // O on its way out, 64 columns at a time: 4 KB a row warp at head dim 64 and wherever no bias takes the space
-  static constexpr bool kStageO = DP == 64 || BIAS == 0;
+  static constexpr bool kStageO = stages_result(DP, BIAS);  // O on its way out, 64 columns at a time: 4 KB a row warp
   static constexpr int kOut = kBias + kBiasStages * kBlk;
   static constexpr int kTotal = kOut + (kStageO ? kTiles * kBlk : 0);
   static constexpr int kDynamic = kTotal + 1024;  // slack for 1024-byte alignment
@@ -936,7 +938,9 @@ int launch_fwd(const fa_params& p, cudaStream_t stream, int* status) {
   fp.o = p.o;
   fp.o_vec32 = reinterpret_cast<uintptr_t>(p.o) % 32 == 0 && p.o_stride[0] % 16 == 0 && p.o_stride[1] % 16 == 0 &&
                p.o_stride[2] % 16 == 0;
-  fp.o_tma = make_tmap_result(&fp.map_o, p.o, p.B, p.M, p.H, p.D, p.o_stride);
+  fp.map_o = fp.map_q;
+  fp.o_tma = stages_result(padded_head_dim(p.D), p.bias_kind) &&
+             make_tmap_result(&fp.map_o, p.o, p.B, p.M, p.H, p.D, p.o_stride);
   fp.lse = p.lse;
   fp.status = status;
   fp.o_sB = p.o_stride[0];
