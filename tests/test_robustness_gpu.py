@@ -483,6 +483,29 @@ def test_first_cuda_call_of_a_thread(M, N, D, device_ok):
     torch.cuda.synchronize()
 
 
+def test_a_refused_layout_leaves_the_context_alone(device_ok):
+    """A layout that the driver cannot encode (a batch stride of 2^41 bytes; nothing is launched) is refused, and the thread's
+    current context stays the one that it was."""
+    from triton_flashattn_b200 import _cabi
+    from triton_flashattn_b200 import flash_attention as fa
+
+    lib, cuda = _cabi.load(), ctypes.CDLL("libcuda.so.1")
+    q, k, v, _, _ = make_inputs(2, 100, 100, 2, 64, BF, None, 73)
+    o, lse = fa._flash_attn_fwd(q, k, v, None, False, 0.1)
+    torch.cuda.synchronize()
+    p = fa._params(q, k, v, o, lse, None, 0, False, 0.1)
+    p.q_stride[0] = 1 << 40
+    before, own, now = ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p()
+    assert cuda.cuCtxGetCurrent(ctypes.byref(before)) == 0
+    assert cuda.cuCtxCreate_v2(ctypes.byref(own), 0, p.device) == 0  # current from here on
+    try:
+        assert lib.fa_fwd(ctypes.byref(p), None) == 6  # FA_ERR_CUDA
+        assert cuda.cuCtxGetCurrent(ctypes.byref(now)) == 0
+    finally:
+        assert cuda.cuCtxDestroy_v2(own) == 0 and cuda.cuCtxSetCurrent(before) == 0
+    assert now.value == own.value
+
+
 @pytest.mark.parametrize("bias_kind,D", [(0, 64), (2, 128), (0, 256), (3, 128)])
 def test_scratch_for_ds_is_bounded(bias_kind, D, device_ok):
     """The scratch a backward asks for: at most 1.5 GiB, and nothing where that holds no problem or too few to fill

@@ -100,9 +100,9 @@ int make_tmap_4d(CUtensorMap* out, const void* base, int elem_bytes, const uint6
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   };
   CUresult r = encode();
-  if (r != CUDA_SUCCESS) {
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {
     // The driver wants a context, and a thread that has made no runtime call yet (the autograd engine's in a program's
-    // first backward) has none bound.
+    // first backward) has none bound.  (A layout that it refuses is another error, and no reason to bind one.)
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = encode();
   }
