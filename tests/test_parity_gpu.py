@@ -47,6 +47,15 @@ def test_small_grid(D, dtype, bias_kind, causal, device_ok):
     check_case(2, 256, 256, 2, D, dtype, bias_kind, causal, seed=1)
 
 
+@pytest.mark.parametrize("M,N,D,causal", [(300, 200, 128, False), (256, 300, 64, True), (200, 130, 256, True), (100, 90, 64, True),
+                                          (40, 50, 32, False), (4, 300, 128, False)])
+@pytest.mark.parametrize("bias_kind", [None, "float", "bool"])
+@pytest.mark.parametrize("sign", [0.0, -1.0])
+def test_scale_of_zero_and_below(M, N, D, causal, bias_kind, sign, device_ok):
+    """The maximum of raw scores is the maximum of the scaled ones only for a positive scale."""
+    check_case(2, M, N, 3, D, BF, bias_kind, causal, seed=3, sm_scale=sign * D ** -0.5)
+
+
 @pytest.mark.parametrize("M,N,causal", [(50, 70, False), (200, 136, False), (200, 200, True),
                                         (128, 384, False), (384, 128, False), (100, 300, True),
                                         (300, 100, True), (1, 1, False), (129, 1, False)])

@@ -377,10 +377,11 @@ def test_causal_units_of_every_length_repeat_bitwise(D, bias_kind, device_ok):
     elif bias_kind != "none":
         bias = torch.randn(B, H, S, S, generator=g, device="cuda", dtype=torch.float32 if bias_kind == "f32" else BF)
     first, lse = fa._flash_attn_fwd(q, k, v, bias, True, D ** -0.5)
+    differing = torch.zeros((), dtype=torch.int64, device="cuda")
     for _ in range(100):
         out, lse2 = fa._flash_attn_fwd(q, k, v, bias, True, D ** -0.5)
-    torch.cuda.synchronize()
-    assert torch.equal(out, first) and torch.equal(lse, lse2)
+        differing += ((out != first).any() | (lse != lse2).any()).long()
+    assert int(differing) == 0, f"{int(differing)} of 100 passes differ"
 
 
 @pytest.mark.parametrize("D,bias_kind,M,N", [(64, "none", 900, 900), (64, "f32", 1030, 300), (128, "16bit", 1100, 700),

@@ -198,6 +198,22 @@ def test_the_reference_classes_take_the_same_kernels(S, kind, device_ok):
 def test_one_launch_backward_equals_the_stages(M, N, D, kind, causal, dtype, B, H, device_ok):
     """One tile of keys: fa_bwd runs everything in one kernel, the three stage entries do it one by one; the same bits,
     delta among them."""
+    assert one_launch_equals_the_stages(M, N, D, kind, causal, dtype, B, H) == (1, 3)  # up to two heads a CTA
+
+
+@pytest.mark.parametrize("cap", [1, 3])
+@pytest.mark.parametrize("M,N,D", [(256, 128, 64), (256, 65, 64), (131, 128, 32), (77, 65, 64)])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("trained", [False, True])
+def test_one_launch_backward_over_many_tiles(M, N, D, causal, trained, cap, device_ok, monkeypatch):
+    """With an fp32 bias a CTA of the one-launch kernel walks any number of heads (here 7 or 20): rings, columns and rows
+    asked for ahead of a tile go round many times."""
+    monkeypatch.setenv("FA_MAX_CTAS", str(cap))
+    launches = one_launch_equals_the_stages(M, N, D, "f32", causal, BF, 5, 4, trained)
+    assert launches == (1, 3)
+
+
+def one_launch_equals_the_stages(M, N, D, kind, causal, dtype, B, H, trained=True):
     from tests.test_robustness_gpu import _bwd_params
     from triton_flashattn_b200 import _cabi
     from triton_flashattn_b200 import flash_attention as fa
@@ -215,7 +231,7 @@ def test_one_launch_backward_equals_the_stages(M, N, D, kind, causal, dtype, B, 
     def run(stages):
         outs = [torch.full_like(t, 7.0) for t in (q, k, v)]
         delta = torch.full_like(lse, 7.0)
-        dbias = fa._new_dbias(bias, q, causal) if kind in ("float", "f32") else None
+        dbias = fa._new_dbias(bias, q, causal) if trained and kind in ("float", "f32") else None
         p, keep = _bwd_params(fa, q, k, v, o, lse, bias, causal, D ** -0.5, do, *outs, dbias, delta)
         ds16 = torch.empty(B, H, M, (N + 7) // 8 * 8, dtype=dtype, device="cuda")
         if kind == "f32":
@@ -228,9 +244,12 @@ def test_one_launch_backward_equals_the_stages(M, N, D, kind, causal, dtype, B, 
 
     one, n_one = run([lib.fa_bwd])
     stages, n_stages = run([lib.fa_bwd_pre, lib.fa_bwd_dkdv, lib.fa_bwd_dq])
-    assert (n_one, n_stages) == (1, 3)  # up to two heads a CTA
-    for a, b, name in zip(one, stages, ("dq", "dk", "dv", "delta", "dbias")):
-        assert torch.equal(a, b), name
+    ws = torch.empty(B * H * M * ((N + 7) // 8 * 8) * 2 if kind == "f32" else 16, dtype=torch.uint8, device="cuda")
+    beside, n_beside = run([lambda p, stream: lib.fa_bwd_workspace(p, ws.data_ptr(), ws.numel(), stream)])  # dS is stored nowhere
+    assert n_beside == n_one
+    for a, b, c, name in zip(one, stages, beside, ("dq", "dk", "dv", "delta", "dbias")):
+        assert torch.equal(a, b) and torch.equal(a, c), name
+    return n_one, n_stages
 
 
 def test_one_launch_backward_takes_and_refuses_what_the_stages_do(device_ok):
