@@ -86,7 +86,7 @@ typedef struct fa_params {
   const void* bias;
   void* dbias;
   float* lse;   /* forward out / backward in: log2-domain log-sum-exp      */
-  float* delta; /* backward scratch: rowsum(o * do), written by fa_bwd_pre or, in one launch, fa_bwd */
+  float* delta; /* backward scratch: rowsum(o * do), written by fa_bwd_pre and by whole backwards */
 
   int64_t q_stride[3];
   int64_t k_stride[3];
@@ -104,7 +104,9 @@ typedef struct fa_params {
    * dtype, required in those cases, ignored otherwise.  The dK/dV stage leaves dS there for
    * the dQ stage (which consumes dS as a 16-bit tensor-core operand, exactly as the reference
    * rounds dS before its dQ product, FA:517).  Same stride rules as dbias.  Contents
-   * afterwards: dS rounded to 16 bits at and below the causal diagonal, unspecified above it. */
+   * after fa_bwd_dkdv and, at any size, fa_bwd: dS rounded to 16 bits at and below the causal
+   * diagonal, unspecified above it.  fa_bwd_workspace with a workspace and fa_small_bwd leave
+   * it alone. */
   void* ds16;
   int64_t ds16_stride[3];
 } fa_params;
@@ -114,8 +116,8 @@ int fa_version(void);
 
 /*
  * Number of kernels this library has launched since it was loaded (forward 1 per call; backward 3:
- * preprocess, dK/dV, dQ, with more parts two more each; short sequences 1; a row copy 1).  For benchmarks and tests that must show the
- * work ran here.  No counterpart in the reference.
+ * preprocess, dK/dV, dQ, with more parts two more each, or 1 where it is one launch (see fa_bwd); a row copy 1).  For
+ * benchmarks and tests that must show the work ran here.  No counterpart in the reference.
  */
 uint64_t fa_launch_count(void);
 
@@ -160,7 +162,10 @@ int fa_pad_rows(void* dst, const int64_t dst_stride[3], const void* src, const i
 int fa_pack_rows(void* dst, const void* src, int64_t pitch, int elem_bytes, int64_t rows, int N, int device, void* stream);
 
 /*
- * Backward, all three stages in order on `stream`.  Replaces _flash_attn_bwd
+ * Backward on `stream`: the three stages below in order, or one launch that does the work of all of them, with `delta` and
+ * `ds16` written as the stages do.  One launch take M, N, D <= 64 (the kernels for short sequences, whose gradients may
+ * differ from the stages' in the last bits) and N <= 128, M <= 256, D <= 64 with an fp32 bias or with B * H of at most
+ * twice the CTAs of a full grid (the same bits as the stages).  Replaces _flash_attn_bwd
  * (FA:688-763): the eager pre-scaled copies of k and bias (FA:699-704) and the
  * zero fill of dbias (FA:799) are folded into the kernels.
  */
@@ -199,7 +204,7 @@ int fa_bwd_workspace(const fa_params* p, void* workspace, uint64_t bytes, void* 
 int fa_bwd_static_scratch(const fa_params* p, void* stream);
 
 /*
- * The three backward stages on their own (per-kernel timing and tests).  Order matters:
+ * The three backward stages on their own, at any size (per-kernel timing and tests).  Order matters:
  * fa_bwd_pre writes `delta`, which the other two read; and when write_dbias is 1 with a
  * 16-bit bias, fa_bwd_dq READS `dbias` (it forms dQ from the dS tiles fa_bwd_dkdv has just
  * stored there), so fa_bwd_dkdv must have run on the same stream before it.

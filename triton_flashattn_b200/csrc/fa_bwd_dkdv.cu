@@ -8,8 +8,8 @@
 // epilogue.  Roles (384 threads):
 //   warps 0-7  "row" threads: warp w works on tensor-memory lanes 32*(w&3)..+31
 //              (query rows of the block) and on the 64-key half (w>>2)
-//   warp 8     TMA producer: K, V per tile; Q ring (2), dO ring; bias tiles, asked
-//              into L2 one step ahead
+//   warp 8     TMA producer: K, V per tile; Q ring (2), dO ring; bias tiles: loaded, or asked
+//              into L2 one step ahead, or (16 bit at head dim 128) both
 //   warp 9     MMA issuer for S and dP, tensor-memory owner
 //   warp 10    MMA issuer for dV and dK
 //   warp 11    bulk tensor stores of dS (into dbias or scratch)
@@ -41,7 +41,8 @@
 // With at most 128 keys one tile holds a whole row of dS, and the ONE_TILE variant (head dims up to 64, up to 256 queries)
 // is the whole backward in one launch: dQ = dS K over the tile of dS that dK reads, into 64 free columns of tensor memory,
 // and delta from the rows of o and dO, which the threads of that query row add up as fa_bwd_pre.cu does (the same bits).
-// It saves two launches, and with an fp32 bias the way of dS through memory, but a tile's chain is longer (see
+// It saves two launches, and with an fp32 bias the way of dS through memory (it is only stored for a caller that gives
+// a ds16), but a tile's chain is longer (see
 // one_tile_takes).
 //
 // Replaces _attn_bwd_dkdv / _attn_bwd_dkdv_inner of the reference
@@ -58,7 +59,7 @@ struct DkdvParams {
   CUtensorMap map_v;
   CUtensorMap map_do;
   CUtensorMap map_dbias;
-  CUtensorMap map_bias;  // only used to prefetch bias tiles into L2
+  CUtensorMap map_bias;  // tiles of a 16-bit bias and, at head dim 64, of a mask; the others are only asked into L2 through it
   const void* bias;
   void* dk;
   void* dv;
@@ -94,7 +95,8 @@ enum DkdvSite { kSiteKV = 1, kSiteQFull, kSiteQEmpty, kSiteDoFull, kSiteDoEmpty,
 
 // Eight row warps, a thread with half a row of a step: what a step costs a warp besides its values (looks at nine
 // barriers, votes, fences, loop) is paid half as often as with sixteen warps and quarters of a row, and 168 registers
-// hold the rest.  Whole backward, us, quarters / halves: no bias B4 H16 S2048 D128 403 / 400, 16 bit B8 H16 S2048 D128 902 / 894,
+// hold the rest, but for ONE_TILE: its eight chunks each of o and dO, asked for ahead of a step, spill (bytes stored / loaded:
+// no bias 66 / 96, 16 bit 150 / 304, mask 102 / 168, fp32 338 / 480; the other variants none).  Whole backward, us, quarters / halves: no bias B4 H16 S2048 D128 403 / 400, 16 bit B8 H16 S2048 D128 902 / 894,
 // D64 742 / 728, mask, causal, B4 H32 S4096 D128 1805 / 1754, fp32 B4 H16 S2048 D128 882 / 867.
 constexpr int kCW = 64;           // columns of a step that a row thread works on
 constexpr int kNG = kCW / 32;     // ... in groups of 32
@@ -352,7 +354,6 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
     if (live) {
       constexpr bool bf = P2::kIsBf16;
       constexpr uint32_t idesc_s = make_idesc(bf, false, false, 128, 128);
-      constexpr bool kSpin = false;
       const uint32_t k_addr = smem_u32(smem + L::kK), v_addr = smem_u32(smem + L::kV);
       const uint32_t q_addr = smem_u32(smem + L::kQ), do_addr = smem_u32(smem + L::kDo);
       const uint64_t k_km = make_sdesc(k_addr, 0, 1024), v_km = make_sdesc(v_addr, 0, 1024);
@@ -371,8 +372,8 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
           const int qs = gs & 1, ds = gs % kDoStages;
           const uint32_t q_par = (gs >> 1) & 1, do_par = (gs / kDoStages) & 1;
           // S_gs: its columns are free once the row threads hold S_{gs-1} in registers
-          ok = gs >= 1 ? wait_all2<kSpin>(&s_free, (gs - 1) & 1, &q_full[qs], q_par, ctx, kSiteSFree, t)
-                       : wait_all1<kSpin>(&q_full[qs], q_par, ctx, kSiteQFull, t);
+          ok = gs >= 1 ? wait_all2<false>(&s_free, (gs - 1) & 1, &q_full[qs], q_par, ctx, kSiteSFree, t)
+                       : wait_all1<false>(&q_full[qs], q_par, ctx, kSiteQFull, t);
           if (!ok) break;
           tc_fence_after();
           if (elect_one()) {
@@ -383,8 +384,8 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
           }
           // dP_gs: same for the dP columns; dO_gs replaces dO_{gs-1} after dV_{gs-1} when
           // single-staged
-          ok = gs >= 1 ? wait_all2<kSpin>(&dp_free, (gs - 1) & 1, &do_full[ds], do_par, ctx, kSiteDpFree, t)
-                       : wait_all1<kSpin>(&do_full[ds], do_par, ctx, kSiteDoFull, t);
+          ok = gs >= 1 ? wait_all2<false>(&dp_free, (gs - 1) & 1, &do_full[ds], do_par, ctx, kSiteDpFree, t)
+                       : wait_all1<false>(&do_full[ds], do_par, ctx, kSiteDoFull, t);
           if (!ok) break;
           tc_fence_after();
           if (elect_one()) {
@@ -411,7 +412,6 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
       const uint64_t do_mn_0 = make_sdesc(do_addr, kBlk, 1024),
                      do_mn_1 = make_sdesc(do_addr + (kDoStages - 1) * L::kTile, kBlk, 1024);
       const uint64_t p_mn = make_sdesc(p_addr, kBlk, 1024), ds_mn = make_sdesc(ds_addr, kBlk, 1024);
-      constexpr bool kSpin = false;
       bool ok = true;
       uint32_t g = 0;
       int bh, nb, i_start, T_steps;
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
           // dV += P^T dO  (dO must have landed: P only depends on S).  The first product of a
           // tile overwrites dV / dK: P and dS of a new tile are only announced by all eight
           // row warps after they have read the previous tile's accumulators.
-          ok = wait_all2<kSpin>(&p_ready, gs & 1, &do_full[ds], (gs / kDoStages) & 1, ctx, kSitePReady, t);
+          ok = wait_all2<false>(&p_ready, gs & 1, &do_full[ds], (gs / kDoStages) & 1, ctx, kSitePReady, t);
           if (!ok) break;
           tc_fence_after();
           if (elect_one()) {
@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
             mma_commit(&do_empty[ds]);
           }
           // dK += dS^T Q
-          ok = wait_all2<kSpin>(&ds_ready, gs & 1, &q_full[qs], (gs >> 1) & 1, ctx, kSiteDsReady, t);
+          ok = wait_all2<false>(&ds_ready, gs & 1, &q_full[qs], (gs >> 1) & 1, ctx, kSiteDsReady, t);
           if (!ok) break;
           tc_fence_after();
           if (elect_one()) {
@@ -734,7 +734,7 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
         if (!ok) break;
         tc_fence_after();
         uint32_t dsu[kCW / 2];
-        // dP is fetched in two halves: fewer registers are live at once
+        // dP is fetched 16 columns at a time: fewer registers are live at once
 #pragma unroll
         for (int hf = 0; hf < kCW / 16; ++hf) {
           uint32_t dp[16];
@@ -758,7 +758,7 @@ __global__ void __launch_bounds__(kThreads, 1) dkdv_kernel(const __grid_constant
             }
           }
           if (BIAS == 3 && p.dbias_f32 != nullptr && m0 + r < p.M) {
-            // the fp32 bias gradient goes out unrounded, 64 contiguous bytes per thread and half
+            // the fp32 bias gradient goes out unrounded, 64 contiguous bytes per thread and fetch
             const int b_ = bh / p.H, h_ = bh - b_ * p.H;
             const int c0 = col0 + hf * 16;
             float* drow = p.dbias_f32 + b_ * p.dbf_sB + h_ * p.dbf_sH + (int64_t)(m0 + r) * p.dbf_sM + c0;

@@ -696,7 +696,7 @@ __device__ __forceinline__ bool wait_warp_polled(uint32_t polled, uint64_t* bar,
   return wait_warp(bar, parity, ctx, site, iter);
 }
 
-// 32 bias values of one row quarter, as raw 16-bit pairs (BIAS == 1), bytes (BIAS == 2) or
+// 32 neighbouring bias values of a row, as raw 16-bit pairs (BIAS == 1), bytes (BIAS == 2) or
 // fp32 words (BIAS == 3).
 template <int BIAS>
 struct BiasRegs {

@@ -5,8 +5,8 @@
 // block they visit.  Roles (384 threads):
 //   warps 0-3   softmax group of tile 0: thread = one query row (= tensor-memory lane)
 //   warps 4-7   softmax group of tile 1
-//   warp 8      TMA producer (converged, an elected lane issues): Q pair per unit, K ring (128-key stages), V ring
-//               (64-key half stages)
+//   warp 8      TMA producer (converged, an elected lane issues): Q pair per unit, K ring (128-key stages, 64-key
+//               half stages at head dim 256), V ring (64-key half stages)
 //   warp 9      MMA issuer of tile 0 (converged, an elected lane issues), tensor-memory owner
 //   warp 10     TMA producer of the bias / mask ring (converged, an elected lane issues).
 //               (Asking TMA to pull the tiles a few units ahead into L2 as well made the
