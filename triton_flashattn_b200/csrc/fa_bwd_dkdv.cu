@@ -969,42 +969,10 @@ DkdvPlan plan_dkdv(const fa_params& p, int n_bh, int sms, bool writes_zeros) {
   const int64_t all = static_cast<int64_t>(n_nblk) * n_bh;
   if (!p.causal || all > 4 * sms) return {false, 0};
   const int n = static_cast<int>(all), zeros = writes_zeros ? 1 : 0;
-  const auto more = [](int& most, int load) { most = load > most ? load : most; };
-
-  // Pairs: a CTA has units c and c + G at most, and their work repeats every n_nblk units (half of that where it is
-  // even), so the first CTAs of those with two units and of those with one stand for all.
-  const int units = (n + 1) / 2, g_pairs = units < sms ? units : sms, period = n_nblk & 1 ? n_nblk : n_nblk / 2;
-  const auto unit_work = [&](int u) {
-    int work = 0;
-    for (int k = 2 * u, pos = k % n_nblk; k < 2 * u + 2 && k < n; ++k, pos = pos + 1 == n_nblk ? 0 : pos + 1)
-      work += tile_work(pos & 1 ? n_nblk - 1 - (pos >> 1) : pos >> 1, n_mblk, zeros);
-    return work;
-  };
-  int pairs = 0;
-  const int with_two = units - g_pairs;
-  for (int c = 0; c < with_two && c < period; ++c) more(pairs, unit_work(c) + unit_work(c + g_pairs));
-  for (int c = with_two; c < g_pairs && c < with_two + period; ++c) more(pairs, unit_work(c));
-
-  // Longest first: along the CTAs the work of even rows falls and that of odd rows rises, so the longest CTA is the first
-  // one, or one at which an odd row comes to a longer key block.
-  const int g = n < sms ? n : sms;
-  const auto load_of = [&](int c) {
-    int load = 0;
-    for (int at = 0, r = 0; at < n; at += g, ++r)
-      if (const int k = at + (r & 1 ? g - 1 - c : c); k < n) load += tile_work(k / n_bh, n_mblk, zeros);
-    return load;
-  };
-  int longest = load_of(0);
-  for (int at = g; at < n; at += 2 * g) {
-    const int last = at + g < n ? at + g - 1 : n - 1;
-    for (int nb = at / n_bh; nb <= last / n_bh; ++nb) {
-      const int k = (nb + 1) * n_bh - 1;
-      more(longest, load_of(at + g - 1 - (k < last ? k : last)));
-    }
-  }
+  const CausalSpans span = causal_spans(n, n_bh, n_nblk, sms, [&](int nb) { return tile_work(nb, n_mblk, zeros); });
   const int margin = p.bias_kind != FA_BIAS_NONE && n > 2 * sms ? 106 : 103;
-  const bool longest_first = 100 * static_cast<int64_t>(pairs) >= margin * static_cast<int64_t>(longest);
-  return {longest_first, longest_first ? longest : pairs};
+  const bool longest_first = 100 * static_cast<int64_t>(span.pairs) >= margin * static_cast<int64_t>(span.longest_first);
+  return {longest_first, longest_first ? span.longest_first : span.pairs};
 }
 
 // One tile of keys and at most two blocks of queries: dQ joins the chain of a step, which a head walks alone (at B1 H8 M4096

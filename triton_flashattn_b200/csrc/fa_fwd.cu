@@ -865,40 +865,10 @@ bool longest_first(const FwdParams& fp, int tiles, int sms, bool bias) {
     const int last = (pair + 1) * tiles < fp.n_mblk ? (pair + 1) * tiles : fp.n_mblk;
     return 4 * (last < nblk ? last : nblk) + 5;
   };
-  const auto more = [](int& most, int load) { most = load > most ? load : most; };
-  // Pairs: the work of a CTA's pairs repeats every np of them (half of that where np is even), so the first CTAs of those
-  // with the most turns and of those with one less stand for all.
-  const int pairs = (n + 1) / 2, g_pairs = pairs < sms ? pairs : sms, period = np & 1 ? np : np / 2;
-  const auto pairs_of = [&](int c) {
-    int load = 0;
-    for (int u = c; u < pairs; u += g_pairs)
-      for (int k = 2 * u, pos = k % np; k < 2 * u + 2 && k < n; ++k, pos = pos + 1 == np ? 0 : pos + 1)
-        load += work(pos & 1 ? pos >> 1 : np - 1 - (pos >> 1));
-    return load;
-  };
-  int by_pairs = 0;
-  const int most_turns = (pairs - 1) % g_pairs + 1;
-  for (int c = 0; c < most_turns && c < period; ++c) more(by_pairs, pairs_of(c));
-  for (int c = most_turns; c < g_pairs && c < most_turns + period; ++c) more(by_pairs, pairs_of(c));
-  // Longest first: along the CTAs the work of even rows falls and that of odd rows rises, so the longest CTA is the first
-  // one, or one at which an odd row comes to a longer unit.
-  const auto load_of = [&](int c) {
-    int load = 0;
-    for (int at = 0, r = 0; at < n; at += sms, ++r)
-      if (const int k = at + (r & 1 ? sms - 1 - c : c); k < n) load += work(np - 1 - k / fp.n_bh);
-    return load;
-  };
-  int longest = load_of(0);
-  for (int at = sms; at < n; at += 2 * sms) {
-    const int last = at + sms < n ? at + sms - 1 : n - 1;
-    for (int level = at / fp.n_bh; level <= last / fp.n_bh; ++level) {
-      const int k = (level + 1) * fp.n_bh - 1;  // the last unit of this length
-      more(longest, load_of(at + sms - 1 - (k < last ? k : last)));
-    }
-  }
+  const CausalSpans span = causal_spans(n, fp.n_bh, np, sms, [&](int level) { return work(np - 1 - level); });
   const int64_t kv_mb = 4 * static_cast<int64_t>(fp.n_bh) * fp.N * fp.D / 1000000;
   const int margin = np <= 3 || kv_mb >= 140 ? 125 : (kv_mb >= 90 ? (bias ? 118 : 110) : (kv_mb >= 40 ? 107 : 104));
-  return 100 * static_cast<int64_t>(by_pairs) >= margin * static_cast<int64_t>(longest);
+  return 100 * static_cast<int64_t>(span.pairs) >= margin * static_cast<int64_t>(span.longest_first);
 }
 
 }  // namespace

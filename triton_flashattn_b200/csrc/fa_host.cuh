@@ -81,6 +81,52 @@ int launch_selftest_timeout(uint32_t limit_us, cudaStream_t stream, int* status)
 // per CTA.
 int persistent_grid(int n_tiles);
 
+// What the longest CTA of a causal launch has to do in the two orders in which persistent CTAs take its n units: n_bh
+// heads of `levels` units each, work(level) falling from level 0 on.
+//   pairs: the units of a head are ordered heavy, light, next heavy, next light, ..., and CTA c takes two neighbours in a
+//     turn, pair c, c + G, ...
+//   longest first: the units are numbered by level, heads inside it, and the CTAs take them in rows, every second row from
+//     the other end.
+struct CausalSpans {
+  int pairs, longest_first;
+};
+template <typename Work>
+inline CausalSpans causal_spans(int n, int n_bh, int levels, int sms, Work work) {
+  CausalSpans span = {0, 0};
+  const auto more = [](int& most, int load) { most = load > most ? load : most; };
+  // Pairs: the work of a CTA's pairs repeats every `levels` of them (half of that where it is even), so the first CTAs of
+  // those with the most turns and of those with one less stand for all.
+  const int pairs = (n + 1) / 2, g_pairs = pairs < sms ? pairs : sms, period = levels & 1 ? levels : levels / 2;
+  const auto pairs_of = [&](int c) {
+    int load = 0;
+    for (int u = c; u < pairs; u += g_pairs)
+      for (int k = 2 * u, pos = k % levels; k < 2 * u + 2 && k < n; ++k, pos = pos + 1 == levels ? 0 : pos + 1)
+        load += work(pos & 1 ? levels - 1 - (pos >> 1) : pos >> 1);
+    return load;
+  };
+  const int most_turns = (pairs - 1) % g_pairs + 1;
+  for (int c = 0; c < most_turns && c < period; ++c) more(span.pairs, pairs_of(c));
+  for (int c = most_turns; c < g_pairs && c < most_turns + period; ++c) more(span.pairs, pairs_of(c));
+  // Longest first: along the CTAs the work of even rows falls and that of odd rows rises, so the longest CTA is the first
+  // one, or one at which an odd row comes to a longer level.
+  const int g = n < sms ? n : sms;
+  const auto load_of = [&](int c) {
+    int load = 0;
+    for (int at = 0, r = 0; at < n; at += g, ++r)
+      if (const int k = at + (r & 1 ? g - 1 - c : c); k < n) load += work(k / n_bh);
+    return load;
+  };
+  span.longest_first = load_of(0);
+  for (int at = g; at < n; at += 2 * g) {
+    const int last = at + g < n ? at + g - 1 : n - 1;
+    for (int level = at / n_bh; level <= last / n_bh; ++level) {
+      const int k = (level + 1) * n_bh - 1;  // the last unit of this level
+      more(span.longest_first, load_of(at + g - 1 - (k < last ? k : last)));
+    }
+  }
+  return span;
+}
+
 // Kernels launched by this library since it was loaded (all devices, all threads).
 extern std::atomic<uint64_t> g_kernel_launches;
 
