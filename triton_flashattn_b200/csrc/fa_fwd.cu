@@ -11,7 +11,7 @@
 //   warp 10     TMA producer of the bias / mask ring (converged, an elected lane issues).
 //               (Asking TMA to pull the tiles a few units ahead into L2 as well made the
 //               kernel 4-5 % slower and was removed.)
-//   warp 11     MMA issuer of tile 1 (converged, an elected lane issues)
+//   warp 11     MMA issuer of tile 1 (converged, an elected lane issues; idle at head dim 256)
 // Tensor memory: S0 | S1 | O0 | O1, 128 columns each.  The 128 score columns of a tile are
 // two halves of 64 that swap roles every key block.  In step c (f = c & 1):
 //   columns [64f, 64f+64)       scores of keys 0-63, read first; afterwards they hold the
@@ -42,7 +42,7 @@
 // raised when it grows by more than 8 (log2 units); only then is O rescaled (by the row's
 // own thread, after the products into it have finished).  Ring stages, tensor-memory
 // buffers and barrier phases run on from unit to unit.  K / V ring stages are handed back
-// by both issuers (their "empty" barriers count two arrivals); an issuer whose tile does
+// by all issuers (their "empty" barriers count one arrival each); an issuer whose tile does
 // not visit a block still waits for its loads and hands the stages back, so that every
 // waiter sees every completion of a barrier it waits on.
 //
@@ -233,10 +233,10 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
   if (tid == 0) {
     abort_flag = 0;
     mbar_init(&q_full, 1);
-    mbar_init(&q_empty, 2);
+    mbar_init(&q_empty, L::kTiles);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&k_full[i], 1);
-      mbar_init(&k_empty[i], 2);
+      mbar_init(&k_empty[i], L::kTiles);
       mbar_init(&s_read[i], 4);
       for (int h = 0; h < 2; ++h) {
         mbar_init(&s_full[i][h], 1);
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
     }
     for (int i = 0; i < 4; ++i) {
       mbar_init(&v_full[i], 1);
-      mbar_init(&v_empty[i], 2);
+      mbar_init(&v_empty[i], L::kTiles);
       mbar_init(&bias_full[0][i], 1);
       mbar_init(&bias_full[1][i], 1);
       mbar_init(&bias_empty[i], 4);
@@ -337,9 +337,12 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
       }
     }
   } else if (warp == 9 || warp == 11) {
-    // ------------------------------------------- MMA issuer of tile slot t (converged, an elected lane issues)
+    // ------------------------------------------- MMA issuer of tile slot t
     // (the whole warp walks the loop converged, one elected lane issues)
-    if (live) {
+    // Head dim 256 has one tile a unit and one issuer.  (The second one, with nothing to issue, used to hand back stages beside
+    // it, behind combined looks that held units of a few key blocks up; us, two / one: 16-bit bias H16 B85 S192 213 / 192, B51
+    // S320 226 / 208, causal B85 S192 200 / 172, B16 S2048 1425 / 1405.)
+    if (live && (L::kTiles == 2 || warp == 9)) {
       const int t = warp == 9 ? 0 : 1;
       // The issuer is on the critical path, and a wait takes some 200 cycles even on a completed barrier, an elect with
       // its reconvergence another 100.  So the three groups of products of a step (P V of the first half, scores of the
