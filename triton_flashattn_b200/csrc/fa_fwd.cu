@@ -352,7 +352,10 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
       // mask D128 371 / 349, D64 334 / 311; B1 H37 S2048 D256 197 / 150 (with the K halves).
       // It polls without suspending at D128 and D256 (D256 149.5, suspended 155.6); at D64 the row threads need the issue
       // slots more (mask 324, suspended 311).  The producers wait suspended for the same reason (mask D128 373 polling,
-      // 346 suspended).
+      // 346 suspended), and so does the issuer where a unit begins and in blocks that only the other tile visits (one tile a
+      // unit, B192 H16 64 x 128 D128: no bias, causal 70.3 / 69.7, 16 bit 107.2 / 104.6; 16 bit causal B85 H16 192 x 256
+      // 112.8 / 110.2).  Where a unit is at most 64 queries over one key block without a bias the looks cost 1 - 4 % against
+      // waits one by one (64 x 64 61.2 / 63.2, 64 x 128 60.0 / 60.5); 128 x 128 70.6 / 67.6, 64 x 256 99.5 / 91.3.
       constexpr bool kSpin = DP > 64;
       constexpr bool bf = P2::kIsBf16;
       constexpr uint32_t idesc_qk = make_idesc(bf, false, false, 128, 64);
@@ -384,7 +387,7 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
       for (int it = 0; ok && unit_at<L::kTiles, LONGEST_FIRST>(p, it, u); ++it) {
         if (u.nmax == 0) continue;
         const int nblk = u.nb(t);
-        ok = wait_all2<kSpin>(&q_full, it & 1, &k_full[k_stage(gk, 0)], k_par(gk), ctx, kSiteQFull, it);
+        ok = wait_all2<false>(&q_full, it & 1, &k_full[k_stage(gk, 0)], k_par(gk), ctx, kSiteQFull, it);
         if (ok && L::kKHalves) ok = wait_all1<kSpin>(&k_full[1], k_par(gk), ctx, kSiteKFull, 0);
         if (!ok) break;
         tc_fence_after();
@@ -416,7 +419,7 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
             ok = L::kKHalves ? wait_all2<kSpin>(&p_full[t][0], cs & 1, vb0, vp0, ctx, kSitePFull, j)
                              : wait_all3<kSpin>(&p_full[t][0], cs & 1, vb0, vp0, kb0, kp0, ctx, kSitePFull, j);
           else
-            ok = wait_all2<kSpin>(vb0, vp0, kb0, kp0, ctx, kSiteVFull, j);
+            ok = wait_all2<false>(vb0, vp0, kb0, kp0, ctx, kSiteVFull, j);
           if (!ok) break;
           tc_fence_after();
           if (elect_one()) {
@@ -446,7 +449,7 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
             ok = L::kKHalves ? wait_all3<kSpin>(&p_full[t][1], cs & 1, vb1, vp1, kb1, kp1, ctx, kSitePFull, j)
                              : wait_all2<kSpin>(&p_full[t][1], cs & 1, vb1, vp1, ctx, kSitePFull, j);
           else
-            ok = wait_all2<kSpin>(vb1, vp1, kb1, kp1, ctx, kSiteVFull, j);
+            ok = wait_all2<false>(vb1, vp1, kb1, kp1, ctx, kSiteVFull, j);
           if (!ok) break;
           tc_fence_after();
           if (elect_one()) {
