@@ -47,6 +47,27 @@ def test_small_grid(D, dtype, bias_kind, causal, device_ok):
     check_case(2, 256, 256, 2, D, dtype, bias_kind, causal, seed=1)
 
 
+@pytest.mark.parametrize("N", [129, 130, 131, 160, 163, 191, 194, 255, 287])
+@pytest.mark.parametrize("kind,D,causal", [("bool", 128, False), ("bool", 128, True), ("f32", 128, False), ("f32", 64, True)])
+def test_right_edge_of_a_bias_read_by_the_row_threads(N, kind, D, causal, device_ok):
+    """A mask at head dim 128 and an fp32 bias come from global memory in words and 16-byte chunks; what stands behind column N
+    in its row, a number here that would show, is not used."""
+    from triton_flashattn_b200 import flash_attention_fn
+
+    M, H = 290, 2
+    q, k, v, bias, do = make_inputs(2, M, N, H, D, BF, "bool" if kind == "bool" else "float", 4)
+    rows = torch.full((2, H, M, 320), 1 if kind == "bool" else float("nan"), dtype=torch.bool if kind == "bool" else torch.float32,
+                      device="cuda")
+    rows[..., :N] = bias
+    bias = rows[..., :N]
+    q, k, v = (t.requires_grad_() for t in (q, k, v))
+    wrt = [q, k, v] + ([bias.requires_grad_()] if kind == "f32" else [])
+    out = flash_attention_fn(q, k, v, bias, causal)
+    grads = torch.autograd.grad(out, wrt, do)
+    ours = dict(zip(("dq", "dk", "dv", "dbias"), grads), out=out.detach())
+    compare(ours, q.detach(), k.detach(), v.detach(), bias.detach(), causal, None, do, BF, label=f"{kind} N{N}: ")
+
+
 @pytest.mark.parametrize("M,N,D,causal", [(300, 200, 128, False), (256, 300, 64, True), (200, 130, 256, True), (100, 90, 64, True),
                                           (40, 50, 32, False), (4, 300, 128, False)])
 @pytest.mark.parametrize("bias_kind", [None, "float", "bool"])
