@@ -72,6 +72,7 @@ struct FwdParams {
   int bias_b_mul, bias_h_mul;
   int n_mblk, n_pairs, n_units;  // query blocks / block pairs per (batch, head); units = pairs * B * H
   int n_bh;                      // B * H
+  int tiles;                     // query tiles per unit
   float sm_scale;
 };
 
@@ -341,9 +342,12 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
     // (the whole warp walks the loop converged, one elected lane issues)
     // Head dim 256 has one tile a unit and one issuer.  (The second one, with nothing to issue, used to hand back stages beside
     // it, behind combined looks that held units of a few key blocks up; us, two / one: 16-bit bias H16 B85 S192 213 / 192, B51
-    // S320 226 / 208, causal B85 S192 200 / 172, B16 S2048 1425 / 1405.)
-    if (live && (L::kTiles == 2 || warp == 9)) {
-      const int t = warp == 9 ? 0 : 1;
+    // S320 226 / 208, causal B85 S192 200 / 172, B16 S2048 1425 / 1405.)  The number of tiles is asked for at run time, except at head dim 64
+    // without a mask, only because of how the compiler then lays the code out; one unit a CTA, H8, us, known / asked: S512
+    // D256 16 bit 15.4 / 15.1, mask 15.0 / 14.7, D128 causal 16 bit 16.3 / 16.1, D64 causal mask 13.5 / 13.2, 16 bit 13.8 / 14.0.
+    constexpr bool kAskTiles = DP > 64 || BIAS == 2;
+    const int t = warp == 9 ? 0 : 1;
+    if (live && t < (kAskTiles ? p.tiles : L::kTiles)) {
       // The issuer is on the critical path, and a wait takes some 200 cycles even on a completed barrier, an elect with
       // its reconvergence another 100.  So the three groups of products of a step (P V of the first half, scores of the
       // next block's first half, P V of the second half with the scores of the next block's second half) have one
@@ -550,7 +554,8 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
             // Without a bias (and a positive scale) the raw q.k is kept and the scale is
             // folded into the exponent below.  A mask scales first, as a bias of zeros does, and so gives the bits of one
             // (folded in as well it rounds once less, with other bits; us, folded / scaled first two at a time: B1 H37 S4096 D128
-            // 344 / 335, D64 318 / 313, causal B4 H32 S4096 D128 670 / 641; one by one 370, 333, 683).
+            // 344 / 335, D64 318 / 313, causal B4 H32 S4096 D128 670 / 641, B1 H8 S512 D128 17.1 / 15.3, D64 12.8 / 13.5; one by one
+            // 370, 333, 683).
             float mul = kLog2e;  // exponent = s * mul - m
             float mx = -INFINITY;  // row maximum of this half
             if (BIAS == 0 && fold_scale) {
@@ -934,6 +939,7 @@ int launch_fwd(const fa_params& p, cudaStream_t stream, int* status) {
   fp.n_pairs = (fp.n_mblk + tiles - 1) / tiles;
   fp.n_units = fp.n_pairs * p.B * p.H;
   fp.n_bh = p.B * p.H;
+  fp.tiles = tiles;
   const int sms = persistent_grid(1 << 30);
   const bool by_length = longest_first(fp, tiles, sms, p.bias_kind != FA_BIAS_NONE);
   const int turns_of = p.causal && !by_length ? (fp.n_units + 1) / 2 : fp.n_units;
