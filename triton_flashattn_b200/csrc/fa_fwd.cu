@@ -342,10 +342,11 @@ __global__ void __launch_bounds__(384, 1) fwd_kernel(const __grid_constant__ Fwd
     // (the whole warp walks the loop converged, one elected lane issues)
     // Head dim 256 has one tile a unit and one issuer.  (The second one, with nothing to issue, used to hand back stages beside
     // it, behind combined looks that held units of a few key blocks up; us, two / one: 16-bit bias H16 B85 S192 213 / 192, B51
-    // S320 226 / 208, causal B85 S192 200 / 172, B16 S2048 1425 / 1405.)  The number of tiles is asked for at run time, except at head dim 64
-    // without a mask, only because of how the compiler then lays the code out; one unit a CTA, H8, us, known / asked: S512
-    // D256 16 bit 15.4 / 15.1, mask 15.0 / 14.7, D128 causal 16 bit 16.3 / 16.1, D64 causal mask 13.5 / 13.2, 16 bit 13.8 / 14.0.
-    constexpr bool kAskTiles = DP > 64 || BIAS == 2;
+    // S320 226 / 208, causal B85 S192 200 / 172, B16 S2048 1425 / 1405.)  Whether the number of tiles is asked for at run
+    // time makes a difference only by how the compiler then lays the code out; us, known / asked, one unit a CTA, H8 S512: D256 16
+    // bit 15.4 / 15.1, mask 15.0 / 14.7, D128 causal 16 bit 16.3 / 16.1, D64 causal mask 13.5 / 13.2, 16 bit 13.8 / 14.0; no bias
+    // causal B2 H32 S4096 D128 256.5 / 257.8.
+    constexpr bool kAskTiles = DP == 256 || (DP == 128 ? BIAS != 0 : BIAS == 2);
     const int t = warp == 9 ? 0 : 1;
     if (live && t < (kAskTiles ? p.tiles : L::kTiles)) {
       // The issuer is on the critical path, and a wait takes some 200 cycles even on a completed barrier, an elect with
