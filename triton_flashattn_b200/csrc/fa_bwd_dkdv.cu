@@ -96,7 +96,7 @@ enum DkdvSite { kSiteKV = 1, kSiteQFull, kSiteQEmpty, kSiteDoFull, kSiteDoEmpty,
 // Eight row warps, a thread with half a row of a step: what a step costs a warp besides its values (looks at nine
 // barriers, votes, fences, loop) is paid half as often as with sixteen warps and quarters of a row, and 168 registers
 // hold the rest, but for ONE_TILE: its eight chunks each of o and dO, asked for ahead of a step, spill (bytes stored / loaded:
-// no bias 66 / 96, 16 bit 150 / 304, mask 102 / 168, fp32 338 / 480; the other variants none).  Whole backward, us, quarters / halves: no bias B4 H16 S2048 D128 403 / 400, 16 bit B8 H16 S2048 D128 902 / 894,
+// no bias 66 / 96, 16 bit 150 / 304, mask 102 / 168, fp32 338 / 480; the other variants 4 / 16 at most).  Whole backward, us, quarters / halves: no bias B4 H16 S2048 D128 403 / 400, 16 bit B8 H16 S2048 D128 902 / 894,
 // D64 742 / 728, mask, causal, B4 H32 S4096 D128 1805 / 1754, fp32 B4 H16 S2048 D128 882 / 867.
 constexpr int kCW = 64;           // columns of a step that a row thread works on
 constexpr int kNG = kCW / 32;     // ... in groups of 32
